@@ -59,6 +59,89 @@ DevArena::~DevArena() {
   for (void* p : ptrs) cudaFree(p);
 }
 
+// ---- coil basis ----------------------------------------------------------------------------
+// Rows of a ring's Gaussian factors ey_q(y) overlap so much (sigma 0.9 of the matrix, centres
+// within 0.6 of it) that they span few dimensions: the constant row (the coil offset's) and at most
+// six more carry every coil of any ring.  Pivoted Gram-Schmidt in FP64 from the constant row takes
+// rows until what remains of every coil is below 1e-9: 7 rows for 12 to 64 coils (2e-10 to 4e-10
+// left; a float32 table of the factors carries 3e-8), 6 for 8 and 10, 4 for 6.  Returns the row
+// count padded to one the kernels are built for (4, 6, 7), or 0 when 7 rows do not suffice; rows
+// [nb - 1][sny] scaled to a largest value of 1, coef [coil][kBasisPad].
+static int coil_basis(const std::vector<double>& ey, int ncoils, int sny, std::vector<float>& rows,
+                      std::vector<float>& coef) {
+  constexpr int kMaxRows = 7;
+  constexpr double kTol = 1e-9;
+  std::vector<double> R(ey);
+  std::vector<std::vector<double>> B;
+  auto remove_mean = [&](double* v) {
+    double m = 0.0;
+    for (int y = 0; y < sny; ++y) m += v[y];
+    m /= sny;
+    for (int y = 0; y < sny; ++y) v[y] -= m;
+  };
+  for (int q = 0; q < ncoils; ++q) remove_mean(&R[(size_t)q * sny]);
+  for (;;) {
+    double worst = 0.0, best = -1.0;
+    int piv = 0;
+    for (int q = 0; q < ncoils; ++q) {
+      double n2 = 0.0;
+      for (int y = 0; y < sny; ++y) {
+        const double v = R[(size_t)q * sny + y];
+        n2 += v * v;
+        worst = std::max(worst, std::fabs(v));
+      }
+      if (n2 > best) {
+        best = n2;
+        piv = q;
+      }
+    }
+    if (worst <= kTol) break;
+    if ((int)B.size() == kMaxRows - 1) return 0;
+    std::vector<double> v(R.begin() + (size_t)piv * sny, R.begin() + (size_t)(piv + 1) * sny);
+    for (int pass = 0; pass < 2; ++pass) {  // twice: the last rows are 1e-6 of the first
+      remove_mean(v.data());
+      for (const auto& b : B) {
+        double d = 0.0;
+        for (int y = 0; y < sny; ++y) d += b[y] * v[y];
+        for (int y = 0; y < sny; ++y) v[y] -= d * b[y];
+      }
+      double n2 = 0.0;
+      for (double x : v) n2 += x * x;
+      const double in = 1.0 / std::sqrt(n2);
+      for (double& x : v) x *= in;
+    }
+    for (int q = 0; q < ncoils; ++q) {
+      double* r = &R[(size_t)q * sny];
+      double d = 0.0;
+      for (int y = 0; y < sny; ++y) d += r[y] * v[y];
+      for (int y = 0; y < sny; ++y) r[y] -= d * v[y];
+    }
+    B.push_back(std::move(v));
+  }
+  const int need = (int)B.size() + 1, nb = need <= 4 ? 4 : need <= 6 ? 6 : 7;
+  rows.assign((size_t)(nb - 1) * sny, 0.f);
+  coef.assign((size_t)ncoils * kBasisPad, 0.f);
+  std::vector<double> scale(B.size());
+  for (size_t r = 0; r < B.size(); ++r) {
+    double m = 0.0;
+    for (double x : B[r]) m = std::max(m, std::fabs(x));
+    scale[r] = m;
+    for (int y = 0; y < sny; ++y) rows[r * sny + y] = (float)(B[r][y] / m);
+  }
+  for (int q = 0; q < ncoils; ++q) {
+    const double* e = &ey[(size_t)q * sny];
+    double mean = 0.0;
+    for (int y = 0; y < sny; ++y) mean += e[y];
+    coef[(size_t)q * kBasisPad + nb - 1] = (float)(mean / sny);
+    for (size_t r = 0; r < B.size(); ++r) {
+      double d = 0.0;
+      for (int y = 0; y < sny; ++y) d += B[r][y] * e[y];
+      coef[(size_t)q * kBasisPad + r] = (float)(d * scale[r]);
+    }
+  }
+  return nb;
+}
+
 // ---- geometry tables -----------------------------------------------------------------------
 // ex/ey: the two factors of the Gaussian ring coil sensitivity (`coil_sensitivity`
 // kspace.rs:226-237) on the sim grid in acquired-voxel units (xa = (x - xoff)/o); tw: the x-stage
@@ -70,6 +153,7 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
   const double xoff = (ox - 1.0) / 2.0, yoff = (oy - 1.0) / 2.0;
   const int xs = nx / 2, sxs = ox * xs;
   std::vector<float> ex((size_t)ncoils * snx), ey((size_t)ncoils * sny);
+  std::vector<double> ey64((size_t)ncoils * sny, 1.0);
   const double sigma = 0.9 * (double)std::max(nx, ny);
   const double r = 0.6 * (double)std::max(nx, ny);
   for (int q = 0; q < ncoils; ++q) {
@@ -86,7 +170,8 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
     }
     for (int y = 0; y < sny; ++y) {
       double d = ((double)y - yoff) / oy - py;
-      ey[(size_t)q * sny + y] = (float)std::exp(-(d * d) / (2.0 * sigma * sigma));
+      ey64[(size_t)q * sny + y] = std::exp(-(d * d) / (2.0 * sigma * sigma));
+      ey[(size_t)q * sny + y] = (float)ey64[(size_t)q * sny + y];
     }
   }
   std::vector<float2> tw((size_t)4 * snx * nx);
@@ -151,6 +236,18 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
     g.ncls = ncls;
     g.cls = (const int*)arena.upload(cls.data(), cls.size() * sizeof(int), st);
     g.eyc = (const float*)arena.upload(eyc.data(), eyc.size() * 4, st);
+  }
+  g.nbas = 0;
+  g.bas = g.bco = nullptr;
+  if (ncoils >= 6) {  // up to 4 coils have kernels of their own; 5 span 6 rows
+    std::vector<float> rows, coef;
+    const int nb = coil_basis(ey64, ncoils, sny, rows, coef);
+    if (nb > 0 && nb <= ncoils) {
+      coef.insert(coef.end(), rows.begin(), rows.end());
+      g.nbas = nb;
+      g.bco = (const float*)arena.upload(coef.data(), coef.size() * 4, st);
+      g.bas = g.bco + (size_t)ncoils * kBasisPad;
+    }
   }
   g.ex = (const float*)arena.upload(ex.data(), ex.size() * 4, st);
   g.ey = (const float*)arena.upload(ey.data(), ey.size() * 4, st);
@@ -482,7 +579,23 @@ void epi_operator_set_fieldmap(EpiOperator* op, const float* fmap) {
 // Selects the y-stages: 0 the exact per-line phasors, 1 / 2 the time-segmented tensor-core
 // contractions in split f16 / split bf16 (built here: segmentation, tables, tensor maps).
 void epi_operator_set_segmented(EpiOperator* op, int precision) {
-  TsPlan* fresh = precision ? ts_plan_build(*op, precision) : nullptr;
+  // the segmented y-stages write coil or class rows: a plan on basis rows is built again without
+  // them, and with them again when the exact path returns
+  std::unique_ptr<EpiPlan> was;
+  if ((precision != 0 && op->plan->basis_nb > 0) || (precision == 0 && op->plan->opt.no_basis)) {
+    EpiPlanOptions o = op->plan->opt;
+    o.no_basis = precision != 0 ? 1 : 0;
+    was.reset(epi_plan_create(op->plan->host_units.data(), op->plan->n_units, op->plan->host_statics.data(),
+                              (int)op->plan->host_statics.size(), &o));
+    std::swap(was, op->plan);
+  }
+  TsPlan* fresh = nullptr;
+  try {
+    fresh = precision ? ts_plan_build(*op, precision) : nullptr;
+  } catch (...) {  // refused: the operator stays as it was
+    if (was) std::swap(was, op->plan);
+    throw;
+  }
   ts_plan_destroy(op->ts);
   op->ts = fresh;
   op->ts_precision = precision;

@@ -25,7 +25,8 @@
 // Kernels, in the order a step runs them:
 //   statics_kernel                     static phase a(x,y) in turns (FP64 per-slice quadratic)
 //   ystage_q_kernel / ystage_kernel    y-stage (staged-input form; per-thread-load fallback);
-//                                      with the 8-coil ring it accumulates 5 ey classes + offset
+//                                      with the 8-coil ring it accumulates 5 ey classes + offset,
+//                                      with other rings of 6 or more coils the rows of a coil basis
 //   xfft_warp_kernel / xfft_kernel /   x-stage: warp-per-row FFT (N = 32..256), shared-memory
 //   xgemm_kernel                       radix-2 FFT (other powers of two), DFT GEMM (other widths)
 //   yadjoint_q_kernel / yadjoint_kernel  y-adjoint (fixed coil or class count; any coil count)
@@ -114,9 +115,9 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 }
 
 // cp.async helpers (16-byte copies zero-fill the bytes past src_bytes)
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
+__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src, int src_bytes = 8) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
@@ -124,6 +125,11 @@ __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_g
 template <int N>
 __device__ __forceinline__ void cp_async_wait_n() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+}
+
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src, int src_bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, int src_bytes) {
@@ -396,9 +402,11 @@ __host__ __device__ __forceinline__ constexpr int fwdq_rows(int nc, bool maps) {
 // NV > 0: the tile holds every coil of the unit and accumulates coil classes instead of coils
 // (NV = classes + 1 for the coil offset): acc_v += ey_v(y) W P, acc_off += W P, and the epilogue
 // expands g_q = s (ex_q acc_cls(q) + off acc_off).
-// cls_rows (with NV): write the class rows G_v = s T_v and G_off = s off T_off ([v][line][x], the
-// layout the class-mode x-stage expands) instead of the coil rows.
-template <int QG, int NV, int NC, bool MAPS>
+// cls_rows (with NV): 1 writes the class rows G_v = s T_v and G_off = s off T_off ([v][line][x],
+// the layout the class-mode x-stage expands) instead of the coil rows; 2 writes basis rows (the
+// unit's eyc holds the coil basis, whose last row is constant), G_v = s T_v for every row.
+// NARROW: some plane or row is not on a 16-byte boundary, so the ring fills by 4-byte copies.
+template <int QG, int NV, int NC, bool MAPS, bool NARROW>
 __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __restrict__ units,
                                                           const Tile* __restrict__ tiles, int cls_rows) {
   constexpr int T = 4, TL = 8;
@@ -438,7 +446,15 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   const int x0 = tl.x0;
   const int nch = (sny + RC - 1) / RC;
   auto issue_rows = [&](int c) {
-    if (c < nch) {
+    if (NARROW && c < nch) {
+      float* dst = ring + (c % kFwdStages) * STAGE;
+      for (int k = tid; k < STAGE; k += 256) {
+        const int pl = k / (RC * 128), r = (k / 128) % RC, xx = x0 + (k & 127), y = c * RC + r;
+        const float* base = plane_s[pl];
+        const bool ok = base != nullptr && y < sny && xx < snx;
+        cp_async4(dst + k, ok ? base + (size_t)y * snx + xx : (const float*)u.g, ok ? 4 : 0);
+      }
+    } else if (c < nch) {
       float* dst = ring + (c % kFwdStages) * STAGE;
 #pragma unroll
       for (int i = 0; i < PPT; ++i) {
@@ -649,7 +665,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
       if (jb + j >= nl) break;
 #pragma unroll
       for (int v = 0; v < NA; ++v) {
-        const float sv = v == NA - 1 ? s * off : s;
+        const float sv = v == NA - 1 && cls_rows == 1 ? s * off : s;
         u.g[((size_t)v * u.n_lines + tl.line0 + jb + j) * snx + x] = make_float2(sv * acc[j][v].x, sv * acc[j][v].y);
       }
     }
@@ -921,8 +937,10 @@ __host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps,
 
 
 // VIRT: the h rows are the NQ = classes + 1 class rows of the class-mode x-adjoint (scale, ex and
-// the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row.
-template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT>
+// the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
+// or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
+// NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
+template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW>
 __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
                                                             const int4* __restrict__ tiles) {
   extern __shared__ __align__(16) float smem[];
@@ -965,7 +983,14 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
   }
   auto issue_chunk = [&](int c, int stage) {
-    if (c < nchunks) {
+    if (NARROW && c < nchunks) {
+      float2* dst = hbuf + stage * STAGE;
+      for (int k = tid; k < STAGE; k += 256) {
+        const int r = k >> 7, xx = x0 + (k & 127), j = c * JC + r / NQ;
+        const bool ok = xx < snx && j < nlines;
+        cp_async8(dst + k, gsrc + (ok ? ((size_t)(r % NQ) * nlines + j) * snx + xx : 0), ok ? 8 : 0);
+      }
+    } else if (c < nchunks) {
       const int rem = nlines - c * JC, jo = c * JC * snx;
       float2* dst = hbuf + stage * STAGE;
 #pragma unroll
@@ -1260,9 +1285,12 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
 //   forward : out[q][row_j][kx] = (1/nvox) sum_x  g[q][j][x] E_j(x)        tw_pol[x][kx]
 //   adjoint : h[q][j][x]        = (1/nvox) conj(E_j(x)) sum_kx conj(tw_pol[x][kx]) r[q][row_j][kx]
 // Each of 256 threads owns 4 rows x 2 columns.
+// nb > 0: g holds the unit's nb basis rows ([r][line][x]).  The forward forms each coil's
+// g_q = ex_q sum_r U_qr G_r + off G_last as it stages A; the adjoint's tile holds every coil of its
+// lines and writes G_r = s sum_q (ex_q U_qr + off [r = last]) h_q.
 template <bool ADJ>
 __global__ void __launch_bounds__(256) xgemm_kernel(const UnitDesc* __restrict__ units,
-                                                    const XTile* __restrict__ tiles) {
+                                                    const XTile* __restrict__ tiles, int nb) {
   __shared__ float2 As[32][33];   // [row][k]
   __shared__ float2 Bs[32][64];   // [k][col]
   __shared__ int lrow[32], lline[32], lq[32];
@@ -1306,7 +1334,19 @@ __global__ void __launch_bounds__(256) xgemm_kernel(const UnitDesc* __restrict__
       float2 v = make_float2(0.f, 0.f);
       if (lq[r] >= 0 && k < K) {
         if (!ADJ) {
-          v = u.g[((size_t)lq[r] * u.n_lines + lline[r]) * snx + k];
+          if (nb > 0) {
+            const float* co = u.geo.bco + lq[r] * kBasisPad;
+            const float2* G = u.g + (size_t)lline[r] * snx + k;
+            const size_t rs = (size_t)u.n_lines * snx;
+            float2 t = make_float2(0.f, 0.f), last = t;
+            for (int b = 0; b < nb; ++b) {
+              last = G[b * rs];
+              t = ffma2(dup2(co[b]), last, t);
+            }
+            v = ffma2(dup2(u.geo.coil_off), last, fmul2(dup2(u.geo.ex[(size_t)lq[r] * snx + k]), t));
+          } else {
+            v = u.g[((size_t)lq[r] * u.n_lines + lline[r]) * snx + k];
+          }
           if (eddy) {
             const double xc = ((double)k - sxs - xoff) / ox;
             double tv = ((double)u.eddy_cx * xc + (double)u.eddy_qx * xc * xc + (double)u.eddy_z) * (double)ldec[r];
@@ -1369,8 +1409,35 @@ __global__ void __launch_bounds__(256) xgemm_kernel(const UnitDesc* __restrict__
           __sincosf(kTwoPiF * (float)tv, &sn, &cs);
           v = make_float2(v.x * cs + v.y * sn, v.y * cs - v.x * sn);
         }
-        u.g[((size_t)lq[r] * u.n_lines + lline[r]) * snx + col] = v;
+        if (nb > 0)
+          Bs[r][tx + 32 * h] = v;  // every thread left the last k chunk's products at a barrier
+        else
+          u.g[((size_t)lq[r] * u.n_lines + lline[r]) * snx + col] = v;
       }
+    }
+  }
+  if (ADJ && nb > 0) {
+    __syncthreads();
+    const float s = u.signal_scale, so = s * u.geo.coil_off;
+    for (int e = threadIdx.x; e < T.nl * 64; e += 256) {
+      const int jj = e >> 6, c = e & 63, col = T.col0 + c;
+      if (col >= N) continue;
+      float2 G[kBasisPad - 1], sum = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int b = 0; b < kBasisPad - 1; ++b) G[b] = make_float2(0.f, 0.f);
+      for (int q = 0; q < T.nq; ++q) {
+        const float2 h = Bs[jj * T.nq + q][c];
+        const float* co = u.geo.bco + (T.q0 + q) * kBasisPad;
+        const float2 w = fmul2(dup2(s * u.geo.ex[(size_t)(T.q0 + q) * snx + col]), h);
+        sum = fadd2(sum, h);
+#pragma unroll
+        for (int b = 0; b < kBasisPad - 1; ++b)
+          if (b < nb) G[b] = ffma2(dup2(co[b]), w, G[b]);
+      }
+      const size_t base = (size_t)T.line[jj] * snx + col, rs = (size_t)u.n_lines * snx;
+#pragma unroll
+      for (int b = 0; b < kBasisPad - 1; ++b)
+        if (b < nb) u.g[base + b * rs] = b == nb - 1 ? ffma2(dup2(so), sum, G[b]) : G[b];
     }
   }
 }
@@ -1492,6 +1559,76 @@ __host__ __device__ constexpr int bitrev_c(int v, int bits) {
 }
 __host__ __device__ constexpr int log2_c(int v) { return v <= 1 ? 0 : 1 + log2_c(v / 2); }
 
+// The transform of one row held by a warp: in, b[bitrev(m)] (E a power of two; else b[m]) is
+// x[lane + 32 m]; out, b[k1] is X[k1 + E bitrev5(lane)].  tw: e^{-i2pi j/N} in shared memory.
+template <int E, bool ADJ>
+__device__ __forceinline__ void warp_row_fft(float2 (&b)[E], const float2* tw, int lane) {
+  constexpr int N = 32 * E;
+  constexpr bool P2 = (E & (E - 1)) == 0;
+  // W(j) = e^{sigma i2pi j/N}: sigma = +1 forward, -1 adjoint
+  auto W = [&](int j) {
+    const float2 w = tw[j];
+    return ADJ ? w : make_float2(w.x, -w.y);
+  };
+  // E-point DFT of the registers: decimation in time from bit-reversed order, or for E not a
+  // power of two the direct sum Y[k1] = sum_m b[m] W^{32 (m k1 mod E)}
+  if (!P2) {
+    float2 y[E];
+#pragma unroll
+    for (int k1 = 0; k1 < E; ++k1) {
+      y[k1] = b[0];
+#pragma unroll
+      for (int m = 1; m < E; ++m) {
+        const float2 v = (m * k1) % E == 0 ? b[m] : cmul(b[m], W(32 * ((m * k1) % E)));
+        y[k1] = make_float2(y[k1].x + v.x, y[k1].y + v.y);
+      }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < E; ++k1) b[k1] = y[k1];
+  }
+#pragma unroll
+  for (int len = 2; len <= (P2 ? E : 1); len <<= 1) {
+#pragma unroll
+    for (int i = 0; i < E; i += len) {
+#pragma unroll
+      for (int p = 0; p < len / 2; ++p) {
+        float2 v = b[i + p + len / 2];
+        const int j = p * (E / len) * 32;
+        if (4 * j == N)  // W(N/4) = sigma i exactly
+          v = ADJ ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x);
+        else if (p != 0)
+          v = cmul(v, W(j));
+        const float2 a = b[i + p];
+        b[i + p] = make_float2(a.x + v.x, a.y + v.y);
+        b[i + p + len / 2] = make_float2(a.x - v.x, a.y - v.y);
+      }
+    }
+  }
+#pragma unroll
+  for (int k1 = 1; k1 < E; ++k1) b[k1] = cmul(b[k1], W(lane * k1));
+  // 32-point DFTs across the lanes: radix-2 decimation in frequency.  The last two stages'
+  // twiddles are exact: 1 at h = 1, and 1 or W(N/4) = sigma i (a swap and a sign) at h = 2.
+#pragma unroll
+  for (int h = 16; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+    const float sg = up ? -1.f : 1.f;
+    const float2 w = h >= 4 && up ? W((lane & (h - 1)) * (N / (2 * h))) : make_float2(1.f, 0.f);
+    const bool quarter = h == 2 && up && (lane & 1);
+#pragma unroll
+    for (int k1 = 0; k1 < E; ++k1) {
+      const float ox_ = __shfl_xor_sync(0xffffffffu, b[k1].x, h);
+      const float oy_ = __shfl_xor_sync(0xffffffffu, b[k1].y, h);
+      const float2 v = make_float2(fmaf(sg, b[k1].x, ox_), fmaf(sg, b[k1].y, oy_));
+      if (h >= 4)
+        b[k1] = cmul(v, w);
+      else if (h == 2)  // times sigma i: -i for the adjoint (e^{-i pi/2}), +i for the forward
+        b[k1] = quarter ? (ADJ ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x)) : v;
+      else
+        b[k1] = v;
+    }
+  }
+}
+
 // CLS (8 coils in 5 classes + offset): a tile is (unit, first line, up to 4 lines) x all 8 coils.
 // Adjoint: warp w transforms coil w of each line into shared memory, and the CTA then writes the
 // 6 class rows G_v = s sum_{q in v} ex_q h_q, G_off = s off sum_q h_q ([v][line][x] in g) that
@@ -1564,11 +1701,6 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
   }
   if (CLS && !ADJ) cp_async_wait0();
   __syncthreads();
-  // W(j) = e^{sigma i2pi j/N}: sigma = +1 forward, -1 adjoint
-  auto W = [&](int j) {
-    const float2 w = tw[j];
-    return ADJ ? w : make_float2(w.x, -w.y);
-  };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ox = N / nx, xs = nx / 2, sxs = ox * xs;
   const double xoff = (ox - 1.0) / 2.0;
@@ -1639,63 +1771,7 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
         b[P2 ? bitrev_c(m, LE) : m] = v;
       }
     }
-    // E-point DFT of the registers: decimation in time from bit-reversed order, or for E not a
-    // power of two the direct sum Y[k1] = sum_m b[m] W^{32 (m k1 mod E)}
-    if (!P2) {
-      float2 y[E];
-#pragma unroll
-      for (int k1 = 0; k1 < E; ++k1) {
-        y[k1] = b[0];
-#pragma unroll
-        for (int m = 1; m < E; ++m) {
-          const float2 v = (m * k1) % E == 0 ? b[m] : cmul(b[m], W(32 * ((m * k1) % E)));
-          y[k1] = make_float2(y[k1].x + v.x, y[k1].y + v.y);
-        }
-      }
-#pragma unroll
-      for (int k1 = 0; k1 < E; ++k1) b[k1] = y[k1];
-    }
-#pragma unroll
-    for (int len = 2; len <= (P2 ? E : 1); len <<= 1) {
-#pragma unroll
-      for (int i = 0; i < E; i += len) {
-#pragma unroll
-        for (int p = 0; p < len / 2; ++p) {
-          float2 v = b[i + p + len / 2];
-          const int j = p * (E / len) * 32;
-          if (4 * j == N)  // W(N/4) = sigma i exactly
-            v = ADJ ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x);
-          else if (p != 0)
-            v = cmul(v, W(j));
-          const float2 a = b[i + p];
-          b[i + p] = make_float2(a.x + v.x, a.y + v.y);
-          b[i + p + len / 2] = make_float2(a.x - v.x, a.y - v.y);
-        }
-      }
-    }
-#pragma unroll
-    for (int k1 = 1; k1 < E; ++k1) b[k1] = cmul(b[k1], W(lane * k1));
-    // 32-point DFTs across the lanes: radix-2 decimation in frequency.  The last two stages'
-    // twiddles are exact: 1 at h = 1, and 1 or W(N/4) = sigma i (a swap and a sign) at h = 2.
-#pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-      const bool up = (lane & h) != 0;
-      const float sg = up ? -1.f : 1.f;
-      const float2 w = h >= 4 && up ? W((lane & (h - 1)) * (N / (2 * h))) : make_float2(1.f, 0.f);
-      const bool quarter = h == 2 && up && (lane & 1);
-#pragma unroll
-      for (int k1 = 0; k1 < E; ++k1) {
-        const float ox_ = __shfl_xor_sync(0xffffffffu, b[k1].x, h);
-        const float oy_ = __shfl_xor_sync(0xffffffffu, b[k1].y, h);
-        const float2 v = make_float2(fmaf(sg, b[k1].x, ox_), fmaf(sg, b[k1].y, oy_));
-        if (h >= 4)
-          b[k1] = cmul(v, w);
-        else if (h == 2)  // times sigma i: -i for the adjoint (e^{-i pi/2}), +i for the forward
-          b[k1] = quarter ? (ADJ ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x)) : v;
-        else
-          b[k1] = v;
-      }
-    }
+    warp_row_fft<E, ADJ>(b, tw, lane);
     const int k2 = __brev(lane) >> 27;
 #pragma unroll
     for (int k1 = 0; k1 < E; ++k1) {
@@ -1749,6 +1825,207 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
       G[5] = make_float2(so * G[5].x, so * G[5].y);
 #pragma unroll
       for (int v = 0; v < 6; ++v) gbuf[((size_t)v * nl + r0 + jl) * N + x] = G[v];
+    }
+  }
+}
+
+// The same x-stage on the rows of a coil basis (nb of them, at most 7), for any coil count: a tile is
+// (unit, first line, lines) x every coil.  Forward: the tile's basis rows G_r ([r][line][x] in g, the
+// y-stage's) are staged once, and each coil's row is formed as the warp loads it,
+//   g_q(x) = ex_q(x) sum_r U_qr G_r(x) + off G_last(x);
+// adjoint: the coils' rows h_q pass through shared memory, at most 32 at a time, and the CTA writes
+//   G_r(x) = s sum_q (ex_q(x) U_qr + off [r = last]) h_q(x).
+// Against one row per coil the forward reads and the adjoint writes nb rows in place of ncoils, and
+// both y-stages run on nb rows.  The coil sums cost 2 (nb + 1) FMAs per row element, about what the
+// row's transform costs, and stay small beside the y-stages (each element serves sny voxels).
+constexpr int kBasisRows = 32;  // coil rows the adjoint holds at a time
+__host__ __device__ constexpr int basis_lines(int ncoils) { return ncoils >= kBasisRows ? 1 : kBasisRows / ncoils; }
+// float2 of dynamic shared memory: tables, reorder rows, then the staged basis or coil rows
+__host__ __device__ constexpr size_t basis_smem(int E, int staged_rows) {
+  return (size_t)(32 * E) * 4 + 8 * (size_t)(33 * E) + (size_t)staged_rows * 32 * E;
+}
+
+template <int E, bool ADJ>
+__global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kernel(const UnitDesc* __restrict__ units,
+                                                            const int4* __restrict__ tiles, int nb) {
+  constexpr int N = 32 * E, LE = log2_c(E);
+  constexpr bool P2 = (E & (E - 1)) == 0;
+  constexpr int NP = N + N / 32;
+  extern __shared__ __align__(16) float2 bsm[];
+  float2* tw = bsm;           // e^{-i2pi j/N}
+  float2* pm = tw + N;        // premodulation per polarity
+  float2* pt = pm + 2 * N;    // post-twiddle per kx (nx <= N)
+  float2* rb = pt + N;        // [8][NP]
+  float2* st = rb + 8 * NP;   // forward: basis rows [line][r][x]; adjoint: coil rows [line][coil][x]
+  __shared__ float co[kMaxCoils * kBasisPad];
+  __shared__ int lrow[kBasisRows], lpol[kBasisRows];
+  __shared__ float ldec[kBasisRows];
+  const int4 t = tiles[blockIdx.x];
+  const UnitDesc& u = units[t.x];
+  const int j0 = t.y, nj = t.z;
+  const int nx = u.nx, nl = u.n_lines, n_rows = u.n_rows, nc = u.ncoils;
+  float2* const ksp = u.kspace;
+  float2* const gbuf = u.g;
+  const float* __restrict__ exg = u.geo.ex;
+  if (!ADJ) {  // issued first: the copies' latency overlaps the table setup
+    constexpr int HN = N / 2;
+    const float4* g4 = reinterpret_cast<const float4*>(gbuf);
+    float4* h4 = reinterpret_cast<float4*>(st);
+    for (int e = threadIdx.x; e < nj * nb * HN; e += 256) {
+      const int jl = e / (nb * HN), r = (e / HN) % nb, x2 = e % HN;
+      cp_async16(h4 + e, g4 + ((size_t)r * nl + j0 + jl) * HN + x2, 16);
+    }
+    cp_async_commit();
+  }
+  const float2* __restrict__ xf = u.geo.xf;
+  for (int k = threadIdx.x; k < N / 2; k += 256) {
+    const float2 w = xf[k];
+    tw[k] = w;
+    tw[k + N / 2] = make_float2(-w.x, -w.y);
+  }
+  const float inv_n = 1.0f / (float)(N * u.sny);
+  for (int k = threadIdx.x; k < 2 * N; k += 256) {
+    const float2 v = xf[N / 2 + k];
+    pm[k] = ADJ ? make_float2(v.x * inv_n, v.y * inv_n) : v;
+  }
+  for (int k = threadIdx.x; k < nx; k += 256) {
+    const float2 v = xf[N / 2 + 2 * N + k];
+    pt[k] = ADJ ? v : make_float2(v.x * inv_n, v.y * inv_n);
+  }
+  for (int k = threadIdx.x; k < nc * kBasisPad; k += 256) co[k] = u.geo.bco[k];
+  if (threadIdx.x < nj) {
+    const LineRec& L = u.lines[j0 + threadIdx.x];
+    lrow[threadIdx.x] = L.row;
+    lpol[threadIdx.x] = L.pol < 0 ? 1 : 0;
+    ldec[threadIdx.x] = L.decay;
+  }
+  if (!ADJ) cp_async_wait0();
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ox = N / nx, xs = nx / 2, sxs = ox * xs;
+  const double xoff = (ox - 1.0) / 2.0;
+  const bool eddy = (u.flags & UF_EDDY) != 0;
+  const int kpos = nx - xs;
+  const float off = u.geo.coil_off;
+  float2* row = rb + warp * NP;
+  auto modulation = [&](int pol, float dec, int x) {  // as xfft_warp_kernel's
+    float2 md = pm[pol * N + x];
+    if (eddy) {
+      const double xc = ((double)x - sxs - xoff) / ox;
+      double tv = ((double)u.eddy_cx * xc + (double)u.eddy_qx * xc * xc + (double)u.eddy_z) * (double)dec;
+      tv -= rint(tv);
+      float sn, cs;
+      __sincosf(kTwoPiF * (float)tv, &sn, &cs);
+      md = cmul(md, make_float2(cs, sn));
+    }
+    return md;
+  };
+  for (int q0 = 0; q0 < nc; q0 += ADJ ? kBasisRows : nc) {
+    const int nq = ADJ ? min(kBasisRows, nc - q0) : nc;
+    const int nr = nj * nq;
+    // adjoint: the next row's k-space samples are loaded while the current one transforms
+    float2 pre[ADJ ? E : 1];
+    auto fetch = [&](int r) {
+      const float2* kr = ksp + ((size_t)(q0 + r % nq) * n_rows + lrow[r / nq]) * nx;
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const int n = lane + 32 * m;
+        const int kx = (n < kpos ? n : n - N) + xs;
+        pre[ADJ ? m : 0] = kx >= 0 && kx < nx ? kr[kx] : make_float2(0.f, 0.f);
+      }
+    };
+    if (ADJ && warp < nr) fetch(warp);
+    for (int r = warp; r < nr; r += 8) {
+      const int jl = r / nq, q = q0 + r % nq, pol = lpol[jl];
+      const float dec = ldec[jl];
+      float2 b[E];
+      if (!ADJ) {
+        const float4 c0 = *reinterpret_cast<const float4*>(co + q * kBasisPad);
+        const float4 c1 = *reinterpret_cast<const float4*>(co + q * kBasisPad + 4);
+        const float cf[kBasisPad] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const float2* cr = st + jl * nb * N;
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          const int x = lane + 32 * m;
+          const float ex = __ldg(exg + q * N + x);
+          float2 a = fmul2(dup2(cf[0]), cr[x]), last = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int v = 1; v < kBasisPad - 1; ++v)
+            if (v < nb) {
+              last = cr[v * N + x];
+              a = ffma2(dup2(cf[v]), last, a);
+            }
+          const float2 g = ffma2(dup2(off), last, fmul2(dup2(ex), a));
+          b[P2 ? bitrev_c(m, LE) : m] = cmul(g, modulation(pol, dec, x));
+        }
+      } else {
+        float2 cur[E];
+#pragma unroll
+        for (int m = 0; m < E; ++m) cur[m] = pre[ADJ ? m : 0];
+        if (r + 8 < nr) fetch(r + 8);
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          const int n = lane + 32 * m;
+          const int kx = (n < kpos ? n : n - N) + xs;
+          float2 v = make_float2(0.f, 0.f);
+          if (kx >= 0 && kx < nx) {
+            const float2 p = pt[kx];
+            v = cmul(cur[m], make_float2(p.x, -p.y));
+          }
+          b[P2 ? bitrev_c(m, LE) : m] = v;
+        }
+      }
+      warp_row_fft<E, ADJ>(b, tw, lane);
+      const int k2 = __brev(lane) >> 27;
+#pragma unroll
+      for (int k1 = 0; k1 < E; ++k1) {
+        const int k = k1 + E * k2;
+        row[k + (k >> 5)] = b[k1];
+      }
+      __syncwarp();
+      if (!ADJ) {
+        float2* out = ksp + ((size_t)q * n_rows + lrow[jl]) * nx;
+        for (int kx = lane; kx < nx; kx += 32) {
+          const int k = kx >= xs ? kx - xs : kx - xs + N;
+          out[kx] = cmul(row[k + (k >> 5)], pt[kx]);
+        }
+      } else {
+        float2* gr = st + (size_t)r * N;
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          const int x = lane + 32 * m;
+          const float2 md = modulation(pol, dec, x);
+          gr[x] = cmul(row[x + (x >> 5)], make_float2(md.x, -md.y));
+        }
+      }
+      __syncwarp();
+    }
+    if (ADJ) {
+      __syncthreads();
+      const float s = u.signal_scale, so = s * off;
+      for (int e = threadIdx.x; e < nj * N; e += 256) {
+        const int jl = e / N, x = e % N;
+        const size_t base = (size_t)(j0 + jl) * N + x, rs = (size_t)nl * N;
+        float2 G[kBasisPad - 1], sum = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int v = 0; v < kBasisPad - 1; ++v)  // past the first 32 coils: on from this thread's own sums
+          G[v] = q0 > 0 && v < nb ? gbuf[base + v * rs] : make_float2(0.f, 0.f);
+        const float2* hr = st + (size_t)jl * nq * N + x;
+        for (int q = 0; q < nq; ++q) {
+          const float2 h = hr[q * N];
+          const float4 c0 = *reinterpret_cast<const float4*>(co + (q0 + q) * kBasisPad);
+          const float4 c1 = *reinterpret_cast<const float4*>(co + (q0 + q) * kBasisPad + 4);
+          const float cf[kBasisPad] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+          const float2 w = fmul2(dup2(s * __ldg(exg + (q0 + q) * N + x)), h);
+          sum = fadd2(sum, h);
+#pragma unroll
+          for (int v = 0; v < kBasisPad - 1; ++v) G[v] = ffma2(dup2(cf[v]), w, G[v]);
+        }
+#pragma unroll
+        for (int v = 0; v < kBasisPad - 1; ++v)
+          if (v < nb) gbuf[base + v * rs] = v == nb - 1 ? ffma2(dup2(so), sum, G[v]) : G[v];
+      }
+      __syncthreads();  // before the next coils' rows overwrite these
     }
   }
 }
@@ -1816,7 +2093,6 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
     p->n_units = n;
     p->host_units.assign(hu, hu + n);
     p->host_statics.assign(hs, hs + ns);
-    p->d_units = (UnitDesc*)dev_upload(p, hu, sizeof(UnitDesc) * n);
     p->n_statics = ns;
     p->d_statics = (StaticDesc*)dev_upload(p, hs, sizeof(StaticDesc) * ns);
     for (int i = 0; i < ns; ++i) p->max_static_n = std::max(p->max_static_n, hs[i].snx * hs[i].sny);
@@ -1837,46 +2113,6 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
     for (int i = 0; i < n; ++i) max_comp = std::max(max_comp, hu[i].ncomp);
     p->nc = max_comp <= 1 ? 1 : max_comp <= 2 ? 2 : max_comp <= 3 ? 3 : max_comp <= 4 ? 4 : 8;
     p->qg = max_coils <= 1 ? 1 : max_coils <= 2 ? 2 : max_coils <= 4 ? 4 : 8;
-    // the staged-input forward serves a pass when every unit has snx % 4 == 0 and 16-byte aligned
-    // input planes (cooperative 16-byte copies)
-    auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
-    for (int pass = 0; pass < 2; ++pass) {
-      bool ok = true;
-      for (int i = 0; i < n; ++i) {
-        const UnitDesc& u = hu[i];
-        if (((u.flags & UF_MAPS) != 0) != (pass == 1)) continue;
-        ok = ok && (u.snx % 4) == 0 && al16(u.phase) && al16(u.fmap) && al16(u.comp) && al16(u.t2map) &&
-             al16(u.timap) && al16(u.log_amp) && (u.ncomp <= 1 || u.comp_stride % 4 == 0) &&
-             (u.ncomp <= 1 || (u.map_stride % 4) == 0);
-      }
-      // eight coils with voxel maps (four or more compartments) or eight compartments take more
-      // registers than the 256-thread CTA leaves: those shapes keep the per-thread-load kernel
-      if (p->qg == 8 && (p->nc == 8 || (pass == 1 && p->nc >= 4))) ok = false;
-      p->fwdq[pass] = ok;
-      // coil classes: every unit with the same 8 coils in 5 classes (the ring) -> 6 accumulators
-      bool cl = ok && n > 0 && p->qg == 8 && (pass == 0 || p->nc <= 3);
-      for (int i = 0; i < n && cl; ++i) {
-        const UnitDesc& u = hu[i];
-        if (((u.flags & UF_MAPS) != 0) != (pass == 1)) continue;
-        cl = u.ncoils == 8 && u.geo.ncls == 5 && u.geo.coil_off != 0.f && u.geo.cls && u.geo.eyc;
-      }
-      p->fwd_nv[pass] = (cl && !p->opt.no_classes) ? 6 : 0;
-    }
-    for (int pass = 0; pass < 2; ++pass) {
-      std::vector<int4> tiles;
-      const int step = p->fwdq[pass] ? 8 : kT;
-      p->y_start[pass].assign(n + 1, 0);
-      for (int i = 0; i < n; ++i) {
-        p->y_start[pass][i] = (int)tiles.size();
-        if (((hu[i].flags & UF_MAPS) != 0) != (pass == 1)) continue;
-        for (int l = 0; l < hu[i].n_lines; l += step)
-          for (int x0 = 0; x0 < hu[i].snx; x0 += 128)
-            for (int q0 = 0; q0 < hu[i].ncoils; q0 += p->qg) tiles.push_back(make_int4(i, l, x0, q0));
-      }
-      p->y_start[pass][n] = (int)tiles.size();
-      p->n_ytiles[pass] = (int)tiles.size();
-      p->d_ytiles[pass] = (int4*)dev_upload(p, tiles.data(), sizeof(int4) * tiles.size());
-    }
     // x-stage as per-row FFTs when every unit has a power-of-two snx with FFT tables
     p->xfft = n > 0 && !p->opt.dft_x;
     for (int i = 0; i < n; ++i) {
@@ -1903,7 +2139,105 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           if (!(N >= 8 && N <= kXfftMaxN && (N & (N - 1)) == 0)) p->xfft = false;
         }
     }
-    if (p->xfft && p->xfft_e < 0) {
+    // The coil basis (coil_basis, driver.cpp) where every unit has one of the same row count: rings of
+    // 6, 7 and 9 or more coils, and of 8 where the class rows have no x-stage (rows past 128 points,
+    // the DFT GEMM).  Its 4 to 7 rows replace the coils in both y-stages, whose work per voxel and
+    // line is the phase plus two FMAs per row: one series of 32 coils (128 x 128 on 256 x 256, 120
+    // units) takes 4.3 ms against 19.3 ms with 32 rows.  The kernels with eight compartments, or four
+    // with voxel maps, have no registers for it; the x-stages that expand the rows are the warp FFT
+    // and, with every coil in one tile (32), the DFT GEMM.
+    {
+      const bool gemm = !p->xfft, warp = p->xfft && p->xfft_e != 0;
+      const bool cls8 = p->xfft && p->xfft_e >= 1 && p->xfft_e <= 4;
+      int nb = n > 0 && !p->opt.no_classes && !p->opt.no_basis && (gemm || warp) && p->nc <= 4 ? hu[0].geo.nbas : 0;
+      bool all8 = true, any_maps = false;
+      for (int i = 0; i < n && nb; ++i) {
+        const UnitDesc& u = hu[i];
+        all8 = all8 && u.ncoils == 8;
+        any_maps = any_maps || (u.flags & UF_MAPS) != 0;
+        if (u.geo.nbas != nb || (gemm && u.ncoils > 32) || (warp && ((uintptr_t)u.g & 15)) ||
+            (long long)u.ncoils * u.n_lines * u.snx >= (1LL << 31))
+          nb = 0;
+      }
+      if ((all8 && cls8) || (any_maps && p->nc > 3)) nb = 0;
+      p->basis_nb = nb;
+    }
+    {  // the kernels read the rows a y-stage runs on as geo.ncls rows of geo.eyc and a constant one
+      std::vector<UnitDesc> du(hu, hu + n);
+      if (p->basis_nb)
+        for (UnitDesc& u : du) {
+          u.geo.ncls = u.geo.nbas - 1;
+          u.geo.eyc = u.geo.bas;
+        }
+      p->d_units = (UnitDesc*)dev_upload(p, du.data(), sizeof(UnitDesc) * n);
+    }
+    // the staged-input forward serves a pass when every unit has snx % 4 == 0 and 16-byte aligned
+    // input planes (cooperative 16-byte copies), and on basis rows also when not (4-byte copies; 12
+    // coils, voxel maps, rows of 150: 0.44 ms against 0.87 ms with the per-thread loads)
+    auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
+    for (int pass = 0; pass < 2; ++pass) {
+      bool ok = true, wide = true;
+      for (int i = 0; i < n; ++i) {
+        const UnitDesc& u = hu[i];
+        if (((u.flags & UF_MAPS) != 0) != (pass == 1)) continue;
+        wide = wide && (u.snx % 4) == 0 && al16(u.phase) && al16(u.fmap) && al16(u.comp) && al16(u.t2map) &&
+             al16(u.timap) && al16(u.log_amp) && (u.ncomp <= 1 || u.comp_stride % 4 == 0) &&
+             (u.ncomp <= 1 || (u.map_stride % 4) == 0);
+      }
+      // eight coils with voxel maps (four or more compartments) or eight compartments take more
+      // registers than the 256-thread CTA leaves: those shapes keep the per-thread-load kernel
+      if (p->qg == 8 && (p->nc == 8 || (pass == 1 && p->nc >= 4))) ok = false;
+      if (!wide && !p->basis_nb) ok = false;
+      p->fwdq[pass] = ok;
+      p->fwd_narrow[pass] = !wide;
+      // coil classes: every unit with the same 8 coils in 5 classes (the ring) -> 6 accumulators
+      bool cl = ok && n > 0 && p->qg == 8 && (pass == 0 || p->nc <= 3);
+      for (int i = 0; i < n && cl; ++i) {
+        const UnitDesc& u = hu[i];
+        if (((u.flags & UF_MAPS) != 0) != (pass == 1)) continue;
+        cl = u.ncoils == 8 && u.geo.ncls == 5 && u.geo.coil_off != 0.f && u.geo.cls && u.geo.eyc;
+      }
+      p->fwd_nv[pass] = p->basis_nb ? p->basis_nb : (cl && !p->opt.no_classes) ? 6 : 0;
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+      std::vector<int4> tiles;
+      const int step = p->fwdq[pass] ? 8 : kT;
+      p->y_start[pass].assign(n + 1, 0);
+      for (int i = 0; i < n; ++i) {
+        p->y_start[pass][i] = (int)tiles.size();
+        if (((hu[i].flags & UF_MAPS) != 0) != (pass == 1)) continue;
+        for (int l = 0; l < hu[i].n_lines; l += step)
+          for (int x0 = 0; x0 < hu[i].snx; x0 += 128)
+            for (int q0 = 0; q0 < (p->basis_nb ? 1 : hu[i].ncoils); q0 += p->qg) tiles.push_back(make_int4(i, l, x0, q0));
+      }
+      p->y_start[pass][n] = (int)tiles.size();
+      p->n_ytiles[pass] = (int)tiles.size();
+      p->d_ytiles[pass] = (int4*)dev_upload(p, tiles.data(), sizeof(int4) * tiles.size());
+    }
+    if (p->xfft && p->basis_nb) {
+      // tiles of a few lines x every coil: by unit, or with mixed widths ordered by width
+      std::vector<int4> ct;
+      auto unit_tiles = [&](int i) {
+        const int step = basis_lines(hu[i].ncoils);
+        p->basis_rows = std::max(p->basis_rows, step * std::min(hu[i].ncoils, kBasisRows));
+        p->basis_lines = std::max(p->basis_lines, step);
+        for (int j0 = 0; j0 < hu[i].n_lines; j0 += step)
+          ct.push_back(make_int4(i, j0, std::min(step, hu[i].n_lines - j0), 0));
+      };
+      if (p->xfft_e > 0) p->c_start.assign(n + 1, 0);
+      for (int E = 1; E <= 8; ++E) {
+        p->ce_first[E] = (int)ct.size();
+        for (int i = 0; i < n; ++i) {
+          if (hu[i].snx != 32 * E) continue;
+          if (p->xfft_e > 0) p->c_start[i] = (int)ct.size();
+          unit_tiles(i);
+        }
+        p->ce_count[E] = (int)ct.size() - p->ce_first[E];
+      }
+      if (p->xfft_e > 0) p->c_start[n] = (int)ct.size();
+      p->n_ctiles = (int)ct.size();
+      p->d_ctiles = (int4*)dev_upload(p, ct.data(), sizeof(int4) * ct.size());
+    } else if (p->xfft && p->xfft_e < 0) {
       // one list ordered by width, no per-unit ranges (such a plan runs whole)
       std::vector<int4> ft;
       for (int E = 1; E <= 8; ++E) {
@@ -1940,7 +2274,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         for (int i = 0; i < n && !any; ++i) any = ((hu[i].flags & UF_MAPS) != 0) == (pass == 1);
         if (any && p->fwd_nv[pass] != 6) fc = false;
       }
-      p->fwd_cls = fc;
+      p->fwd_cls = fc || p->basis_nb > 0;
     }
     // x-stage GEMM tiles, from host copies of the line tables (one copy per distinct table)
     std::map<const LineRec*, std::vector<LineRec>> host_lines;
@@ -1964,12 +2298,14 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->d_gtiles[dir] = dev_upload(p, xt.data(), sizeof(XTile) * xt.size());
     }
     // the fixed-coil-count y-adjoint serves a pass when every unit has the same coil count (1, 2,
-    // 4 or 8), an even snx and 16-byte aligned h rows (cooperative 16-byte copies)
+    // 4 or 8), an even snx and 16-byte aligned h rows (cooperative 16-byte copies), and on basis rows
+    // any of them (8-byte copies where some row is not so)
     int nq_all = n > 0 ? hu[0].ncoils : 0;
-    for (int i = 0; i < n; ++i)
-      if (hu[i].ncoils != nq_all || (hu[i].snx & 1) || ((uintptr_t)hu[i].g & 15) ||
-          (long long)hu[i].ncoils * hu[i].n_lines * hu[i].snx >= (1LL << 31))
-        nq_all = 0;
+    for (int i = 0; i < n; ++i) {
+      if (hu[i].ncoils != nq_all || (long long)hu[i].ncoils * hu[i].n_lines * hu[i].snx >= (1LL << 31)) nq_all = 0;
+      p->adj_narrow = p->adj_narrow || (hu[i].snx & 1) || ((uintptr_t)hu[i].g & 15);
+    }
+    if (p->adj_narrow) nq_all = 0;
     if (nq_all != 1 && nq_all != 2 && nq_all != 4 && nq_all != 8) nq_all = 0;
     // coil classes in the adjoint: every unit has the 8-coil ring (5 classes + offset), rows of
     // at most 128 points in the warp FFT, and the fixed-count y-adjoint for its shape
@@ -1979,14 +2315,14 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         const UnitDesc& u = hu[i];
         cl = u.ncoils == 8 && u.geo.ncls == 5 && u.geo.coil_off != 0.f && u.geo.cls && u.geo.eyc;
       }
-      p->adj_cls = cl && !p->opt.no_classes;
+      p->adj_cls = (cl && !p->opt.no_classes) || p->basis_nb > 0;
     }
     for (int pass = 0; pass < 4; ++pass) {
       bool maps = pass & 1, grads = pass & 2;
-      p->adjq[pass] = p->adj_cls ? 6 : (maps && p->nc == 8) ? 0 : nq_all;
+      p->adjq[pass] = p->basis_nb ? p->basis_nb : p->adj_cls ? 6 : (maps && p->nc == 8) ? 0 : nq_all;
       // rows per thread: the built-in choice, or 2 where 4 would be (the tunable)
       int ty = adjq_rows_v(p->nc, maps, p->adj_cls);
-      if (p->opt.adj_rows == 2 && ty == 4) ty = 2;
+      if (p->opt.adj_rows == 2 && ty == 4 && !(p->basis_nb && p->adj_narrow)) ty = 2;
       p->adj_ty[pass] = ty;
       const int step = p->adjq[pass] ? 2 * ty : kTY;
       std::vector<int4> yt;
@@ -2003,7 +2339,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->n_atiles[pass] = (int)yt.size();
       p->d_atiles[pass] = (int4*)dev_upload(p, yt.data(), sizeof(int4) * yt.size());
     }
-    if (p->adj_cls || p->fwd_cls) {  // the class x-stage tiles: 4 lines x the 8 coils
+    if (!p->basis_nb && (p->adj_cls || p->fwd_cls)) {  // the class x-stage tiles: 4 lines x the 8 coils
       std::vector<int4> ct;
       p->c_start.assign(n + 1, 0);
       for (int i = 0; i < n; ++i) {
@@ -2065,21 +2401,33 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
                                           (size_t)p->max_sny * (8 + (QG + 3) / 4 * 4));
       bool launched = false;
       const int NVv = p->fwd_nv[pass];
-#define MRSIM_YF(QGV, NVV, NCV, M)                                                      \
-  if (QG == QGV && NVv == NVV && NCv == NCV && maps == M) {                             \
-    auto k = ystage_q_kernel<QGV, NVV, NCV, M>;                                         \
+      const bool narrow = p->fwd_narrow[pass];
+#define MRSIM_YFW(QGV, NVV, NCV, M, W)                                                  \
+  if (QG == QGV && NVv == NVV && NCv == NCV && maps == M && narrow == W) {              \
+    auto k = ystage_q_kernel<QGV, NVV, NCV, M, W>;                                      \
     set_smem(k, smq);                                                                   \
-    k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles, p->fwd_cls ? 1 : 0);          \
+    k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles, p->basis_nb ? 2 : p->fwd_cls ? 1 : 0);  \
     launched = true;                                                                    \
   }
+#define MRSIM_YF(QGV, NVV, NCV, M) MRSIM_YFW(QGV, NVV, NCV, M, false)
+#define MRSIM_YFB(NVV) MRSIM_YFW(8, NVV, 1, false, true) MRSIM_YFW(8, NVV, 2, false, true) \
+  MRSIM_YFW(8, NVV, 3, false, true) MRSIM_YFW(8, NVV, 4, false, true) MRSIM_YFW(8, NVV, 1, true, true) \
+  MRSIM_YFW(8, NVV, 2, true, true) MRSIM_YFW(8, NVV, 3, true, true)
+      MRSIM_YFB(4) MRSIM_YFB(6) MRSIM_YFB(7)
 #define MRSIM_YFQ(NCV, M) MRSIM_YF(1, 0, NCV, M) MRSIM_YF(2, 0, NCV, M) MRSIM_YF(4, 0, NCV, M) MRSIM_YF(8, 0, NCV, M)
 #define MRSIM_YFN(M) MRSIM_YFQ(1, M) MRSIM_YFQ(2, M) MRSIM_YFQ(3, M) MRSIM_YFQ(4, M) MRSIM_YFQ(8, M)
       MRSIM_YFN(false) MRSIM_YFN(true)
       MRSIM_YF(8, 6, 1, false) MRSIM_YF(8, 6, 2, false) MRSIM_YF(8, 6, 3, false) MRSIM_YF(8, 6, 4, false)
       MRSIM_YF(8, 6, 1, true) MRSIM_YF(8, 6, 2, true) MRSIM_YF(8, 6, 3, true)
+      MRSIM_YF(8, 4, 1, false) MRSIM_YF(8, 4, 2, false) MRSIM_YF(8, 4, 3, false) MRSIM_YF(8, 4, 4, false)
+      MRSIM_YF(8, 4, 1, true) MRSIM_YF(8, 4, 2, true) MRSIM_YF(8, 4, 3, true)
+      MRSIM_YF(8, 7, 1, false) MRSIM_YF(8, 7, 2, false) MRSIM_YF(8, 7, 3, false) MRSIM_YF(8, 7, 4, false)
+      MRSIM_YF(8, 7, 1, true) MRSIM_YF(8, 7, 2, true) MRSIM_YF(8, 7, 3, true)
 #undef MRSIM_YFN
 #undef MRSIM_YFQ
 #undef MRSIM_YF
+#undef MRSIM_YFB
+#undef MRSIM_YFW
       if (!launched) fail("no forward kernel instance for this unit shape");
       MRSIM_CUDA(cudaGetLastError());
       continue;
@@ -2106,7 +2454,38 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
 
 namespace {
 void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) {
-  if ((adj && p->adj_cls) || (!adj && p->fwd_cls)) {
+  if (p->basis_nb && p->xfft) {
+    if (p->xfft_e < 0 && !(u0 == 0 && (u1 < 0 || u1 == p->n_units)))
+      fail("a plan of mixed row widths runs its units whole");
+    const TileRange R = tile_range(p->c_start, p->n_ctiles, u0, u1);
+    for (int E = 1; E <= 8; ++E) {
+      if (p->ce_count[E] == 0) continue;
+      // one width: the tiles of the unit range; mixed widths: the width's whole list
+      const int first = p->xfft_e > 0 ? R.t0 : p->ce_first[E], count = p->xfft_e > 0 ? R.n : p->ce_count[E];
+      if (count == 0) continue;
+      const int4* tiles = p->d_ctiles + first;
+      const size_t sm = sizeof(float2) * basis_smem(E, adj ? p->basis_rows : p->basis_lines * p->basis_nb);
+#define MRSIM_XB(EV, ADJ)                                                                 \
+  case EV: {                                                                              \
+    auto k = xfft_basis_kernel<EV, ADJ>;                                                  \
+    set_smem(k, sm);                                                                      \
+    k<<<(unsigned)count, 256, sm, st>>>(p->d_units, tiles, p->basis_nb);                  \
+    break;                                                                                \
+  }
+#define MRSIM_XBA(ADJ) MRSIM_XB(1, ADJ) MRSIM_XB(2, ADJ) MRSIM_XB(3, ADJ) MRSIM_XB(4, ADJ) \
+  MRSIM_XB(5, ADJ) MRSIM_XB(6, ADJ) MRSIM_XB(7, ADJ) MRSIM_XB(8, ADJ)
+      if (adj) {
+        switch (E) { MRSIM_XBA(true) }
+      } else {
+        switch (E) { MRSIM_XBA(false) }
+      }
+#undef MRSIM_XBA
+#undef MRSIM_XB
+      MRSIM_CUDA(cudaGetLastError());
+    }
+    return;
+  }
+  if (!p->basis_nb && ((adj && p->adj_cls) || (!adj && p->fwd_cls))) {
     const TileRange R = tile_range(p->c_start, p->n_ctiles, u0, u1);
     if (R.n == 0) return;
     const int4* tiles = p->d_ctiles + R.t0;
@@ -2185,9 +2564,9 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
   if (R.n == 0) return;
   const XTile* tiles = (const XTile*)p->d_gtiles[dir] + R.t0;
   if (adj)
-    xgemm_kernel<true><<<(unsigned)R.n, 256, 0, st>>>(p->d_units, tiles);
+    xgemm_kernel<true><<<(unsigned)R.n, 256, 0, st>>>(p->d_units, tiles, p->basis_nb);
   else
-    xgemm_kernel<false><<<(unsigned)R.n, 256, 0, st>>>(p->d_units, tiles);
+    xgemm_kernel<false><<<(unsigned)R.n, 256, 0, st>>>(p->d_units, tiles, p->basis_nb);
   MRSIM_CUDA(cudaGetLastError());
 }
 }  // namespace
@@ -2212,33 +2591,38 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
       bool launched = false;
       const bool virt = p->adj_cls;
       // the built-in rows per thread, and 2 rows where the built-in choice is 4
-#define MRSIM_AQV(NQV, NCV, M, G, V)                                                    \
-  if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V) {               \
+#define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
+  if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V && p->adj_narrow == W) { \
     if (TYv == adjq_rows_v(NCV, M, V)) {                                                \
-      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V>;            \
+      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W>;         \
       set_smem(k, smq);                                                                 \
       k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
       launched = true;                                                                  \
-    } else if (adjq_rows_v(NCV, M, V) == 4 && TYv == 2) {                               \
-      auto k = yadjoint_q_kernel<NQV, 2, NCV, M, G, V>;                                 \
+    } else if (!W && adjq_rows_v(NCV, M, V) == 4 && TYv == 2) {                         \
+      auto k = yadjoint_q_kernel<NQV, 2, NCV, M, G, V, false>;                          \
       set_smem(k, smq);                                                                 \
       k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
       launched = true;                                                                  \
     }                                                                                   \
   }
+#define MRSIM_AQV(NQV, NCV, M, G, V) MRSIM_AQW(NQV, NCV, M, G, V, false)
 #define MRSIM_AQ(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, false)
 #define MRSIM_AQC(NCV, M, G) MRSIM_AQ(1, NCV, M, G) MRSIM_AQ(2, NCV, M, G) MRSIM_AQ(4, NCV, M, G) MRSIM_AQ(8, NCV, M, G)
 #define MRSIM_AQN(M, G) MRSIM_AQC(1, M, G) MRSIM_AQC(2, M, G) MRSIM_AQC(3, M, G) MRSIM_AQC(4, M, G)
-#define MRSIM_AQK(M, G) MRSIM_AQV(6, 1, M, G, true) MRSIM_AQV(6, 2, M, G, true) MRSIM_AQV(6, 3, M, G, true) \
-  MRSIM_AQV(6, 4, M, G, true)
+#define MRSIM_AQK(M, G) MRSIM_AQL(4, M, G) MRSIM_AQL(6, M, G) MRSIM_AQL(7, M, G)
+#define MRSIM_AQB(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, true) MRSIM_AQW(NQV, NCV, M, G, true, true)
+#define MRSIM_AQL(NQV, M, G) MRSIM_AQB(NQV, 1, M, G) MRSIM_AQB(NQV, 2, M, G) MRSIM_AQB(NQV, 3, M, G) MRSIM_AQB(NQV, 4, M, G)
       MRSIM_AQN(false, false) MRSIM_AQN(true, false) MRSIM_AQN(false, true) MRSIM_AQN(true, true)
       MRSIM_AQC(8, false, false) MRSIM_AQC(8, false, true)
       MRSIM_AQK(false, false) MRSIM_AQK(true, false) MRSIM_AQK(false, true) MRSIM_AQK(true, true)
 #undef MRSIM_AQK
+#undef MRSIM_AQL
+#undef MRSIM_AQB
 #undef MRSIM_AQN
 #undef MRSIM_AQC
 #undef MRSIM_AQ
 #undef MRSIM_AQV
+#undef MRSIM_AQW
       if (!launched) fail("no adjoint kernel instance for this unit shape");
       MRSIM_CUDA(cudaGetLastError());
       continue;

@@ -15,6 +15,7 @@ namespace mrsim {
 
 constexpr int kMaxComp = 8;   // compartments per unit handled by the kernels
 constexpr int kMaxCoils = 64; // coils per series
+constexpr int kBasisPad = 8;  // floats of a coil's basis coefficients (at most 7 rows)
 constexpr int kXfftMaxN = 2048; // largest power-of-two snx of the FFT x-stage (one CTA holds 2048 points)
 
 // An error carrying the library status code; the ABI layer turns it into (status, message).
@@ -57,6 +58,12 @@ struct GeoTab {
   int ncls;
   const int* cls;     // [coil] class index
   const float* eyc;   // [class][sny] the class rows
+  // coil basis: every coil's ey row as a combination of nbas rows, the last of them constant,
+  //   ey_q(y) = sum_{r < nbas - 1} bco[q][r] bas_r(y) + bco[q][nbas - 1]
+  // (coil_basis, driver.cpp; nbas = 0: none).  bco rows are kBasisPad floats.
+  int nbas;
+  const float* bas;   // [nbas - 1][sny]
+  const float* bco;   // [coil][kBasisPad]
 };
 
 // One unit of work: one slice of one volume, all echoes.  Device pointers throughout.
@@ -153,6 +160,7 @@ struct EpiPlanOptions {
   int no_classes = 0;
   int dft_x = 0;
   int adj_rows = 0;
+  int no_basis = 0;  // no coil basis (the time-segmented y-stages write coil or class rows)
 };
 // Device-resident unit descriptors and tile lists, built once; executing a plan only launches
 // kernels on a stream (no host copies, no synchronisation), so it can be captured in a graph.
@@ -184,12 +192,19 @@ struct EpiPlan {
   int4* d_ctiles = nullptr;
   int n_ctiles = 0;
   std::vector<int> c_start;
+  // coil basis (> 0: its rows): both y-stages run on basis rows instead of coils, the x-stages
+  // expand and contract them, through the warp FFT or the DFT GEMM
+  int basis_nb = 0;
+  int basis_rows = 0, basis_lines = 0;         // most coil rows, most lines of an x-stage tile
+  int ce_first[9] = {0}, ce_count[9] = {0};  // per width E, as fe_first / fe_count, of d_ctiles
   int4* d_ftiles = nullptr;
   int n_ftiles = 0;
   // forward y-stage pass (maps) served by the staged-input kernel (8 lines per tile)
   bool fwdq[2] = {false, false};
   // ... and accumulating coil classes: their count plus the coil offset row, or 0
   int fwd_nv[2] = {0, 0};
+  bool fwd_narrow[2] = {false, false};  // ... its rows copied 4 bytes at a time (16 otherwise)
+  bool adj_narrow = false;                // the fixed-count y-adjoint's rows 8 at a time
   // y-adjoint pass (maps | grads << 1) served by the fixed-coil-count kernel: its coil count, or 0
   // for the general kernel
   int adjq[4] = {0, 0, 0, 0};
