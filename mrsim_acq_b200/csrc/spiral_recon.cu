@@ -349,6 +349,11 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
     fft_lines(d_tf, m, m, 1, m, (size_t)m * m, 1, tw_2n, -1, st);
     fft_lines(d_tf, m, m, m, 1, (size_t)m * m, 1, tw_2n, -1, st);
     MRSIM_CUDA(cudaGetLastError());
+    if (spiral_iter_fits(n)) {
+      d_tfp = (double2*)A.alloc((size_t)m * m * 16);
+      if (d_keep) d_keepp = (unsigned char*)A.alloc((size_t)n * n);
+      spiral_iter_tables(d_tf, d_keep, n, d_tfp, d_keepp, st);
+    }
   }
   // the power iteration (grid_recon.rs:178-197) from the reference's fixed pseudo-random start
   {
@@ -362,13 +367,23 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
       c.x = rnd();
       c.y = rnd();
     }
-    Scratch sc = scratch(T, 1);
     double2* v = (double2*)T.upload(v0.data(), v0.size() * 16, st);
-    double2* u = (double2*)T.alloc(v0.size() * 16);
     double* d_ss = (double*)T.alloc(16);
     double lam = 0.0, ss[2];
     power_iterations = 0;
-    for (int it = 0; it < kPowerIterations; ++it) {
+    Scratch sc{};
+    double2* u = nullptr;
+    if (d_tfp) {
+      spiral_power(n, d_tfp, d_keepp, tw_2n, v, d_ss, kPowerIterations, kPowerTol, st);
+      MRSIM_CUDA(cudaMemcpyAsync(ss, d_ss, 16, cudaMemcpyDeviceToHost, st));
+      MRSIM_CUDA(cudaStreamSynchronize(st));
+      lam = ss[0];
+      power_iterations = (int)ss[1];
+    } else {
+      sc = scratch(T, 1);
+      u = (double2*)T.alloc(v0.size() * 16);
+    }
+    for (int it = 0; it < (d_tfp ? 0 : kPowerIterations); ++it) {
       sumsq_kernel<<<1, 256, 0, st>>>(v, n * n, d_ss);
       normal(v, u, 1, sc, st);
       sumsq_kernel<<<1, 256, 0, st>>>(u, n * n, d_ss + 1);
@@ -377,7 +392,7 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
       const double nv = std::sqrt(ss[0]), nu = std::sqrt(ss[1]);
       const double next = nu / nv;
       scale_kernel<<<grid1((size_t)n * n), 256, 0, st>>>(u, 1.0 / nu, (size_t)n * n, v);
-      const bool done = std::fabs(next - lam) <= 1e-10 * next;
+      const bool done = std::fabs(next - lam) <= kPowerTol * next;
       lam = next;
       ++power_iterations;
       if (done) break;
@@ -451,35 +466,47 @@ void SpiralRecon::images(const double2* d_data, int batch, double2* d_x) {
   DevArena T;
   const double sc = 1.0 / ((double)n * n);
   double2* r = (double2*)T.alloc((size_t)batch * nn * 16);
-  double2* dir = (double2*)T.alloc((size_t)batch * nn * 16);
-  double2* nd = (double2*)T.alloc((size_t)batch * nn * 16);
   {
     DevArena W;
     double2* wts = (double2*)W.alloc((size_t)batch * npts * 16);
     weight_samples_kernel<<<grid1(npts, batch), 256, 0, st>>>(d_data, d_win, d_w, sc, npts, wts);
     double2* work = (double2*)W.alloc((size_t)batch * g.nf0 * g.nf1 * 16);
     nufft_type1<double>(g, d_k, npts, bins_k, wts, batch, npts, r, nn, work, -1, st);
-    project(r, batch, st);
+    if (!d_tfp) project(r, batch, st);
     MRSIM_CUDA(cudaStreamSynchronize(st));  // W's buffers are freed on return
   }
   std::vector<double> r0(batch), rn(batch);
-  sumsq(r, batch, r0.data(), st);
   const double hi = lambda_hi, lo = lambda_hi / kappa;
   const double theta = (hi + lo) / 2.0, delta = (hi - lo) / 2.0;
-  const double sigma1 = theta / delta;
-  double rho = 1.0 / sigma1;
-  MRSIM_CUDA(cudaMemsetAsync(d_x, 0, (size_t)batch * nn * 16, st));
-  scale_kernel<<<grid1((size_t)batch * nn), 256, 0, st>>>(r, 1.0 / theta, (size_t)batch * nn, dir);
-  Scratch s = scratch(T, batch);
-  for (int it = 0; it < iterations; ++it) {
-    normal(dir, nd, batch, s, st);
-    const double rho1 = 1.0 / (2.0 * sigma1 - rho);
-    cheb_update_kernel<<<grid1((size_t)batch * nn), 256, 0, st>>>(d_x, r, dir, nd, (size_t)batch * nn, rho1 * rho,
-                                                                  2.0 * rho1 / delta);
-    rho = rho1;
+  if (d_tfp) {
+    double* d_n = (double*)T.alloc((size_t)batch * 16);
+    spiral_chebyshev(n, batch, d_tfp, d_keepp, tw_2n, r, d_x, d_n, theta, delta, iterations, st);
+    std::vector<double> norms(2 * (size_t)batch);
+    MRSIM_CUDA(cudaMemcpyAsync(norms.data(), d_n, norms.size() * 8, cudaMemcpyDeviceToHost, st));
+    MRSIM_CUDA(cudaStreamSynchronize(st));
+    for (int b = 0; b < batch; ++b) {
+      r0[b] = norms[2 * b];
+      rn[b] = norms[2 * b + 1];
+    }
+  } else {
+    double2* dir = (double2*)T.alloc((size_t)batch * nn * 16);
+    double2* nd = (double2*)T.alloc((size_t)batch * nn * 16);
+    sumsq(r, batch, r0.data(), st);
+    const double sigma1 = theta / delta;
+    double rho = 1.0 / sigma1;
+    MRSIM_CUDA(cudaMemsetAsync(d_x, 0, (size_t)batch * nn * 16, st));
+    scale_kernel<<<grid1((size_t)batch * nn), 256, 0, st>>>(r, 1.0 / theta, (size_t)batch * nn, dir);
+    Scratch s = scratch(T, batch);
+    for (int it = 0; it < iterations; ++it) {
+      normal(dir, nd, batch, s, st);
+      const double rho1 = 1.0 / (2.0 * sigma1 - rho);
+      cheb_update_kernel<<<grid1((size_t)batch * nn), 256, 0, st>>>(d_x, r, dir, nd, (size_t)batch * nn, rho1 * rho,
+                                                                    2.0 * rho1 / delta);
+      rho = rho1;
+    }
+    MRSIM_CUDA(cudaGetLastError());
+    sumsq(r, batch, rn.data(), st);
   }
-  MRSIM_CUDA(cudaGetLastError());
-  sumsq(r, batch, rn.data(), st);
   for (int b = 0; b < batch; ++b) {
     const double a = std::sqrt(r0[b]), z = std::sqrt(rn[b]);
     if (!(z <= (1.0 + 1e-6) * a + 1e-300)) {

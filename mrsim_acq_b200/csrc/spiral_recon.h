@@ -16,8 +16,20 @@ constexpr int kDcfIterations = 10;
 constexpr int kLsIterations = 80;
 constexpr double kLsKappa = 100.0;
 constexpr int kPowerIterations = 1000;
+constexpr double kPowerTol = 1e-10;
 constexpr double kLambdaMargin = 1.1;
-constexpr int kMaxBatch = 256;  // images per pass through the Chebyshev loop
+constexpr int kMaxBatch = 592;  // images per pass through the Chebyshev iteration: four waves of 148
+
+// The iterations as one launch each, for n = 32, 64, 96, 128 (spiral_iter.cu): tables permuted from
+// the circulant's transform and the band (NULL: none); norms [batch][2] = |r|^2 before and after; out
+// = lambda and the iterations taken.
+bool spiral_iter_fits(int n);
+void spiral_iter_tables(const double2* tf, const unsigned char* keep, int n, double2* tfp, unsigned char* keepp,
+                        cudaStream_t st);
+void spiral_chebyshev(int n, int batch, const double2* tfp, const unsigned char* keepp, const double2* tw2, double2* r,
+                      double2* x, double* norms, double theta, double delta, int iterations, cudaStream_t st);
+void spiral_power(int n, const double2* tfp, const unsigned char* keepp, const double2* tw2, double2* v0, double* out,
+                  int iterations, double tol, cudaStream_t st);
 
 struct SpiralRecon {
   mrsim_context* ctx;
@@ -36,6 +48,8 @@ struct SpiralRecon {
   double* d_win = nullptr;  // window per sample
   unsigned char* d_keep = nullptr;
   double2* d_tf = nullptr;  // transform of the Toeplitz kernel's circulant, 2n x 2n
+  double2* d_tfp = nullptr;  // where spiral_iter_fits(n): it and the band in the iterations' order
+  unsigned char* d_keepp = nullptr;
   std::vector<double> w_host, k_host;
 
   struct Scratch {

@@ -202,3 +202,54 @@ def test_parameter_errors(gpu_ctx):
     rec = S.SpiralRecon(k, 16, iterations=5, ctx=gpu_ctx)
     with pytest.raises(MrsimError, match="rings of 3"):
         rec.reconstruct_rings(np.zeros((4, len(k))), 3, np.ones(4))
+
+
+# ---- the one-launch iterations ------------------------------------------------------------------------
+@pytest.mark.parametrize("n,band,iterations,batch", [(32, True, 9, 3), (32, False, 5, 1), (64, True, 80, 2),
+                                                     (64, False, 6, 5), (64, True, 0, 1), (96, True, 7, 2),
+                                                     (96, False, 4, 1), (128, True, 6, 2), (128, False, 3, 1)])
+def test_one_launch_iterations_match_the_operator_in_numpy(gpu_ctx, n, band, iterations, batch):
+    """Every grid the one-launch iterations serve (clusters of 1, 2 and 4 blocks), with and without the
+    band, against the power and Chebyshev iterations of the nonuniform sums themselves in FP64."""
+    rng = np.random.default_rng(n + iterations)
+    k = design(n, 4, 0.008 * (32.0 / n) ** 2)[1]
+    k = k[::max(1, len(k) // 1200)]
+    d = rng.normal(size=(batch, len(k))) + 1j * rng.normal(size=(batch, len(k)))
+    rec = S.SpiralRecon(k, n, iterations=iterations, band_limited=band, ctx=gpu_ctx)
+    got, w = rec.image(d), rec.weights()
+    X = np.arange(n) - n // 2
+    ex, ey = np.exp(1j * TAU * np.outer(k[:, 0], X) / n), np.exp(1j * TAU * np.outer(k[:, 1], X) / n)
+    f = np.fft.fftfreq(n, 1.0 / n)
+    keep = np.hypot(*np.meshgrid(f, f)) <= np.hypot(k[:, 0], k[:, 1]).max()
+
+    def q(x):
+        return np.fft.ifft2(np.fft.fft2(x) * keep) if band else x
+
+    def ah(v):
+        return ((ey.conj() * v[:, None]).T @ ex.conj()) / n ** 2
+
+    def normal(x):
+        return q(ah(w * (((ex @ q(x).T) * ey).sum(1) / n ** 2)))
+
+    g = uniform(0x9E3779B97F4A7C15)
+    v = np.array([complex(g(), g()) for _ in range(n * n)]).reshape(n, n)
+    lam, its = 0.0, 0
+    while its < 1000:
+        u = normal(v)
+        nxt = np.linalg.norm(u) / np.linalg.norm(v)
+        v, done, lam, its = u / np.linalg.norm(u), abs(nxt - lam) <= 1e-10 * nxt, nxt, its + 1
+        if done:
+            break
+    assert abs(rec.lambda_hi - 1.1 * lam) <= 1e-9 * lam
+    hi, lo = rec.lambda_hi, rec.lambda_hi / 100.0
+    theta, delta = (hi + lo) / 2, (hi - lo) / 2
+    for b in range(batch):
+        r, x, rho = q(ah(w * d[b])), np.zeros((n, n), complex), delta / theta
+        dr = r / theta
+        for _ in range(iterations):
+            x = x + dr
+            r = r - normal(dr)
+            rho1 = 1.0 / (2.0 * theta / delta - rho)
+            dr, rho = rho1 * rho * dr + 2.0 * rho1 / delta * r, rho1
+        assert np.linalg.norm(got[b] - x) <= 1e-8 * max(np.linalg.norm(x), 1e-300)
+
