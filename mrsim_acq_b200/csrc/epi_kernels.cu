@@ -2033,10 +2033,13 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
 template <class K>
 void set_smem(K kernel, size_t bytes) {
   // past 48 KB of static + dynamic shared memory the launch needs the dynamic opt-in
+  // (the whole limit, so that threads launching one kernel with different sizes never lower it
+  // between another's opt-in and launch)
   cudaFuncAttributes fa;
   MRSIM_CUDA(cudaFuncGetAttributes(&fa, kernel));
   if (bytes + fa.sharedSizeBytes > 48 * 1024)
-    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    227 * 1024 - (int)fa.sharedSizeBytes));
 }
 
 }  // namespace

@@ -219,7 +219,9 @@ void TsegDevice::fit(const std::vector<std::pair<double, double>>& rates, const 
   while (TJ > 1 && smem_of(TJ) > kFitSmemBudget) TJ /= 2;
   const size_t smem = smem_of(TJ);
   if (smem > 227 * 1024) fail("the time segmentation's rate grid is too large for the device fit");
-  MRSIM_CUDA(cudaFuncSetAttribute(tseg_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the whole limit whatever this fit needs: fits run on several threads at once, and one that set a
+  // smaller size between another's opt-in and launch would make that launch fail
+  MRSIM_CUDA(cudaFuncSetAttribute(tseg_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   FitArgs a;
   a.tau = d_->tau;
   a.rate = d_->rate;

@@ -160,3 +160,20 @@ def test_spiral_shot_images_match_the_oracle(gpu_ctx, name):
                                                   kz_opts=c["kzo"], shot_images=si)
     z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
     assert rel_l2(z, vols.T.ravel()) <= 1e-5, name
+
+
+def test_slices_planned_on_several_threads(gpu_ctx):
+    """Every slice with a fieldmap range of its own: the planner's fits run on several host threads at
+    once, with different shared memory sizes (one lowering the kernel's opt-in between another's
+    opt-in and launch failed the call, not on every run)."""
+    n, nz = 16, 24
+    tr = K3.EchoTrain(etl=nz, esp_ms=12.0, refocusing_deg=180.0, kz_order=K3.KzOrder.Centric, kz_segments=1)
+    vox = np.arange(n * n * nz)
+    x, y, z = (vox % n) / n, ((vox // n) % n) / n, vox // (n * n)
+    img = np.exp(-((x - 0.5) ** 2 + (y - 0.5) ** 2) / 0.05).astype(np.float32)
+    fmap = ((10.0 + 8.0 * z) * (x - 0.5)).astype(np.float32)
+    args = ((n, n, nz), (n, n, nz), 1, [img], [T2.uniform(80.0)], [T2.uniform(1300.0)], fmap, None,
+            Acquisition(n_coils=2, signal_scale=1.0), tr, K3.SpiralReadout(4, 4.0, 0.008, 1.2, K3.KzSampling(1.0, 1)))
+    first = K3.spiral_samples_3d(*args, ctx=gpu_ctx)
+    for _ in range(20):
+        assert np.array_equal(K3.spiral_samples_3d(*args, ctx=gpu_ctx), first)
