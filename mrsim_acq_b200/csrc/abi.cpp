@@ -65,7 +65,13 @@ int on_ctx(mrsim_context* ctx, F&& f) {
     need(ctx, "context");
     std::lock_guard<std::mutex> lk(ctx->mu);
     MRSIM_CUDA(cudaSetDevice(ctx->device));
-    f();
+    try {
+      f();
+    } catch (...) {
+      // copies that the call had queued may still read or write the caller's page-locked buffers
+      cudaStreamSynchronize(ctx->stream);
+      throw;
+    }
   });
 }
 }  // namespace
@@ -91,7 +97,7 @@ int recon_call(mrsim_spiral_recon* rec, const double* in, size_t in_elems, doubl
     need(in, "samples");
     need(out, "out");
     cudaStream_t st = rec->impl->ctx->stream;
-    mrsim::DevArena T;
+    mrsim::DevArena T(rec->impl->ctx);
     double2* din = (double2*)T.upload(in, in_elems * 16, st);
     double2* dout = (double2*)T.alloc(out_elems * 16);
     f(din, dout);
@@ -152,7 +158,16 @@ int mrsim_context_create(int device, mrsim_context** out) {
     try {
       MRSIM_CUDA(cudaSetDevice(device));
       MRSIM_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      MRSIM_CUDA(cudaMemPoolCreate(&ctx->pool, &props));
+      uint64_t keep = mrsim::kPoolKeep;
+      MRSIM_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     } catch (...) {
+      if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+      if (ctx->stream) cudaStreamDestroy(ctx->stream);
       delete ctx;
       throw;
     }
@@ -170,6 +185,7 @@ int mrsim_context_destroy(mrsim_context* ctx) {
     for (auto& e : ctx->slot_ev)
       if (e) cudaEventDestroy(e);
     if (ctx->host_pinned) cudaFreeHost(ctx->host_pinned);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
   });
@@ -688,11 +704,10 @@ int mrsim_epi_batch_download(mrsim_epi_batch* b, int32_t series, float* kspace, 
     const mrsim::EpiOperator* o = b->impl->ops[series].get();
     cudaStream_t st = b->impl->ctx->stream;
     if (kspace)
-      MRSIM_CUDA(cudaMemcpyAsync(kspace, o->d_kspace, o->kspace_elems * sizeof(float2), cudaMemcpyDeviceToHost, st));
+      mrsim::copy_pageable_d2h(b->impl->ctx, kspace, o->d_kspace, o->kspace_elems * sizeof(float2), st);
     if (comp_grad)
-      MRSIM_CUDA(cudaMemcpyAsync(comp_grad, o->d_comp_grad,
-                                 (size_t)o->nv * o->nz * o->ncomp * o->snx * o->sny * sizeof(float2),
-                                 cudaMemcpyDeviceToHost, st));
+      mrsim::copy_pageable_d2h(b->impl->ctx, comp_grad, o->d_comp_grad,
+                               (size_t)o->nv * o->nz * o->ncomp * o->snx * o->sny * sizeof(float2), st);
     MRSIM_CUDA(cudaStreamSynchronize(st));
   });
 }
@@ -770,7 +785,7 @@ int mrsim_resample_by_pose(mrsim_context* ctx, const float* src, const int64_t* 
     check_dims(dims, 1);
     cudaStream_t st = ctx->stream;
     const size_t n = (size_t)(dims[0] * dims[1] * dims[2]);
-    mrsim::DevArena A;
+    mrsim::DevArena A(ctx);
     float* in = (float*)A.upload(src, n * 4, st);
     float* o = (float*)A.alloc(n * 4);
     mrsim::resample_poses_device(in, o, dims, 1, 1, 1, dims[0], dims[0] * dims[1], 0, 0, v2w, pose, st, A);
@@ -790,7 +805,7 @@ int mrsim_apply_motion(mrsim_context* ctx, float* const* images, int64_t ncomp, 
     cudaStream_t st = ctx->stream;
     const HostSeries H = host_strides(dims, n_volumes);
     const size_t per = (size_t)H.sc;
-    mrsim::DevArena A;
+    mrsim::DevArena A(ctx);
     float* in = (float*)A.alloc(per * ncomp * 4);
     float* o = (float*)A.alloc(per * ncomp * 4);
     for (int64_t c = 0; c < ncomp; ++c)
@@ -818,7 +833,7 @@ int mrsim_apply_multiband_motion(mrsim_context* ctx, float* const* images, int64
     cudaStream_t st = ctx->stream;
     const HostSeries H = host_strides(dims, n_volumes);
     const size_t per = (size_t)H.sc;
-    mrsim::DevArena A;
+    mrsim::DevArena A(ctx);
     float* in = (float*)A.alloc(per * std::max<int64_t>(ncomp, 1) * 4);
     float* o = (float*)A.alloc(per * std::max<int64_t>(ncomp, 1) * 4);
     for (int64_t c = 0; c < ncomp; ++c)
@@ -845,7 +860,7 @@ int mrsim_epi_operator_apply_motion(mrsim_epi_operator* op, const double* v2w, c
     // the pre-motion images, then the moved ones back into the operator's buffer
     float* scratch = (float*)mrsim::workspace(o->ctx, 21, n * 4);
     MRSIM_CUDA(cudaMemcpyAsync(scratch, o->d_images, n * 4, cudaMemcpyDeviceToDevice, st));
-    mrsim::DevArena A;
+    mrsim::DevArena A(o->ctx);
     mrsim::resample_poses_device(scratch, o->d_images, dims, o->nv, o->ncomp, 1, o->snx, o->ncomp * plane,
                                  (long long)o->nz * o->ncomp * plane, plane, v2w, poses, st, A);
     MRSIM_CUDA(cudaStreamSynchronize(st));  // the pose tables (in A) are read by the kernel
@@ -907,7 +922,7 @@ int mrsim_tseg_plan(const double* tau_ms, int64_t n_tau, double t_ms, const doub
 int mrsim_tseg_plan_device(mrsim_context* ctx, const double* tau_ms, int64_t n_tau, double t_ms, const double d[2],
                            const double f[2], int64_t l_capacity, double* tau_l, double* b, mrsim_tseg_info* info) {
   return on_ctx(ctx, [&] {
-    mrsim::TsegDevice dev(ctx->stream);
+    mrsim::TsegDevice dev(ctx, ctx->stream);
     tseg_plan_out(&dev, tau_ms, n_tau, t_ms, d, f, l_capacity, tau_l, b, info);
   });
 }

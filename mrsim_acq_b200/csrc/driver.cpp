@@ -46,7 +46,11 @@ void* workspace(mrsim_context* ctx, int slot, size_t bytes) {
 void* DevArena::alloc(size_t bytes) {
   void* p = nullptr;
   if (bytes == 0) bytes = 16;
-  MRSIM_CUDA(cudaMalloc(&p, bytes));
+  ptrs.reserve(ptrs.size() + 1);
+  if (ctx)
+    MRSIM_CUDA(cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream));
+  else
+    MRSIM_CUDA(cudaMalloc(&p, bytes));
   ptrs.push_back(p);
   return p;
 }
@@ -56,7 +60,12 @@ void* DevArena::upload(const void* src, size_t bytes, cudaStream_t st) {
   return p;
 }
 DevArena::~DevArena() {
-  for (void* p : ptrs) cudaFree(p);
+  for (void* p : ptrs) {
+    if (ctx)
+      cudaFreeAsync(p, ctx->stream);
+    else
+      cudaFree(p);
+  }
 }
 
 // ---- coil basis ----------------------------------------------------------------------------
@@ -148,7 +157,11 @@ static int coil_basis(const std::vector<double>& ey, int ncoils, int sny, std::v
 // twiddles e^{i2pi (kx - xs + gh)(x - sxs - xoff)/snx} for gh = +ghost, -ghost (`XStage::new`,
 // kspace.rs:1069-1110), with the k.r part from the exact integer index (kx-xs)(2(x-sxs)-(o-1))
 // mod 2 snx, stored [pol][x][kx] then transposed [pol][kx][x].
-GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, double ghost, cudaStream_t st) {
+//
+// The tables go up as one copy.  dft: the twiddles of the DFT GEMM too; a plan of one geometry whose
+// rows have FFT tables never reads them, and their 2 snx nx sincos cost more than the rest.
+GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, double ghost, cudaStream_t st,
+                 bool dft) {
   const int ox = snx / nx, oy = sny / ny;
   const double xoff = (ox - 1.0) / 2.0, yoff = (oy - 1.0) / 2.0;
   const int xs = nx / 2, sxs = ox * xs;
@@ -174,10 +187,12 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
       ey[(size_t)q * sny + y] = (float)ey64[(size_t)q * sny + y];
     }
   }
-  std::vector<float2> tw((size_t)4 * snx * nx);
+  const bool fft = (snx >= 8 && snx <= kXfftMaxN && (snx & (snx - 1)) == 0) || (snx % 32 == 0 && snx <= 256);
+  if (!fft) dft = true;
+  std::vector<float2> tw(dft ? (size_t)4 * snx * nx : 0);
   const double c = (double)sxs + xoff;
   const long long m2 = 2LL * snx;
-  for (int pol = 0; pol < 2; ++pol) {
+  for (int pol = 0; pol < 2 && dft; ++pol) {
     const double gh = pol == 0 ? ghost : -ghost;
     for (int x = 0; x < snx; ++x) {
       const long long X = 2LL * (x - sxs) - (ox - 1);
@@ -194,8 +209,16 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
     }
   }
   GeoTab g;
-  g.xf = nullptr;
-  if ((snx >= 8 && snx <= kXfftMaxN && (snx & (snx - 1)) == 0) || (snx % 32 == 0 && snx <= 256)) {
+  std::memset(&g, 0, sizeof g);
+  std::vector<char> blob;  // every table, each from a 16-byte boundary
+  auto put = [&](const void* src, size_t bytes) {
+    const size_t at = blob.size();
+    blob.resize(at + (bytes + 15) / 16 * 16);
+    std::memcpy(blob.data() + at, src, bytes);
+    return at;
+  };
+  size_t o_xf = 0, o_bco = 0, o_bas = 0;
+  if (fft) {
     // the factored x-stage: tw[x][kx] = premod_pol(x) * e^{i2pi (kx-xs) x/snx} * post(kx)
     std::vector<float2> xf((size_t)snx / 2 + 2 * (size_t)snx + nx);
     for (int k = 0; k < snx / 2; ++k) {
@@ -218,12 +241,12 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
       turns -= std::rint(turns);
       xf[(size_t)snx / 2 + 2 * (size_t)snx + kx] = make_float2((float)std::cos(kTau * turns), (float)std::sin(kTau * turns));
     }
-    g.xf = (const float2*)arena.upload(xf.data(), xf.size() * sizeof(float2), st);
+    o_xf = put(xf.data(), xf.size() * sizeof(float2));
   }
+  // coil classes of bitwise-equal ey rows
+  std::vector<int> cls(ncoils, -1);
+  std::vector<float> eyc;
   {
-    // coil classes of bitwise-equal ey rows
-    std::vector<int> cls(ncoils, -1);
-    std::vector<float> eyc;
     int ncls = 0;
     for (int q = 0; q < ncoils; ++q) {
       for (int q2 = 0; q2 < q && cls[q] < 0; ++q2)
@@ -234,24 +257,30 @@ GeoTab build_geo(DevArena& arena, int snx, int sny, int nx, int ny, int ncoils, 
       }
     }
     g.ncls = ncls;
-    g.cls = (const int*)arena.upload(cls.data(), cls.size() * sizeof(int), st);
-    g.eyc = (const float*)arena.upload(eyc.data(), eyc.size() * 4, st);
   }
-  g.nbas = 0;
-  g.bas = g.bco = nullptr;
+  const size_t o_cls = put(cls.data(), cls.size() * sizeof(int)), o_eyc = put(eyc.data(), eyc.size() * 4);
   if (ncoils >= 6) {  // up to 4 coils have kernels of their own; 5 span 6 rows
     std::vector<float> rows, coef;
     const int nb = coil_basis(ey64, ncoils, sny, rows, coef);
     if (nb > 0 && nb <= ncoils) {
-      coef.insert(coef.end(), rows.begin(), rows.end());
       g.nbas = nb;
-      g.bco = (const float*)arena.upload(coef.data(), coef.size() * 4, st);
-      g.bas = g.bco + (size_t)ncoils * kBasisPad;
+      o_bco = put(coef.data(), coef.size() * 4);
+      o_bas = put(rows.data(), rows.size() * 4);
     }
   }
-  g.ex = (const float*)arena.upload(ex.data(), ex.size() * 4, st);
-  g.ey = (const float*)arena.upload(ey.data(), ey.size() * 4, st);
-  g.tw = (const float2*)arena.upload(tw.data(), tw.size() * sizeof(float2), st);
+  const size_t o_ex = put(ex.data(), ex.size() * 4), o_ey = put(ey.data(), ey.size() * 4);
+  const size_t o_tw = put(tw.data(), tw.size() * sizeof(float2));
+  const char* d = (const char*)arena.upload(blob.data(), blob.size(), st);
+  g.xf = fft ? (const float2*)(d + o_xf) : nullptr;
+  g.cls = (const int*)(d + o_cls);
+  g.eyc = (const float*)(d + o_eyc);
+  if (g.nbas) {
+    g.bco = (const float*)(d + o_bco);
+    g.bas = (const float*)(d + o_bas);
+  }
+  g.ex = (const float*)(d + o_ex);
+  g.ey = (const float*)(d + o_ey);
+  g.tw = dft ? (const float2*)(d + o_tw) : nullptr;
   g.coil_off = ncoils <= 1 ? 0.f : 0.15f;
   return g;
 }
@@ -568,10 +597,10 @@ void epi_operator_set_fieldmap(EpiOperator* op, const float* fmap) {
   cudaStream_t st = op->ctx->stream;
   const size_t n = (size_t)op->nz * op->snx * op->sny;
   MRSIM_CUDA(cudaMemcpyAsync(op->d_fmap, fmap, n * 4, cudaMemcpyHostToDevice, st));
-  op->h_fmap.assign(fmap, fmap + n);
+  op->h_fmap.clear();  // read back when a segmentation is planned
   MRSIM_CUDA(cudaStreamSynchronize(st));
   if (op->ts && op->acq.do_distortions) {
-    const auto mm = std::minmax_element(op->h_fmap.begin(), op->h_fmap.end());
+    const auto mm = std::minmax_element(fmap, fmap + n);
     if (*mm.first < op->ts->fmin || *mm.second > op->ts->fmax) epi_operator_set_segmented(op, op->ts_precision);
   }
 }
@@ -588,6 +617,12 @@ void epi_operator_set_segmented(EpiOperator* op, int precision) {
     was.reset(epi_plan_create(op->plan->host_units.data(), op->plan->n_units, op->plan->host_statics.data(),
                               (int)op->plan->host_statics.size(), &o));
     std::swap(was, op->plan);
+  }
+  if (precision && op->h_fmap.empty()) {
+    op->h_fmap.resize((size_t)op->nz * op->snx * op->sny);
+    MRSIM_CUDA(cudaMemcpyAsync(op->h_fmap.data(), op->d_fmap, op->h_fmap.size() * 4, cudaMemcpyDeviceToHost,
+                               op->ctx->stream));
+    MRSIM_CUDA(cudaStreamSynchronize(op->ctx->stream));
   }
   TsPlan* fresh = nullptr;
   try {

@@ -2077,27 +2077,58 @@ constexpr int kTY = 4;
 }  // namespace
 
 EpiPlan::~EpiPlan() {
-  for (void* p : allocs) cudaFree(p);
+  for (void* p : allocs) {
+    if (pool_stream)
+      cudaFreeAsync(p, pool_stream);
+    else
+      cudaFree(p);
+  }
 }
 
-static void* dev_upload(EpiPlan* p, const void* src, size_t bytes) {
-  void* d = nullptr;
-  if (bytes == 0) return nullptr;
-  MRSIM_CUDA(cudaMalloc(&d, bytes));
-  p->allocs.push_back(d);
-  MRSIM_CUDA(cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice));
-  return d;
-}
+namespace {
+// A plan's arrays, gathered on the host and sent up as one allocation and one copy.
+struct PlanArrays {
+  std::vector<char> blob;
+  std::vector<std::pair<void**, size_t>> slots;
+  template <class T>
+  void add(T** slot, const void* src, size_t bytes) {
+    *slot = nullptr;
+    if (bytes == 0) return;
+    const size_t at = blob.size();
+    blob.resize(at + (bytes + 255) / 256 * 256);
+    std::memcpy(blob.data() + at, src, bytes);
+    slots.emplace_back((void**)slot, at);
+  }
+  void send(EpiPlan* p, mrsim_context* ctx) {
+    if (blob.empty()) return;
+    void* d = nullptr;
+    p->allocs.reserve(1);
+    if (ctx) {
+      MRSIM_CUDA(cudaMallocFromPoolAsync(&d, blob.size(), ctx->pool, ctx->stream));
+      p->pool_stream = ctx->stream;
+      p->allocs.push_back(d);
+      MRSIM_CUDA(cudaMemcpyAsync(d, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+      MRSIM_CUDA(cudaMalloc(&d, blob.size()));
+      p->allocs.push_back(d);
+      MRSIM_CUDA(cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    }
+    for (auto& s : slots) *s.first = (char*)d + s.second;
+  }
+};
+}  // namespace
 
-EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns, const EpiPlanOptions* opt) {
+EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns, const EpiPlanOptions* opt,
+                         mrsim_context* ctx) {
   EpiPlan* p = new EpiPlan();
+  PlanArrays arrays;
   try {
     if (opt) p->opt = *opt;
     p->n_units = n;
     p->host_units.assign(hu, hu + n);
     p->host_statics.assign(hs, hs + ns);
     p->n_statics = ns;
-    p->d_statics = (StaticDesc*)dev_upload(p, hs, sizeof(StaticDesc) * ns);
+    arrays.add(&p->d_statics, hs, sizeof(StaticDesc) * ns);
     for (int i = 0; i < ns; ++i) p->max_static_n = std::max(p->max_static_n, hs[i].snx * hs[i].sny);
     int max_coils = 0;
     for (int i = 0; i < n; ++i) {
@@ -2172,7 +2203,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           u.geo.ncls = u.geo.nbas - 1;
           u.geo.eyc = u.geo.bas;
         }
-      p->d_units = (UnitDesc*)dev_upload(p, du.data(), sizeof(UnitDesc) * n);
+      arrays.add(&p->d_units, du.data(), sizeof(UnitDesc) * n);
     }
     // the staged-input forward serves a pass when every unit has snx % 4 == 0 and 16-byte aligned
     // input planes (cooperative 16-byte copies), and on basis rows also when not (4-byte copies; 12
@@ -2215,7 +2246,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->y_start[pass][n] = (int)tiles.size();
       p->n_ytiles[pass] = (int)tiles.size();
-      p->d_ytiles[pass] = (int4*)dev_upload(p, tiles.data(), sizeof(int4) * tiles.size());
+      arrays.add(&p->d_ytiles[pass], tiles.data(), sizeof(int4) * tiles.size());
     }
     if (p->xfft && p->basis_nb) {
       // tiles of a few lines x every coil: by unit, or with mixed widths ordered by width
@@ -2239,7 +2270,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       if (p->xfft_e > 0) p->c_start[n] = (int)ct.size();
       p->n_ctiles = (int)ct.size();
-      p->d_ctiles = (int4*)dev_upload(p, ct.data(), sizeof(int4) * ct.size());
+      arrays.add(&p->d_ctiles, ct.data(), sizeof(int4) * ct.size());
     } else if (p->xfft && p->xfft_e < 0) {
       // one list ordered by width, no per-unit ranges (such a plan runs whole)
       std::vector<int4> ft;
@@ -2254,7 +2285,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->f_start.clear();
       p->n_ftiles = (int)ft.size();
-      p->d_ftiles = (int4*)dev_upload(p, ft.data(), sizeof(int4) * ft.size());
+      arrays.add(&p->d_ftiles, ft.data(), sizeof(int4) * ft.size());
     } else if (p->xfft) {
       std::vector<int4> ft;
       p->f_start.assign(n + 1, 0);
@@ -2266,7 +2297,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->f_start[n] = (int)ft.size();
       p->n_ftiles = (int)ft.size();
-      p->d_ftiles = (int4*)dev_upload(p, ft.data(), sizeof(int4) * ft.size());
+      arrays.add(&p->d_ftiles, ft.data(), sizeof(int4) * ft.size());
     }
     // coil classes through the forward x-stage: every unit's y-stage runs in class mode and the
     // rows have at most 128 points
@@ -2298,7 +2329,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->g_start[dir][n] = (int)xt.size();
       p->n_gtiles[dir] = (int)xt.size();
-      p->d_gtiles[dir] = dev_upload(p, xt.data(), sizeof(XTile) * xt.size());
+      arrays.add(&p->d_gtiles[dir], xt.data(), sizeof(XTile) * xt.size());
     }
     // the fixed-coil-count y-adjoint serves a pass when every unit has the same coil count (1, 2,
     // 4 or 8), an even snx and 16-byte aligned h rows (cooperative 16-byte copies), and on basis rows
@@ -2340,7 +2371,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->a_start[pass][n] = (int)yt.size();
       p->n_atiles[pass] = (int)yt.size();
-      p->d_atiles[pass] = (int4*)dev_upload(p, yt.data(), sizeof(int4) * yt.size());
+      arrays.add(&p->d_atiles[pass], yt.data(), sizeof(int4) * yt.size());
     }
     if (!p->basis_nb && (p->adj_cls || p->fwd_cls)) {  // the class x-stage tiles: 4 lines x the 8 coils
       std::vector<int4> ct;
@@ -2351,8 +2382,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->c_start[n] = (int)ct.size();
       p->n_ctiles = (int)ct.size();
-      p->d_ctiles = (int4*)dev_upload(p, ct.data(), sizeof(int4) * ct.size());
+      arrays.add(&p->d_ctiles, ct.data(), sizeof(int4) * ct.size());
     }
+    arrays.send(p, ctx);
   } catch (...) {
     delete p;
     throw;

@@ -348,12 +348,13 @@ static int most_variants(const mrsim_acquisition_3d_input& in) {
 // The acquired 3D k-space (before spikes and noise) of volumes g0..g1 into k3 [gl][q][p][ky][kx].
 static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_acquisition& acq,
                          const mrsim_phase_model* phase, const float* d_lw, int g0, int g1,
-                         const std::vector<uint8_t>& mask, float2* k3, cudaStream_t st,
+                         const std::vector<uint8_t>& mask, float2* k3, mrsim_context* ctx,
                          const ShotVariants* V = nullptr) {
+  cudaStream_t st = ctx->stream;
   const int ngl = g1 - g0, nsrc = (int)P.srcs.size(), nz = P.nz, nc = P.nc;
   const int nvar = V ? V->nvar : 1;
   const size_t per = (size_t)P.nx * P.ny;
-  DevArena C;
+  DevArena C(ctx);
   mrsim_acquisition norel = acq;
   norel.do_relaxation = 0;
   norel.noise_variance = 0.0;
@@ -373,7 +374,7 @@ static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_a
   MRSIM_CUDA(cudaMemsetAsync(K, 0, nunit * nc * per * sizeof(float2), st));
   float2* gs = (float2*)C.alloc(std::max<size_t>(1, nunit * nc * std::max(n_lines, 1) * P.snx) * sizeof(float2));
   float* ph = (float*)C.alloc(std::max<size_t>(1, nunit * P.plane) * 4);
-  GeoTab geo = build_geo(C, P.snx, P.sny, P.nx, P.ny, nc, acq.ghost_offset, st);
+  GeoTab geo = build_geo(C, P.snx, P.sny, P.nx, P.ny, nc, acq.ghost_offset, st, false);
   mrsim_phase_model zero;
   std::memset(&zero, 0, sizeof zero);
   Batch Bc, Bv;
@@ -414,8 +415,8 @@ static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_a
         }
       }
   if (n_lines > 0) {
-    run_forward(Bc, st);
-    run_forward(Bv, st);
+    run_forward(Bc, ctx);
+    run_forward(Bv, ctx);
   }
   // the z-DFT, weights, compartment sum and sampling
   std::vector<unsigned char> rows(P.ny);
@@ -442,7 +443,6 @@ static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_a
   a.nvar = nvar;
   grase_zdft_kernel<<<grid3(per, nz, ngl * nc), 256, 0, st>>>(a);
   MRSIM_CUDA(cudaGetLastError());
-  MRSIM_CUDA(cudaStreamSynchronize(st));  // C's buffers are freed on return
 }
 
 // spikes and noise per (volume, partition, coil) (`partitions_to_slices` kspace3d.rs:235-262)
@@ -479,7 +479,7 @@ void grase_observed(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, co
   cudaStream_t st = ctx->stream;
   GrasePlan P = make_plan(in, acq, train, ro);
   if (g < 0 || g >= (int)in.n_volumes) fail("volume index out of range");
-  DevArena A;
+  DevArena A(ctx);
   GraseInputs I = upload_inputs(A, P, in, in.images, (int)in.n_volumes, acq, st);
   const float* d_lw = nullptr;
   if (in.line_weights) {
@@ -490,7 +490,7 @@ void grase_observed(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, co
   const size_t per = (size_t)P.nx * P.ny;
   float2* k3 = (float2*)A.alloc((size_t)P.nc * P.nz * per * sizeof(float2));
   ShotVariants V = input_sets(A, P, in, g, g + 1, st);
-  grase_kspace(P, I, acq, in.phase, d_lw, g, g + 1, P.mask, k3, st, &V);
+  grase_kspace(P, I, acq, in.phase, d_lw, g, g + 1, P.mask, k3, ctx, &V);
   copy_pageable_d2h(ctx, out, k3, (size_t)P.nc * P.nz * per * sizeof(float2), st);
   MRSIM_CUDA(cudaStreamSynchronize(st));
 }
@@ -504,7 +504,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
   const size_t per = (size_t)nx * ny;
   const int accel = (int)std::max<int64_t>(acq.accel, 1);
   const int nvar = most_variants(in);
-  DevArena A;
+  DevArena A(ctx);
   if (nvar > 1) (void)input_sets(A, P, in, 0, nv, st, false);  // every volume's sets checked before any work
   GraseInputs I = upload_inputs(A, P, in, in.images, nv, acq, st);
   const float* d_lw = nullptr;
@@ -522,7 +522,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     acq_cal.accel = 1;
     acq_cal.n_spikes = 0;
     GrasePlan Pc = make_plan(in, acq_cal, train, ro);
-    DevArena C;
+    DevArena C(ctx);
     const float* const* cal_images = in.images;
     int cal_nv = nv;
     uint64_t cal_seed = seed;
@@ -534,7 +534,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     }
     GraseInputs Ic = upload_inputs(C, Pc, in, cal_images, cal_nv, acq_cal, st);
     float2* k3 = (float2*)C.alloc((size_t)nc * nz * per * sizeof(float2));
-    grase_kspace(Pc, Ic, acq_cal, in.phase, nullptr, 0, 1, Pc.mask, k3, st);
+    grase_kspace(Pc, Ic, acq_cal, in.phase, nullptr, 0, 1, Pc.mask, k3, ctx);
     grase_noise(C, Pc, k3, 0, 1, cal_seed ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
     float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
     grase_izdft_kernel<<<grid3(per, nz, nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
@@ -555,10 +555,10 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
   const int vchunk = (int)std::max<size_t>(1, std::min<size_t>(std::max(nv, 1), budget / std::max<size_t>(1, bytes_per_vol)));
   for (int g0 = 0; g0 < nv; g0 += vchunk) {
     const int g1 = std::min(nv, g0 + vchunk), ngl = g1 - g0;
-    DevArena C;
+    DevArena C(ctx);
     float2* k3 = (float2*)C.alloc((size_t)ngl * nc * nz * per * sizeof(float2));
     ShotVariants V = input_sets(C, P, in, g0, g1, st);
-    grase_kspace(P, I, acq, in.phase, d_lw, g0, g1, P.mask, k3, st, &V);
+    grase_kspace(P, I, acq, in.phase, d_lw, g0, g1, P.mask, k3, ctx, &V);
     grase_noise(C, P, k3, g0, g1, seed, P.mask, acq, st);
     float2* sl = (float2*)C.alloc((size_t)ngl * nz * nc * per * sizeof(float2));
     grase_izdft_kernel<<<grid3(per, nz, ngl * nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
@@ -776,7 +776,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
     if (e > 0 && !(train.echo_times_ms[e] > train.echo_times_ms[e - 1]))
       fail("the echo times must increase strictly");
   }
-  DevArena A;
+  DevArena A(ctx);
   const float2* d_zk = (const float2*)A.upload(P.zk.data(), P.zk.size() * sizeof(float2), st);
   ReconTables T = build_recon_tables(A, nx, ny, nc, acq, st);
   const size_t w_per_slice = (size_t)(accel - 1) * nc * 6 * nc;
@@ -798,7 +798,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
     GrasePlan Pc = P;
     Pc.mask = sampling_mask(nx, ny, acq_cal);
     for (int c = 0; c < P.ncomp; ++c) Pc.used[c] = ref.images[c] != nullptr;
-    DevArena C;
+    DevArena C(ctx);
     const float* d_lw = nullptr;
     GraseInputs Ic = upload_ge_volume(C, Pc, in, ref, acq, &d_lw, st);
     for (int e = 0; e < n_echoes; ++e) {
@@ -807,7 +807,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       mrsim_acquisition ae = acq_cal;
       ae.t_echo = te;
       float2* k3 = (float2*)C.alloc((size_t)nc * nz * per * sizeof(float2));
-      grase_kspace(Pc, Ic, ae, in.phase, d_lw, 0, 1, Pc.mask, k3, st);
+      grase_kspace(Pc, Ic, ae, in.phase, d_lw, 0, 1, Pc.mask, k3, ctx);
       grase_noise(C, Pc, k3, 0, 1, (seed ^ echo_salt((uint64_t)e)) ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
       float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
       grase_izdft_kernel<<<grid3(per, nz, nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
@@ -826,7 +826,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
     GeVolumeData v = fetch_ge_volume(in, g, n_exc_lines);
     GrasePlan Pg = P;
     for (int c = 0; c < P.ncomp; ++c) Pg.used[c] = v.images[c] != nullptr;
-    DevArena C;
+    DevArena C(ctx);
     const float* d_lw = nullptr;
     GraseInputs I = upload_ge_volume(C, Pg, in, v, acq, &d_lw, st);
     const ShotVariants V = upload_sets(C, Pg, {v.sets}, {v.n_sets}, g, st);
@@ -835,9 +835,9 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       ge_echo(Pg, acq, te);
       mrsim_acquisition ae = acq;
       ae.t_echo = te;
-      DevArena E;
+      DevArena E(ctx);
       float2* k3 = (float2*)E.alloc((size_t)nc * nz * per * sizeof(float2));
-      grase_kspace(Pg, I, ae, in.phase, d_lw, 0, 1, Pg.mask, k3, st, &V);
+      grase_kspace(Pg, I, ae, in.phase, d_lw, 0, 1, Pg.mask, k3, ctx, &V);
       // the noise and spikes of echo e on its own streams (echo 0 unsalted)
       grase_noise(E, Pg, k3, g, g + 1, seed ^ echo_salt((uint64_t)e), Pg.mask, acq, st);
       float2* sl = (float2*)E.alloc((size_t)nz * nc * per * sizeof(float2));

@@ -138,10 +138,15 @@ struct mrsim_context {
   void* host_pinned = nullptr;  // page-locked staging slots of the pageable copies (host_copy.cpp)
   size_t host_pinned_n = 0;
   std::vector<cudaEvent_t> slot_ev;  // per slot: its last copy
+  // stream-ordered memory of the host calls (DevArena on a context): kept between calls up to
+  // mrsim::kPoolKeep bytes, given back above that and when the context ends
+  cudaMemPool_t pool = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
 namespace mrsim {
+
+constexpr unsigned long long kPoolKeep = 2ull << 30;
 
 // Workspace slot `slot` of at least `bytes` (grow-only, device memory of the context's device).
 void* workspace(mrsim_context* ctx, int slot, size_t bytes);
@@ -215,10 +220,13 @@ struct EpiPlan {
   EpiPlanOptions opt;
   std::vector<StaticDesc> host_statics;
   std::vector<void*> allocs;
+  cudaStream_t pool_stream = nullptr;  // the arrays came from a context's pool: freed on this stream
   ~EpiPlan();
 };
+// With `ctx` its arrays come from the context's pool and are freed on its stream, after the work
+// queued there: for a plan that runs on that stream and ends with the call.
 EpiPlan* epi_plan_create(const UnitDesc* units, int n, const StaticDesc* statics, int ns,
-                         const EpiPlanOptions* opt = nullptr);
+                         const EpiPlanOptions* opt = nullptr, mrsim_context* ctx = nullptr);
 // The x-stage tiles of one unit (dir 0 forward, 1 adjoint); `lines` is a host copy of its table.
 void append_xtiles(std::vector<XTile>& out, const UnitDesc& u, int unit_index, const LineRec* lines, int dir);
 // Each launcher covers units [u0, u1) of the plan (u1 < 0: every unit).

@@ -24,32 +24,48 @@ namespace mrsim {
 ReconTables build_recon_tables(DevArena& A, int nx, int ny, int nc, const mrsim_acquisition& acq, cudaStream_t st) {
   ReconTables T;
   const int xs = nx / 2, ys = ny / 2;
-  std::vector<float2> ex(nx), ey(ny);
+  const size_t per = (size_t)nx * ny;
+  // one allocation and one copy: DFT tables, sensitivities, Roemer denominator, window
+  const bool win = acq.window_kind != MRSIM_WINDOW_NONE;
+  const size_t o_sens = 2 * ((size_t)nx + ny), o_inv = o_sens + nc * per, o_win = o_inv + per;
+  std::vector<float> host(o_win + (win ? per : 0));
+  float2* ex = (float2*)host.data();
+  float2* ey = ex + nx;
   for (int m = 0; m < nx; ++m) ex[m] = make_float2((float)std::cos(-kTau * m / nx), (float)std::sin(-kTau * m / nx));
   for (int m = 0; m < ny; ++m) ey[m] = make_float2((float)std::cos(-kTau * m / ny), (float)std::sin(-kTau * m / ny));
-  T.ex_tab = (float2*)A.upload(ex.data(), ex.size() * sizeof(float2), st);
-  T.ey_tab = (float2*)A.upload(ey.data(), ey.size() * sizeof(float2), st);
   // `coil_sensitivity` on the acquired grid and the Roemer denominator (kspace.rs:1343-1373)
-  T.sens_host.assign((size_t)nc * nx * ny, 0.f);
-  std::vector<double> ssum((size_t)nx * ny, 0.0);
-  for (int q = 0; q < nc; ++q)
-    for (int i = 0; i < nx * ny; ++i) {
-      double s = coil_sensitivity(q, nc, (double)(i % nx), (double)(i / nx), nx, ny);
-      T.sens_host[(size_t)q * nx * ny + i] = (float)s;
+  T.sens_host.assign(nc * per, 0.f);
+  std::vector<double> ssum(per, 0.0);
+  // the Gaussian factors per axis: one exponential per coil and column or row in place of one per
+  // coil and voxel (the product is within 2 ulp of it in FP64)
+  std::vector<double> gx(nx, 1.0), gy(ny, 1.0);
+  for (int q = 0; q < nc; ++q) {
+    if (nc > 1) {
+      const double big = (double)std::max(nx, ny), r = 0.6 * big, w = 2.0 * (0.9 * big) * (0.9 * big);
+      const double ang = kTau * (double)q / (double)nc;
+      const double px = (double)nx / 2.0 + r * std::cos(ang), py = (double)ny / 2.0 + r * std::sin(ang);
+      for (int x = 0; x < nx; ++x) gx[x] = std::exp(-((double)x - px) * ((double)x - px) / w);
+      for (int y = 0; y < ny; ++y) gy[y] = std::exp(-((double)y - py) * ((double)y - py) / w);
+    }
+    for (size_t i = 0; i < per; ++i) {
+      const double s = nc > 1 ? gx[i % nx] * gy[i / nx] + 0.15 : 1.0;
+      T.sens_host[q * per + i] = (float)s;
       ssum[i] += s * s;
     }
-  std::vector<float> inv((size_t)nx * ny);
-  for (int i = 0; i < nx * ny; ++i) inv[i] = (float)(1.0 / std::max(ssum[i], 1e-12));
-  T.sens = (float*)A.upload(T.sens_host.data(), T.sens_host.size() * 4, st);
-  T.inv_ssum = (float*)A.upload(inv.data(), inv.size() * 4, st);
-  if (acq.window_kind != MRSIM_WINDOW_NONE) {
-    std::vector<float> w((size_t)nx * ny);
+  }
+  std::copy(T.sens_host.begin(), T.sens_host.end(), host.begin() + o_sens);
+  for (size_t i = 0; i < per; ++i) host[o_inv + i] = (float)(1.0 / std::max(ssum[i], 1e-12));
+  if (win)
     for (int ky = 0; ky < ny; ++ky)
       for (int kx = 0; kx < nx; ++kx)
-        w[(size_t)ky * nx + kx] =
+        host[o_win + (size_t)ky * nx + kx] =
             (float)window_at(acq, ((double)kx - xs) / (double)nx, ((double)ky - ys) / (double)ny);
-    T.window = (float*)A.upload(w.data(), w.size() * 4, st);
-  }
+  float* d = (float*)A.upload(host.data(), host.size() * 4, st);
+  T.ex_tab = (float2*)d;
+  T.ey_tab = T.ex_tab + nx;
+  T.sens = d + o_sens;
+  T.inv_ssum = d + o_inv;
+  if (win) T.window = d + o_win;
   // the lines GRAPPA synthesises (`GrappaKernel::apply`, kspace.rs:1605-1632)
   const int accel = (int)std::max<int64_t>(acq.accel, 1);
   if (accel > 1) {
@@ -141,13 +157,12 @@ void add_unit(Batch& B, const UnitInputs& in, int snx, int sny, int nx, int ny, 
   B.statics.push_back(sd);
 }
 
-void run_forward(const Batch& B, cudaStream_t st) {
+void run_forward(const Batch& B, mrsim_context* ctx) {
   if (B.units.empty()) return;
   std::unique_ptr<EpiPlan> plan(epi_plan_create(B.units.data(), (int)B.units.size(), B.statics.data(),
-                                                (int)B.statics.size()));
-  epi_plan_statics(plan.get(), st);
-  epi_plan_forward(plan.get(), st);
-  MRSIM_CUDA(cudaStreamSynchronize(st));  // the plan's device memory is freed on return
+                                                (int)B.statics.size(), nullptr, ctx));
+  epi_plan_statics(plan.get(), ctx->stream);
+  epi_plan_forward(plan.get(), ctx->stream);
 }
 
 // Uniform relaxation weights of a line (kspace.rs:886-903), with T2' from Acquisition::t_inhom
@@ -276,6 +291,7 @@ bool uniform_relaxation(const mrsim_t2* t2, const mrsim_t2* ti, int ncomp) {
 // =============================================================================================
 // Per slice (`simulate_slice_with`, kspace.rs:1271-1284)
 struct SliceState {
+  explicit SliceState(mrsim_context* ctx) : A(ctx) {}
   DevArena A;
   int snx, sny, nx, ny, ncomp, nc;
   float2* k = nullptr;  // [coil][ny][nx]
@@ -339,14 +355,13 @@ static void slice_forward_into(mrsim_context* ctx, SliceState& S, const mrsim_sl
   ui.nz_full = (int)inp.nz;
   ui.has_eddy = inp.has_eddy_drive != 0;
   for (int i = 0; i < 3; ++i) ui.grad[i] = inp.eddy_drive[i];
-  GeoTab geo = build_geo(A, snx, sny, nx, ny, nc, acq.ghost_offset, st);
+  GeoTab geo = build_geo(A, snx, sny, nx, ny, nc, acq.ghost_offset, st, false);
   Batch B;
   add_unit(B, ui, snx, sny, nx, ny, ncomp, nc, maps, t2u, tiu, geo, acq);
-  if (!lines.empty()) run_forward(B, st);
+  if (!lines.empty()) run_forward(B, ctx);
   else {
-    std::unique_ptr<EpiPlan> plan(epi_plan_create(B.units.data(), 1, B.statics.data(), 1));
+    std::unique_ptr<EpiPlan> plan(epi_plan_create(B.units.data(), 1, B.statics.data(), 1, nullptr, ctx));
     epi_plan_statics(plan.get(), st);
-    MRSIM_CUDA(cudaStreamSynchronize(st));
   }
   std::vector<int> rows;
   for (auto& L : lines) rows.push_back(L.ky);
@@ -359,7 +374,7 @@ static void slice_forward_into(mrsim_context* ctx, SliceState& S, const mrsim_sl
 
 std::vector<float2> slice_forward2(mrsim_context* ctx, const mrsim_slice_input& inp, const mrsim_acquisition& acq,
                                    const LineTimingTab* timing, const double* log_amp) {
-  SliceState S;
+  SliceState S(ctx);
   S.snx = (int)inp.sim[0];
   S.sny = (int)inp.sim[1];
   S.nx = (int)inp.acq_matrix[0];
@@ -391,7 +406,7 @@ void simulate_slice_full(mrsim_context* ctx, const mrsim_slice_input& inp, const
   const int nc = (int)std::max<int64_t>(acq.n_coils, 1);
   const int accel = (int)std::max<int64_t>(acq.accel, 1);
   const size_t per = (size_t)nx * ny;
-  SliceState S;
+  SliceState S(ctx);
   S.snx = (int)inp.sim[0];
   S.sny = (int)inp.sim[1];
   S.nx = nx;
@@ -403,7 +418,7 @@ void simulate_slice_full(mrsim_context* ctx, const mrsim_slice_input& inp, const
   // seed salted by SEED_SALT_GRAPPA_CAL, without eddy and preparation drives (kspace.rs:1253-1284)
   float2* W = nullptr;
   if (accel > 1) {
-    SliceState R;
+    SliceState R(ctx);
     R.snx = S.snx;
     R.sny = S.sny;
     R.nx = nx;
@@ -533,7 +548,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
            " slices");
     captured.push_back((int)opts.kspace_slices[i]);
   }
-  DevArena A;
+  DevArena A(ctx);
   // ---- inputs on the device (kept in `cache` for a later call with the same arrays)
   const size_t per_comp = nvox_sim * nv;
   const std::vector<const float*> img_from(images, images + (images ? ncomp : 0));
@@ -584,7 +599,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
     t2u[c] = c < ncomp ? in.t2[c].value : 1.f;
     tiu[c] = c < ncomp ? (in.t_inhom ? in.t_inhom[c].value : (float)acq.t_inhom) : 1.f;
   }
-  GeoTab geo = build_geo(A, snx, sny, nx, ny, nc, acq.ghost_offset, st);
+  GeoTab geo = build_geo(A, snx, sny, nx, ny, nc, acq.ghost_offset, st, false);
   ReconTables T = build_recon_tables(A, nx, ny, nc, acq, st);
   const int accel = (int)std::max<int64_t>(acq.accel, 1);
 
@@ -641,7 +656,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
       std::vector<LineRec> L;
       lines_for(L, acq_cal, nx, ny, false, uniform, ncomp, t2u, tiu, in.t_inhom != nullptr, nullptr);
       const LineRec* dl = (const LineRec*)A.upload(L.data(), std::max<size_t>(1, L.size()) * sizeof(LineRec), st);
-      DevArena C;
+      DevArena C(ctx);
       float2* ck = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
       MRSIM_CUDA(cudaMemsetAsync(ck, 0, (size_t)nz * nc * per * sizeof(float2), st));
       float2* cg = (float2*)C.alloc(std::max<size_t>(1, (size_t)nz * nc * L.size() * snx) * sizeof(float2));
@@ -669,7 +684,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
         const uint64_t seed = ((uint64_t)ui.z * 0x9E37ull) ^ cal_seed ^ kSeedSaltGrappaCal;
         for (int q = 0; q < nc; ++q) specs.push_back({ck + ((size_t)zl * nc + q) * per, seed, q, 0});
       }
-      if (!L.empty()) run_forward(B, st);
+      if (!L.empty()) run_forward(B, ctx);
       std::vector<int> crow;
       for (auto& r : L) crow.push_back(r.ky);
       run_noise(C, specs, crow, {}, nx, ny, acq_cal, st);
@@ -709,7 +724,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
   for (int g0 = 0; g0 < nv; g0 += vchunk) {
     const int g1 = std::min(nv, g0 + vchunk);
     const int nunit = (g1 - g0) * nz;
-    DevArena C;
+    DevArena C(ctx);
     float2* ks = (float2*)C.alloc((size_t)nunit * nc * per * sizeof(float2));
     MRSIM_CUDA(cudaMemsetAsync(ks, 0, (size_t)nunit * nc * per * sizeof(float2), st));
     float2* gs = (float2*)C.alloc(std::max<size_t>(1, (size_t)nunit * nc * max_lines * snx) * sizeof(float2));
@@ -775,7 +790,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
         jobs.push_back(J);
       }
     }
-    run_forward(B, st);
+    run_forward(B, ctx);
     run_noise(C, specs, rows, picks, nx, ny, acq, st);
     for (int g = g0; g < g1; ++g)
       for (int s = 0; s < nsl; ++s) {

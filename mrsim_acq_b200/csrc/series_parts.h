@@ -55,7 +55,8 @@ struct UnitInputs {
 
 void add_unit(Batch& B, const UnitInputs& in, int snx, int sny, int nx, int ny, int ncomp, int ncoils, bool maps,
               const float* t2u, const float* tiu, const GeoTab& geo, const mrsim_acquisition& acq);
-void run_forward(const Batch& B, cudaStream_t st);
+// Forward of the batch, queued on the context's stream.
+void run_forward(const Batch& B, mrsim_context* ctx);
 // Line records of the acquired lines (uniform relaxation weights when `uniform`).
 void lines_for(std::vector<LineRec>& out, const mrsim_acquisition& acq, int nx, int ny, bool eddy, bool uniform,
                int ncomp, const float* t2u, const float* tiu, bool has_tinhom, const LineTimingTab* timing);

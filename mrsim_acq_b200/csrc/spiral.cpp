@@ -154,7 +154,7 @@ void nufft1_host(mrsim_context* ctx, int n, int k_lo, int n_out, double tol, con
     fail("output band must sit inside the coarse Nyquist band");
   if (n <= 0 || n > 4096) fail("NUFFT period must be in 1..4096");
   cudaStream_t st = ctx->stream;
-  DevArena A;
+  DevArena A(ctx);
   Nufft1Grid g;
   g.n = n;
   g.nf = 2 * n;
@@ -180,7 +180,7 @@ void nufft1_host(mrsim_context* ctx, int n, int k_lo, int n_out, double tol, con
 void nufft2_host(mrsim_context* ctx, int type, int n0, int n1, int m_lo0, int m_lo1, int m_out0, int m_out1, double tol,
                  const double* u, int npts, const float* in, int sign, float* out) {
   cudaStream_t st = ctx->stream;
-  DevArena A;
+  DevArena A(ctx);
   NufftGrid g = make_nufft<float>(A, n0, n1, m_lo0, m_lo1, m_out0, m_out1, tol, st);
   const size_t nm = (size_t)m_out0 * m_out1;
   if (npts == 0) {  // no points: type 2 has no values, type 1 all-zero modes
@@ -265,7 +265,7 @@ void spiral_exact_host(mrsim_context* ctx, const mrsim_slice_input& inp, const m
       dec[(size_t)c * n + i] = (float)decay_rate(inp, acq, c, i);
     }
   }
-  DevArena A;
+  DevArena A(ctx);
   SpiralExactArgs a;
   std::memset(&a, 0, sizeof a);
   a.k = (const double*)A.upload(k, (size_t)npts * 2 * 8, st);
@@ -326,7 +326,7 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
   std::vector<double> tau(tau_ms, tau_ms + ntau);
   TsegPlan plan;
   {
-    TsegDevice dev(st);
+    TsegDevice dev(ctx, st);
     plan = tseg_plan(tau, t_ms, rect_d, rect_f, &dev);
   }
   SegmentedInfo info;
@@ -349,7 +349,7 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
     if (tau_idx[j] < 0 || tau_idx[j] >= ntau) fail("sample-time index out of range");
     tidx[j] = (int)tau_idx[j];
   }
-  DevArena A;
+  DevArena A(ctx);
   NufftGrid g = make_nufft<float>(A, snx, sny, -sxs, -sys, snx, sny, 1e-12, st);
   const float2* dx = (const float2*)A.upload(x.data(), n * sizeof(float2), st);
   const float2* drate = (const float2*)A.upload(rate.data(), n * sizeof(float2), st);

@@ -621,7 +621,7 @@ static void build_sources(SpiralPlan3& P, const mrsim_acquisition& acq) {
 
 static SpiralPlan3 make_spiral_plan(const mrsim_acquisition_3d_input& in, const mrsim_acquisition& acq,
                                     const mrsim_echo_train& train, const mrsim_spiral_readout& ro, int rows,
-                                    cudaStream_t st) {
+                                    mrsim_context* ctx) {
   SpiralPlan3 P;
   P.nc = (int)std::max<int64_t>(acq.n_coils, 1);
   if (P.nc > kMaxCoils) fail("more than 64 coils");
@@ -693,7 +693,7 @@ static SpiralPlan3 make_spiral_plan(const mrsim_acquisition_3d_input& in, const 
     try {
       MRSIM_CUDA(cudaSetDevice(dev_id));
       MRSIM_CUDA(cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking));
-      TsegDevice dev(ws);
+      TsegDevice dev(ctx, ws);
       for (int i; (i = next.fetch_add(1)) < (int)keys.size();) {
         try {
           const double d[2] = {keys[i][0], keys[i][1]}, f[2] = {keys[i][2], keys[i][3]};
@@ -859,10 +859,11 @@ static SpiralVariants spiral_sets(DevArena& A, const SpiralPlan3& P, const mrsim
 
 // Every coil's samples of volume g before noise: out [q][p][nsamp].
 static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, const float* d_lw, float2* out,
-                           cudaStream_t st, const SpiralVariants* V = nullptr) {
+                           mrsim_context* ctx, const SpiralVariants* V = nullptr) {
+  cudaStream_t st = ctx->stream;
   const int nsrc = (int)P.srcs.size(), nz = P.nz, nsamp = P.nsamp, ring = P.ring;
   const int nvar = V ? V->nvar : 1;
-  DevArena C;
+  DevArena C(ctx);
   NufftGrid grid = make_nufft<float>(C, P.snx, P.sny, -P.o * (P.n / 2), -P.o * (P.n / 2), P.snx, P.sny, 1e-12, st);
   const double* d_k = (const double*)C.upload(P.table.traj.k.data(), P.table.traj.k.size() * 8, st);
   const float2* d_stat = (const float2*)C.upload(P.stat.data(), P.stat.size() * sizeof(float2), st);
@@ -913,7 +914,7 @@ static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, c
     MRSIM_CUDA(cudaMemcpyAsync(d_base, base.data(), base.size() * 4, cudaMemcpyHostToDevice, st));
     MRSIM_CUDA(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * 4, cudaMemcpyHostToDevice, st));
     MRSIM_CUDA(cudaMemcpyAsync(d_off, off.data(), off.size() * sizeof(size_t), cudaMemcpyHostToDevice, st));
-    DevArena Z;
+    DevArena Z(ctx);
     const double* tl0 = pc.l ? (const double*)Z.upload(pc.tau_l.data(), pc.tau_l.size() * 8, st) : nullptr;
     const double* tl1 = pv.l ? (const double*)Z.upload(pv.tau_l.data(), pv.tau_l.size() * 8, st) : nullptr;
     const double* b0 = pc.l ? (const double*)Z.upload(pc.b.data(), pc.b.size() * 8, st) : nullptr;
@@ -925,7 +926,6 @@ static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, c
     seg_combine_kernel<<<g3(nsamp, nslot, 1), 256, 0, st>>>(segout, d_base, d_plan, b0, b1, pc.l, pv.l, P.ns, nsamp,
                                                             d_stat, k2, d_off);
     MRSIM_CUDA(cudaGetLastError());
-    MRSIM_CUDA(cudaStreamSynchronize(st));  // Z's tables are freed at the end of the iteration
   }
   // the z-DFT with the rings' profiles, amplitudes and line weights
   std::vector<float2> zkq((size_t)P.rows * nz * nz);
@@ -1057,7 +1057,7 @@ static KzKernel kz_fit(mrsim_context* ctx, const Spiral3dTable& T, int accel, co
            "]: too few partitions for a kz acceleration of " + std::to_string(accel));
     }
     if (nfeat * ncol > 24 * 256) fail("too many coils for the kz kernel (at most 16 x 4 sources)");
-    DevArena A;
+    DevArena A(ctx);
     KzFitArgs a;
     a.k = d_cal;
     a.t_list = (const int*)A.upload(tl.data(), tl.size() * 4, st);
@@ -1101,7 +1101,7 @@ static KzKernel kz_fit(mrsim_context* ctx, const Spiral3dTable& T, int accel, co
 static void kz_fill(mrsim_context* ctx, const KzKernel& K, int accel, float2* d_k, int nc, int nz, int nsamp) {
   cudaStream_t st = ctx->stream;
   if (K.targets.empty()) return;
-  DevArena A;
+  DevArena A(ctx);
   std::vector<KzFillJob> jobs;
   for (const auto& tg : K.targets) {
     auto it = K.where.find(std::make_pair(tg.d, tg.pat));
@@ -1129,9 +1129,9 @@ void spiral3d_samples(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
                       int g, float* out) {
   cudaStream_t st = ctx->stream;
   const int rows = opts ? (int)opts->coil_rows : 1;
-  SpiralPlan3 P = make_spiral_plan(in, acq, train, ro, rows, st);
+  SpiralPlan3 P = make_spiral_plan(in, acq, train, ro, rows, ctx);
   if (g < 0 || g >= (int)in.n_volumes) fail("volume index out of range");
-  DevArena A;
+  DevArena A(ctx);
   SpiralInputs I = upload_spiral_inputs(A, P, in, in.images, (int)in.n_volumes, acq, st);
   const float* d_lw = nullptr;
   if (in.line_weights) {
@@ -1142,7 +1142,7 @@ void spiral3d_samples(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
   float2* k = (float2*)A.alloc((size_t)P.nc * P.nz * P.nsamp * sizeof(float2));
   for (int h = 0; h < (int)in.n_volumes; ++h) (void)spiral_sets(A, P, in, h, st, false);  // every volume's sets checked
   const SpiralVariants V = spiral_sets(A, P, in, g, st);
-  spiral_samples(P, I, g, d_lw, k, st, &V);
+  spiral_samples(P, I, g, d_lw, k, ctx, &V);
   copy_pageable_d2h(ctx, out, k, (size_t)P.nc * P.nz * P.nsamp * sizeof(float2), st);
   MRSIM_CUDA(cudaStreamSynchronize(st));
 }
@@ -1152,10 +1152,10 @@ void spiral3d_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
                       uint64_t seed, float* mag, float* ph) {
   cudaStream_t st = ctx->stream;
   const int rows = opts ? (int)opts->coil_rows : 1;
-  SpiralPlan3 P = make_spiral_plan(in, acq, train, ro, rows, st);
+  SpiralPlan3 P = make_spiral_plan(in, acq, train, ro, rows, ctx);
   const int nv = (int)in.n_volumes, nz = P.nz, nc = P.nc, n = P.n, nsamp = P.nsamp;
   const double sigma = std::sqrt(acq.noise_variance / (double)((size_t)n * n));
-  DevArena A;
+  DevArena A(ctx);
   for (int g = 0; g < nv; ++g) (void)spiral_sets(A, P, in, g, st, false);  // every volume's sets checked first
   SpiralInputs I = upload_spiral_inputs(A, P, in, in.images, nv, acq, st);
   const float* d_lw = nullptr;
@@ -1189,15 +1189,15 @@ void spiral3d_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
     Pc.table = spiral_lines(ctr, cro, n, n, nz);
     Pc.modes = resolve_modes(in.t2, in.t1, in.t_inhom, P.ncomp, acq, ctr, P.nvox);
     build_sources(Pc, acq);
-    DevArena C;
+    DevArena C(ctx);
     SpiralInputs Ic = upload_spiral_inputs(C, Pc, in, opts->calibration_images, 1, acq, st);
     float2* ck = (float2*)C.alloc((size_t)nc * nz * nsamp * sizeof(float2));
-    spiral_samples(Pc, Ic, 0, nullptr, ck, st);
+    spiral_samples(Pc, Ic, 0, nullptr, ck, ctx);
     spiral_noise(C, Pc, Pc.table.acquired, ck, 0, opts->calibration_seed ^ kSeedSaltKzcal, sigma, st);
     kzk = kz_fit(ctx, P.table, accel, ck, nc, nsamp);
   }
   const bool pocs = ro.kz.partial_fourier < 1.0 && P.table.band_start > 0 && opts && opts->pocs;
-  SpiralRecon rec(ctx, P.table.traj.k.data(), nsamp, n, acq, kLsIterations, kLsKappa, true);
+  SpiralRecon rec(ctx, P.table.traj.k.data(), nsamp, n, acq, kLsIterations, kLsKappa, true, true);
   const size_t nn = (size_t)n * n;
   float* d_mag = (float*)A.alloc(std::max<size_t>(1, nn * nz * nv) * 4);
   float* d_ph = (float*)A.alloc(std::max<size_t>(1, nn * nz * nv) * 4);
@@ -1206,10 +1206,10 @@ void spiral3d_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
     for (int q = 0; q < nc; ++q) zs_zq[(size_t)z * nc + q] = P.zsens[(size_t)q * nz + z];
   const float2* d_zk = (const float2*)A.upload(P.zk.data(), P.zk.size() * sizeof(float2), st);
   for (int g = 0; g < nv; ++g) {
-    DevArena C;
+    DevArena C(ctx);
     float2* k = (float2*)C.alloc((size_t)nc * nz * nsamp * sizeof(float2));
     const SpiralVariants V = spiral_sets(C, P, in, g, st);
-    spiral_samples(P, I, g, d_lw, k, st, &V);
+    spiral_samples(P, I, g, d_lw, k, ctx, &V);
     spiral_noise(C, P, P.table.acquired, k, g, seed, sigma, st);
     if (accel > 1) kz_fill(ctx, kzk, accel, k, nc, nz, nsamp);
     double2* vol = (double2*)C.alloc(nn * nz * sizeof(double2));

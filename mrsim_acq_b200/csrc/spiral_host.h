@@ -6,6 +6,8 @@
 #include <utility>
 #include <vector>
 
+struct mrsim_context;
+
 namespace mrsim {
 
 struct SpiralTraj {
@@ -34,7 +36,8 @@ struct TsegPlan {
 // search over L and m stay on the host.  One object serves the plans of one call on one stream.
 class TsegDevice {
  public:
-  explicit TsegDevice(cudaStream_t st);
+  // its memory comes from the context's pool in the order of `st` (any stream of the device)
+  TsegDevice(mrsim_context* ctx, cudaStream_t st);
   ~TsegDevice();
   TsegDevice(const TsegDevice&) = delete;
   TsegDevice& operator=(const TsegDevice&) = delete;
@@ -49,6 +52,7 @@ class TsegDevice {
  private:
   struct Bufs;
   cudaStream_t st_;
+  cudaMemPool_t pool_;
   Bufs* d_;
   int n_tau_ = 0, l_ = 0;
 };

@@ -269,8 +269,9 @@ dim3 grid1(size_t n, int batch = 1) { return dim3((unsigned)std::max<size_t>(1, 
 
 // ---- SpiralRecon ------------------------------------------------------------------------------------
 SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, const mrsim_acquisition& win_acq,
-                         int iterations_, double kappa_, bool band_limited)
-    : ctx(c), n(n_), npts(npts_), iterations(iterations_), kappa(kappa_), band(band_limited) {
+                         int iterations_, double kappa_, bool band_limited, bool call_scoped)
+    : ctx(c), n(n_), npts(npts_), iterations(iterations_), kappa(kappa_), band(band_limited),
+      A(call_scoped ? c : nullptr) {
   cudaStream_t st = ctx->stream;
   if (n <= 0 || n > 1024) fail("spiral reconstruction matrix must be in 1..1024");
   if (npts <= 0) fail("a spiral reconstruction needs samples");
@@ -283,7 +284,7 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
   d_k = (double*)A.upload(k, (size_t)npts * 2 * 8, st);
   bins_k = nufft_bins2(A, g.nf0, g.nf1, g.w, k, npts, st);
   d_w = (double*)A.alloc((size_t)npts * 8);
-  DevArena T;
+  DevArena T(ctx);
   // Pipe-Menon (grid_recon.rs:54-66)
   {
     std::vector<double> ones(npts, 1.0);
@@ -438,7 +439,7 @@ void SpiralRecon::normal(const double2* x, double2* out, int batch, const Scratc
 }
 
 void SpiralRecon::sumsq(const double2* v, int batch, double* out, cudaStream_t st) const {
-  DevArena T;
+  DevArena T(ctx);
   double* d = (double*)T.alloc((size_t)batch * 8);
   sumsq_kernel<<<batch, 256, 0, st>>>(v, n * n, d);
   MRSIM_CUDA(cudaMemcpyAsync(out, d, (size_t)batch * 8, cudaMemcpyDeviceToHost, st));
@@ -448,7 +449,7 @@ void SpiralRecon::sumsq(const double2* v, int batch, double* out, cudaStream_t s
 // `gridding` (grid_recon.rs:231-236): n^2 A^H W d, no window
 void SpiralRecon::gridding(const double2* d_data, int batch, double2* d_out) {
   cudaStream_t st = ctx->stream;
-  DevArena T;
+  DevArena T(ctx);
   const double sc = 1.0 / ((double)n * n);
   double2* wts = (double2*)T.alloc((size_t)batch * npts * 16);
   weight_samples_kernel<<<grid1(npts, batch), 256, 0, st>>>(d_data, nullptr, d_w, sc, npts, wts);
@@ -463,11 +464,11 @@ void SpiralRecon::gridding(const double2* d_data, int batch, double2* d_out) {
 void SpiralRecon::images(const double2* d_data, int batch, double2* d_x) {
   cudaStream_t st = ctx->stream;
   const size_t nn = (size_t)n * n;
-  DevArena T;
+  DevArena T(ctx);
   const double sc = 1.0 / ((double)n * n);
   double2* r = (double2*)T.alloc((size_t)batch * nn * 16);
   {
-    DevArena W;
+    DevArena W(ctx);
     double2* wts = (double2*)W.alloc((size_t)batch * npts * 16);
     weight_samples_kernel<<<grid1(npts, batch), 256, 0, st>>>(d_data, d_win, d_w, sc, npts, wts);
     double2* work = (double2*)W.alloc((size_t)batch * g.nf0 * g.nf1 * 16);
@@ -527,7 +528,7 @@ void SpiralRecon::rings(const double2* d_coil, int n_part, int ncoils, int ring,
   if (ring < 1 || ncoils % ring != 0) fail("the coils do not divide into rings of " + std::to_string(ring));
   const int rows = ncoils / ring;
   const size_t nn = (size_t)n * n;
-  DevArena T;
+  DevArena T(ctx);
   double* dz = (double*)T.upload(zsens, (size_t)n_part * ncoils * 8, st);
   std::vector<double> z2((size_t)n_part * ring, 0.0), sens((size_t)ring * nn);
   for (int p = 0; p < n_part; ++p)

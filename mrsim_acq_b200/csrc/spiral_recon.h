@@ -57,9 +57,10 @@ struct SpiralRecon {
     double2* tmp;
   };
 
-  // `SpiralRecon::with_params` (grid_recon.rs:152-198); the window is win_acq's.
+  // `SpiralRecon::with_params` (grid_recon.rs:152-198); the window is win_acq's.  call_scoped: it ends
+  // with the call that made it, so its memory comes from the context's pool.
   SpiralRecon(mrsim_context* ctx, const double* k, int npts, int n, const mrsim_acquisition& win_acq,
-              int iterations, double kappa, bool band_limited);
+              int iterations, double kappa, bool band_limited, bool call_scoped = false);
   Scratch scratch(DevArena& T, int batch) const;
   void project(double2* x, int batch, cudaStream_t st) const;
   void normal(const double2* x, double2* out, int batch, const Scratch& s, cudaStream_t st) const;

@@ -779,7 +779,7 @@ TsPlan* ts_plan_build(const EpiOperator& op, int precision) {
   const int snx = op.snx, sny = op.sny, nx = op.nx, ny = op.ny, ncomp = op.ncomp;
   const mrsim_acquisition& acq = op.acq;
   cudaStream_t st = op.ctx->stream;
-  TsegDevice fitdev(st);  // the segmentation fits' per-sample work
+  TsegDevice fitdev(op.ctx, st);  // the segmentation fits' per-sample work
 
   // coil classes (the geometry's bitwise-equal ey rows) plus the offset row
   std::vector<float> eyc((size_t)op.geo.ncls * sny);

@@ -135,12 +135,12 @@ __global__ void __launch_bounds__(kFitThreads) tseg_fit_kernel(FitArgs a) {
 }
 
 template <class T>
-void grow(T*& p, size_t& cap, size_t n) {
+void grow(cudaMemPool_t pool, cudaStream_t st, T*& p, size_t& cap, size_t n) {
   if (n <= cap) return;
-  if (p) MRSIM_CUDA(cudaFree(p));
+  if (p) MRSIM_CUDA(cudaFreeAsync(p, st));
   p = nullptr;
   cap = 0;
-  MRSIM_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
+  MRSIM_CUDA(cudaMallocFromPoolAsync((void**)&p, std::max<size_t>(n, 1) * sizeof(T), pool, st));
   cap = n;
 }
 
@@ -155,18 +155,18 @@ struct TsegDevice::Bufs {
   std::vector<double> stage;  // host staging of the flattened factors
 };
 
-TsegDevice::TsegDevice(cudaStream_t st) : st_(st), d_(new Bufs) {}
+TsegDevice::TsegDevice(mrsim_context* ctx, cudaStream_t st) : st_(st), pool_(ctx->pool), d_(new Bufs) {}
 
 TsegDevice::~TsegDevice() {
   for (void* p : {(void*)d_->tau, (void*)d_->rate, (void*)d_->left, (void*)d_->right, (void*)d_->sig,
                   (void*)d_->cols, (void*)d_->b, (void*)d_->maxes})
-    if (p) cudaFree(p);
+    if (p) cudaFreeAsync(p, st_);
   delete d_;
 }
 
 void TsegDevice::set_times(const std::vector<double>& tau) {
   n_tau_ = (int)tau.size();
-  grow(d_->tau, d_->c_tau, tau.size());
+  grow(pool_, st_, d_->tau, d_->c_tau, tau.size());
   if (!tau.empty())
     MRSIM_CUDA(cudaMemcpyAsync(d_->tau, tau.data(), tau.size() * sizeof(double), cudaMemcpyHostToDevice, st_));
 }
@@ -200,13 +200,13 @@ void TsegDevice::fit(const std::vector<std::pair<double, double>>& rates, const 
   p += R;
   double* pc = p;
   for (int i = 0; i < l2; ++i) std::memcpy(p + (size_t)i * g2, cols[i].data(), g2 * sizeof(double));
-  grow(d_->rate, d_->c_rate, (size_t)g);
-  grow(d_->left, d_->c_left, (size_t)R * g2);
-  grow(d_->right, d_->c_right, (size_t)R * l2);
-  grow(d_->sig, d_->c_sig, (size_t)R);
-  grow(d_->cols, d_->c_cols, (size_t)l2 * g2);
-  grow(d_->b, d_->c_b, (size_t)n_tau_ * l2);
-  grow(d_->maxes, d_->c_max, 2);
+  grow(pool_, st_, d_->rate, d_->c_rate, (size_t)g);
+  grow(pool_, st_, d_->left, d_->c_left, (size_t)R * g2);
+  grow(pool_, st_, d_->right, d_->c_right, (size_t)R * l2);
+  grow(pool_, st_, d_->sig, d_->c_sig, (size_t)R);
+  grow(pool_, st_, d_->cols, d_->c_cols, (size_t)l2 * g2);
+  grow(pool_, st_, d_->b, d_->c_b, (size_t)n_tau_ * l2);
+  grow(pool_, st_, d_->maxes, d_->c_max, 2);
   MRSIM_CUDA(cudaMemcpyAsync(d_->rate, s.data(), (size_t)g * sizeof(double2), cudaMemcpyHostToDevice, st_));
   MRSIM_CUDA(cudaMemcpyAsync(d_->left, pl, (size_t)R * g2 * sizeof(double), cudaMemcpyHostToDevice, st_));
   MRSIM_CUDA(cudaMemcpyAsync(d_->right, pr, (size_t)R * l2 * sizeof(double), cudaMemcpyHostToDevice, st_));
