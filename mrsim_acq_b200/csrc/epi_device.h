@@ -1,0 +1,157 @@
+// epi_device.h — what the EPI kernels share (epi_ystage.cu, epi_yadjoint.cu, epi_kernels.cu): packed
+// arithmetic, the reduced phase, asynchronous copies, and the shapes of the staged kernels' tiles.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "mrsim_internal.h"
+
+// Template flags select whole code paths (packed or scalar, class or coil accumulators); the paths
+// an instance does not take leave loops the front end reports as unreachable.
+#pragma nv_diag_suppress 128
+
+namespace mrsim {
+
+namespace {
+
+constexpr float kTwoPiF = 6.28318530717958647692f;
+
+// The reduced phase s + f t in turns (s = static phase + k.r term, |s| <= 1 turn; f the voxel's
+// off-resonance in Hz; t = t_hi + t_lo the line time in s, |f t| < 2^22) with one rounding to an
+// integer: n = round(s + f t_hi) by adding and subtracting 1.5 * 2^23 (the FMA's rounded value
+// serves only to choose n), r = f t_hi - n from one FMA of the exact product (|r| < 2: one rounding
+// of at most ulp(1)/2), and
+//   theta = (r + s) + f t_lo,   |theta| <= 1/2 + ulps,
+// whose last two roundings are at most ulp(1/2)/2 each.
+__device__ __forceinline__ float phase_turns(float s, float f, float t_hi, float t_lo) {
+  const float nn = __fsub_rn(12582912.0f, __fadd_rn(fmaf(f, t_hi, s), 12582912.0f));  // -n
+  return fmaf(f, t_lo, __fadd_rn(fmaf(f, t_hi, nn), s));
+}
+
+// Packed FP32 pairs (sm_100 add/sub/mul/fma.rn.f32x2): one instruction for two lanes, each lane
+// rounding exactly like the scalar operation, so a packed computation is bitwise the scalar one.
+__device__ __forceinline__ unsigned long long pk2(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 upk2(unsigned long long r) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
+  return d;
+}
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
+  return upk2(d);
+}
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
+  return upk2(d);
+}
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
+  return upk2(d);
+}
+__device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
+  return upk2(d);
+}
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// The reduced phase s + f t (s = static phase + k.r term, |s| <= 1 turn, t = t_hi + t_lo) on a pair
+// of lanes with one rounding to an integer: n = round(s + f t_hi) (the FMA's rounded value serves
+// only to choose n), r = f t_hi - n from one FMA of the exact product (|r| < 2: one rounding of
+// at most ulp(1)/2), and
+//   theta = (r + s) + f t_lo,   |theta| <= 1/2 + ulps,
+// whose last two roundings are at most ulp(1/2)/2 each: six packed operations.
+__device__ __forceinline__ float2 phase_turns2(float2 s, float2 f, float2 t_hi, float2 t_lo) {
+  const float2 M = dup2(12582912.0f);
+  const float2 nn = fsub2(M, fadd2(ffma2(f, t_hi, s), M));  // -n
+  const float2 r = ffma2(f, t_hi, nn);
+  return ffma2(f, t_lo, fadd2(r, s));
+}
+
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
+}
+
+// cp.async helpers (16-byte copies zero-fill the bytes past src_bytes)
+__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src, int src_bytes = 8) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
+__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_n() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+}
+
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src, int src_bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
+}
+
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, int src_bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
+}
+
+constexpr int kT = 4;   // lines per tile of ystage_kernel
+constexpr int kTY = 4;  // rows per tile of yadjoint_kernel
+
+// ystage_q_kernel: ring stages, and input planes and rows per stage
+constexpr int kFwdStages = 3;
+__host__ __device__ __forceinline__ constexpr int fwdq_planes(int nc, bool maps) { return maps ? 3 + 3 * nc : 2 + nc; }
+__host__ __device__ __forceinline__ constexpr int fwdq_rows(int nc, bool maps) {
+  return fwdq_planes(nc, maps) <= 5 ? 8 : fwdq_planes(nc, maps) <= 12 ? 4 : 2;
+}
+
+// Lines per h chunk of yadjoint_kernel for `ncoils` coils (16 coil-lines per chunk, at least one line).
+__host__ __device__ __forceinline__ int adjoint_chunk_lines(int ncoils) { return ncoils >= 16 ? 1 : 16 / ncoils; }
+
+// yadjoint_q_kernel: ring stages, lines per chunk, floats of a line record
+constexpr int kAdjStages = 3;
+__host__ __device__ __forceinline__ constexpr int adjq_chunk_lines(int nq) { return nq >= 16 ? 1 : 16 / nq; }
+__host__ __device__ __forceinline__ constexpr int adjq_line_floats(int nc, bool maps) {
+  return ((maps ? 5 : 4 + 3 * nc) + 3) / 4 * 4;
+}
+// rows per thread: 4 with class decay and up to 3 compartments, else 2 (registers)
+__host__ __device__ __forceinline__ constexpr int adjq_rows(int nc, bool maps) { return !maps && nc <= 3 ? 4 : 2; }
+// ... the same with coil-class rows (two rows per thread in 80 registers and three CTAs per SM
+// measured 30 % slower than four rows: the per-line loads then serve half the rows)
+__host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps, bool virt) {
+  return adjq_rows(nc, maps);
+}
+
+template <class K>
+void set_smem(K kernel, size_t bytes) {
+  // past 48 KB of static + dynamic shared memory the launch needs the dynamic opt-in
+  // (the whole limit, so that threads launching one kernel with different sizes never lower it
+  // between another's opt-in and launch)
+  cudaFuncAttributes fa;
+  MRSIM_CUDA(cudaFuncGetAttributes(&fa, kernel));
+  if (bytes + fa.sharedSizeBytes > 48 * 1024)
+    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    227 * 1024 - (int)fa.sharedSizeBytes));
+}
+
+// The tiles of units [u0, u1) in a list with per-unit starts `start` (empty: the whole list).
+struct TileRange {
+  int t0, n;
+};
+TileRange tile_range(const std::vector<int>& start, int n_tiles, int u0, int u1) {
+  if (start.empty() || (u0 == 0 && (u1 < 0 || u1 == (int)start.size() - 1))) return {0, n_tiles};
+  if (u1 < 0) u1 = (int)start.size() - 1;
+  if (u0 < 0 || u0 > u1 || u1 >= (int)start.size()) fail("unit range outside the plan");
+  return {start[u0], start[u1] - start[u0]};
+}
+
+}  // namespace
+
+}  // namespace mrsim

@@ -24,12 +24,13 @@
 //
 // Kernels, in the order a step runs them:
 //   statics_kernel                     static phase a(x,y) in turns (FP64 per-slice quadratic)
-//   ystage_q_kernel / ystage_kernel    y-stage (staged-input form; per-thread-load fallback);
+//   ystage_q_kernel / ystage_kernel    y-stage (epi_ystage.cu: staged-input form; per-thread-load fallback);
 //                                      with the 8-coil ring it accumulates 5 ey classes + offset,
 //                                      with other rings of 6 or more coils the rows of a coil basis
 //   xfft_warp_kernel / xfft_kernel /   x-stage: warp-per-row FFT (N = 32..256), shared-memory
 //   xgemm_kernel                       radix-2 FFT (other powers of two), DFT GEMM (other widths)
-//   yadjoint_q_kernel / yadjoint_kernel  y-adjoint (fixed coil or class count; any coil count)
+//   yadjoint_q_kernel / yadjoint_kernel  y-adjoint (epi_yadjoint.cu: fixed coil or class count; any
+//                                      coil count)
 // The class-mode and packed (f32x2) paths are exact rearrangements: equal ey rows, and lanes that
 // round like the scalar operations.
 #include <cuda_runtime.h>
@@ -39,103 +40,12 @@
 #include <cstring>
 #include <map>
 
+#include "epi_device.h"
 #include "mrsim_internal.h"
-
-// Template flags select whole code paths (packed or scalar, class or coil accumulators); the paths
-// an instance does not take leave loops the front end reports as unreachable.
-#pragma nv_diag_suppress 128
 
 namespace mrsim {
 
 namespace {
-
-constexpr float kTwoPiF = 6.28318530717958647692f;
-
-// The reduced phase s + f t in turns (s = static phase + k.r term, |s| <= 1 turn; f the voxel's
-// off-resonance in Hz; t = t_hi + t_lo the line time in s, |f t| < 2^22) with one rounding to an
-// integer: n = round(s + f t_hi) by adding and subtracting 1.5 * 2^23 (the FMA's rounded value
-// serves only to choose n), r = f t_hi - n from one FMA of the exact product (|r| < 2: one rounding
-// of at most ulp(1)/2), and
-//   theta = (r + s) + f t_lo,   |theta| <= 1/2 + ulps,
-// whose last two roundings are at most ulp(1/2)/2 each.
-__device__ __forceinline__ float phase_turns(float s, float f, float t_hi, float t_lo) {
-  const float nn = __fsub_rn(12582912.0f, __fadd_rn(fmaf(f, t_hi, s), 12582912.0f));  // -n
-  return fmaf(f, t_lo, __fadd_rn(fmaf(f, t_hi, nn), s));
-}
-
-// Packed FP32 pairs (sm_100 add/sub/mul/fma.rn.f32x2): one instruction for two lanes, each lane
-// rounding exactly like the scalar operation, so a packed computation is bitwise the scalar one.
-__device__ __forceinline__ unsigned long long pk2(float2 a) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-  return r;
-}
-__device__ __forceinline__ float2 upk2(unsigned long long r) {
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
-  return d;
-}
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
-
-// The reduced phase s + f t (s = static phase + k.r term, |s| <= 1 turn, t = t_hi + t_lo) on a pair
-// of lanes with one rounding to an integer: n = round(s + f t_hi) (the FMA's rounded value serves
-// only to choose n), r = f t_hi - n from one FMA of the exact product (|r| < 2: one rounding of
-// at most ulp(1)/2), and
-//   theta = (r + s) + f t_lo,   |theta| <= 1/2 + ulps,
-// whose last two roundings are at most ulp(1/2)/2 each: six packed operations.
-__device__ __forceinline__ float2 phase_turns2(float2 s, float2 f, float2 t_hi, float2 t_lo) {
-  const float2 M = dup2(12582912.0f);
-  const float2 nn = fsub2(M, fadd2(ffma2(f, t_hi, s), M));  // -n
-  const float2 r = ffma2(f, t_hi, nn);
-  return ffma2(f, t_lo, fadd2(r, s));
-}
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
-}
-
-// cp.async helpers (16-byte copies zero-fill the bytes past src_bytes)
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src, int src_bytes = 8) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_n() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src, int src_bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
-}
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, int src_bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
-}
 
 // ---------------------------------------------------------------------------------------------
 // statics: a(x,y) = frac( (phi0 + eddy object phase) / 2pi ) in FP64, stored as f32 turns.
@@ -196,1086 +106,6 @@ __global__ void statics_kernel(const StaticDesc* descs) {
     double tt = p0 * inv_tau;
     tt -= rint(tt);
     out[i] = (float)tt;
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// y-stage of the forward.  One CTA = (unit, T lines, 128 columns, QG coils); one thread per
-// column x accumulates T*QG complex sums over every sim row y.
-struct Tile {
-  int unit, line0, x0, q0;
-};
-
-template <int T, int QG, int NC, bool MAPS>
-__global__ void __launch_bounds__(128, 4) ystage_kernel(const UnitDesc* __restrict__ units,
-                                                        const Tile* __restrict__ tiles) {
-  // A CTA of 128 threads: one column each, T lines x QG coils per thread.
-  constexpr int LG = 1;
-  constexpr int TL = LG * T;  // lines per CTA
-  static_assert(T == 4, "the phase table is read as float4");
-  extern __shared__ __align__(16) float smem[];
-  const Tile tl = tiles[blockIdx.x];
-  const UnitDesc& u = units[tl.unit];
-  const int snx = u.snx, sny = u.sny;
-  const int ncomp = u.ncomp;
-  float* Bt = smem;                 // [sny][TL] phase terms per (row, line)
-  float* Ey = smem + sny * TL;      // [sny][QGP] (QGP = QG rounded up to 4)
-  constexpr int QGP = (QG + 3) / 4 * 4;
-  __shared__ float rel_s[TL][kMaxComp];
-  __shared__ float tinh_s[TL], trf_s[TL];
-  __shared__ float thi_s[TL], tlo_s[TL];
-
-  const int nl = min(TL, u.n_lines - tl.line0);
-  const int ys = u.ny / 2;
-  const int oy = sny / u.ny;
-  const int sys = oy * ys;
-  for (int idx = threadIdx.x; idx < sny * TL; idx += blockDim.x) {
-    const int y = idx / TL, j = idx % TL;
-    float v = 0.f;
-    if (j < nl) {
-      const LineRec& L = u.lines[tl.line0 + j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
-      if (u.flags & UF_EDDY) {
-        const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
-        tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
-      }
-      tv -= rint(tv);
-      v = (float)tv;
-    }
-    Bt[idx] = v;
-  }
-  for (int idx = threadIdx.x; idx < QGP * sny; idx += blockDim.x) {
-    const int y = idx / QGP, qq = idx % QGP;
-    const int q = tl.q0 + qq;
-    Ey[idx] = (qq < QG && q < u.ncoils) ? u.geo.ey[(size_t)q * sny + y] : 0.f;
-  }
-  if (threadIdx.x < TL) {
-    const int j = threadIdx.x;
-    if (j < nl) {
-      const LineRec& L = u.lines[tl.line0 + j];
-      thi_s[j] = L.t_hi;
-      tlo_s[j] = L.t_lo;
-      tinh_s[j] = L.inhom_ms;
-      trf_s[j] = L.trf_ms;
-      for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = L.rel[c];
-    } else {
-      thi_s[j] = tlo_s[j] = tinh_s[j] = trf_s[j] = 0.f;
-      for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = 0.f;
-    }
-  }
-  __syncthreads();
-
-  const int col = threadIdx.x & 127, lg = threadIdx.x >> 7;
-  const int jb = lg * T;  // this thread's first line within the CTA
-  const int x = tl.x0 + col;
-  const bool xok = x < snx;
-  const int xs_ = xok ? x : 0;
-  float exq[QG];
-  const float off = u.geo.coil_off;
-#pragma unroll
-  for (int qq = 0; qq < QG; ++qq) {
-    const int q = tl.q0 + qq;
-    exq[qq] = (xok && q < u.ncoils) ? u.geo.ex[(size_t)q * snx + x] : 0.f;
-  }
-  float thi[T], tlo[T], relr[T][NC];
-#pragma unroll
-  for (int j = 0; j < T; ++j) {
-    thi[j] = thi_s[jb + j];
-    tlo[j] = tlo_s[jb + j];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) relr[j][c] = rel_s[jb + j][c];
-  }
-  float2 acc[T][QG];
-#pragma unroll
-  for (int j = 0; j < T; ++j)
-#pragma unroll
-    for (int qq = 0; qq < QG; ++qq) acc[j][qq] = make_float2(0.f, 0.f);
-
-  const bool distort = (u.flags & UF_DISTORT) != 0;
-  const float* __restrict__ comp = u.comp;
-  const float* __restrict__ fmap = u.fmap;
-  const float* __restrict__ phase = u.phase;
-  // row y's inputs, prefetched one row ahead
-  float na = 0.f, nf = 0.f, nm[NC];
-  {
-    const int i = xs_;
-    na = phase ? __ldg(phase + i) : 0.f;
-    nf = distort ? __ldg(fmap + i) : 0.f;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) nm[c] = c < ncomp ? __ldg(comp + (size_t)c * u.comp_stride + i) : 0.f;
-  }
-  for (int y = 0; y < sny; ++y) {
-    const int i = xs_ + snx * y;
-    const float a = na, f = nf;
-    float m[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) m[c] = nm[c];
-    if (y + 1 < sny) {
-      const int i1 = i + snx;
-      na = phase ? __ldg(phase + i1) : 0.f;
-      nf = distort ? __ldg(fmap + i1) : 0.f;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) nm[c] = c < ncomp ? __ldg(comp + (size_t)c * u.comp_stride + i1) : 0.f;
-    }
-    float r2[MAPS ? NC : 1], r2i[MAPS ? NC : 1];
-    float la = 0.f;
-    if (MAPS) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        r2[MAPS ? c : 0] = r2i[MAPS ? c : 0] = 0.f;
-        if (c < ncomp) {
-          const float t2 = u.t2map ? __ldg(u.t2map + (size_t)c * u.map_stride + i) : u.t2u[c];
-          const float ti = u.timap ? __ldg(u.timap + (size_t)c * u.map_stride + i) : u.tiu[c];
-          r2[MAPS ? c : 0] = 1.0f / t2;
-          r2i[MAPS ? c : 0] = 1.0f / ti;
-        }
-      }
-      if (u.log_amp) la = __ldg(u.log_amp + i);
-    }
-    float amp[QG];
-#pragma unroll
-    for (int q4 = 0; q4 < QGP; q4 += 4) {
-      const float4 e4 = *reinterpret_cast<const float4*>(Ey + y * QGP + q4);
-      const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (q4 + k < QG) amp[q4 + k] = fmaf(exq[q4 + k], ev[k], off);
-    }
-    const float4 b4 = *reinterpret_cast<const float4*>(Bt + y * TL + jb);
-    const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-    for (int j = 0; j < T; ++j) {
-      const float th = phase_turns(a + bt[j], f, thi[j], tlo[j]);
-      float sn, cs;
-      __sincosf(kTwoPiF * th, &sn, &cs);
-      float W = 0.f;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (c < ncomp) {
-          float r;
-          if (MAPS)
-            r = __expf(la - trf_s[jb + j] * r2[MAPS ? c : 0] - tinh_s[jb + j] * r2i[MAPS ? c : 0]);
-          else
-            r = relr[j][c];
-          W = fmaf(r, m[c], W);
-        }
-      }
-      const float wr = W * cs, wi = W * sn;
-#pragma unroll
-      for (int qq = 0; qq < QG; ++qq) {
-        acc[j][qq].x = fmaf(amp[qq], wr, acc[j][qq].x);
-        acc[j][qq].y = fmaf(amp[qq], wi, acc[j][qq].y);
-      }
-    }
-  }
-  if (!xok) return;
-  const float s = u.signal_scale;
-#pragma unroll
-  for (int qq = 0; qq < QG; ++qq) {
-    const int q = tl.q0 + qq;
-    if (q >= u.ncoils) break;
-#pragma unroll
-    for (int j = 0; j < T; ++j) {
-      if (jb + j < nl)
-        u.g[((size_t)q * u.n_lines + tl.line0 + jb + j) * snx + x] = make_float2(acc[j][qq].x * s, acc[j][qq].y * s);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// y-stage of the forward with the per-row inputs staged in shared memory (every unit of the plan
-// has snx % 4 == 0 and 16-byte aligned input planes).  Same sums as ystage_kernel:
-//   * a CTA of 256 threads covers 128 columns x 8 lines (two groups of 4 lines, one column each)
-//     x QG coils, so each row's inputs serve 8 lines;
-//   * the inputs of RC rows (static phase, fieldmap, compartments, and with voxel maps T2, T2',
-//     log amplitude) arrive through a 3-stage ring filled by cooperative 16-byte cp.async, one
-//     barrier per RC rows, in place of per-thread global loads one row ahead.
-constexpr int kFwdStages = 3;
-__host__ __device__ __forceinline__ constexpr int fwdq_planes(int nc, bool maps) { return maps ? 3 + 3 * nc : 2 + nc; }
-__host__ __device__ __forceinline__ constexpr int fwdq_rows(int nc, bool maps) {
-  return fwdq_planes(nc, maps) <= 5 ? 8 : fwdq_planes(nc, maps) <= 12 ? 4 : 2;
-}
-
-// NV > 0: the tile holds every coil of the unit and accumulates coil classes instead of coils
-// (NV = classes + 1 for the coil offset): acc_v += ey_v(y) W P, acc_off += W P, and the epilogue
-// expands g_q = s (ex_q acc_cls(q) + off acc_off).
-// cls_rows (with NV): 1 writes the class rows G_v = s T_v and G_off = s off T_off ([v][line][x],
-// the layout the class-mode x-stage expands) instead of the coil rows; 2 writes basis rows (the
-// unit's eyc holds the coil basis, whose last row is constant), G_v = s T_v for every row.
-// NARROW: some plane or row is not on a 16-byte boundary, so the ring fills by 4-byte copies.
-template <int QG, int NV, int NC, bool MAPS, bool NARROW>
-__global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __restrict__ units,
-                                                          const Tile* __restrict__ tiles, int cls_rows) {
-  constexpr int T = 4, TL = 8;
-  constexpr int NA = NV ? NV : QG;             // accumulators per line
-  constexpr int NPL = fwdq_planes(NC, MAPS);
-  constexpr int RC = fwdq_rows(NC, MAPS);
-  constexpr int STAGE = NPL * RC * 128;        // floats per stage
-  constexpr int PIECES = NPL * RC * 32;        // 16-byte pieces per stage
-  constexpr int PPT = (PIECES + 255) / 256;
-  constexpr int QGP = (NA + 3) / 4 * 4;
-  // plane order: 0 static phase, 1 fieldmap, 2.. compartments, then T2, T2' maps and log amplitude
-  constexpr int P_COMP = 2, P_T2 = 2 + NC, P_TI = 2 + 2 * NC, P_LA = 2 + 3 * NC;
-  extern __shared__ __align__(16) float smem[];
-  float* ring = smem;                           // [stage][plane][RC][128]
-  float* Bt = ring + kFwdStages * STAGE;        // [sny][TL]
-  const Tile tl = tiles[blockIdx.x];
-  const UnitDesc& u = units[tl.unit];
-  const int snx = u.snx, sny = u.sny, ncomp = u.ncomp;
-  float* Ey = Bt + sny * TL;                    // [sny][QGP]: ey per coil, or per class and 1
-  __shared__ const float* plane_s[NPL];
-  __shared__ float rel_s[TL][kMaxComp];
-  __shared__ float tinh_s[TL], trf_s[TL], thi_s[TL], tlo_s[TL];
-  const int tid = threadIdx.x;
-  const bool distort = (u.flags & UF_DISTORT) != 0;
-  if (tid < NPL) {
-    const float* pp = nullptr;
-    const int k = tid;
-    if (k == 0) pp = u.phase;
-    else if (k == 1) pp = distort ? u.fmap : nullptr;
-    else if (k < P_T2) pp = (k - P_COMP) < ncomp ? u.comp + (size_t)(k - P_COMP) * u.comp_stride : nullptr;
-    else if (k < P_TI) pp = ((k - P_T2) < ncomp && u.t2map) ? u.t2map + (size_t)(k - P_T2) * u.map_stride : nullptr;
-    else if (k < P_LA) pp = ((k - P_TI) < ncomp && u.timap) ? u.timap + (size_t)(k - P_TI) * u.map_stride : nullptr;
-    else pp = u.log_amp;
-    plane_s[k] = pp;
-  }
-  __syncthreads();
-  const int x0 = tl.x0;
-  const int nch = (sny + RC - 1) / RC;
-  auto issue_rows = [&](int c) {
-    if (NARROW && c < nch) {
-      float* dst = ring + (c % kFwdStages) * STAGE;
-      for (int k = tid; k < STAGE; k += 256) {
-        const int pl = k / (RC * 128), r = (k / 128) % RC, xx = x0 + (k & 127), y = c * RC + r;
-        const float* base = plane_s[pl];
-        const bool ok = base != nullptr && y < sny && xx < snx;
-        cp_async4(dst + k, ok ? base + (size_t)y * snx + xx : (const float*)u.g, ok ? 4 : 0);
-      }
-    } else if (c < nch) {
-      float* dst = ring + (c % kFwdStages) * STAGE;
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) {
-        const int k = tid + 256 * i;
-        if (PIECES % 256 == 0 || k < PIECES) {
-          const int pl = k / (RC * 32), rem = k % (RC * 32);
-          const int r = rem >> 5, c4 = (rem & 31) * 4;
-          // absent planes (no static phase, no distortion, compartments past ncomp) and rows
-          // or columns past the plane zero-fill: the row loop reads every plane unconditionally
-          const float* base = plane_s[pl];
-          const int y = c * RC + r, xx = x0 + c4;
-          const bool ok = base != nullptr && y < sny && xx < snx;
-          cp_async16(dst + (pl * RC + r) * 128 + c4, ok ? base + (size_t)y * snx + xx : (const float*)u.g, ok ? 16 : 0);
-        }
-      }
-    }
-    cp_async_commit();
-  };
-#pragma unroll
-  for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(c);
-
-  const int nl = min(TL, u.n_lines - tl.line0);
-  const int ys = u.ny / 2;
-  const int oy = sny / u.ny;
-  const int sys = oy * ys;
-  for (int idx = tid; idx < sny * TL; idx += 256) {
-    const int y = idx / TL, j = idx % TL;
-    float v = 0.f;
-    if (j < nl) {
-      const LineRec& L = u.lines[tl.line0 + j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
-      if (u.flags & UF_EDDY) {
-        const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
-        tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
-      }
-      tv -= rint(tv);
-      v = (float)tv;
-    }
-    Bt[idx] = v;
-  }
-  for (int idx = tid; idx < QGP * sny; idx += 256) {
-    const int y = idx / QGP, qq = idx % QGP;
-    if (NV) {
-      const int nc = u.geo.ncls;
-      Ey[idx] = qq < nc ? u.geo.eyc[(size_t)qq * sny + y] : (qq == nc ? 1.f : 0.f);
-    } else {
-      const int q = tl.q0 + qq;
-      Ey[idx] = (qq < QG && q < u.ncoils) ? u.geo.ey[(size_t)q * sny + y] : 0.f;
-    }
-  }
-  if (tid < TL) {
-    const int j = tid;
-    if (j < nl) {
-      const LineRec& L = u.lines[tl.line0 + j];
-      thi_s[j] = L.t_hi;
-      tlo_s[j] = L.t_lo;
-      tinh_s[j] = L.inhom_ms;
-      trf_s[j] = L.trf_ms;
-      for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = c < ncomp ? L.rel[c] : 0.f;
-    } else {
-      thi_s[j] = tlo_s[j] = tinh_s[j] = trf_s[j] = 0.f;
-      for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = 0.f;
-    }
-  }
-  __syncthreads();
-
-  const int col = tid & 127, lg = tid >> 7;
-  const int jb = lg * T;
-  const int x = x0 + col;
-  const bool xok = x < snx;
-  const float off = u.geo.coil_off;
-  float exq[NV ? 1 : QG];
-  if (!NV) {
-#pragma unroll
-    for (int qq = 0; qq < QG; ++qq) {
-      const int q = tl.q0 + qq;
-      exq[NV ? 0 : qq] = (xok && q < u.ncoils) ? u.geo.ex[(size_t)q * snx + x] : 0.f;
-    }
-  }
-  float thi[T], tlo[T], relr[T][MAPS ? 1 : NC], trf[MAPS ? T : 1], tinh[MAPS ? T : 1];
-#pragma unroll
-  for (int j = 0; j < T; ++j) {
-    thi[j] = thi_s[jb + j];
-    tlo[j] = tlo_s[jb + j];
-    if (MAPS) {
-      trf[MAPS ? j : 0] = trf_s[jb + j];
-      tinh[MAPS ? j : 0] = tinh_s[jb + j];
-    } else {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) relr[j][MAPS ? 0 : c] = rel_s[jb + j][c];
-    }
-  }
-  const bool has_t2 = MAPS && plane_s[P_T2] != nullptr, has_ti = MAPS && plane_s[P_TI] != nullptr;
-  const bool has_la = MAPS && plane_s[P_LA] != nullptr;
-  float2 acc[T][NA];
-#pragma unroll
-  for (int j = 0; j < T; ++j)
-#pragma unroll
-    for (int qq = 0; qq < NA; ++qq) acc[j][qq] = make_float2(0.f, 0.f);
-
-  for (int c = 0; c < nch; ++c) {
-    cp_async_wait_n<kFwdStages - 2>();
-    __syncthreads();  // rows of chunk c landed; every thread is done with chunk c - 1
-    issue_rows(c + kFwdStages - 1);
-    const float* S = ring + (c % kFwdStages) * STAGE + col;
-    const int rn = min(RC, sny - c * RC);
-    for (int r = 0; r < rn; ++r) {
-      const int y = c * RC + r;
-      const float a = S[(0 * RC + r) * 128];
-      const float f = S[(1 * RC + r) * 128];
-      float m[NC];
-#pragma unroll
-      for (int cc = 0; cc < NC; ++cc) m[cc] = S[((P_COMP + cc) * RC + r) * 128];
-      float r2[MAPS ? NC : 1], r2i[MAPS ? NC : 1];
-      float la = 0.f;
-      if (MAPS) {
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          r2[MAPS ? cc : 0] = r2i[MAPS ? cc : 0] = 0.f;
-          if (cc < ncomp) {
-            const float t2 = has_t2 ? S[((P_T2 + cc) * RC + r) * 128] : u.t2u[cc];
-            const float ti = has_ti ? S[((P_TI + cc) * RC + r) * 128] : u.tiu[cc];
-            r2[MAPS ? cc : 0] = 1.0f / t2;
-            r2i[MAPS ? cc : 0] = 1.0f / ti;
-          }
-        }
-        if (has_la) la = S[(P_LA * RC + r) * 128];
-      }
-      float amp[NA];
-#pragma unroll
-      for (int q4 = 0; q4 < QGP; q4 += 4) {
-        const float4 e4 = *reinterpret_cast<const float4*>(Ey + y * QGP + q4);
-        const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (q4 + k < NA) amp[q4 + k] = NV ? ev[k] : fmaf(exq[NV ? 0 : q4 + k], ev[k], off);
-      }
-      const float4 b4 = *reinterpret_cast<const float4*>(Bt + y * TL + jb);
-      const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
-      if (NV && !MAPS) {
-        // lines (0, 1) and (2, 3) as packed pairs: the same arithmetic, two lanes per instruction
-        const float2 a2 = dup2(a), f2 = dup2(f);
-#pragma unroll
-        for (int jp = 0; jp < T; jp += 2) {
-          float2 th = phase_turns2(fadd2(a2, make_float2(bt[jp], bt[jp + 1])), f2,
-                                   make_float2(thi[jp], thi[jp + 1]), make_float2(tlo[jp], tlo[jp + 1]));
-          th = fmul2(dup2(kTwoPiF), th);
-          float s0, c0, s1, c1;
-          __sincosf(th.x, &s0, &c0);
-          __sincosf(th.y, &s1, &c1);
-          float2 W = fmul2(make_float2(relr[jp][MAPS ? 0 : 0], relr[jp + 1][MAPS ? 0 : 0]), dup2(m[0]));
-#pragma unroll
-          for (int cc = 1; cc < NC; ++cc)
-            W = ffma2(make_float2(relr[jp][MAPS ? 0 : cc], relr[jp + 1][MAPS ? 0 : cc]), dup2(m[cc]), W);
-          const float2 w0 = fmul2(dup2(W.x), make_float2(c0, s0)), w1 = fmul2(dup2(W.y), make_float2(c1, s1));
-#pragma unroll
-          for (int qq = 0; qq < NA - 1; ++qq) {
-            acc[jp][qq] = ffma2(dup2(amp[qq]), w0, acc[jp][qq]);
-            acc[jp + 1][qq] = ffma2(dup2(amp[qq]), w1, acc[jp + 1][qq]);
-          }
-          acc[jp][NA - 1] = fadd2(acc[jp][NA - 1], w0);
-          acc[jp + 1][NA - 1] = fadd2(acc[jp + 1][NA - 1], w1);
-        }
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < T; ++j) {
-        const float th = phase_turns(a + bt[j], f, thi[j], tlo[j]);
-        float sn, cs;
-        __sincosf(kTwoPiF * th, &sn, &cs);
-        float W = 0.f;
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          if (!MAPS || cc < ncomp) {  // class decay: rel and m are 0 past ncomp
-            float rr;
-            if (MAPS)
-              rr = __expf(la - trf[MAPS ? j : 0] * r2[MAPS ? cc : 0] - tinh[MAPS ? j : 0] * r2i[MAPS ? cc : 0]);
-            else
-              rr = relr[j][MAPS ? 0 : cc];
-            W = fmaf(rr, m[cc], W);
-          }
-        }
-        const float wr = W * cs, wi = W * sn;
-#pragma unroll
-        for (int qq = 0; qq < NA; ++qq) {
-          if (NV && qq == NA - 1) {  // the coil-offset row is all ones
-            acc[j][qq].x += wr;
-            acc[j][qq].y += wi;
-          } else if (NV) {
-            acc[j][qq] = ffma2(make_float2(amp[qq], amp[qq]), make_float2(wr, wi), acc[j][qq]);
-          } else {
-            acc[j][qq].x = fmaf(amp[qq], wr, acc[j][qq].x);
-            acc[j][qq].y = fmaf(amp[qq], wi, acc[j][qq].y);
-          }
-        }
-      }
-    }
-  }
-  cp_async_wait0();
-  if (!xok) return;
-  const float s = u.signal_scale;
-  if (NV && cls_rows) {
-#pragma unroll
-    for (int j = 0; j < T; ++j) {
-      if (jb + j >= nl) break;
-#pragma unroll
-      for (int v = 0; v < NA; ++v) {
-        const float sv = v == NA - 1 && cls_rows == 1 ? s * off : s;
-        u.g[((size_t)v * u.n_lines + tl.line0 + jb + j) * snx + x] = make_float2(sv * acc[j][v].x, sv * acc[j][v].y);
-      }
-    }
-    return;
-  }
-  if (NV) {
-    // expand the classes to the unit's coils (all in this tile)
-    for (int q = 0; q < u.ncoils; ++q) {
-      const int cl = u.geo.cls[q];
-      const float e = s * u.geo.ex[(size_t)q * snx + x], o = s * off;
-#pragma unroll
-      for (int j = 0; j < T; ++j) {
-        float2 v = acc[j][0];
-#pragma unroll
-        for (int k = 1; k < NA - 1; ++k)
-          if (cl == k) v = acc[j][k];
-        if (jb + j < nl)
-          u.g[((size_t)q * u.n_lines + tl.line0 + jb + j) * snx + x] =
-              make_float2(fmaf(e, v.x, o * acc[j][NA - 1].x), fmaf(e, v.y, o * acc[j][NA - 1].y));
-      }
-    }
-    return;
-  }
-#pragma unroll
-  for (int qq = 0; qq < QG; ++qq) {
-    const int q = tl.q0 + qq;
-    if (q >= u.ncoils) break;
-#pragma unroll
-    for (int j = 0; j < T; ++j) {
-      if (jb + j < nl)
-        u.g[((size_t)q * u.n_lines + tl.line0 + jb + j) * snx + x] = make_float2(acc[j][qq].x * s, acc[j][qq].y * s);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// y-adjoint: per voxel, over every line j and coil q:
-//   H_j = s * sum_q (ex_q ey_q + off) h_q[j][x];   Z_j = conj(e^{i2pi theta_j}) H_j
-//   comp_grad_c = sum_j rel_cj Z_j                          (A^H r, complex)
-//   fmap_grad   = 4 pi sum_c m_c Im(sum_j t_j rel_cj Z_j)   (dL/dfmap, L = sum |r|^2)
-//   r2_grad_c   = -2 m_c Re(sum_j trf_j rel_cj Z_j)         (dL/dR2_c)
-// A CTA of 128 threads covers 128 columns x TY rows (one column each).  The line table sits in
-// shared memory; h arrives by cp.async in double-buffered chunks of JC lines x every coil.
-// The number of lines per h chunk for `ncoils` coils (16 coil-lines per chunk, at least one line).
-__host__ __device__ __forceinline__ int adjoint_chunk_lines(int ncoils) { return ncoils >= 16 ? 1 : 16 / ncoils; }
-
-template <int TY, int NC, bool MAPS, bool GRADS>
-__global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restrict__ units,
-                                                       const int4* __restrict__ tiles) {
-  extern __shared__ __align__(16) float smem[];
-  static_assert(TY == 4, "the row tables are read as float4");
-  constexpr int ROWS = TY;
-  const int4 tl = tiles[blockIdx.x];  // unit, y0, x0
-  const UnitDesc& u = units[tl.x];
-  const int snx = u.snx, sny = u.sny, ncomp = u.ncomp, nlines = u.n_lines, ncoils = u.ncoils;
-  const int y0 = tl.y;
-  const int JC = adjoint_chunk_lines(ncoils);
-  // shared layout: h buffers (2 x JC x ncoils x 128 float2), then floats
-  float2* hbuf = reinterpret_cast<float2*>(smem);
-  float* Bt = reinterpret_cast<float*>(hbuf + 2 * JC * ncoils * 128);  // [nlines][ROWS]
-  float* Ey = Bt + nlines * ROWS;                                        // [ncoils][ROWS]
-  float* Ex = Ey + ncoils * ROWS;                                        // [ncoils][128], scale folded
-  float* Lt = Ex + ncoils * 128;                                         // [nlines][LF] line table
-  constexpr int LF = 5 + NC;  // t_hi, t_lo, trf, inhom, t_phase, rel[NC]
-  const int ys = u.ny / 2;
-  const int oy = sny / u.ny;
-  const int sys = oy * ys;
-  const int col = threadIdx.x;
-  const int x = tl.z + col;
-  const bool xok = x < snx;
-  const float2* __restrict__ hcol = u.g + (xok ? x : 0);
-  const size_t qstride = (size_t)nlines * snx;
-  // the first h chunk is in flight while the tables fill
-  auto issue_chunk = [&](int c, int buf) {
-    const int j0 = c * JC;
-    for (int jj = 0; jj < JC; ++jj) {
-      const int j = j0 + jj;
-      if (j >= nlines) break;
-      for (int q = 0; q < ncoils; ++q)
-        cp_async8(hbuf + ((size_t)(buf * JC + jj) * ncoils + q) * 128 + col, hcol + q * qstride + (size_t)j * snx);
-    }
-    cp_async_commit();
-  };
-  const int nchunks = (nlines + JC - 1) / JC;
-  if (nchunks > 0) issue_chunk(0, 0);
-  for (int idx = threadIdx.x; idx < nlines * ROWS; idx += blockDim.x) {
-    const int j = idx / ROWS, r = idx % ROWS;
-    const int y = y0 + r;
-    float v = 0.f;
-    if (y < sny) {
-      const LineRec& L = u.lines[j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
-      if (u.flags & UF_EDDY) {
-        const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
-        tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
-      }
-      tv -= rint(tv);
-      v = (float)tv;
-    }
-    Bt[idx] = v;
-  }
-  for (int idx = threadIdx.x; idx < ncoils * ROWS; idx += blockDim.x) {
-    const int q = idx / ROWS, r = idx % ROWS;
-    const int y = y0 + r;
-    Ey[idx] = y < sny ? u.geo.ey[(size_t)q * sny + y] : 0.f;
-  }
-  for (int idx = threadIdx.x; idx < ncoils * 128; idx += blockDim.x) {
-    const int q = idx / 128, c = idx % 128;
-    const int xx = tl.z + c;
-    Ex[idx] = xx < snx ? u.signal_scale * u.geo.ex[(size_t)q * snx + xx] : 0.f;
-  }
-  for (int j = threadIdx.x; j < nlines; j += blockDim.x) {
-    const LineRec& L = u.lines[j];
-    float* e = Lt + j * LF;
-    e[0] = L.t_hi;
-    e[1] = L.t_lo;
-    e[2] = L.trf_ms;
-    e[3] = L.inhom_ms;
-    e[4] = L.t_hi + L.t_lo;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) e[5 + c] = L.rel[c];
-  }
-  __syncthreads();
-  const bool active = xok && y0 < sny;
-  const bool distort = (u.flags & UF_DISTORT) != 0;
-  float a[TY], f[TY], r2[TY][MAPS ? NC : 1], r2i[TY][MAPS ? NC : 1], la[TY];
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty) {
-    const int y = min(y0 + ty, sny - 1);
-    const int i = (xok ? x : 0) + snx * y;
-    a[ty] = u.phase ? __ldg(u.phase + i) : 0.f;
-    f[ty] = distort ? __ldg(u.fmap + i) : 0.f;
-    la[ty] = (MAPS && u.log_amp) ? __ldg(u.log_amp + i) : 0.f;
-    if (MAPS) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        r2[ty][MAPS ? c : 0] = r2i[ty][MAPS ? c : 0] = 0.f;
-        if (c < ncomp) {
-          const float t2 = u.t2map ? __ldg(u.t2map + (size_t)c * u.map_stride + i) : u.t2u[c];
-          const float ti = u.timap ? __ldg(u.timap + (size_t)c * u.map_stride + i) : u.tiu[c];
-          r2[ty][MAPS ? c : 0] = 1.0f / t2;
-          r2i[ty][MAPS ? c : 0] = 1.0f / ti;
-        }
-      }
-    }
-  }
-  float2 cg[TY][NC];
-  float Uy[TY][GRADS ? NC : 1], Vx[TY][GRADS ? NC : 1];
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      cg[ty][c] = make_float2(0.f, 0.f);
-      if (GRADS) Uy[ty][GRADS ? c : 0] = Vx[ty][GRADS ? c : 0] = 0.f;
-    }
-  const float soff = u.signal_scale * u.geo.coil_off;
-  for (int c = 0; c < nchunks; ++c) {
-    const int buf = c & 1;
-    if (c + 1 < nchunks) {
-      issue_chunk(c + 1, buf ^ 1);
-      cp_async_wait1();
-    } else {
-      cp_async_wait0();
-    }
-    // each thread reads back only its own column, which it copied itself: no barrier needed
-    const int j0 = c * JC;
-    const int jn = min(JC, nlines - j0);
-    for (int jj = 0; jj < jn; ++jj) {
-      const int j = j0 + jj;
-      const float* e = Lt + j * LF;
-      const float thi = e[0], tlo = e[1], trf = e[2], tinh = e[3], tph = e[4];
-      // (Re, Im) pairs in packed f32x2 arithmetic: each lane rounds as the scalar product, sum and
-      // fused multiply-add do, so the sums are bitwise the scalar ones in half the issue slots
-      float2 H[TY];
-      float2 hs = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int ty = 0; ty < TY; ++ty) H[ty] = make_float2(0.f, 0.f);
-      const float2* hb = hbuf + (size_t)(buf * JC + jj) * ncoils * 128 + col;
-#pragma unroll 4
-      for (int q = 0; q < ncoils; ++q) {
-        const float2 h = hb[q * 128];
-        const float ex = Ex[q * 128 + col];
-        hs = fadd2(hs, h);
-        const float2 uu = fmul2(dup2(ex), h);
-        const float4 e4 = *reinterpret_cast<const float4*>(Ey + q * ROWS);
-        const float ey[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int ty = 0; ty < TY; ++ty) H[ty] = ffma2(dup2(ey[ty]), uu, H[ty]);
-      }
-      const float hsr = hs.x, hsi = hs.y;
-      const float4 b4 = *reinterpret_cast<const float4*>(Bt + j * ROWS);
-      const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-      for (int ty = 0; ty < TY; ++ty) {
-        const float hr = fmaf(soff, hsr, H[ty].x), hi = fmaf(soff, hsi, H[ty].y);
-        const float th = phase_turns(a[ty] + bt[ty], f[ty], thi, tlo);
-        float sn, cs;
-        __sincosf(kTwoPiF * th, &sn, &cs);
-        const float zr = fmaf(cs, hr, sn * hi);  // Z = conj(P) * H
-        const float zi = fmaf(cs, hi, -sn * hr);
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          if (cc < ncomp) {
-            float r;
-            if (MAPS)
-              r = __expf(la[ty] - trf * r2[ty][MAPS ? cc : 0] - tinh * r2i[ty][MAPS ? cc : 0]);
-            else
-              r = e[5 + cc];
-            cg[ty][cc].x = fmaf(r, zr, cg[ty][cc].x);
-            cg[ty][cc].y = fmaf(r, zi, cg[ty][cc].y);
-            if (GRADS) {
-              Uy[ty][GRADS ? cc : 0] = fmaf(r * tph, zi, Uy[ty][GRADS ? cc : 0]);
-              Vx[ty][GRADS ? cc : 0] = fmaf(r * trf, zr, Vx[ty][GRADS ? cc : 0]);
-            }
-          }
-        }
-      }
-    }
-  }
-  if (!active) return;
-  const size_t plane = (size_t)snx * sny;
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty) {
-    const int y = y0 + ty;
-    if (y >= sny) break;
-    const size_t i = (size_t)x + (size_t)snx * y;
-    float fg = 0.f;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (c >= ncomp) break;
-      u.comp_grad[c * plane + i] = cg[ty][c];
-      if (GRADS) {
-        const float m = __ldg(u.comp + (size_t)c * u.comp_stride + i);
-        fg = fmaf(m, Uy[ty][GRADS ? c : 0], fg);
-        if (u.r2_grad) u.r2_grad[c * plane + i] = -2.0f * m * Vx[ty][GRADS ? c : 0];
-      }
-    }
-    if (GRADS && u.fmap_grad) u.fmap_grad[i] = distort ? 4.0f * 3.14159265358979f * fg : 0.f;
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// y-adjoint for a compile-time coil count NQ (every unit of the plan has NQ coils, an even snx and
-// 16-byte aligned h rows).  Same sums as yadjoint_kernel, reorganised so the per-(line, voxel)
-// work is the coil combination and the phase:
-//   * a CTA of 256 threads covers 128 columns x 2*TY rows (two groups of TY rows, one column each;
-//     TY = 4 with class decay, 2 with voxel maps, whose rates take the registers);
-//   * amp_q(x, y) = s * (ex_q(x) ey_q(y) + off) of the thread's TY rows sits in registers, so the
-//     coil combination is 2 FMAs per (coil, row) from one shared load of h per coil;
-//   * h arrives through a 3-stage ring of JC-line chunks (every coil, 128 columns) filled by
-//     cooperative 16-byte cp.async, one barrier per chunk;
-//   * the line table carries rel_cj, rel_cj * t_j and rel_cj * trf_j (class decay), so every
-//     accumulator update is one FMA.
-constexpr int kAdjStages = 3;
-__host__ __device__ __forceinline__ constexpr int adjq_chunk_lines(int nq) { return nq >= 16 ? 1 : 16 / nq; }
-__host__ __device__ __forceinline__ constexpr int adjq_line_floats(int nc, bool maps) {
-  return ((maps ? 5 : 4 + 3 * nc) + 3) / 4 * 4;
-}
-// rows per thread: 4 with class decay and up to 3 compartments, else 2 (registers)
-__host__ __device__ __forceinline__ constexpr int adjq_rows(int nc, bool maps) { return !maps && nc <= 3 ? 4 : 2; }
-// ... the same with coil-class rows (two rows per thread in 80 registers and three CTAs per SM
-// measured 30 % slower than four rows: the per-line loads then serve half the rows)
-__host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps, bool virt) {
-  return adjq_rows(nc, maps);
-}
-
-
-// VIRT: the h rows are the NQ = classes + 1 class rows of the class-mode x-adjoint (scale, ex and
-// the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
-// or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
-// NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
-template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW>
-__global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
-                                                            const int4* __restrict__ tiles) {
-  extern __shared__ __align__(16) float smem[];
-  static_assert(TY == 2 || TY == 4, "the row phases are read as one float2 / float4");
-  constexpr int ROWS = 2 * TY;
-  constexpr int JC = adjq_chunk_lines(NQ);
-  constexpr int LF = adjq_line_floats(NC, MAPS);
-  constexpr int STAGE = JC * NQ * 128;        // float2 per stage
-  constexpr int PIECES = JC * NQ * 64;        // 16-byte pieces per stage
-  constexpr int PPT = (PIECES + 255) / 256;   // pieces per thread
-  const int4 tl = tiles[blockIdx.x];          // unit, y0, x0
-  const UnitDesc& u = units[tl.x];
-  const int snx = u.snx, sny = u.sny, ncomp = u.ncomp, nlines = u.n_lines;
-  const int y0 = tl.y, x0 = tl.z;
-  float2* hbuf = reinterpret_cast<float2*>(smem);
-  float* Bt = reinterpret_cast<float*>(hbuf + kAdjStages * STAGE);  // [nlines][ROWS]
-  // the line tables cover whole chunks (zero entries past nlines), so the packed path runs every
-  // line of a chunk without a branch
-  const int nlp = (nlines + JC - 1) / JC * JC;
-  float* Lt = Bt + nlp * ROWS;                                       // [nlp][LF]
-  const int tid = threadIdx.x;
-  const int col = tid & 127, rg = tid >> 7;
-  const int x = x0 + col;
-  const bool xok = x < snx;
-  const int nchunks = (nlines + JC - 1) / JC;
-
-  // This thread's 16-byte pieces k = tid + 256 i of a chunk: row r = k / 64 = (line jj, coil q),
-  // column pair 2 (k % 64); the destination is float2 2k of the stage.  The source offset of
-  // each piece for the chunk's first line (or -1 past snx) sits in a per-thread shared table, so
-  // a chunk costs one shared load, a compare and a select per piece.  (The plan keeps
-  // NQ * lines * snx below 2^31.)
-  __shared__ int ptab[PPT * 256];
-  const float2* __restrict__ gsrc = u.g;
-#pragma unroll
-  for (int i = 0; i < PPT; ++i) {
-    const int k = tid + 256 * i;
-    if (PIECES % 256 == 0 || k < PIECES) {
-      const int r = k >> 6, xx = x0 + (k & 63) * 2;
-      ptab[i * 256 + tid] = xx < snx ? ((r % NQ) * nlines + r / NQ) * snx + xx : -1;
-    }
-  }
-  auto issue_chunk = [&](int c, int stage) {
-    if (NARROW && c < nchunks) {
-      float2* dst = hbuf + stage * STAGE;
-      for (int k = tid; k < STAGE; k += 256) {
-        const int r = k >> 7, xx = x0 + (k & 127), j = c * JC + r / NQ;
-        const bool ok = xx < snx && j < nlines;
-        cp_async8(dst + k, gsrc + (ok ? ((size_t)(r % NQ) * nlines + j) * snx + xx : 0), ok ? 8 : 0);
-      }
-    } else if (c < nchunks) {
-      const int rem = nlines - c * JC, jo = c * JC * snx;
-      float2* dst = hbuf + stage * STAGE;
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) {
-        const int k = tid + 256 * i;
-        if (PIECES % 256 == 0 || k < PIECES) {
-          const int o = ptab[i * 256 + tid];
-          const bool ok = o >= 0 && ((tid >> 6) + 4 * i) / NQ < rem;
-          cp_async16(dst + 2 * k, gsrc + (ok ? o + jo : 0), ok ? 16 : 0);
-        }
-      }
-    }
-    cp_async_commit();
-  };
-#pragma unroll
-  for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(c, c);
-
-  const int ys = u.ny / 2;
-  const int oy = sny / u.ny;
-  const int sys = oy * ys;
-  for (int idx = tid; idx < nlp * ROWS; idx += 256) {
-    const int j = idx / ROWS, r = idx % ROWS;
-    const int y = y0 + r;
-    float v = 0.f;
-    if (y < sny && j < nlines) {
-      const LineRec& L = u.lines[j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
-      if (u.flags & UF_EDDY) {
-        const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
-        tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
-      }
-      tv -= rint(tv);
-      v = (float)tv;
-    }
-    Bt[idx] = v;
-  }
-  for (int j = tid; j < nlp; j += 256) {
-    float* e = Lt + j * LF;
-    if (j >= nlines) {
-#pragma unroll
-      for (int k = 0; k < LF; ++k) e[k] = 0.f;
-      continue;
-    }
-    const LineRec& L = u.lines[j];
-    const float tph = L.t_hi + L.t_lo;
-    e[0] = L.t_hi;
-    e[1] = L.t_lo;
-    e[2] = L.trf_ms;
-    e[3] = L.inhom_ms;
-    if (MAPS) {
-      e[4] = tph;
-    } else {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {  // zero weights past ncomp: those accumulators stay 0
-        const float r = c < ncomp ? L.rel[c] : 0.f;
-        e[4 + c] = r;
-        e[4 + NC + c] = r * tph;
-        e[4 + 2 * NC + c] = r * L.trf_ms;
-      }
-    }
-  }
-
-  // per-thread constants of its 4 rows
-  const bool distort = (u.flags & UF_DISTORT) != 0;
-  const int xs_ = xok ? x : 0;
-  const float s = u.signal_scale, off = u.geo.coil_off;
-  float amp[TY][NQ];
-  float a[TY], f[TY];
-  float r2[TY][MAPS ? NC : 1], r2i[TY][MAPS ? NC : 1], la[TY];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const float ex = VIRT ? 0.f : u.geo.ex[(size_t)q * snx + xs_];
-#pragma unroll
-    for (int ty = 0; ty < TY; ++ty) {
-      const int y = min(y0 + rg * TY + ty, sny - 1);
-      if (VIRT)
-        amp[ty][q] = q < NQ - 1 ? u.geo.eyc[(size_t)q * sny + y] : 1.f;
-      else
-        amp[ty][q] = s * fmaf(ex, u.geo.ey[(size_t)q * sny + y], off);
-    }
-  }
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty) {
-    const int y = min(y0 + rg * TY + ty, sny - 1);
-    const int i = xs_ + snx * y;
-    a[ty] = u.phase ? __ldg(u.phase + i) : 0.f;
-    f[ty] = distort ? __ldg(u.fmap + i) : 0.f;
-    la[ty] = (MAPS && u.log_amp) ? __ldg(u.log_amp + i) : 0.f;
-    if (MAPS) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        r2[ty][MAPS ? c : 0] = r2i[ty][MAPS ? c : 0] = 0.f;
-        if (c < ncomp) {
-          const float t2 = u.t2map ? __ldg(u.t2map + (size_t)c * u.map_stride + i) : u.t2u[c];
-          const float ti = u.timap ? __ldg(u.timap + (size_t)c * u.map_stride + i) : u.tiu[c];
-          r2[ty][MAPS ? c : 0] = 1.0f / t2;
-          r2i[ty][MAPS ? c : 0] = 1.0f / ti;
-        }
-      }
-    }
-  }
-  // PK (class rows, class decay, 4 rows): rows (0, 1) and (2, 3) run as packed f32x2 pairs, with
-  // accumulators pcx/pcy/puy/pvx[pair][c] holding the two rows' Re/Im comp sums, t- and trf-sums
-  constexpr bool PK = VIRT && !MAPS;
-  constexpr int NPR = PK ? TY / 2 : 1;  // row pairs
-  float2 pcx[NPR][NC], pcy[NPR][NC], puy[NPR][NC], pvx[NPR][NC];
-  if (PK) {
-#pragma unroll
-    for (int pp = 0; pp < NPR; ++pp)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) pcx[pp][c] = pcy[pp][c] = puy[pp][c] = pvx[pp][c] = make_float2(0.f, 0.f);
-  }
-  float2 cg[TY][NC];
-  float Uy[TY][GRADS ? NC : 1], Vx[TY][GRADS ? NC : 1];
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      cg[ty][c] = make_float2(0.f, 0.f);
-      if (GRADS) Uy[ty][GRADS ? c : 0] = Vx[ty][GRADS ? c : 0] = 0.f;
-    }
-
-  int s_use = 0, s_issue = kAdjStages - 1;  // stages of chunk c and of chunk c + stages - 1
-  for (int c = 0; c < nchunks; ++c) {
-    cp_async_wait_n<kAdjStages - 2>();
-    __syncthreads();  // chunk c landed for every thread; every thread is done with chunk c - 1
-    issue_chunk(c + kAdjStages - 1, s_issue);
-    s_issue = s_issue + 1 == kAdjStages ? 0 : s_issue + 1;
-    const float2* hs = hbuf + s_use * STAGE + col;
-    s_use = s_use + 1 == kAdjStages ? 0 : s_use + 1;
-    const int j0 = c * JC;
-#pragma unroll
-    for (int jj = 0; jj < JC; ++jj) {
-      const int j = j0 + jj;
-      if (!PK && j >= nlines) break;  // (the packed path reads the zero entries instead)
-      const float* e = Lt + j * LF;
-      const float4 e0 = *reinterpret_cast<const float4*>(e);
-      const float thi = e0.x, tlo = e0.y, trf = e0.z, tinh = e0.w;
-      if (PK) {
-        float2 Hx[NPR], Hy[NPR];  // [pair] = rows (2p, 2p + 1); starts from the offset row (amplitude 1)
-        {
-          const float2 h = hs[(jj * NQ + NQ - 1) * 128];
-#pragma unroll
-          for (int pp = 0; pp < NPR; ++pp) {
-            Hx[pp] = dup2(h.x);
-            Hy[pp] = dup2(h.y);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NQ - 1; ++q) {
-          const float2 h = hs[(jj * NQ + q) * 128];
-          const float2 hx = dup2(h.x), hy = dup2(h.y);
-#pragma unroll
-          for (int pp = 0; pp < NPR; ++pp) {
-            const float2 am = make_float2(amp[2 * pp][q], amp[(2 * pp + 1) % TY][q]);
-            Hx[pp] = ffma2(am, hx, Hx[pp]);
-            Hy[pp] = ffma2(am, hy, Hy[pp]);
-          }
-        }
-        float2 btp[NPR];
-        if (TY == 4) {
-          const float4 b4 = *reinterpret_cast<const float4*>(Bt + j * ROWS + rg * TY);
-          btp[0] = make_float2(b4.x, b4.y);
-          btp[NPR - 1] = make_float2(b4.z, b4.w);
-        } else {
-          btp[0] = *reinterpret_cast<const float2*>(Bt + j * ROWS + rg * TY);
-        }
-        const float2 thi2 = dup2(thi), tlo2 = dup2(tlo);
-#pragma unroll
-        for (int pp = 0; pp < NPR; ++pp) {
-          const int t0 = 2 * pp, t1 = (2 * pp + 1) % TY;
-          const float2 bt2 = btp[pp];
-          float2 th = phase_turns2(fadd2(make_float2(a[t0], a[t1]), bt2), make_float2(f[t0], f[t1]), thi2, tlo2);
-          th = fmul2(dup2(kTwoPiF), th);
-          float s0, c0, s1, c1;
-          __sincosf(th.x, &s0, &c0);
-          __sincosf(th.y, &s1, &c1);
-          const float2 cs2 = make_float2(c0, c1), sn2 = make_float2(s0, s1);
-          const float2 zr = ffma2(cs2, Hx[pp], fmul2(sn2, Hy[pp]));  // Z = conj(P) H per row
-          const float2 zi = ffma2(cs2, Hy[pp], fsub2(dup2(0.f), fmul2(sn2, Hx[pp])));
-#pragma unroll
-          for (int cc = 0; cc < NC; ++cc) {
-            const float2 r = dup2(e[4 + cc]);
-            pcx[PK ? pp : 0][cc] = ffma2(r, zr, pcx[PK ? pp : 0][cc]);
-            pcy[PK ? pp : 0][cc] = ffma2(r, zi, pcy[PK ? pp : 0][cc]);
-            if (GRADS) {
-              puy[PK ? pp : 0][cc] = ffma2(dup2(e[4 + NC + cc]), zi, puy[PK ? pp : 0][cc]);
-              pvx[PK ? pp : 0][cc] = ffma2(dup2(e[4 + 2 * NC + cc]), zr, pvx[PK ? pp : 0][cc]);
-            }
-          }
-        }
-        continue;
-      }
-      float2 H[TY];
-      {
-        const float2 h = hs[jj * NQ * 128];
-#pragma unroll
-        for (int ty = 0; ty < TY; ++ty) H[ty] = make_float2(amp[ty][0] * h.x, amp[ty][0] * h.y);
-      }
-#pragma unroll
-      for (int q = 1; q < NQ; ++q) {
-        const float2 h = hs[(jj * NQ + q) * 128];
-#pragma unroll
-        for (int ty = 0; ty < TY; ++ty) {
-          H[ty].x = fmaf(amp[ty][q], h.x, H[ty].x);
-          H[ty].y = fmaf(amp[ty][q], h.y, H[ty].y);
-        }
-      }
-      float bt[TY];
-      if (TY == 4) {
-        const float4 b4 = *reinterpret_cast<const float4*>(Bt + j * ROWS + rg * TY);
-        bt[0] = b4.x, bt[1] = b4.y, bt[TY > 2 ? 2 : 0] = b4.z, bt[TY > 3 ? 3 : 0] = b4.w;
-      } else {
-        const float2 b2 = *reinterpret_cast<const float2*>(Bt + j * ROWS + rg * TY);
-        bt[0] = b2.x, bt[1] = b2.y;
-      }
-      const float tph = MAPS ? e[4] : 0.f;
-#pragma unroll
-      for (int ty = 0; ty < TY; ++ty) {
-        const float th = phase_turns(a[ty] + bt[ty], f[ty], thi, tlo);
-        float sn, cs;
-        __sincosf(kTwoPiF * th, &sn, &cs);
-        const float zr = fmaf(cs, H[ty].x, sn * H[ty].y);  // Z = conj(P) * H
-        const float zi = fmaf(cs, H[ty].y, -sn * H[ty].x);
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          if (!MAPS || cc < ncomp) {
-            float r, rt, rf;
-            if (MAPS) {
-              r = __expf(la[ty] - trf * r2[ty][MAPS ? cc : 0] - tinh * r2i[ty][MAPS ? cc : 0]);
-              rt = r * tph;
-              rf = r * trf;
-            } else {
-              r = e[4 + cc];
-              rt = e[4 + NC + cc];
-              rf = e[4 + 2 * NC + cc];
-            }
-            cg[ty][cc].x = fmaf(r, zr, cg[ty][cc].x);
-            cg[ty][cc].y = fmaf(r, zi, cg[ty][cc].y);
-            if (GRADS) {
-              Uy[ty][GRADS ? cc : 0] = fmaf(rt, zi, Uy[ty][GRADS ? cc : 0]);
-              Vx[ty][GRADS ? cc : 0] = fmaf(rf, zr, Vx[ty][GRADS ? cc : 0]);
-            }
-          }
-        }
-      }
-    }
-  }
-  cp_async_wait0();
-  if (!xok) return;
-  if (PK) {
-#pragma unroll
-    for (int ty = 0; ty < TY; ++ty)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const int pp = PK ? (ty >> 1) % NPR : 0;
-        const bool hi = ty & 1;
-        cg[ty][c] = make_float2(hi ? pcx[pp][c].y : pcx[pp][c].x, hi ? pcy[pp][c].y : pcy[pp][c].x);
-        if (GRADS) {
-          Uy[ty][GRADS ? c : 0] = hi ? puy[pp][c].y : puy[pp][c].x;
-          Vx[ty][GRADS ? c : 0] = hi ? pvx[pp][c].y : pvx[pp][c].x;
-        }
-      }
-  }
-  const size_t plane = (size_t)snx * sny;
-#pragma unroll
-  for (int ty = 0; ty < TY; ++ty) {
-    const int y = y0 + rg * TY + ty;
-    if (y >= sny) break;
-    const size_t i = (size_t)x + (size_t)snx * y;
-    float fg = 0.f;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (c >= ncomp) break;
-      u.comp_grad[c * plane + i] = cg[ty][c];
-      if (GRADS) {
-        const float m = __ldg(u.comp + (size_t)c * u.comp_stride + i);
-        fg = fmaf(m, Uy[ty][GRADS ? c : 0], fg);
-        if (u.r2_grad) u.r2_grad[c * plane + i] = -2.0f * m * Vx[ty][GRADS ? c : 0];
-      }
-    }
-    if (GRADS && u.fmap_grad) u.fmap_grad[i] = distort ? 4.0f * 3.14159265358979f * fg : 0.f;
   }
 }
 
@@ -2030,18 +860,6 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
   }
 }
 
-template <class K>
-void set_smem(K kernel, size_t bytes) {
-  // past 48 KB of static + dynamic shared memory the launch needs the dynamic opt-in
-  // (the whole limit, so that threads launching one kernel with different sizes never lower it
-  // between another's opt-in and launch)
-  cudaFuncAttributes fa;
-  MRSIM_CUDA(cudaFuncGetAttributes(&fa, kernel));
-  if (bytes + fa.sharedSizeBytes > 48 * 1024)
-    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024 - (int)fa.sharedSizeBytes));
-}
-
 }  // namespace
 
 // ---- plans and launchers ----------------------------------------------------------------------
@@ -2070,11 +888,6 @@ void append_xtiles(std::vector<XTile>& out, const UnitDesc& u, int unit_index, c
         }
   }
 }
-
-namespace {
-constexpr int kT = 4;
-constexpr int kTY = 4;
-}  // namespace
 
 EpiPlan::~EpiPlan() {
   for (void* p : allocs) {
@@ -2392,19 +1205,6 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
   return p;
 }
 
-namespace {
-// The tiles of units [u0, u1) in a list with per-unit starts `start` (empty: the whole list).
-struct TileRange {
-  int t0, n;
-};
-TileRange tile_range(const std::vector<int>& start, int n_tiles, int u0, int u1) {
-  if (start.empty() || (u0 == 0 && (u1 < 0 || u1 == (int)start.size() - 1))) return {0, n_tiles};
-  if (u1 < 0) u1 = (int)start.size() - 1;
-  if (u0 < 0 || u0 > u1 || u1 >= (int)start.size()) fail("unit range outside the plan");
-  return {start[u0], start[u1] - start[u0]};
-}
-}  // namespace
-
 void epi_plan_statics(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
   if (u1 < 0) u1 = p->n_statics;
   if (u0 < 0 || u0 > u1 || u1 > p->n_statics) fail("unit range outside the plan");
@@ -2422,69 +1222,6 @@ void epi_plan_forward(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
 void epi_plan_adjoint(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
   epi_plan_adjoint_xstage(p, st, u0, u1);
   epi_plan_adjoint_ystage(p, st, u0, u1);
-}
-
-void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
-  for (int pass = 0; pass < 2; ++pass) {
-    const TileRange R = tile_range(p->y_start[pass], p->n_ytiles[pass], u0, u1);
-    if (R.n == 0) continue;
-    const Tile* tiles = (const Tile*)p->d_ytiles[pass] + R.t0;
-    const bool maps = pass == 1;
-    const int QG = p->qg, NCv = p->nc;
-    if (p->fwdq[pass]) {
-      const size_t smq = sizeof(float) * ((size_t)kFwdStages * fwdq_planes(NCv, maps) * fwdq_rows(NCv, maps) * 128 +
-                                          (size_t)p->max_sny * (8 + (QG + 3) / 4 * 4));
-      bool launched = false;
-      const int NVv = p->fwd_nv[pass];
-      const bool narrow = p->fwd_narrow[pass];
-#define MRSIM_YFW(QGV, NVV, NCV, M, W)                                                  \
-  if (QG == QGV && NVv == NVV && NCv == NCV && maps == M && narrow == W) {              \
-    auto k = ystage_q_kernel<QGV, NVV, NCV, M, W>;                                      \
-    set_smem(k, smq);                                                                   \
-    k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles, p->basis_nb ? 2 : p->fwd_cls ? 1 : 0);  \
-    launched = true;                                                                    \
-  }
-#define MRSIM_YF(QGV, NVV, NCV, M) MRSIM_YFW(QGV, NVV, NCV, M, false)
-#define MRSIM_YFB(NVV) MRSIM_YFW(8, NVV, 1, false, true) MRSIM_YFW(8, NVV, 2, false, true) \
-  MRSIM_YFW(8, NVV, 3, false, true) MRSIM_YFW(8, NVV, 4, false, true) MRSIM_YFW(8, NVV, 1, true, true) \
-  MRSIM_YFW(8, NVV, 2, true, true) MRSIM_YFW(8, NVV, 3, true, true)
-      MRSIM_YFB(4) MRSIM_YFB(6) MRSIM_YFB(7)
-#define MRSIM_YFQ(NCV, M) MRSIM_YF(1, 0, NCV, M) MRSIM_YF(2, 0, NCV, M) MRSIM_YF(4, 0, NCV, M) MRSIM_YF(8, 0, NCV, M)
-#define MRSIM_YFN(M) MRSIM_YFQ(1, M) MRSIM_YFQ(2, M) MRSIM_YFQ(3, M) MRSIM_YFQ(4, M) MRSIM_YFQ(8, M)
-      MRSIM_YFN(false) MRSIM_YFN(true)
-      MRSIM_YF(8, 6, 1, false) MRSIM_YF(8, 6, 2, false) MRSIM_YF(8, 6, 3, false) MRSIM_YF(8, 6, 4, false)
-      MRSIM_YF(8, 6, 1, true) MRSIM_YF(8, 6, 2, true) MRSIM_YF(8, 6, 3, true)
-      MRSIM_YF(8, 4, 1, false) MRSIM_YF(8, 4, 2, false) MRSIM_YF(8, 4, 3, false) MRSIM_YF(8, 4, 4, false)
-      MRSIM_YF(8, 4, 1, true) MRSIM_YF(8, 4, 2, true) MRSIM_YF(8, 4, 3, true)
-      MRSIM_YF(8, 7, 1, false) MRSIM_YF(8, 7, 2, false) MRSIM_YF(8, 7, 3, false) MRSIM_YF(8, 7, 4, false)
-      MRSIM_YF(8, 7, 1, true) MRSIM_YF(8, 7, 2, true) MRSIM_YF(8, 7, 3, true)
-#undef MRSIM_YFN
-#undef MRSIM_YFQ
-#undef MRSIM_YF
-#undef MRSIM_YFB
-#undef MRSIM_YFW
-      if (!launched) fail("no forward kernel instance for this unit shape");
-      MRSIM_CUDA(cudaGetLastError());
-      continue;
-    }
-    const size_t sm = sizeof(float) * (size_t)p->max_sny * (kT + (QG + 3) / 4 * 4);
-    bool launched = false;
-#define MRSIM_Y(QGV, NCV, M)                                                            \
-  if (QG == QGV && NCv == NCV && maps == M) {                                           \
-    auto k = ystage_kernel<kT, QGV, NCV, M>;                                            \
-    set_smem(k, sm);                                                                    \
-    k<<<(unsigned)R.n, 128, sm, st>>>(p->d_units, tiles);                               \
-    launched = true;                                                                    \
-  }
-#define MRSIM_YQ(NCV, M) MRSIM_Y(1, NCV, M) MRSIM_Y(2, NCV, M) MRSIM_Y(4, NCV, M) MRSIM_Y(8, NCV, M)
-#define MRSIM_YN(M) MRSIM_YQ(1, M) MRSIM_YQ(2, M) MRSIM_YQ(3, M) MRSIM_YQ(4, M) MRSIM_YQ(8, M)
-    MRSIM_YN(false) MRSIM_YN(true)
-#undef MRSIM_YN
-#undef MRSIM_YQ
-#undef MRSIM_Y
-    if (!launched) fail("no forward kernel instance for this unit shape");
-    MRSIM_CUDA(cudaGetLastError());
-  }
 }
 
 namespace {
@@ -2609,77 +1346,5 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
 void epi_plan_forward_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1) { launch_xstage(p, st, u0, u1, false); }
 
 void epi_plan_adjoint_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1) { launch_xstage(p, st, u0, u1, true); }
-
-void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
-  for (int pass = 0; pass < 4; ++pass) {
-    const TileRange R = tile_range(p->a_start[pass], p->n_atiles[pass], u0, u1);
-    if (R.n == 0) continue;
-    const int4* tiles = p->d_atiles[pass] + R.t0;
-    const bool maps = pass & 1, grads = (pass & 2) != 0;
-    const int NCv = p->nc;
-    if (p->adjq[pass]) {
-      const int NQv = p->adjq[pass];
-      const int TYv = p->adj_ty[pass];
-      const size_t smq = sizeof(float2) * (size_t)kAdjStages * adjq_chunk_lines(NQv) * NQv * 128 +
-                         sizeof(float) * (size_t)(p->max_lines + adjq_chunk_lines(NQv)) *
-                             (2 * TYv + adjq_line_floats(NCv, maps));
-      bool launched = false;
-      const bool virt = p->adj_cls;
-      // the built-in rows per thread, and 2 rows where the built-in choice is 4
-#define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
-  if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V && p->adj_narrow == W) { \
-    if (TYv == adjq_rows_v(NCV, M, V)) {                                                \
-      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W>;         \
-      set_smem(k, smq);                                                                 \
-      k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
-      launched = true;                                                                  \
-    } else if (!W && adjq_rows_v(NCV, M, V) == 4 && TYv == 2) {                         \
-      auto k = yadjoint_q_kernel<NQV, 2, NCV, M, G, V, false>;                          \
-      set_smem(k, smq);                                                                 \
-      k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
-      launched = true;                                                                  \
-    }                                                                                   \
-  }
-#define MRSIM_AQV(NQV, NCV, M, G, V) MRSIM_AQW(NQV, NCV, M, G, V, false)
-#define MRSIM_AQ(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, false)
-#define MRSIM_AQC(NCV, M, G) MRSIM_AQ(1, NCV, M, G) MRSIM_AQ(2, NCV, M, G) MRSIM_AQ(4, NCV, M, G) MRSIM_AQ(8, NCV, M, G)
-#define MRSIM_AQN(M, G) MRSIM_AQC(1, M, G) MRSIM_AQC(2, M, G) MRSIM_AQC(3, M, G) MRSIM_AQC(4, M, G)
-#define MRSIM_AQK(M, G) MRSIM_AQL(4, M, G) MRSIM_AQL(6, M, G) MRSIM_AQL(7, M, G)
-#define MRSIM_AQB(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, true) MRSIM_AQW(NQV, NCV, M, G, true, true)
-#define MRSIM_AQL(NQV, M, G) MRSIM_AQB(NQV, 1, M, G) MRSIM_AQB(NQV, 2, M, G) MRSIM_AQB(NQV, 3, M, G) MRSIM_AQB(NQV, 4, M, G)
-      MRSIM_AQN(false, false) MRSIM_AQN(true, false) MRSIM_AQN(false, true) MRSIM_AQN(true, true)
-      MRSIM_AQC(8, false, false) MRSIM_AQC(8, false, true)
-      MRSIM_AQK(false, false) MRSIM_AQK(true, false) MRSIM_AQK(false, true) MRSIM_AQK(true, true)
-#undef MRSIM_AQK
-#undef MRSIM_AQL
-#undef MRSIM_AQB
-#undef MRSIM_AQN
-#undef MRSIM_AQC
-#undef MRSIM_AQ
-#undef MRSIM_AQV
-#undef MRSIM_AQW
-      if (!launched) fail("no adjoint kernel instance for this unit shape");
-      MRSIM_CUDA(cudaGetLastError());
-      continue;
-    }
-    size_t sm = sizeof(float2) * (size_t)2 * p->max_hchunk * 128 +
-                sizeof(float) * ((size_t)kTY * (p->max_lines + p->max_coils) + 128 * (size_t)p->max_coils +
-                                 (size_t)p->max_lines * (5 + NCv));
-    bool launched = false;
-#define MRSIM_A(NCV, M, G)                                                              \
-  if (NCv == NCV && maps == M && grads == G) {                                          \
-    auto k = yadjoint_kernel<kTY, NCV, M, G>;                                           \
-    set_smem(k, sm);                                                                    \
-    k<<<(unsigned)R.n, 128, sm, st>>>(p->d_units, tiles);                               \
-    launched = true;                                                                    \
-  }
-#define MRSIM_AN(M, G) MRSIM_A(1, M, G) MRSIM_A(2, M, G) MRSIM_A(3, M, G) MRSIM_A(4, M, G) MRSIM_A(8, M, G)
-    MRSIM_AN(false, false) MRSIM_AN(true, false) MRSIM_AN(false, true) MRSIM_AN(true, true)
-#undef MRSIM_AN
-#undef MRSIM_A
-    if (!launched) fail("no adjoint kernel instance for this unit shape");
-    MRSIM_CUDA(cudaGetLastError());
-  }
-}
 
 }  // namespace mrsim
