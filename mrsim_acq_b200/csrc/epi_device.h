@@ -2,6 +2,7 @@
 // arithmetic, the reduced phase, asynchronous copies, and the shapes of the staged kernels' tiles.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "mrsim_internal.h"
@@ -11,6 +12,8 @@
 #pragma nv_diag_suppress 128
 
 namespace mrsim {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -79,6 +82,13 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// The k.r phase (K Y mod m2) / m2 in turns of line K (ky - ys) and row Y (2(y - sys) - (oy - 1)),
+// m2 = 2 sny: an exact integer index, in 32 bits wherever the product fits.
+__device__ __forceinline__ double kr_turns(int K, int Y, int m2) {
+  const int r = m2 <= 65536 ? (K * Y) % m2 : (int)(((long long)K * Y) % m2);
+  return (double)r / (double)m2;
+}
+
 // cp.async helpers (16-byte copies zero-fill the bytes past src_bytes)
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src, int src_bytes = 8) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -127,6 +137,43 @@ __host__ __device__ __forceinline__ constexpr int adjq_rows(int nc, bool maps) {
 // measured 30 % slower than four rows: the per-line loads then serve half the rows)
 __host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps, bool virt) {
   return adjq_rows(nc, maps);
+}
+
+// How many blocks share one tile of a y-stage (a cluster; each takes a part of the rows or lines and
+// the partial sums meet in distributed shared memory).  A plan of few tiles leaves most of the chip
+// idle and its blocks walk their rows or lines one after another: the count that makes waves times
+// steps smallest, with two blocks resident per SM, `steps` row or line steps in a tile and about
+// `setup` steps' worth of tables and reduction in a block.  Fixed by the whole plan, so that ranges of
+// its units give the same bits.
+inline int split_blocks(long long tiles, int steps, int max_split, double setup) {
+  int best = 1;
+  double least = 1e300;
+  for (int s = 1; s <= max_split; s *= 2) {
+    const double waves = (double)((tiles * s + 295) / 296);
+    const double cost = waves * ((double)steps / s + (s > 1 ? setup : 0.5 * setup));
+    if (cost < 0.9 * least) {  // a gain worth the exchange
+      least = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
+// A launch of `blocks` blocks in clusters of `cluster` (1: none).
+template <class K, class... A>
+void launch_split(K kernel, unsigned blocks, int cluster, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  MRSIM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 template <class K>

@@ -1059,6 +1059,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->y_start[pass][n] = (int)tiles.size();
       p->n_ytiles[pass] = (int)tiles.size();
+      // (not where this kernel expands classes to coils, whose epilogue holds every class of a line)
+      if (p->fwdq[pass] && pass == 0 && !p->fwd_narrow[pass] && n > 0)
+        p->fwd_split[pass] = split_blocks(p->n_ytiles[pass], p->max_sny, std::min(8, p->max_sny / 16), 16.0);
       arrays.add(&p->d_ytiles[pass], tiles.data(), sizeof(int4) * tiles.size());
     }
     if (p->xfft && p->basis_nb) {
@@ -1122,6 +1125,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         if (any && p->fwd_nv[pass] != 6) fc = false;
       }
       p->fwd_cls = fc || p->basis_nb > 0;
+      if (p->fwd_nv[0] && !p->fwd_cls) p->fwd_split[0] = 1;
     }
     // x-stage GEMM tiles, from host copies of the line tables (one copy per distinct table)
     std::map<const LineRec*, std::vector<LineRec>> host_lines;
@@ -1184,6 +1188,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->a_start[pass][n] = (int)yt.size();
       p->n_atiles[pass] = (int)yt.size();
+      if (p->adjq[pass] && !maps && !p->adj_narrow && ty == adjq_rows_v(p->nc, maps, p->adj_cls))
+        p->adj_split[pass] = split_blocks(p->n_atiles[pass], p->max_lines,
+                                          std::min(8, p->max_lines / adjq_chunk_lines(p->adjq[pass])), 8.0);
       arrays.add(&p->d_atiles[pass], yt.data(), sizeof(int4) * yt.size());
     }
     if (!p->basis_nb && (p->adj_cls || p->fwd_cls)) {  // the class x-stage tiles: 4 lines x the 8 coils

@@ -59,10 +59,7 @@ __global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restric
     float v = 0.f;
     if (y < sny) {
       const LineRec& L = u.lines[j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
+      double tv = kr_turns(L.ky - ys, 2 * (y - sys) - (oy - 1), 2 * sny);
       if (u.flags & UF_EDDY) {
         const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
         tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
@@ -230,7 +227,9 @@ __global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restric
 // the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
 // or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
 // NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
-template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW>
+// SPLIT: the blocks of a cluster share the tile's lines; each leaves its sums in shared memory and
+// adds up, over the cluster in rank order, and stores the rows rank, rank + blocks, ... of the tile.
+template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW, bool SPLIT>
 __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
                                                             const int4* __restrict__ tiles) {
   extern __shared__ __align__(16) float smem[];
@@ -241,7 +240,9 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   constexpr int STAGE = JC * NQ * 128;        // float2 per stage
   constexpr int PIECES = JC * NQ * 64;        // 16-byte pieces per stage
   constexpr int PPT = (PIECES + 255) / 256;   // pieces per thread
-  const int4 tl = tiles[blockIdx.x];          // unit, y0, x0
+  const int nsplit = SPLIT ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
+  const int rank = SPLIT ? (int)cooperative_groups::this_cluster().block_rank() : 0;
+  const int4 tl = tiles[SPLIT ? blockIdx.x / nsplit : blockIdx.x];  // unit, y0, x0
   const UnitDesc& u = units[tl.x];
   const int snx = u.snx, sny = u.sny, ncomp = u.ncomp, nlines = u.n_lines;
   const int y0 = tl.y, x0 = tl.z;
@@ -255,7 +256,8 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   const int col = tid & 127, rg = tid >> 7;
   const int x = x0 + col;
   const bool xok = x < snx;
-  const int nchunks = (nlines + JC - 1) / JC;
+  const int nch_all = (nlines + JC - 1) / JC;
+  const int cb = SPLIT ? nch_all * rank / nsplit : 0, nchunks = SPLIT ? nch_all * (rank + 1) / nsplit : nch_all;
 
   // This thread's 16-byte pieces k = tid + 256 i of a chunk: row r = k / 64 = (line jj, coil q),
   // column pair 2 (k % 64); the destination is float2 2k of the stage.  The source offset of
@@ -296,21 +298,19 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     cp_async_commit();
   };
 #pragma unroll
-  for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(c, c);
+  for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
 
   const int ys = u.ny / 2;
   const int oy = sny / u.ny;
   const int sys = oy * ys;
-  for (int idx = tid; idx < nlp * ROWS; idx += 256) {
+  const int line0 = SPLIT ? cb * JC : 0, line1 = SPLIT ? nchunks * JC : nlp;  // this block's lines
+  for (int idx = line0 * ROWS + tid; idx < line1 * ROWS; idx += 256) {
     const int j = idx / ROWS, r = idx % ROWS;
     const int y = y0 + r;
     float v = 0.f;
     if (y < sny && j < nlines) {
       const LineRec& L = u.lines[j];
-      const long long K = L.ky - ys;
-      const long long Y = 2LL * (y - sys) - (oy - 1);
-      const long long m2 = 2LL * sny;
-      double tv = (double)((K * Y) % m2) / (double)m2;
+      double tv = kr_turns(L.ky - ys, 2 * (y - sys) - (oy - 1), 2 * sny);
       if (u.flags & UF_EDDY) {
         const double yc = ((double)y - sys - (oy - 1) / 2.0) / oy;
         tv += ((double)u.eddy_cy * yc + (double)u.eddy_qy * yc * yc) * (double)L.decay;
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
     Bt[idx] = v;
   }
-  for (int j = tid; j < nlp; j += 256) {
+  for (int j = line0 + tid; j < line1; j += 256) {
     float* e = Lt + j * LF;
     if (j >= nlines) {
 #pragma unroll
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
 
   int s_use = 0, s_issue = kAdjStages - 1;  // stages of chunk c and of chunk c + stages - 1
-  for (int c = 0; c < nchunks; ++c) {
+  for (int c = cb; c < nchunks; ++c) {
     cp_async_wait_n<kAdjStages - 2>();
     __syncthreads();  // chunk c landed for every thread; every thread is done with chunk c - 1
     issue_chunk(c + kAdjStages - 1, s_issue);
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
   }
   cp_async_wait0();
-  if (!xok) return;
+  if (!SPLIT && !xok) return;
   if (PK) {
 #pragma unroll
     for (int ty = 0; ty < TY; ++ty)
@@ -549,6 +549,50 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
       }
   }
   const size_t plane = (size_t)snx * sny;
+  if (SPLIT) {
+    constexpr int NF = GRADS ? 4 : 2;  // sums per compartment
+    __syncthreads();                   // every thread is done with the ring
+    float* part = smem;                // [row][compartment][sum][thread]
+#pragma unroll
+    for (int ty = 0; ty < TY; ++ty)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        float* o = part + (ty * NC + c) * NF * 256 + tid;
+        o[0] = cg[ty][c].x;
+        o[256] = cg[ty][c].y;
+        if (GRADS) {
+          o[512] = Uy[ty][GRADS ? c : 0];
+          o[768] = Vx[ty][GRADS ? c : 0];
+        }
+      }
+    cooperative_groups::this_cluster().sync();
+    for (int ty = rank; ty < TY; ty += nsplit) {
+      const int y = y0 + rg * TY + ty;
+      const bool store = xok && y < sny;
+      const size_t i = store ? (size_t)x + (size_t)snx * y : 0;
+      float fg = 0.f;
+      for (int c = 0; c < ncomp; ++c) {
+        float t[NF];
+#pragma unroll
+        for (int k = 0; k < NF; ++k) t[k] = 0.f;
+        for (int r = 0; r < nsplit; ++r) {
+          const float* o = cooperative_groups::this_cluster().map_shared_rank(part, r) + (ty * NC + c) * NF * 256 + tid;
+#pragma unroll
+          for (int k = 0; k < NF; ++k) t[k] += o[256 * k];
+        }
+        if (!store) continue;
+        u.comp_grad[c * plane + i] = make_float2(t[0], t[1]);
+        if (GRADS) {
+          const float m = __ldg(u.comp + (size_t)c * u.comp_stride + i);
+          fg = fmaf(m, t[NF - 2], fg);
+          if (u.r2_grad) u.r2_grad[c * plane + i] = -2.0f * m * t[NF - 1];
+        }
+      }
+      if (GRADS && store && u.fmap_grad) u.fmap_grad[i] = distort ? 4.0f * 3.14159265358979f * fg : 0.f;
+    }
+    cooperative_groups::this_cluster().sync();  // no block leaves while another reads its sums
+    return;
+  }
 #pragma unroll
   for (int ty = 0; ty < TY; ++ty) {
     const int y = y0 + rg * TY + ty;
@@ -586,16 +630,23 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
                              (2 * TYv + adjq_line_floats(NCv, maps));
       bool launched = false;
       const bool virt = p->adj_cls;
+      const int split = p->adj_split[pass];
+      const size_t smsplit = std::max(smq, sizeof(float) * 256 * (size_t)TYv * NCv * (grads ? 4 : 2));
       // the built-in rows per thread, and 2 rows where the built-in choice is 4
 #define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
   if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V && p->adj_narrow == W) { \
-    if (TYv == adjq_rows_v(NCV, M, V)) {                                                \
-      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W>;         \
+    if (TYv == adjq_rows_v(NCV, M, V) && !M && !W && split > 1) {                       \
+      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, !M && !W>;   \
+      set_smem(k, smsplit);                                                             \
+      launch_split(k, (unsigned)R.n * split, split, smsplit, st, p->d_units, tiles);    \
+      launched = true;                                                                  \
+    } else if (TYv == adjq_rows_v(NCV, M, V)) {                                         \
+      auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, false>;  \
       set_smem(k, smq);                                                                 \
       k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
       launched = true;                                                                  \
     } else if (!W && adjq_rows_v(NCV, M, V) == 4 && TYv == 2) {                         \
-      auto k = yadjoint_q_kernel<NQV, 2, NCV, M, G, V, false>;                          \
+      auto k = yadjoint_q_kernel<NQV, 2, NCV, M, G, V, false, false>;                   \
       set_smem(k, smq);                                                                 \
       k<<<(unsigned)R.n, 256, smq, st>>>(p->d_units, tiles);                            \
       launched = true;                                                                  \
