@@ -667,9 +667,7 @@ EpiBatch* epi_batch_create(mrsim_context* ctx, int n, const mrsim_acquisition_in
     const EpiPlan& p = *b->ops.back()->plan;
     b->unit0.push_back((int)units.size());
     units.insert(units.end(), p.host_units.begin(), p.host_units.end());
-    std::vector<StaticDesc> sd(p.n_statics);
-    MRSIM_CUDA(cudaMemcpy(sd.data(), p.d_statics, sizeof(StaticDesc) * sd.size(), cudaMemcpyDeviceToHost));
-    statics.insert(statics.end(), sd.begin(), sd.end());
+    statics.insert(statics.end(), p.host_statics.begin(), p.host_statics.end());
     b->samples += b->ops.back()->samples_per_step;
   }
   b->plan.reset(epi_plan_create(units.data(), (int)units.size(), statics.data(), (int)statics.size()));

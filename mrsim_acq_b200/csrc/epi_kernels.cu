@@ -925,6 +925,7 @@ struct PlanArrays {
       MRSIM_CUDA(cudaMalloc(&d, blob.size()));
       p->allocs.push_back(d);
       MRSIM_CUDA(cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+      MRSIM_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the plan runs on streams that do not wait for this one
     }
     for (auto& s : slots) *s.first = (char*)d + s.second;
   }
@@ -1139,7 +1140,14 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         auto it = host_lines.find(hu[i].lines);
         if (it == host_lines.end()) {
           std::vector<LineRec> L(nl);
-          MRSIM_CUDA(cudaMemcpy(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost));
+          // the table's upload may still be queued on the context's stream
+          if (ctx) {
+            MRSIM_CUDA(cudaMemcpyAsync(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost, ctx->stream));
+            MRSIM_CUDA(cudaStreamSynchronize(ctx->stream));
+          } else {
+            MRSIM_CUDA(cudaDeviceSynchronize());
+            MRSIM_CUDA(cudaMemcpy(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost));
+          }
           it = host_lines.emplace(hu[i].lines, std::move(L)).first;
         }
         append_xtiles(xt, hu[i], i, it->second.data(), dir);

@@ -81,3 +81,14 @@ def test_eight_ring_coils_match_the_oracle(idx, gpu_ctx):
     for q in range(8):
         want = oracle.build_coil_kspace(inp, acq, q, 8)
         assert rel_l2(got[q], want) <= TOL, f"{name} coil {q}: rel-L2 {rel_l2(got[q], want):.2e}"
+
+
+def test_calls_in_turn_give_the_same_bits(gpu_ctx):
+    """One-slice calls of one shape with different line tables, in turn: the plan of each reads its own
+    table (rows in the DFT GEMM; the copy once ran beside the table's upload, and a call in about
+    150,000 took the tiles of the call before)."""
+    cs = [c for c in cases.literal_sum_cases() if c[0].startswith("8x9o3")]
+    first = [api.build_coil_kspaces(inp, acq.replace(n_coils=nc), ctx=gpu_ctx) for _, inp, acq, _, nc in cs]
+    for _ in range(40):
+        for (name, inp, acq, _, nc), want in zip(cs, first):
+            assert np.array_equal(api.build_coil_kspaces(inp, acq.replace(n_coils=nc), ctx=gpu_ctx), want), name
