@@ -82,6 +82,18 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// The kernels of a step are launched so that one may start while the one before it still runs
+// (programmatic dependent launch): its blocks take their place as the last blocks of the one before
+// drain, read the tables that no kernel writes, and wait here before they touch anything else.  Every
+// kernel of the chain waits, so what a kernel sees after it is what in-order launches give; copies and
+// kernels that do not call grid_begin are waited for before a launch starts, as always.  A step of
+// one slice is five launches of 3 to 8 us; the overlap takes the launch gaps and table setups out of
+// its chain (39.9 -> 21.0 us).  Launches of more than kChainTiles tiles keep kernels without the wait,
+// which cost a 1200-unit step 1.5 % and gave it nothing.
+constexpr int kChainTiles = 4 * 296;
+__device__ __forceinline__ void grid_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void grid_wait() { cudaGridDependencySynchronize(); }
+
 // The k.r phase (K Y mod m2) / m2 in turns of line K (ky - ys) and row Y (2(y - sys) - (oy - 1)),
 // m2 = 2 sny: an exact integer index, in 32 bits wherever the product fits.
 __device__ __forceinline__ double kr_turns(int K, int Y, int m2) {
@@ -159,20 +171,23 @@ inline int split_blocks(long long tiles, int steps, int max_split, double setup)
   return best;
 }
 
-// A launch of `blocks` blocks in clusters of `cluster` (1: none).
+// A launch of 256-thread blocks in clusters of `cluster` (1: none) that may start while the kernel
+// before it still runs (`overlap`); the kernel calls grid_begin and grid_wait.
 template <class K, class... A>
-void launch_split(K kernel, unsigned blocks, int cluster, size_t smem, cudaStream_t st, A... args) {
+void launch_chained(K kernel, dim3 blocks, int cluster, size_t smem, cudaStream_t st, bool overlap, A... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks);
+  cfg.gridDim = blocks;
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)cluster;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   MRSIM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
@@ -181,6 +196,7 @@ void set_smem(K kernel, size_t bytes) {
   // past 48 KB of static + dynamic shared memory the launch needs the dynamic opt-in
   // (the whole limit, so that threads launching one kernel with different sizes never lower it
   // between another's opt-in and launch)
+  if (bytes <= 40 * 1024) return;  // no kernel here has 8 KB of static shared memory beside dynamic
   cudaFuncAttributes fa;
   MRSIM_CUDA(cudaFuncGetAttributes(&fa, kernel));
   if (bytes + fa.sharedSizeBytes > 48 * 1024)

@@ -52,6 +52,7 @@ namespace {
 // phi0 = phase0[i] (explicit) or the phase model `PhaseModel::at` (phase.rs:141) sampled by
 // `phase_slice` (kspace.rs:1156-1180).
 __global__ void statics_kernel(const StaticDesc* descs) {
+  grid_begin();
   const StaticDesc& d = descs[blockIdx.y];
   const int n = d.snx * d.sny;
   const double inv_tau = 0.15915494309189533577;
@@ -97,6 +98,7 @@ __global__ void statics_kernel(const StaticDesc* descs) {
       cy += e[1] / oy;
     }
   }
+  grid_wait();  // the step before may still read this phase
   const double* __restrict__ phase0 = d.phase0;
   float* __restrict__ out = d.out;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -490,9 +492,14 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
   float2* const gbuf = u.g;
   // forward: the 8 coils' ex rows ([q][x]) after the class rows of at most 4 lines (24 N float2)
   float* exs = CLS ? reinterpret_cast<float*>(hsm + 24 * N) : nullptr;
-  if (CLS && !ADJ) {  // the tile's class rows, [line][v][x], as 16-byte asynchronous copies issued
-                      // first, so that their latency overlaps the table setup (N is even and the
-                      // rows of g start on 16-byte boundaries); then the ex rows
+  grid_begin();
+  // a small launch fills its tables while the kernel before it ends; a larger one issues its row copies
+  // first, which then fly while the tables fill
+  const bool fill = ADJ || gridDim.x <= kChainTiles;
+  if (!fill) grid_wait();
+  // forward: the tile's class rows, [line][v][x], as 16-byte asynchronous copies (N is even and the
+  // rows of g start on 16-byte boundaries)
+  auto stage_rows = [&] {
     constexpr int HN = N / 2;
     const float4* g4 = reinterpret_cast<const float4*>(gbuf);
     float4* h4 = reinterpret_cast<float4*>(hsm);
@@ -501,8 +508,10 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
       cp_async16(h4 + e, g4 + ((size_t)v * nl + r0 + jl) * HN + x2, 16);
     }
     cp_async_commit();
+  };
+  if (CLS && !ADJ && !fill) stage_rows();
+  if (CLS && !ADJ)
     for (int e = threadIdx.x; e < 8 * N; e += 256) exs[e] = u.geo.ex[e];
-  }
   const float2* __restrict__ xf = u.geo.xf;
   for (int k = threadIdx.x; k < N / 2; k += 256) {
     const float2 w = xf[k];
@@ -529,6 +538,8 @@ __global__ void __launch_bounds__(256, E <= 4 ? 4 : 2) xfft_warp_kernel(const Un
     rpol[r] = L.pol < 0 ? 1 : 0;
     rdec[r] = L.decay;
   }
+  if (fill) grid_wait();
+  if (CLS && !ADJ && fill) stage_rows();
   if (CLS && !ADJ) cp_async_wait0();
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -697,7 +708,7 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
   float2* const ksp = u.kspace;
   float2* const gbuf = u.g;
   const float* __restrict__ exg = u.geo.ex;
-  if (!ADJ) {  // issued first: the copies' latency overlaps the table setup
+  auto stage_rows = [&] {
     constexpr int HN = N / 2;
     const float4* g4 = reinterpret_cast<const float4*>(gbuf);
     float4* h4 = reinterpret_cast<float4*>(st);
@@ -706,7 +717,11 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
       cp_async16(h4 + e, g4 + ((size_t)r * nl + j0 + jl) * HN + x2, 16);
     }
     cp_async_commit();
-  }
+  };
+  grid_begin();
+  const bool fill = ADJ || gridDim.x <= kChainTiles;
+  if (!fill) grid_wait();
+  if (!ADJ && !fill) stage_rows();
   const float2* __restrict__ xf = u.geo.xf;
   for (int k = threadIdx.x; k < N / 2; k += 256) {
     const float2 w = xf[k];
@@ -729,6 +744,8 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
     lpol[threadIdx.x] = L.pol < 0 ? 1 : 0;
     ldec[threadIdx.x] = L.decay;
   }
+  if (fill) grid_wait();
+  if (!ADJ && fill) stage_rows();
   if (!ADJ) cp_async_wait0();
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1061,15 +1078,21 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->y_start[pass][n] = (int)tiles.size();
       p->n_ytiles[pass] = (int)tiles.size();
       // (not where this kernel expands classes to coils, whose epilogue holds every class of a line)
-      if (p->fwdq[pass] && pass == 0 && !p->fwd_narrow[pass] && n > 0)
+      p->fwd_small[pass] = p->fwdq[pass] && pass == 0 && !p->fwd_narrow[pass] && p->n_ytiles[pass] <= kChainTiles;
+      if (p->fwd_small[pass])
         p->fwd_split[pass] = split_blocks(p->n_ytiles[pass], p->max_sny, std::min(8, p->max_sny / 16), 16.0);
       arrays.add(&p->d_ytiles[pass], tiles.data(), sizeof(int4) * tiles.size());
     }
+    // x-stage tiles of 32 rows, or where those would not fill the chip (two blocks per SM) of one line of
+    // every coil, or one row per warp
+    long long x_rows = 0;
+    for (int i = 0; i < n; ++i) x_rows += (long long)hu[i].ncoils * hu[i].n_lines;
+    const bool few = x_rows < 296 * 32;
     if (p->xfft && p->basis_nb) {
       // tiles of a few lines x every coil: by unit, or with mixed widths ordered by width
       std::vector<int4> ct;
       auto unit_tiles = [&](int i) {
-        const int step = basis_lines(hu[i].ncoils);
+        const int step = few ? 1 : basis_lines(hu[i].ncoils);
         p->basis_rows = std::max(p->basis_rows, step * std::min(hu[i].ncoils, kBasisRows));
         p->basis_lines = std::max(p->basis_lines, step);
         for (int j0 = 0; j0 < hu[i].n_lines; j0 += step)
@@ -1109,7 +1132,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       for (int i = 0; i < n; ++i) {
         p->f_start[i] = (int)ft.size();
         const int rows = hu[i].ncoils * hu[i].n_lines;
-        const int per = p->xfft_e ? 32 : std::min(256, kXfftMaxN / hu[i].snx);
+        const int per = p->xfft_e ? (few ? 8 : 32) : std::min(256, kXfftMaxN / hu[i].snx);
         for (int r0 = 0; r0 < rows; r0 += per) ft.push_back(make_int4(i, r0, std::min(per, rows - r0), 0));
       }
       p->f_start[n] = (int)ft.size();
@@ -1126,7 +1149,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         if (any && p->fwd_nv[pass] != 6) fc = false;
       }
       p->fwd_cls = fc || p->basis_nb > 0;
-      if (p->fwd_nv[0] && !p->fwd_cls) p->fwd_split[0] = 1;
+      if (p->fwd_nv[0] && !p->fwd_cls) p->fwd_small[0] = false;
     }
     // x-stage GEMM tiles, from host copies of the line tables (one copy per distinct table)
     std::map<const LineRec*, std::vector<LineRec>> host_lines;
@@ -1196,7 +1219,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->a_start[pass][n] = (int)yt.size();
       p->n_atiles[pass] = (int)yt.size();
-      if (p->adjq[pass] && !maps && !p->adj_narrow && ty == adjq_rows_v(p->nc, maps, p->adj_cls))
+      p->adj_small[pass] = p->adjq[pass] && !maps && !p->adj_narrow && ty == adjq_rows_v(p->nc, maps, p->adj_cls) &&
+                           p->n_atiles[pass] <= kChainTiles;
+      if (p->adj_small[pass])
         p->adj_split[pass] = split_blocks(p->n_atiles[pass], p->max_lines,
                                           std::min(8, p->max_lines / adjq_chunk_lines(p->adjq[pass])), 8.0);
       arrays.add(&p->d_atiles[pass], yt.data(), sizeof(int4) * yt.size());
@@ -1206,7 +1231,8 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->c_start.assign(n + 1, 0);
       for (int i = 0; i < n; ++i) {
         p->c_start[i] = (int)ct.size();
-        for (int j0 = 0; j0 < hu[i].n_lines; j0 += 4) ct.push_back(make_int4(i, j0, std::min(4, hu[i].n_lines - j0), 0));
+        for (int j0 = 0, step = few ? 1 : 4; j0 < hu[i].n_lines; j0 += step)
+          ct.push_back(make_int4(i, j0, std::min(step, hu[i].n_lines - j0), 0));
       }
       p->c_start[n] = (int)ct.size();
       p->n_ctiles = (int)ct.size();
@@ -1224,9 +1250,10 @@ void epi_plan_statics(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
   if (u1 < 0) u1 = p->n_statics;
   if (u0 < 0 || u0 > u1 || u1 > p->n_statics) fail("unit range outside the plan");
   if (u1 == u0) return;
-  dim3 grid(std::min(8, (p->max_static_n + 255) / 256), u1 - u0);  // a few voxels per thread
-  statics_kernel<<<grid, 256, 0, st>>>(p->d_statics + u0);
-  MRSIM_CUDA(cudaGetLastError());
+  // a few voxels per thread: eight blocks per unit, or more where the units are few
+  const int per_unit = std::max(8, 592 / (u1 - u0));
+  launch_chained(statics_kernel, dim3(std::min(per_unit, (p->max_static_n + 255) / 256), u1 - u0), 1, 0, st,
+                 u1 - u0 <= 148, (const StaticDesc*)(p->d_statics + u0));
 }
 
 void epi_plan_forward(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
@@ -1256,7 +1283,7 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
   case EV: {                                                                              \
     auto k = xfft_basis_kernel<EV, ADJ>;                                                  \
     set_smem(k, sm);                                                                      \
-    k<<<(unsigned)count, 256, sm, st>>>(p->d_units, tiles, p->basis_nb);                  \
+    launch_chained(k, dim3((unsigned)count), 1, sm, st, count <= kChainTiles, p->d_units, tiles, p->basis_nb);  \
     break;                                                                                \
   }
 #define MRSIM_XBA(ADJ) MRSIM_XB(1, ADJ) MRSIM_XB(2, ADJ) MRSIM_XB(3, ADJ) MRSIM_XB(4, ADJ) \
@@ -1279,10 +1306,10 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
     const unsigned g = (unsigned)R.n;
 #define MRSIM_XC(ADJ)                                                                             \
   switch (p->xfft_e) {                                                                            \
-    case 1: xfft_warp_kernel<1, ADJ, true><<<g, 256, 0, st>>>(p->d_units, tiles); break;          \
-    case 2: xfft_warp_kernel<2, ADJ, true><<<g, 256, 0, st>>>(p->d_units, tiles); break;          \
-    case 3: xfft_warp_kernel<3, ADJ, true><<<g, 256, 0, st>>>(p->d_units, tiles); break;          \
-    default: xfft_warp_kernel<4, ADJ, true><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    default: launch_chained(xfft_warp_kernel<4, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
   }
     if (adj) {
       MRSIM_XC(true)
@@ -1301,14 +1328,14 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
       const unsigned g = (unsigned)p->fe_count[E];
 #define MRSIM_XE(ADJ)                                                                               \
   switch (E) {                                                                                      \
-    case 1: xfft_warp_kernel<1, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 2: xfft_warp_kernel<2, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 3: xfft_warp_kernel<3, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 4: xfft_warp_kernel<4, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 5: xfft_warp_kernel<5, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 6: xfft_warp_kernel<6, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    case 7: xfft_warp_kernel<7, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;           \
-    default: xfft_warp_kernel<8, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;          \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    default: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
   }
       if (adj) {
         MRSIM_XE(true)
@@ -1327,14 +1354,14 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
     const unsigned g = (unsigned)R.n;
 #define MRSIM_XF(ADJ)                                                                             \
   switch (p->xfft_e) {                                                                            \
-    case 1: xfft_warp_kernel<1, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 2: xfft_warp_kernel<2, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 3: xfft_warp_kernel<3, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 4: xfft_warp_kernel<4, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 5: xfft_warp_kernel<5, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 6: xfft_warp_kernel<6, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 7: xfft_warp_kernel<7, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
-    case 8: xfft_warp_kernel<8, ADJ, false><<<g, 256, 0, st>>>(p->d_units, tiles); break;         \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 8: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
     default: xfft_kernel<ADJ><<<g, 256, 0, st>>>(p->d_units, tiles);                              \
   }
     if (adj) {

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restric
 // the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
 // or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
 // NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
-// SPLIT: the blocks of a cluster share the tile's lines; each leaves its sums in shared memory and
+// SPLIT: a small launch, chained to the kernel before it: the blocks of a cluster share the tile's lines; each leaves its sums in shared memory and
 // adds up, over the cluster in rank order, and stores the rows rank, rank + blocks, ... of the tile.
 template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW, bool SPLIT>
 __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   constexpr int STAGE = JC * NQ * 128;        // float2 per stage
   constexpr int PIECES = JC * NQ * 64;        // 16-byte pieces per stage
   constexpr int PPT = (PIECES + 255) / 256;   // pieces per thread
+  if (SPLIT) grid_begin();
   const int nsplit = SPLIT ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
   const int rank = SPLIT ? (int)cooperative_groups::this_cluster().block_rank() : 0;
   const int4 tl = tiles[SPLIT ? blockIdx.x / nsplit : blockIdx.x];  // unit, y0, x0
@@ -297,8 +298,10 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
     cp_async_commit();
   };
+  if (!SPLIT) {  // (as in the forward: a small launch fills its tables first)
 #pragma unroll
-  for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
+    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
+  }
 
   const int ys = u.ny / 2;
   const int oy = sny / u.ny;
@@ -346,6 +349,11 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
   }
 
+  if (SPLIT) {
+    grid_wait();
+#pragma unroll
+    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
+  }
   // per-thread constants of its 4 rows
   const bool distort = (u.flags & UF_DISTORT) != 0;
   const int xs_ = xok ? x : 0;
@@ -630,15 +638,16 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
                              (2 * TYv + adjq_line_floats(NCv, maps));
       bool launched = false;
       const bool virt = p->adj_cls;
+      const bool small = p->adj_small[pass];
       const int split = p->adj_split[pass];
       const size_t smsplit = std::max(smq, sizeof(float) * 256 * (size_t)TYv * NCv * (grads ? 4 : 2));
       // the built-in rows per thread, and 2 rows where the built-in choice is 4
 #define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
   if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V && p->adj_narrow == W) { \
-    if (TYv == adjq_rows_v(NCV, M, V) && !M && !W && split > 1) {                       \
+    if (TYv == adjq_rows_v(NCV, M, V) && !M && !W && small) {                           \
       auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, !M && !W>;   \
       set_smem(k, smsplit);                                                             \
-      launch_split(k, (unsigned)R.n * split, split, smsplit, st, p->d_units, tiles);    \
+      launch_chained(k, dim3((unsigned)R.n * split), split, smsplit, st, true, p->d_units, tiles);   \
       launched = true;                                                                  \
     } else if (TYv == adjq_rows_v(NCV, M, V)) {                                         \
       auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, false>;  \

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(128, 4) ystage_kernel(const UnitDesc* __restri
 // the layout the class-mode x-stage expands) instead of the coil rows; 2 writes basis rows (the
 // unit's eyc holds the coil basis, whose last row is constant), G_v = s T_v for every row.
 // NARROW: some plane or row is not on a 16-byte boundary, so the ring fills by 4-byte copies.
-// SPLIT: the blocks of a cluster share the tile's rows (not with classes expanded to coils here); each
+// SPLIT: a small launch, chained to the kernel before it, in which the blocks of a cluster share the tile's rows (not with classes expanded to coils here); each
 // leaves its sums in shared memory and adds up a share of the (line, row) pairs over the cluster, in
 // rank order.  One slice of one coil (64 lines on 128 x 128) has 8 tiles: 23.2 us walked whole.
 template <int QG, int NV, int NC, bool MAPS, bool NARROW, bool SPLIT>
@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   extern __shared__ __align__(16) float smem[];
   float* ring = smem;                           // [stage][plane][RC][128]
   float* Bt = ring + kFwdStages * STAGE;        // [sny][TL]
+  if (SPLIT) grid_begin();
   const int nsplit = SPLIT ? (int)cg::this_cluster().num_blocks() : 1;
   const int rank = SPLIT ? (int)cg::this_cluster().block_rank() : 0;
   const Tile tl = tiles[SPLIT ? blockIdx.x / nsplit : blockIdx.x];
@@ -276,8 +277,12 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
     }
     cp_async_commit();
   };
+  // the first rows fly while the tables fill; a small launch fills its tables while the kernel before
+  // it still runs instead
+  if (!SPLIT) {
 #pragma unroll
-  for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(cb + c);
+    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(cb + c);
+  }
 
   const int nl = min(TL, u.n_lines - tl.line0);
   const int ys = u.ny / 2;
@@ -322,6 +327,11 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
       thi_s[j] = tlo_s[j] = tinh_s[j] = trf_s[j] = 0.f;
       for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = 0.f;
     }
+  }
+  if (SPLIT) {
+    grid_wait();
+#pragma unroll
+    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(cb + c);
   }
   __syncthreads();
 
@@ -537,14 +547,15 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
       bool launched = false;
       const int NVv = p->fwd_nv[pass];
       const bool narrow = p->fwd_narrow[pass];
+      const bool small = p->fwd_small[pass];
       const int split = p->fwd_split[pass], rows_kind = p->basis_nb ? 2 : p->fwd_cls ? 1 : 0;
       const size_t smsplit = std::max(smq, sizeof(float2) * 256 * kT * (size_t)std::max(NVv, QG));
 #define MRSIM_YFW(QGV, NVV, NCV, M, W)                                                  \
   if (QG == QGV && NVv == NVV && NCv == NCV && maps == M && narrow == W) {              \
-    if (!M && !W && split > 1) {                                                        \
+    if (!M && !W && small) {                                                            \
       auto k = ystage_q_kernel<QGV, NVV, NCV, M, W, !M && !W>;                          \
       set_smem(k, smsplit);                                                             \
-      launch_split(k, (unsigned)R.n * split, split, smsplit, st, p->d_units, tiles, rows_kind);   \
+      launch_chained(k, dim3((unsigned)R.n * split), split, smsplit, st, true, p->d_units, tiles, rows_kind);  \
     } else {                                                                            \
       auto k = ystage_q_kernel<QGV, NVV, NCV, M, W, false>;                             \
       set_smem(k, smq);                                                                 \
