@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "mrsim_internal.h"
+#include "row_fft.h"
 
 // Template flags select whole code paths (packed or scalar, class or coil accumulators); the paths
 // an instance does not take leave loops the front end reports as unreachable.
@@ -76,10 +77,6 @@ __device__ __forceinline__ float2 phase_turns2(float2 s, float2 f, float2 t_hi, 
   const float2 nn = fsub2(M, fadd2(ffma2(f, t_hi, s), M));  // -n
   const float2 r = ffma2(f, t_hi, nn);
   return ffma2(f, t_lo, fadd2(r, s));
-}
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
 // The kernels of a step are launched so that one may start while the one before it still runs

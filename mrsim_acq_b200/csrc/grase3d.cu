@@ -46,56 +46,107 @@ struct ZdftArgs {
 
 // out = sampling * sum_c lw(g, shot, c) * (w_c(p, ky) * sum_z K[var(p, ky)][src(c, p)][z] zk[p][z]), var
 // the images the line's shot saw (`Plan::kspace` kspace3d.rs:206-232)
-__global__ void grase_zdft_kernel(const ZdftArgs a) {
-  const int per = a.nx * a.ny;
-  const int p = blockIdx.y;
+//
+// A thread serves ZT partitions of its column: with kZTile of them a slice's sample is read once for all
+// (it was read once per partition: 3.2 GB through L2 for 32 coils x 32 partitions x 3 compartments of
+// 64 x 64: 640 us, here 149).  Per-shot images and per-echo sources give partitions different ones: ZT = 1.  The
+// tile's z kernel sits in shared memory ([z][partition]); the sums run in z order.
+constexpr int kZTile = 8;
+template <int ZT>
+__global__ void __launch_bounds__(256) grase_zdft_kernel(const ZdftArgs a) {
+  extern __shared__ __align__(16) float2 zks[];
+  const int per = a.nx * a.ny, nz = a.nz;
+  const int p0 = blockIdx.y * ZT;
   const int gq = blockIdx.z;  // gl * nc + q
   const int gl = gq / a.nc, q = gq % a.nc;
+  for (int t = threadIdx.x; t < nz * ZT; t += blockDim.x) {
+    const int z = t / ZT, p = p0 + t % ZT;
+    zks[t] = p < nz ? a.zk[p * nz + z] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  const size_t zstride = (size_t)a.nc * per;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < per; i += gridDim.x * blockDim.x) {
     const int ky = i / a.nx;
-    float2 v = make_float2(0.f, 0.f);
+    float2 v[ZT];
+#pragma unroll
+    for (int t = 0; t < ZT; ++t) v[t] = make_float2(0.f, 0.f);
     if (a.row_acquired[ky]) {
+      const int var = ZT == 1 && a.line_var ? a.line_var[((size_t)gl * nz + p0) * a.ny + ky] : 0;
       for (int c = 0; c < a.ncomp; ++c) {
-        const int s = a.src[c * a.nz + p];
-        const int var = a.line_var ? a.line_var[((size_t)gl * a.nz + p) * a.ny + ky] : 0;
         const float2* Kc =
-            a.K + ((size_t)((gl * a.nvar + var) * a.nsrc + s) * a.nz) * a.nc * per + (size_t)q * per + i;
-        float ar = 0.f, ai = 0.f;
-        for (int z = 0; z < a.nz; ++z) {
-          const float2 k = Kc[(size_t)z * a.nc * per];
-          const float2 e = a.zk[p * a.nz + z];
-          ar += k.x * e.x - k.y * e.y;
-          ai += k.x * e.y + k.y * e.x;
+            a.K + (size_t)((gl * a.nvar + var) * a.nsrc + a.src[c * nz + p0]) * nz * zstride + (size_t)q * per + i;
+        float ar[ZT], ai[ZT];
+#pragma unroll
+        for (int t = 0; t < ZT; ++t) ar[t] = ai[t] = 0.f;
+#pragma unroll 4
+        for (int z = 0; z < nz; ++z) {
+          const float2 k = Kc[z * zstride];
+#pragma unroll
+          for (int t = 0; t < ZT; ++t) {
+            const float2 e = zks[z * ZT + t];
+            ar[t] += k.x * e.x - k.y * e.y;
+            ai[t] += k.x * e.y + k.y * e.x;
+          }
         }
-        const float w = a.wc[((size_t)c * a.nz + p) * a.ny + ky];
-        ar *= w;
-        ai *= w;
-        const float l = a.lw ? a.lw[((size_t)(a.g0 + gl) * a.n_shots + a.shot[p * a.ny + ky]) * a.ncomp + c] : 1.f;
-        v.x += ar * l;
-        v.y += ai * l;
+#pragma unroll
+        for (int t = 0; t < ZT; ++t) {
+          const int p = min(p0 + t, nz - 1);
+          const float w = a.wc[((size_t)c * nz + p) * a.ny + ky];
+          const float l = a.lw ? a.lw[((size_t)(a.g0 + gl) * a.n_shots + a.shot[p * a.ny + ky]) * a.ncomp + c] : 1.f;
+          v[t].x += ar[t] * w * l;
+          v[t].y += ai[t] * w * l;
+        }
       }
     }
-    a.out[(((size_t)gl * a.nc + q) * a.nz + p) * per + i] = v;
+#pragma unroll
+    for (int t = 0; t < ZT; ++t)
+      if (p0 + t < nz) a.out[(((size_t)gl * a.nc + q) * nz + p0 + t) * per + i] = v[t];
   }
 }
 
-// slices[gl][z][q] = (1/nz) sum_p k3[gl][q][p] conj(zk[p][z])
-__global__ void grase_izdft_kernel(const float2* __restrict__ k3, const float2* __restrict__ zk, int nx, int ny,
-                                   int nz, int nc, float2* __restrict__ slices) {
+// slices[gl][z][q] = (1/nz) sum_p k3[gl][q][p] conj(zk[p][z]), kZTile slices to a thread as above
+__global__ void __launch_bounds__(256) grase_izdft_kernel(const float2* __restrict__ k3, const float2* __restrict__ zk,
+                                                          int nx, int ny, int nz, int nc, float2* __restrict__ slices) {
+  extern __shared__ __align__(16) float2 zks[];
   const int per = nx * ny;
-  const int z = blockIdx.y;
+  const int z0 = blockIdx.y * kZTile;
   const int gq = blockIdx.z, gl = gq / nc, q = gq % nc;
+  for (int t = threadIdx.x; t < nz * kZTile; t += blockDim.x) {
+    const int p = t / kZTile, z = z0 + t % kZTile;
+    zks[t] = z < nz ? zk[p * nz + z] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
   const float inv = 1.0f / (float)nz;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < per; i += gridDim.x * blockDim.x) {
-    float ar = 0.f, ai = 0.f;
+    float ar[kZTile], ai[kZTile];
+#pragma unroll
+    for (int t = 0; t < kZTile; ++t) ar[t] = ai[t] = 0.f;
+#pragma unroll 4
     for (int p = 0; p < nz; ++p) {
       const float2 k = k3[(((size_t)gl * nc + q) * nz + p) * per + i];
-      const float2 e = zk[p * nz + z];
-      ar += k.x * e.x + k.y * e.y;
-      ai += k.y * e.x - k.x * e.y;
+#pragma unroll
+      for (int t = 0; t < kZTile; t += 2) {
+        const float4 e = *reinterpret_cast<const float4*>(zks + p * kZTile + t);
+        ar[t] += k.x * e.x + k.y * e.y;
+        ai[t] += k.y * e.x - k.x * e.y;
+        ar[t + 1] += k.x * e.z + k.y * e.w;
+        ai[t + 1] += k.y * e.z - k.x * e.w;
+      }
     }
-    slices[(((size_t)gl * nz + z) * nc + q) * per + i] = make_float2(ar * inv, ai * inv);
+#pragma unroll
+    for (int t = 0; t < kZTile; ++t)
+      if (z0 + t < nz)
+        slices[(((size_t)gl * nz + z0 + t) * nc + q) * per + i] = make_float2(ar[t] * inv, ai[t] * inv);
   }
+}
+
+// the tile's z kernel in shared memory, opted in past 48 KB (more than 768 partitions)
+template <class K>
+size_t z_smem(K kernel, int nz) {
+  const size_t n = sizeof(float2) * kZTile * (size_t)nz;
+  if (n > 48 * 1024)
+    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+  return n;
 }
 
 // combined [gl][z][ny][nx] -> magnitude / phase at vox * nv + g
@@ -441,7 +492,14 @@ static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_a
   a.g0 = g0;
   a.line_var = V ? V->d_line_var : nullptr;
   a.nvar = nvar;
-  grase_zdft_kernel<<<grid3(per, nz, ngl * nc), 256, 0, st>>>(a);
+  bool one_source = a.line_var == nullptr;  // every partition of a compartment reads the same images
+  for (int c = 0; c < P.ncomp; ++c)
+    for (int p = 1; p < nz; ++p) one_source = one_source && P.src_of[(size_t)c * nz + p] == P.src_of[(size_t)c * nz];
+  if (one_source)
+    grase_zdft_kernel<kZTile><<<grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), 256,
+                                z_smem(grase_zdft_kernel<kZTile>, nz), st>>>(a);
+  else
+    grase_zdft_kernel<1><<<grid3(per, nz, ngl * nc), 256, z_smem(grase_zdft_kernel<1>, nz), st>>>(a);
   MRSIM_CUDA(cudaGetLastError());
 }
 
@@ -537,7 +595,8 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     grase_kspace(Pc, Ic, acq_cal, in.phase, nullptr, 0, 1, Pc.mask, k3, ctx);
     grase_noise(C, Pc, k3, 0, 1, cal_seed ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
     float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
-    grase_izdft_kernel<<<grid3(per, nz, nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
+    grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
+        k3, d_zk, nx, ny, nz, nc, sl);
     std::vector<float2*> refs;
     for (int z = 0; z < nz; ++z) refs.push_back(sl + (size_t)z * nc * per);
     W = fit_grappa(A, refs, nx, ny, nc, acq_cal, accel, (int)acq.acs_lines, st);
@@ -561,7 +620,8 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     grase_kspace(P, I, acq, in.phase, d_lw, g0, g1, P.mask, k3, ctx, &V);
     grase_noise(C, P, k3, g0, g1, seed, P.mask, acq, st);
     float2* sl = (float2*)C.alloc((size_t)ngl * nz * nc * per * sizeof(float2));
-    grase_izdft_kernel<<<grid3(per, nz, ngl * nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
+    grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
+        k3, d_zk, nx, ny, nz, nc, sl);
     float2* comb = (float2*)C.alloc((size_t)ngl * nz * per * sizeof(float2));
     std::vector<ReconJob> jobs;
     for (int gl = 0; gl < ngl; ++gl)
@@ -583,7 +643,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
       }
     const ReconJob* d_jobs = (const ReconJob*)C.upload(jobs.data(), jobs.size() * sizeof(ReconJob), st);
     if (accel > 1) launch_grappa_apply(d_jobs, (int)jobs.size(), T.fills, T.n_fills, nx, nc, st);
-    launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, false, st);
+    launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, nc, false, st);
     volume_output_kernel<<<1024, 256, 0, st>>>(comb, g0, ngl, nv, per * nz, d_mag, d_ph);
     MRSIM_CUDA(cudaGetLastError());
     MRSIM_CUDA(cudaStreamSynchronize(st));
@@ -810,7 +870,8 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       grase_kspace(Pc, Ic, ae, in.phase, d_lw, 0, 1, Pc.mask, k3, ctx);
       grase_noise(C, Pc, k3, 0, 1, (seed ^ echo_salt((uint64_t)e)) ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
       float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
-      grase_izdft_kernel<<<grid3(per, nz, nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
+      grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
+          k3, d_zk, nx, ny, nz, nc, sl);
       std::vector<float2*> refs;
       for (int z = 0; z < nz; ++z) refs.push_back(sl + (size_t)z * nc * per);
       W[e] = fit_grappa(A, refs, nx, ny, nc, acq_cal, accel, (int)acq.acs_lines, st);
@@ -841,7 +902,8 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       // the noise and spikes of echo e on its own streams (echo 0 unsalted)
       grase_noise(E, Pg, k3, g, g + 1, seed ^ echo_salt((uint64_t)e), Pg.mask, acq, st);
       float2* sl = (float2*)E.alloc((size_t)nz * nc * per * sizeof(float2));
-      grase_izdft_kernel<<<grid3(per, nz, nc), 256, 0, st>>>(k3, d_zk, nx, ny, nz, nc, sl);
+      grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
+          k3, d_zk, nx, ny, nz, nc, sl);
       float2* comb = (float2*)E.alloc((size_t)nz * per * sizeof(float2));
       std::vector<ReconJob> jobs;
       for (int z = 0; z < nz; ++z) {
@@ -862,7 +924,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       }
       const ReconJob* d_jobs = (const ReconJob*)E.upload(jobs.data(), jobs.size() * sizeof(ReconJob), st);
       if (accel > 1) launch_grappa_apply(d_jobs, (int)jobs.size(), T.fills, T.n_fills, nx, nc, st);
-      launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, false, st);
+      launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, nc, false, st);
       volume_output_kernel<<<1024, 256, 0, st>>>(comb, g, 1, nv, per * nz, d_mag[e], d_ph[e]);
       MRSIM_CUDA(cudaGetLastError());
       MRSIM_CUDA(cudaStreamSynchronize(st));

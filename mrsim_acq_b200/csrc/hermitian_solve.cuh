@@ -27,7 +27,8 @@ __device__ __forceinline__ HsCd hs_recip(HsCd d) {
 }
 
 // W: [n][n + nrhs] in global memory; fre/fim: n doubles each; xs: nrhs * 2n doubles (solution
-// scratch); out: [nrhs][n] complex f32.  red_v / red_i: blockDim.x-entry shared arrays.  Every
+// scratch); out: [nrhs][n] complex f32.  red_v / red_i: shared arrays of an
+// entry per warp.  W and the scratch may be in shared memory.  blockDim.x is a multiple of 32.  Every
 // thread of the block calls it.
 __device__ inline void hermitian_solve_block(double2* W, int n, int nrhs, double* fre, double* fim, double* xs,
                                              float2* out, double* red_v, int* red_i) {
@@ -44,13 +45,25 @@ __device__ inline void hermitian_solve_block(double2* W, int n, int nrhs, double
         bi = r;
       }
     }
-    red_v[threadIdx.x] = best;
-    red_i[threadIdx.x] = bi;
+    // (largest value, then lowest row, in any order of comparison)
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+      const double o = __shfl_xor_sync(0xffffffffu, best, h);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, h);
+      if (o > best || (o == best && oi < bi)) {
+        best = o;
+        bi = oi;
+      }
+    }
+    if ((threadIdx.x & 31) == 0) {
+      red_v[threadIdx.x >> 5] = best;
+      red_i[threadIdx.x >> 5] = bi;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       double b = red_v[0];
       int p = red_i[0];
-      for (int t = 1; t < (int)blockDim.x; ++t)
+      for (int t = 1; t < (int)blockDim.x / 32; ++t)
         if (red_v[t] > b || (red_v[t] == b && red_i[t] < p)) {
           b = red_v[t];
           p = red_i[t];
@@ -76,37 +89,50 @@ __device__ inline void hermitian_solve_block(double2* W, int n, int nrhs, double
       fim[r] = f.im;
     }
     __syncthreads();
-    const int rows = n - col - 1, width = cols - col;
-    for (int e = threadIdx.x; e < rows * width; e += blockDim.x) {
-      const int r = col + 1 + e / width, c = col + e % width;
-      const double2 p = W[(size_t)col * cols + c];
-      const HsCd s = hs_mul({fre[r], fim[r]}, {p.x, p.y});
-      double2 h = W[(size_t)r * cols + c];
-      h.x = __dsub_rn(h.x, s.re);
-      h.y = __dsub_rn(h.y, s.im);
-      W[(size_t)r * cols + c] = h;
+    // a warp per row, lanes along it
+    for (int r = col + 1 + (int)(threadIdx.x >> 5); r < n; r += blockDim.x >> 5) {
+      const HsCd f = {fre[r], fim[r]};
+      for (int c = col + (int)(threadIdx.x & 31); c < cols; c += 32) {
+        const double2 p = W[(size_t)col * cols + c];
+        const HsCd s = hs_mul(f, {p.x, p.y});
+        double2 h = W[(size_t)r * cols + c];
+        h.x = __dsub_rn(h.x, s.re);
+        h.y = __dsub_rn(h.y, s.im);
+        W[(size_t)r * cols + c] = h;
+      }
     }
     __syncthreads();
   }
-  // back substitution, one thread per right-hand side
-  for (int q = threadIdx.x; q < nrhs; q += blockDim.x) {
+  // back substitution, one warp per right-hand side: the lanes form 32 products at a time, and every
+  // lane subtracts them in the reference's order (column by column)
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < nrhs; q += blockDim.x >> 5) {
     double* xre = xs + (size_t)q * 2 * n;
     double* xim = xre + n;
     for (int col = n - 1; col >= 0; --col) {
       const double2 b = W[(size_t)col * cols + n + q];
       HsCd s = {b.x, b.y};
-      for (int c = col + 1; c < n; ++c) {
-        const double2 h = W[(size_t)col * cols + c];
-        const HsCd t = hs_mul({h.x, h.y}, {xre[c], xim[c]});
-        s.re = __dsub_rn(s.re, t.re);
-        s.im = __dsub_rn(s.im, t.im);
+      for (int c0 = col + 1; c0 < n; c0 += 32) {
+        HsCd t = {0.0, 0.0};
+        if (c0 + lane < n) {
+          const double2 h = W[(size_t)col * cols + c0 + lane];
+          t = hs_mul({h.x, h.y}, {xre[c0 + lane], xim[c0 + lane]});
+        }
+        const int m = n - c0 < 32 ? n - c0 : 32;
+        for (int l = 0; l < m; ++l) {
+          s.re = __dsub_rn(s.re, __shfl_sync(0xffffffffu, t.re, l));
+          s.im = __dsub_rn(s.im, __shfl_sync(0xffffffffu, t.im, l));
+        }
       }
       const double2 d = W[(size_t)col * cols + col];
       const HsCd x = hs_mul(s, hs_recip({d.x, d.y}));
-      xre[col] = x.re;
-      xim[col] = x.im;
+      if (lane == 0) {
+        xre[col] = x.re;
+        xim[col] = x.im;
+      }
+      __syncwarp();
     }
-    for (int f = 0; f < n; ++f) out[(size_t)q * n + f] = make_float2((float)xre[f], (float)xim[f]);
+    for (int f = lane; f < n; f += 32) out[(size_t)q * n + f] = make_float2((float)xre[f], (float)xim[f]);
   }
 }
 

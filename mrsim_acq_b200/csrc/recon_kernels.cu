@@ -4,6 +4,7 @@
 // :1457-1491), GRAPPA apply (kspace.rs:1605-1632), the radial window (kspace.rs:1327-1342), the
 // centred inverse 2D DFT (`inverse_2d`, kspace.rs:1428-1453) and the Roemer combine
 // (kspace.rs:1343-1373).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -11,7 +12,9 @@
 #include <algorithm>
 
 #include "hermitian_solve.cuh"
+#include "mrsim_internal.h"
 #include "recon_kernels.h"
+#include "row_fft.h"
 
 namespace mrsim {
 
@@ -30,48 +33,70 @@ __device__ __forceinline__ float2 feature(const float2* __restrict__ k, int nx, 
   return k[(size_t)ci * nx * ny + (size_t)sl * nx + kxs];
 }
 
-// One thread per entry of [A^H A | A^H b]: FP64 sums over the reference band in the reference's
-// order (band line, then readout point).
-__global__ void grappa_normal_kernel(const GrappaSystem* __restrict__ sys) {
-  const GrappaSystem& S = sys[blockIdx.y];
-  const int nf = 6 * S.nc;
-  const int cols = nf + S.nc;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nf * cols) return;
-  const int i = e / cols, j = e % cols;
+// The normal equations [A^H A | A^H b], FP64 sums over the reference band in the reference's order (band
+// line, then readout point): a block of 16 x 16 entries of one system, one thread each.  A chunk of
+// readout points' features (16 of the rows, 16 of the columns) is gathered and widened to FP64 once in
+// shared memory for all 256 entries; bound by that memory (two 16-byte reads per four FMAs).  30
+// systems of 8 coils, 23 band lines x 64 points: 219 us, 614 with a gather per entry and term.
+constexpr int kNormTile = 16, kNormChunk = 32;
+__global__ void __launch_bounds__(256) grappa_normal_kernel(const GrappaSystem* __restrict__ sys) {
+  __shared__ double2 fi_s[kNormChunk][kNormTile], fj_s[kNormChunk][kNormTile];
+  const GrappaSystem& S = sys[blockIdx.z];
+  const int nf = 6 * S.nc, nc = S.nc, nx = S.nx, ny = S.ny;
+  const int cols = nf + nc;
+  const int i0 = blockIdx.y * kNormTile, j0 = blockIdx.x * kNormTile;
+  if (i0 >= nf || j0 >= cols) return;
+  const int ti = threadIdx.x / kNormTile, tj = threadIdx.x % kNormTile;
   double ar = 0.0, ai = 0.0;
   for (int b = S.acs_lo; b < S.acs_hi; ++b) {
     const int s0 = b, s1 = b + S.accel, tgt = b + S.d;
     if (s1 > S.acs_hi || tgt > S.acs_hi || !(S.lines[s0] && S.lines[s1] && S.lines[tgt])) continue;
-    for (int kx = 0; kx < S.nx; ++kx) {
-      const float2 fi = feature(S.k, S.nx, S.ny, S.nc, s0, s1, kx, i);
-      float2 fj;
-      if (j < nf)
-        fj = feature(S.k, S.nx, S.ny, S.nc, s0, s1, kx, j);
-      else
-        fj = S.k[(size_t)(j - nf) * S.nx * S.ny + (size_t)tgt * S.nx + kx];
-      const double xr = fi.x, xi = -(double)fi.y, yr = fj.x, yi = fj.y;
-      ar += xr * yr - xi * yi;
-      ai += xr * yi + xi * yr;
+    for (int k0 = 0; k0 < nx; k0 += kNormChunk) {
+      const int nk = min(kNormChunk, nx - k0);
+      for (int e = threadIdx.x; e < 2 * kNormTile * kNormChunk; e += 256) {
+        // neighbouring threads take neighbouring readout points of one feature
+        const int kk = e % kNormChunk, f = e / kNormChunk, side = f / kNormTile, ff = f % kNormTile;
+        const int c = (side ? j0 : i0) + ff;
+        double2 v = make_double2(0.0, 0.0);
+        if (kk < nk && c < (side ? cols : nf)) {
+          const float2 x = c < nf ? feature(S.k, nx, ny, nc, s0, s1, k0 + kk, c)
+                                  : S.k[(size_t)(c - nf) * nx * ny + (size_t)tgt * nx + k0 + kk];
+          v = make_double2((double)x.x, (double)x.y);
+        }
+        (side ? fj_s : fi_s)[kk][ff] = v;
+      }
+      __syncthreads();
+      for (int kk = 0; kk < nk; ++kk) {
+        const double2 a = fi_s[kk][ti], y = fj_s[kk][tj];
+        const double xi = -a.y;
+        ar += a.x * y.x - xi * y.y;
+        ai += a.x * y.y + xi * y.x;
+      }
+      __syncthreads();
     }
   }
-  S.work[(size_t)i * cols + j] = make_double2(ar, ai);
+  if (i0 + ti < nf && j0 + tj < cols) S.work[(size_t)(i0 + ti) * cols + j0 + tj] = make_double2(ar, ai);
 }
 
 // One CTA per system: scale by the mean diagonal, add the Tikhonov term, then the pivoted
-// Gaussian elimination of [H | B] with every right-hand side at once (hermitian_solve.cuh).
-__global__ void __launch_bounds__(256) grappa_solve_kernel(const GrappaSystem* __restrict__ sys, double lambda) {
+// Gaussian elimination of [H | B] with every right-hand side at once (hermitian_solve.cuh), in shared
+// memory where the system fits (16 coils; `shared`): its steps are a chain, and through global memory
+// each took 15 us (30 systems of 48 unknowns: 711 us, here 145).
+__global__ void __launch_bounds__(256) grappa_solve_kernel(const GrappaSystem* __restrict__ sys, double lambda,
+                                                           int shared) {
+  extern __shared__ __align__(16) unsigned char gs_smem[];
   const GrappaSystem& S = sys[blockIdx.x];
   const int nf = 6 * S.nc, nc = S.nc;
   const int cols = nf + nc;
-  double2* W = S.work;
+  double2* W = shared ? reinterpret_cast<double2*>(gs_smem) : S.work;
+  double* scratch = shared ? reinterpret_cast<double*>(W + (size_t)nf * cols) : S.fscratch;
   __shared__ double red_v[256];
   __shared__ int red_i[256];
   __shared__ double s_scale;
   __shared__ int s_zero;
   if (threadIdx.x == 0) {
     double sum = 0.0;
-    for (int i = 0; i < nf; ++i) sum += W[(size_t)i * cols + i].x;
+    for (int i = 0; i < nf; ++i) sum += S.work[(size_t)i * cols + i].x;
     double mean = sum / (double)nf;
     s_zero = !(mean > 0.0);
     s_scale = s_zero ? 0.0 : 1.0 / mean;
@@ -83,35 +108,75 @@ __global__ void __launch_bounds__(256) grappa_solve_kernel(const GrappaSystem* _
   }
   const double sc = s_scale;
   for (int e = threadIdx.x; e < nf * cols; e += blockDim.x) {  // (scale, then add: two roundings)
-    double2 v = W[e];
+    double2 v = S.work[e];
     v.x = __dmul_rn(v.x, sc);
     v.y = __dmul_rn(v.y, sc);
     if (e / cols == e % cols) v.x = __dadd_rn(v.x, lambda);
     W[e] = v;
   }
   __syncthreads();
-  hermitian_solve_block(W, nf, nc, S.fscratch, S.fscratch + nf, S.fscratch + 2 * nf, S.weights, red_v, red_i);
+  hermitian_solve_block(W, nf, nc, scratch, scratch + nf, scratch + 2 * nf, S.weights, red_v, red_i);
 }
 
-// GRAPPA apply: one thread per (missing line, kx, output coil) of one (unit, echo).
-__global__ void grappa_apply_kernel(const ReconJob* __restrict__ jobs, const int4* __restrict__ fills, int n_fills) {
+// GRAPPA apply: one thread per (missing line, kx) of one (unit, echo) and eight output coils at a time:
+// a source sample is read once for the eight, and their weights come from shared memory ([feature][8],
+// one offset d at a time).  600 units, 8 coils, 23 lines of 64: 117 us, 697 with a thread per output
+// coil.
+constexpr int kApplyCoils = 8;
+__global__ void __launch_bounds__(256) grappa_apply_kernel(const ReconJob* __restrict__ jobs,
+                                                           const int4* __restrict__ fills, int n_fills) {
+  extern __shared__ __align__(16) float2 wts[];  // [6 nc][kApplyCoils]
   const ReconJob& J = jobs[blockIdx.y];
   const int nx = J.nx, ny = J.ny, nc = J.nc, nf = 6 * nc;
-  const int total = n_fills * nx * nc;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int co = e % nc;
-    const int kx = (e / nc) % nx;
-    const int4 fl = fills[e / (nc * nx)];  // ky, d, s0, s1
-    const float2* w = J.grappa_w + ((size_t)(fl.y - 1) * nc + co) * nf;
-    float vr = 0.f, vi = 0.f;
-    for (int f = 0; f < nf; ++f) {
-      const float2 x = feature(J.k, nx, ny, nc, fl.z, fl.w, kx, f);
-      const float2 ww = w[f];
-      vr = vr + (ww.x * x.x - ww.y * x.y);
-      vi = vi + (ww.x * x.y + ww.y * x.x);
-    }
-    J.k[(size_t)co * nx * ny + (size_t)fl.x * nx + kx] = make_float2(vr, vi);
+  const size_t per = (size_t)nx * ny;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int first = blockIdx.x * blockDim.x / nx;
+  const int last = min(n_fills - 1, (int)((blockIdx.x + 1) * blockDim.x - 1) / nx);
+  if (first >= n_fills) return;
+  const bool mine = e < n_fills * nx;
+  const int kx = e % nx;
+  const int4 fl = fills[min(e / nx, n_fills - 1)];  // ky, d, s0, s1 (by d)
+  int kxs[3];
+#pragma unroll
+  for (int ki = 0; ki < 3; ++ki) {
+    const int x = kx + ki - 1;
+    kxs[ki] = x < 0 ? x + nx : (x >= nx ? x - nx : x);
   }
+  for (int d = fills[first].y; d <= fills[last].y; ++d)
+    for (int co0 = 0; co0 < nc; co0 += kApplyCoils) {
+      __syncthreads();  // every thread is done with the weights before
+      for (int t = threadIdx.x; t < nf * kApplyCoils; t += blockDim.x) {
+        const int c = t / nf, f = t % nf;
+        wts[f * kApplyCoils + c] =
+            co0 + c < nc ? J.grappa_w[((size_t)(d - 1) * nc + co0 + c) * nf + f] : make_float2(0.f, 0.f);
+      }
+      __syncthreads();
+      if (!mine || fl.y != d) continue;
+      float vr[kApplyCoils], vi[kApplyCoils];
+#pragma unroll
+      for (int c = 0; c < kApplyCoils; ++c) vr[c] = vi[c] = 0.f;
+#pragma unroll
+      for (int li = 0; li < 2; ++li)
+#pragma unroll
+        for (int ki = 0; ki < 3; ++ki) {
+          const float2* src = J.k + (size_t)(li == 0 ? fl.z : fl.w) * nx + kxs[ki];
+          const float2* w = wts + (li * 3 + ki) * nc * kApplyCoils;
+          for (int ci = 0; ci < nc; ++ci) {
+            const float2 x = src[ci * per];
+#pragma unroll
+            for (int c = 0; c < kApplyCoils; c += 2) {
+              const float4 w2 = *reinterpret_cast<const float4*>(w + ci * kApplyCoils + c);
+              vr[c] = vr[c] + (w2.x * x.x - w2.y * x.y);
+              vi[c] = vi[c] + (w2.x * x.y + w2.y * x.x);
+              vr[c + 1] = vr[c + 1] + (w2.z * x.x - w2.w * x.y);
+              vi[c + 1] = vi[c + 1] + (w2.z * x.y + w2.w * x.x);
+            }
+          }
+        }
+#pragma unroll
+      for (int c = 0; c < kApplyCoils; ++c)
+        if (co0 + c < nc) J.k[(co0 + c) * per + (size_t)fl.x * nx + kx] = make_float2(vr[c], vi[c]);
+    }
 }
 
 // Window, inverse DFT and Roemer combine of one (unit, echo): one CTA per block of YB image rows.
@@ -204,6 +269,106 @@ __global__ void __launch_bounds__(256) recon_combine_kernel(const ReconJob* __re
   }
 }
 
+// The same by FFTs, for matrices of 32 E points per axis (E <= 4): a cluster of blocks per (unit, echo),
+// each taking every S-th coil.  A coil's k-space is windowed and row-transformed by a warp per row as it
+// is read, column-transformed in shared memory, and added to the block's Roemer sums in registers;
+// the cluster adds those in rank order.  With xs = nx/2 and ys = ny/2 multiples of 16 the centred
+// transform is the plain one between sign flips: e^{-i2pi (k - s)(x - s)/n} = (-1)^(k + x) e^{-i2pi kx/n}.
+// One cluster of S = 1 per unit fills the chip from 592 units on; fewer units share their coils among up to
+// 8 blocks.  600 units of 64 x 64 x 8 coils: 208 us, 0.76 TB/s of k-space; as direct sums 2142
+// us (64-term sums at 12 % of the FMA rate).
+template <int EX, int EY>
+struct ReconShape {
+  static constexpr int NX = 32 * EX, NY = 32 * EY, LD = NX + 1;
+  static constexpr int T = NX * NY >= 8192 ? 512 : 256, NW = T / 32, NP = NX * NY / T;
+  static constexpr size_t smem = sizeof(float2) * ((size_t)NY * LD + NX + NY);
+};
+
+template <int EX, int EY>
+__global__ void __launch_bounds__(ReconShape<EX, EY>::T) recon_fft_kernel(const ReconJob* __restrict__ jobs) {
+  using R = ReconShape<EX, EY>;
+  constexpr int NX = R::NX, NY = R::NY, LD = R::LD, T = R::T, NW = R::NW, NP = R::NP;
+  constexpr int LX = log2_c(EX), LY = log2_c(EY);
+  constexpr bool PX = (EX & (EX - 1)) == 0, PY = (EY & (EY - 1)) == 0;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* img = sm;             // [NY][LD]
+  float2* twx = img + NY * LD;  // e^{-i2pi j/NX}
+  float2* twy = twx + NX;
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const ReconJob& J = jobs[blockIdx.x / S];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nc = J.nc;
+  for (int i = tid; i < NX; i += T) twx[i] = J.ex_tab[i];
+  for (int i = tid; i < NY; i += T) twy[i] = J.ey_tab[i];
+  float2 acc[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) acc[p] = make_float2(0.f, 0.f);
+  __syncthreads();
+  const int k2 = (int)(__brev(lane) >> 27);
+  for (int q = rank; q < nc; q += S) {
+    const float2* kq = J.k + (size_t)q * NX * NY;
+    for (int ky = warp; ky < NY; ky += NW) {
+      float2 b[EX];
+#pragma unroll
+      for (int m = 0; m < EX; ++m) {
+        const int kx = lane + 32 * m;
+        float2 v = kq[ky * NX + kx];
+        float w = J.window ? J.window[ky * NX + kx] : 1.f;
+        w = ((kx + ky) & 1) ? -w : w;
+        b[PX ? bitrev_c(m, LX) : m] = make_float2(v.x * w, v.y * w);
+      }
+      warp_row_fft<EX, true>(b, twx, lane);
+#pragma unroll
+      for (int k1 = 0; k1 < EX; ++k1) img[ky * LD + k1 + EX * k2] = b[k1];
+    }
+    __syncthreads();
+    for (int x = warp; x < NX; x += NW) {
+      float2 b[EY];
+#pragma unroll
+      for (int m = 0; m < EY; ++m) b[PY ? bitrev_c(m, LY) : m] = img[(lane + 32 * m) * LD + x];
+      warp_row_fft<EY, true>(b, twy, lane);
+#pragma unroll
+      for (int k1 = 0; k1 < EY; ++k1) img[(k1 + EY * k2) * LD + x] = b[k1];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int i = tid + p * T, y = i / NX, x = i % NX;
+      float2 v = img[y * LD + x];
+      if ((x + y) & 1) v = make_float2(-v.x, -v.y);
+      if (J.coil_images) J.coil_images[(size_t)q * NX * NY + i] = v;
+      const float s = J.sens[(size_t)q * NX * NY + i];
+      acc[p].x = fmaf(s, v.x, acc[p].x);
+      acc[p].y = fmaf(s, v.y, acc[p].y);
+    }
+    __syncthreads();
+  }
+  if (S == 1) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int i = tid + p * T;
+      const float inv = J.inv_ssum[i];
+      J.combined[i] = make_float2(acc[p].x * inv, acc[p].y * inv);
+    }
+    return;
+  }
+  float2* part = img;  // [pixel]
+#pragma unroll
+  for (int p = 0; p < NP; ++p) part[tid + p * T] = acc[p];
+  cl.sync();
+  for (int i = rank * T + tid; i < NX * NY; i += S * T) {
+    float2 v = cl.map_shared_rank(part, 0)[i];
+    for (int r = 1; r < S; ++r) {
+      const float2 o = cl.map_shared_rank(part, r)[i];
+      v.x += o.x;
+      v.y += o.y;
+    }
+    const float inv = J.inv_ssum[i];
+    J.combined[i] = make_float2(v.x * inv, v.y * inv);
+  }
+  cl.sync();  // no block leaves while another reads its sums
+}
+
 __global__ void window_copy_kernel(const ReconJob* __restrict__ jobs) {
   const ReconJob& J = jobs[blockIdx.y];
   if (!J.reconstructed) return;  // only the captured slices keep their reconstructed k-space
@@ -221,28 +386,75 @@ __global__ void window_copy_kernel(const ReconJob* __restrict__ jobs) {
 
 }  // namespace
 
+namespace {
+template <int EX, int EY>
+void launch_recon_fft(const ReconJob* d_jobs, int n_jobs, int nc, cudaStream_t st) {
+  using R = ReconShape<EX, EY>;
+  auto k = recon_fft_kernel<EX, EY>;
+  if (R::smem > 48 * 1024)
+    MRSIM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem));
+  int S = 1;
+  while (2 * S <= std::min(8, nc) && (long long)n_jobs * 2 * S <= 592) S *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(n_jobs * S));
+  cfg.blockDim = dim3(R::T);
+  cfg.dynamicSmemBytes = R::smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)S;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  MRSIM_CUDA(cudaLaunchKernelEx(&cfg, k, d_jobs));
+}
+
+template <int EX>
+void launch_recon_fft_y(int ey, const ReconJob* d_jobs, int n_jobs, int nc, cudaStream_t st) {
+  switch (ey) {
+    case 1: launch_recon_fft<EX, 1>(d_jobs, n_jobs, nc, st); break;
+    case 2: launch_recon_fft<EX, 2>(d_jobs, n_jobs, nc, st); break;
+    case 3: launch_recon_fft<EX, 3>(d_jobs, n_jobs, nc, st); break;
+    default: launch_recon_fft<EX, 4>(d_jobs, n_jobs, nc, st); break;
+  }
+}
+}  // namespace
+
 void launch_grappa_fit(const GrappaSystem* d_sys, int n_sys, int max_nc, double lambda, cudaStream_t st) {
   if (n_sys <= 0) return;
   const int nf = 6 * max_nc, cols = nf + max_nc;
-  dim3 grid((nf * cols + 127) / 128, n_sys);
-  grappa_normal_kernel<<<grid, 128, 0, st>>>(d_sys);
-  grappa_solve_kernel<<<n_sys, 256, 0, st>>>(d_sys, lambda);
+  const dim3 grid((cols + kNormTile - 1) / kNormTile, (nf + kNormTile - 1) / kNormTile, n_sys);
+  grappa_normal_kernel<<<grid, 256, 0, st>>>(d_sys);
+  const size_t smem = (size_t)nf * cols * sizeof(double2) + (size_t)(2 * nf + max_nc * 2 * nf) * sizeof(double);
+  constexpr size_t kMost = 216 * 1024;  // beside 3 KB of static shared memory
+  const bool shared = smem <= kMost;
+  if (shared && smem > 40 * 1024)
+    MRSIM_CUDA(cudaFuncSetAttribute(grappa_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+  grappa_solve_kernel<<<n_sys, 256, shared ? smem : 0, st>>>(d_sys, lambda, shared ? 1 : 0);
 }
 
 void launch_grappa_apply(const ReconJob* d_jobs, int n_jobs, const int4* d_fills, int n_fills, int nx, int nc,
                          cudaStream_t st) {
   if (n_jobs <= 0 || n_fills <= 0) return;
-  const int total = n_fills * nx * nc;
-  dim3 grid(std::min((total + 255) / 256, 1024), n_jobs);
-  grappa_apply_kernel<<<grid, 256, 0, st>>>(d_jobs, d_fills, n_fills);
+  const dim3 grid(((long long)n_fills * nx + 255) / 256, n_jobs);
+  grappa_apply_kernel<<<grid, 256, sizeof(float2) * 6 * nc * kApplyCoils, st>>>(d_jobs, d_fills, n_fills);
 }
 
-void launch_recon_combine(const ReconJob* d_jobs, int n_jobs, int nx, int ny, bool capture_reconstructed,
+void launch_recon_combine(const ReconJob* d_jobs, int n_jobs, int nx, int ny, int nc, bool capture_reconstructed,
                           cudaStream_t st) {
   if (n_jobs <= 0) return;
   if (capture_reconstructed) {
     dim3 g(64, n_jobs);
     window_copy_kernel<<<g, 256, 0, st>>>(d_jobs);
+  }
+  if (nx % 32 == 0 && ny % 32 == 0 && nx <= 128 && ny <= 128) {
+    switch (nx / 32) {
+      case 1: launch_recon_fft_y<1>(ny / 32, d_jobs, n_jobs, nc, st); break;
+      case 2: launch_recon_fft_y<2>(ny / 32, d_jobs, n_jobs, nc, st); break;
+      case 3: launch_recon_fft_y<3>(ny / 32, d_jobs, n_jobs, nc, st); break;
+      default: launch_recon_fft_y<4>(ny / 32, d_jobs, n_jobs, nc, st); break;
+    }
+    return;
   }
   const int YB = std::max(1, std::min(8, 1024 / nx));
   dim3 grid((ny + YB - 1) / YB, n_jobs);

@@ -12,7 +12,7 @@ struct GrappaSystem {
   const uint8_t* lines;    // ny acquired-line flags of the reference scan (device)
   int nx, ny, nc, accel, d, acs_lo, acs_hi, pad;
   double2* work;           // nf*(nf+nc) FP64 complex: [A^H A | A^H b]
-  double* fscratch;        // 2*nf + nc*2*nf FP64
+  double* fscratch;        // 2*nf + nc*2*nf FP64 (used where the system does not fit shared memory)
   float2* weights;         // out: [nc][nf] complex f32 for this d
 };
 
@@ -32,10 +32,11 @@ struct ReconJob {
 };
 
 void launch_grappa_fit(const GrappaSystem* d_sys, int n_sys, int max_nc, double lambda, cudaStream_t st);
-// fills: (ky, d, s0, s1) of every line GRAPPA synthesises (the same for every job of the launch)
+// fills: (ky, d, s0, s1) of every line GRAPPA synthesises, by d (the same for every job of the launch)
 void launch_grappa_apply(const ReconJob* d_jobs, int n_jobs, const int4* d_fills, int n_fills, int nx, int nc,
                          cudaStream_t st);
-void launch_recon_combine(const ReconJob* d_jobs, int n_jobs, int nx, int ny, bool capture_reconstructed,
+// nc: the coils of every job
+void launch_recon_combine(const ReconJob* d_jobs, int n_jobs, int nx, int ny, int nc, bool capture_reconstructed,
                           cudaStream_t st);
 
 }  // namespace mrsim

@@ -457,7 +457,7 @@ void simulate_slice_full(mrsim_context* ctx, const mrsim_slice_input& inp, const
   J.nc = nc;
   const ReconJob* d_job = (const ReconJob*)A.upload(&J, sizeof J, st);
   if (accel > 1) launch_grappa_apply(d_job, 1, T.fills, T.n_fills, nx, nc, st);
-  launch_recon_combine(d_job, 1, nx, ny, out.reconstructed != nullptr, st);
+  launch_recon_combine(d_job, 1, nx, ny, nc, out.reconstructed != nullptr, st);
   MRSIM_CUDA(cudaGetLastError());
   MRSIM_CUDA(cudaMemcpyAsync(out.combined, J.combined, per * sizeof(float2), cudaMemcpyDeviceToHost, st));
   if (out.coil_images)
@@ -801,7 +801,7 @@ void acquire_series(mrsim_context* ctx, const mrsim_acquisition_input& in, const
       }
     const ReconJob* d_jobs = (const ReconJob*)C.upload(jobs.data(), jobs.size() * sizeof(ReconJob), st);
     if (accel > 1) launch_grappa_apply(d_jobs, (int)jobs.size(), T.fills, T.n_fills, nx, nc, st);
-    launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, cap_rec != nullptr, st);
+    launch_recon_combine(d_jobs, (int)jobs.size(), nx, ny, nc, cap_rec != nullptr, st);
     MRSIM_CUDA(cudaGetLastError());
     for (int g = g0; g < g1; ++g)
       for (int s = 0; s < nsl; ++s)
