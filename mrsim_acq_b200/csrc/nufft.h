@@ -76,6 +76,20 @@ void nufft_type1(const NufftGridT<R>& g, const double* u, int npts, const NufftB
                  const typename Vec2<R>::type* wts, int batch, size_t w_stride, typename Vec2<R>::type* modes,
                  size_t mode_stride, typename Vec2<R>::type* work, int sign, cudaStream_t st);
 
+// Type 2 of a batch of FP32 mode grids (packed [item][m1][m0]) at points ordered by window origin
+// (nufft_tiled.cu), sign +1: out[point][item].  grid: batch fine grids; tmp: batch x m_out1 x nf0.
+struct NufftPoints {
+  const double* u = nullptr;
+  int npts = 0, tiles0 = 0, max_items = 0;
+  int4* items = nullptr;
+  int* n_items = nullptr;
+  const int* pts = nullptr;
+};
+bool nufft_tiled_fits(const NufftGrid& g);
+NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, cudaStream_t st);
+void nufft_type2_tiled(const NufftGrid& g, const float2* modes, int batch, const NufftPoints& P, float2* out,
+                       float2* grid, float2* tmp, cudaStream_t st);
+
 // The 1D type-1 NUFFT (`Nufft1`, nufft.rs:25-112) in FP64: sources at `pos` (cells, period n),
 // outputs at integer frequencies k_lo .. k_lo + n_out, F[k] = sum_j w_j e^{+i2pi k pos_j / n}, for
 // nw weight vectors sharing the positions.  corr and tw on the device; work holds nw fine grids.
@@ -110,7 +124,8 @@ void spiral_exact(const SpiralExactArgs& a, cudaStream_t st);
 
 void segment_images(const float2* x, const float2* rate, int nvox, const double* tau_l, int L, float2* out,
                     cudaStream_t st);
+// seg [l][point], or with by_point [point][l]
 void segment_combine(const float2* seg, int npts, int L, const int* tau_idx, const double* b, const float2* stat,
-                     float2* out, cudaStream_t st);
+                     float2* out, bool by_point, cudaStream_t st);
 
 }  // namespace mrsim

@@ -13,6 +13,7 @@
 
 #include <algorithm>
 
+#include "es_taps.cuh"
 #include "nufft.h"
 
 namespace mrsim {
@@ -34,28 +35,6 @@ template <>
 __device__ __forceinline__ double2 mk2<double>(double a, double b) {
   return make_double2(a, b);
 }
-__device__ __forceinline__ float es_exp(float x) { return __expf(x); }
-__device__ __forceinline__ double es_exp(double x) { return exp(x); }
-
-constexpr int kWMax = 16;
-
-// First fine cell and the w taps of coordinate u (period n) on a fine grid of nf = 2n cells.
-template <class R>
-__device__ __forceinline__ int es_taps(double u, int nf, int w, R beta, R* k) {
-  const double half = 0.5 * w;
-  double p = fmod(2.0 * u, (double)nf);
-  if (p < 0.0) p += nf;
-  const int m0 = (int)floor(p - half) + 1;
-  const R ih = (R)(1.0 / half);
-#pragma unroll
-  for (int i = 0; i < kWMax; ++i) {
-    if (i >= w) break;
-    const R z = (R)((double)(m0 + i) - p) * ih;
-    k[i] = fabs(z) < (R)1 ? es_exp(beta * (sqrt((R)1 - z * z) - (R)1)) : (R)0;
-  }
-  return m0;
-}
-
 template <class R>
 __global__ void place_kernel(const NufftGridT<R> g, const typename Vec2<R>::type* __restrict__ modes,
                              typename Vec2<R>::type* __restrict__ grid, int batch, size_t mode_stride,
@@ -435,12 +414,12 @@ __global__ void segment_images_kernel(const float2* __restrict__ x, const float2
 // out_j = stat_j * sum_l b[tau_idx_j][l] * seg[l][j]
 __global__ void segment_combine_kernel(const float2* __restrict__ seg, int npts, int L, const int* __restrict__ tau_idx,
                                        const double* __restrict__ b, const float2* __restrict__ stat,
-                                       float2* __restrict__ out) {
+                                       float2* __restrict__ out, int by_point) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < npts; j += gridDim.x * blockDim.x) {
     const double* bj = b + (size_t)tau_idx[j] * L * 2;
     float re = 0.f, im = 0.f;
     for (int l = 0; l < L; ++l) {
-      const float2 v = seg[(size_t)l * npts + j];
+      const float2 v = seg[by_point ? (size_t)j * L + l : (size_t)l * npts + j];
       const float br = (float)bj[2 * l], bi = (float)bj[2 * l + 1];
       re = fmaf(br, v.x, fmaf(-bi, v.y, re));
       im = fmaf(br, v.y, fmaf(bi, v.x, im));
@@ -540,8 +519,8 @@ void segment_images(const float2* x, const float2* rate, int nvox, const double*
 }
 
 void segment_combine(const float2* seg, int npts, int L, const int* tau_idx, const double* b, const float2* stat,
-                     float2* out, cudaStream_t st) {
-  segment_combine_kernel<<<(npts + 255) / 256, 256, 0, st>>>(seg, npts, L, tau_idx, b, stat, out);
+                     float2* out, bool by_point, cudaStream_t st) {
+  segment_combine_kernel<<<(npts + 255) / 256, 256, 0, st>>>(seg, npts, L, tau_idx, b, stat, out, by_point ? 1 : 0);
 }
 
 }  // namespace mrsim

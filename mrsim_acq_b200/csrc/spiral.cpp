@@ -359,12 +359,18 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
   const double* du = (const double*)A.upload(k, (size_t)npts * 2 * 8, st);
   float2* seg = (float2*)A.alloc((size_t)L * npts * sizeof(float2));
   float2* work = (float2*)A.alloc((size_t)L * g.nf0 * g.nf1 * sizeof(float2));
-  nufft_type2<float>(g, imgs, L, n, du, npts, seg, npts, work, 1, nullptr, st);
+  const bool tiled = nufft_tiled_fits(g);
+  if (tiled) {
+    float2* tmp = (float2*)A.alloc((size_t)L * g.m_out1 * g.nf0 * sizeof(float2));
+    nufft_type2_tiled(g, imgs, L, nufft_points(A, g, du, npts, st), seg, work, tmp, st);
+  } else {
+    nufft_type2<float>(g, imgs, L, n, du, npts, seg, npts, work, 1, nullptr, st);
+  }
   const double* db = (const double*)A.upload(plan.b.data(), plan.b.size() * 8, st);
   const float2* dstat = (const float2*)A.upload(stat.data(), stat.size() * sizeof(float2), st);
   const int* dti = (const int*)A.upload(tidx.data(), tidx.size() * 4, st);
   float2* dout = (float2*)A.alloc((size_t)npts * sizeof(float2));
-  segment_combine(seg, npts, L, dti, db, dstat, dout, st);
+  segment_combine(seg, npts, L, dti, db, dstat, dout, tiled, st);
   MRSIM_CUDA(cudaGetLastError());
   MRSIM_CUDA(cudaMemcpyAsync(out, dout, (size_t)npts * sizeof(float2), cudaMemcpyDeviceToHost, st));
   MRSIM_CUDA(cudaStreamSynchronize(st));

@@ -157,23 +157,24 @@ __global__ void seg_images_kernel(const SegSlot* __restrict__ slots, const float
   }
 }
 
-// k2[slot][j] = stat_j sum_l b[j % ns][l] seg_out[slot][l][j]
+// k2[slot][j] = stat_j sum_l b[j % ns][l] seg_out[slot][l][j] (items > 0: seg_out[j][items], the slot's
+// segments in a run)
 __global__ void seg_combine_kernel(const float2* __restrict__ seg, const int* __restrict__ slot_base,
                                    const int* __restrict__ slot_plan, const double* __restrict__ b0,
                                    const double* __restrict__ b1, int L0, int L1, int ns, int nsamp,
                                    const float2* __restrict__ stat, float2* __restrict__ k2,
-                                   const size_t* __restrict__ k2_off) {
+                                   const size_t* __restrict__ k2_off, int items) {
   const int s = blockIdx.y;
   const int plan = slot_plan[s];
   const int L = plan ? L1 : L0;
   const double* b = plan ? b1 : b0;
-  const float2* sg = seg + (size_t)slot_base[s] * nsamp;
+  const float2* sg = seg + (size_t)slot_base[s] * (items ? 1 : nsamp);
   float2* out = k2 + k2_off[s];
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nsamp; j += gridDim.x * blockDim.x) {
     const double* bj = b + (size_t)(j % ns) * L * 2;
     float re = 0.f, im = 0.f;
     for (int l = 0; l < L; ++l) {
-      const float2 v = sg[(size_t)l * nsamp + j];
+      const float2 v = sg[items ? (size_t)j * items + l : (size_t)l * nsamp + j];
       const float br = (float)bj[2 * l], bi = (float)bj[2 * l + 1];
       re += br * v.x - bi * v.y;
       im += br * v.y + bi * v.x;
@@ -572,7 +573,8 @@ struct SpiralPlan3 {
   Spiral3dTable table;
   std::vector<CompMode> modes;
   bool any_class = false, any_voxel = false;
-  std::vector<TsegPlan> class_plan, voxel_plan;  // per slice (empty if the mode is unused)
+  std::vector<TsegPlan> plans;               // the distinct segmentations
+  std::vector<int> cls_of, vox_of;           // per slice: its plan in each mode (-1: the mode is unused)
   std::vector<float2> zk;
   std::vector<double2> zk_d;
   struct Src {
@@ -660,8 +662,6 @@ static SpiralPlan3 make_spiral_plan(const mrsim_acquisition_3d_input& in, const 
   P.modes = resolve_modes(in.t2, in.t1, in.t_inhom, P.ncomp, acq, train, P.nvox);
   for (auto& m : P.modes) (m.voxel ? P.any_voxel : P.any_class) = true;
   build_sources(P, acq);
-  P.class_plan.resize(P.nz);
-  P.voxel_plan.resize(P.nz);
   // per-slice certified segmentations: each distinct rate rectangle planned once (slices that
   // share one get the same plan bit for bit), the distinct ones on up to 16 host threads, each
   // with its fits' per-sample work on the device on a stream of its own; the first failure in
@@ -719,10 +719,9 @@ static SpiralPlan3 make_spiral_plan(const mrsim_acquisition_3d_input& in, const 
   if (setup_err) std::rethrow_exception(setup_err);
   for (auto& e : errs)
     if (e) std::rethrow_exception(e);
-  for (int z = 0; z < P.nz; ++z) {
-    if (cls_of[z] >= 0) P.class_plan[z] = plans[cls_of[z]];
-    if (vox_of[z] >= 0) P.voxel_plan[z] = plans[vox_of[z]];
-  }
+  P.plans = std::move(plans);
+  P.cls_of = cls_of;
+  P.vox_of = vox_of;
   // the centred z-DFT kernel, the ring z profiles, the object phase, the half-cell phase
   const double zs = (double)(P.nz / 2);
   P.zk.resize((size_t)P.nz * P.nz);
@@ -869,62 +868,73 @@ static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, c
   const float2* d_stat = (const float2*)C.upload(P.stat.data(), P.stat.size() * sizeof(float2), st);
   float2* k2 = (float2*)C.alloc((size_t)nvar * ring * nsrc * nz * nsamp * sizeof(float2));
   MRSIM_CUDA(cudaMemsetAsync(k2, 0, (size_t)nvar * ring * nsrc * nz * nsamp * sizeof(float2), st));
-  // per slice: slots (a, s) with their plans
-  int Lmax = 1;
-  for (int z = 0; z < nz; ++z) Lmax = std::max({Lmax, P.class_plan[z].l, P.voxel_plan[z].l});
+  // per slice: slots (a, s) with their plans; the plans' tables and every slice's slots go up once, so
+  // the slices are launches alone
+  auto plan_at = [&](int i) -> const TsegPlan* { return i >= 0 ? &P.plans[i] : nullptr; };
   const int nslot = nvar * ring * nsrc;
-  float2* seg = (float2*)C.alloc((size_t)nslot * Lmax * P.plane * sizeof(float2));
-  float2* segout = (float2*)C.alloc((size_t)nslot * Lmax * nsamp * sizeof(float2));
-  float2* work = (float2*)C.alloc((size_t)nslot * Lmax * grid.nf0 * grid.nf1 * sizeof(float2));
-  SegSlot* d_slots = (SegSlot*)C.alloc((size_t)nslot * sizeof(SegSlot));
-  int* d_base = (int*)C.alloc((size_t)nslot * 4);
-  int* d_plan = (int*)C.alloc((size_t)nslot * 4);
-  size_t* d_off = (size_t*)C.alloc((size_t)nslot * sizeof(size_t));
+  std::vector<const double*> d_tl(P.plans.size()), d_b(P.plans.size());
+  for (size_t i = 0; i < P.plans.size(); ++i) {
+    d_tl[i] = (const double*)C.upload(P.plans[i].tau_l.data(), P.plans[i].tau_l.size() * 8, st);
+    d_b[i] = (const double*)C.upload(P.plans[i].b.data(), P.plans[i].b.size() * 8, st);
+  }
+  std::vector<SegSlot> slots((size_t)nz * nslot);
+  std::vector<int> base((size_t)nz * nslot), plan((size_t)nz * nslot), tot(nz, 0);
+  std::vector<size_t> off((size_t)nz * nslot);
+  int most = 1;
   for (int z = 0; z < nz; ++z) {
-    const TsegPlan& pc = P.class_plan[z];
-    const TsegPlan& pv = P.voxel_plan[z];
-    std::vector<SegSlot> slots(nslot);
-    std::vector<int> base(nslot), plan(nslot);
-    std::vector<size_t> off(nslot);
-    int tot = 0;
+    const TsegPlan *pc = plan_at(P.cls_of[z]), *pv = plan_at(P.vox_of[z]);
     for (int v = 0; v < nvar; ++v)
-    for (int a = 0; a < ring; ++a)
-      for (int s = 0; s < nsrc; ++s) {
-        const int i = (v * ring + a) * nsrc + s;
-        const SpiralPlan3::Src& S = P.srcs[s];
-        const bool voxel = P.modes[S.c].voxel;
-        SegSlot& sl = slots[i];
-        std::memset(&sl, 0, sizeof sl);
-        sl.comp = v > 0 ? V->img[(size_t)v][S.c] + (size_t)z * P.plane
-                        : I.img + (((size_t)g * nz + z) * P.ncomp + S.c) * P.plane;
-        sl.amp = I.amp + (size_t)a * P.plane;
-        sl.plan = voxel ? 1 : 0;
-        if (voxel) {
-          const int etl = (int)P.modes[S.c].maps.size();
-          sl.la = I.lna + ((size_t)S.c * etl + (S.e - 1)) * P.nvox + (size_t)z * P.plane;
-          sl.decay = I.decay + (size_t)S.c * P.nvox + (size_t)z * P.plane;
+      for (int a = 0; a < ring; ++a)
+        for (int s = 0; s < nsrc; ++s) {
+          const int i = (v * ring + a) * nsrc + s;
+          const size_t at = (size_t)z * nslot + i;
+          const SpiralPlan3::Src& S = P.srcs[s];
+          const bool voxel = P.modes[S.c].voxel;
+          SegSlot& sl = slots[at];
+          std::memset(&sl, 0, sizeof sl);
+          sl.comp = v > 0 ? V->img[(size_t)v][S.c] + (size_t)z * P.plane
+                          : I.img + (((size_t)g * nz + z) * P.ncomp + S.c) * P.plane;
+          sl.amp = I.amp + (size_t)a * P.plane;
+          sl.plan = voxel ? 1 : 0;
+          if (voxel) {
+            const int etl = (int)P.modes[S.c].maps.size();
+            sl.la = I.lna + ((size_t)S.c * etl + (S.e - 1)) * P.nvox + (size_t)z * P.plane;
+            sl.decay = I.decay + (size_t)S.c * P.nvox + (size_t)z * P.plane;
+          }
+          base[at] = tot[z];
+          plan[at] = sl.plan;
+          tot[z] += voxel ? (pv ? pv->l : 0) : (pc ? pc->l : 0);
+          off[at] = (((size_t)(v * ring + a) * nsrc + s) * nz + z) * nsamp;
         }
-        base[i] = tot;
-        plan[i] = sl.plan;
-        tot += voxel ? pv.l : pc.l;
-        off[i] = ((((size_t)v * ring + a) * nsrc + s) * nz + z) * nsamp;
-      }
-    if (tot == 0) continue;
-    MRSIM_CUDA(cudaMemcpyAsync(d_slots, slots.data(), slots.size() * sizeof(SegSlot), cudaMemcpyHostToDevice, st));
-    MRSIM_CUDA(cudaMemcpyAsync(d_base, base.data(), base.size() * 4, cudaMemcpyHostToDevice, st));
-    MRSIM_CUDA(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * 4, cudaMemcpyHostToDevice, st));
-    MRSIM_CUDA(cudaMemcpyAsync(d_off, off.data(), off.size() * sizeof(size_t), cudaMemcpyHostToDevice, st));
-    DevArena Z(ctx);
-    const double* tl0 = pc.l ? (const double*)Z.upload(pc.tau_l.data(), pc.tau_l.size() * 8, st) : nullptr;
-    const double* tl1 = pv.l ? (const double*)Z.upload(pv.tau_l.data(), pv.tau_l.size() * 8, st) : nullptr;
-    const double* b0 = pc.l ? (const double*)Z.upload(pc.b.data(), pc.b.size() * 8, st) : nullptr;
-    const double* b1 = pv.l ? (const double*)Z.upload(pv.b.data(), pv.b.size() * 8, st) : nullptr;
-    seg_images_kernel<<<g3(P.plane, nslot, 1), 256, 0, st>>>(d_slots, I.cis0 + (size_t)z * P.plane,
+    most = std::max(most, tot[z]);
+  }
+  const SegSlot* d_slots = (const SegSlot*)C.upload(slots.data(), slots.size() * sizeof(SegSlot), st);
+  const int* d_base = (const int*)C.upload(base.data(), base.size() * 4, st);
+  const int* d_plan = (const int*)C.upload(plan.data(), plan.size() * 4, st);
+  const size_t* d_off = (const size_t*)C.upload(off.data(), off.size() * sizeof(size_t), st);
+  const bool tiled = nufft_tiled_fits(grid);
+  float2* seg = (float2*)C.alloc((size_t)most * P.plane * sizeof(float2));
+  float2* segout = (float2*)C.alloc((size_t)most * nsamp * sizeof(float2));
+  float2* work = (float2*)C.alloc((size_t)most * grid.nf0 * grid.nf1 * sizeof(float2));
+  float2* tmp = tiled ? (float2*)C.alloc((size_t)most * grid.m_out1 * grid.nf0 * sizeof(float2)) : nullptr;
+  NufftPoints points;
+  if (tiled) points = nufft_points(C, grid, d_k, nsamp, st);
+  for (int z = 0; z < nz; ++z) {
+    if (tot[z] == 0) continue;
+    const TsegPlan *pc = plan_at(P.cls_of[z]), *pv = plan_at(P.vox_of[z]);
+    const int lc = pc ? pc->l : 0, lv = pv ? pv->l : 0;
+    const double *tl0 = pc ? d_tl[P.cls_of[z]] : nullptr, *tl1 = pv ? d_tl[P.vox_of[z]] : nullptr;
+    const double *b0 = pc ? d_b[P.cls_of[z]] : nullptr, *b1 = pv ? d_b[P.vox_of[z]] : nullptr;
+    const size_t at = (size_t)z * nslot;
+    seg_images_kernel<<<g3(P.plane, nslot, 1), 256, 0, st>>>(d_slots + at, I.cis0 + (size_t)z * P.plane,
                                                              I.fmap ? I.fmap + (size_t)z * P.plane : nullptr, tl0, tl1,
-                                                             pc.l, pv.l, (int)P.plane, seg, d_base);
-    nufft_type2<float>(grid, seg, tot, P.plane, d_k, nsamp, segout, nsamp, work, 1, nullptr, st);
-    seg_combine_kernel<<<g3(nsamp, nslot, 1), 256, 0, st>>>(segout, d_base, d_plan, b0, b1, pc.l, pv.l, P.ns, nsamp,
-                                                            d_stat, k2, d_off);
+                                                             lc, lv, (int)P.plane, seg, d_base + at);
+    if (tiled)
+      nufft_type2_tiled(grid, seg, tot[z], points, segout, work, tmp, st);
+    else
+      nufft_type2<float>(grid, seg, tot[z], P.plane, d_k, nsamp, segout, nsamp, work, 1, nullptr, st);
+    seg_combine_kernel<<<g3(nsamp, nslot, 1), 256, 0, st>>>(segout, d_base + at, d_plan + at, b0, b1, lc, lv, P.ns,
+                                                            nsamp, d_stat, k2, d_off + at, tiled ? tot[z] : 0);
     MRSIM_CUDA(cudaGetLastError());
   }
   // the z-DFT with the rings' profiles, amplitudes and line weights

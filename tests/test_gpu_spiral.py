@@ -323,3 +323,29 @@ def test_nufft1_integer_positions_reduce_to_the_dft(gpu_ctx):
 def test_nufft1_refuses_a_band_outside_nyquist(gpu_ctx):
     with pytest.raises(MrsimError, match="coarse Nyquist band"):
         S.Nufft1(16, -9, 16, 1e-12, ctx=gpu_ctx).run(np.zeros(3), [np.zeros(3, complex)])
+
+
+@pytest.mark.parametrize("sx,sy,npts,fmax", [(32, 32, 1, 20.0), (64, 96, 1003, 150.0), (128, 32, 517, 300.0),
+                                             (96, 128, 2001, 60.0)])
+def test_tiled_type2_matches_the_oracle(gpu_ctx, sx, sy, npts, fmax):
+    # fine grids of whole tiles: windows that wrap on both axes, crowded origins (more points than a
+    # group), and segment counts on both sides of 16 and 32
+    rng = np.random.default_rng(sx + npts)
+    x, y = np.meshgrid((np.arange(sx) + 0.5) / sx, (np.arange(sy) + 0.5) / sy)
+    img = np.exp(-((x - 0.4) ** 2 + (y - 0.5) ** 2) / 0.02).astype(np.float32).ravel()
+    fmap = (fmax * (x - 0.2 * y)).astype(np.float32).ravel()
+    inp = SliceInput(compartments=[img], t2=[T2.uniform(70.0)], fmap=fmap, sim=(sx, sy), acq_matrix=(sx, sy))
+    k = (rng.random((npts, 2)) - 0.5) * [sx, sy]
+    k[: min(npts, 11)] = [0.26, -0.49]
+    if npts > 24:
+        k[20:24] = [[-sx / 2, sy / 2], [sx / 2, -sy / 2], [-sx / 2 + 1e-9, sy / 2 - 1e-9], [0.0, 0.0]]
+    tau_ms = np.linspace(0.0, 30.0, 41)
+    ti = rng.integers(0, 41, npts)
+    rect = S.RateRect((0.0, 0.0), (float(fmap.min()), float(fmap.max())))
+    plan = S.tseg_plan(tau_ms, 30.0, rect)
+    acq = _acq(n_coils=1, do_relaxation=False)
+    got, info = S.spiral_segmented_forward(inp, acq, 0, 1, k, ti, tau_ms, 30.0, rect, None, False, ctx=gpu_ctx)
+    assert info["l"] == plan.l
+    want = O.spiral_segmented(inp, acq, 0, 1, k, ti, plan.tau_l, plan.b, None, False)
+    assert rel_l2(got, want) <= 1e-5
+    assert np.abs(got - want).max() <= 5e-6 * np.abs(want).max()
