@@ -69,12 +69,15 @@ NufftBins nufft_bins2(DevArena& A, int nf0, int nf1, int w, const double* u_host
 NufftBins nufft_bins1(DevArena& A, int nf, int w, const double* pos_host, int npos, cudaStream_t st);
 
 // Type 1 (nufft.rs:225-256): modes[b][m] = sum_j w[b][j] e^{sign i2pi (...)}.  The fine grid is
-// spread without atomics: each cell sums its points in point order (the reference's order), so
-// the result is the same on every run.  `bins` from nufft_bins2 over the same points.
+// spread without atomics: each cell sums its points in an order that the points alone set, so
+// the result is the same on every run.  `bins` from nufft_bins2 over the same points.  taps: scratch
+// of nufft_spread_taps bytes for a batch of many items (NULL: none, when that is 0).
 template <class R>
 void nufft_type1(const NufftGridT<R>& g, const double* u, int npts, const NufftBins& bins,
                  const typename Vec2<R>::type* wts, int batch, size_t w_stride, typename Vec2<R>::type* modes,
-                 size_t mode_stride, typename Vec2<R>::type* work, int sign, cudaStream_t st);
+                 size_t mode_stride, typename Vec2<R>::type* work, int sign, cudaStream_t st,
+                 void* taps = nullptr);
+size_t nufft_spread_taps(const NufftGridT<double>& g, int npts, int batch);
 
 // Type 2 of a batch of FP32 mode grids (packed [item][m1][m0]) at points ordered by window origin
 // (nufft_tiled.cu), sign +1: out[point][item].  grid: batch fine grids; tmp: batch x m_out1 x nf0.

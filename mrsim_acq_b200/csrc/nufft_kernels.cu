@@ -212,15 +212,18 @@ __device__ __forceinline__ int ring_offset(int c, int a, int n) {
 
 constexpr int kSpreadChunk = 64;  // points whose taps a spread block holds at a time
 
-// Type 1 spreading without atomics: one block per 8 x 8 tile of the fine grid (one thread per
-// cell) and group of up to kBatchBlock batch items (the taps formed once for the group).  The tile's points (nufft_bins2: every point whose window can reach the
-// tile, in point order) pass through shared memory in chunks with their taps; each thread adds
-// the contributions to its own cell point after point, cell += w_j (k0 k1) as the reference does
-// (nufft.rs:236-250), and stores the cell once.  The sum order is fixed, so the grid is the same
-// on every run; a window that wraps onto a cell twice (a fine grid narrower than the kernel) adds
-// both taps in tap order.
+// Type 1 spreading without atomics: one block per 8 x 8 tile of the fine grid and group of up to
+// kBatchBlock batch items (the taps formed once for the group).  The tile's points (nufft_bins2: every
+// point whose window can reach the tile, in point order) pass through shared memory in chunks with
+// their taps; the block's kSpreadParts parts (a thread per cell each) take every kSpreadParts-th point of
+// a chunk, add w_j (k0 k1) (nufft.rs:236-250) to their own sums, and the parts are added in order at
+// the end: a tile's points are one serial chain of additions per cell otherwise, and at one item a few
+// hundred tiles of 64 threads leave the chip idle (65,536 points on a 128 x 128 fine grid: 0.97 ms
+// with one part, 0.38 with four).  The order is fixed, so the grid is the same on every run; a window that
+// wraps onto a cell twice (a fine grid narrower than the kernel) adds both taps.
+constexpr int kSpreadParts = 4, kCellsPerTile = kSpreadTile * kSpreadTile;
 template <class R>
-__global__ void __launch_bounds__(kSpreadTile * kSpreadTile)
+__global__ void __launch_bounds__(kCellsPerTile * kSpreadParts)
     spread_tile_kernel(const NufftGridT<R> g, typename Vec2<R>::type* __restrict__ grid, const double* __restrict__ u,
                        const typename Vec2<R>::type* __restrict__ wts, size_t grid_stride, size_t w_stride,
                        const NufftBins bins, int batch) {
@@ -228,9 +231,11 @@ __global__ void __launch_bounds__(kSpreadTile * kSpreadTile)
   __shared__ R sk0[kSpreadChunk][kWMax], sk1[kSpreadChunk][kWMax];
   __shared__ int sa0[kSpreadChunk], sa1[kSpreadChunk];
   __shared__ V sw[kBatchBlock][kSpreadChunk];
+  __shared__ V sums[kSpreadParts - 1][kCellsPerTile];
   const int b0 = blockIdx.y * kBatchBlock, nb = min(kBatchBlock, batch - b0), tile = blockIdx.x;
-  const int c0 = (tile % bins.tiles0) * kSpreadTile + (int)threadIdx.x % kSpreadTile;
-  const int c1 = (tile / bins.tiles0) * kSpreadTile + (int)threadIdx.x / kSpreadTile;
+  const int cell = (int)threadIdx.x % kCellsPerTile, part = (int)threadIdx.x / kCellsPerTile;
+  const int c0 = (tile % bins.tiles0) * kSpreadTile + cell % kSpreadTile;
+  const int c1 = (tile / bins.tiles0) * kSpreadTile + cell / kSpreadTile;
   const bool mine = c0 < g.nf0 && c1 < g.nf1;
   const int w = g.w;
   R re[kBatchBlock], im[kBatchBlock];
@@ -239,17 +244,21 @@ __global__ void __launch_bounds__(kSpreadTile * kSpreadTile)
   const int p0 = bins.start[tile], p1 = bins.start[tile + 1];
   for (int base = p0; base < p1; base += kSpreadChunk) {
     const int n = min(kSpreadChunk, p1 - base);
-    if ((int)threadIdx.x < n) {
-      const int t = threadIdx.x, j = bins.pts[base + t];
-      sa0[t] = es_taps<R>(u[2 * j], g.nf0, w, g.beta, sk0[t]);
-      sa1[t] = es_taps<R>(u[2 * j + 1], g.nf1, w, g.beta, sk1[t]);
+    // the two axes' taps and the weights by different threads
+    const int t = (int)threadIdx.x % kSpreadChunk, job = (int)threadIdx.x / kSpreadChunk;
+    if (t < n) {
+      const int j = bins.pts[base + t];
+      if (job == 0) sa0[t] = es_taps<R>(u[2 * j], g.nf0, w, g.beta, sk0[t]);
+      if (job == 1) sa1[t] = es_taps<R>(u[2 * j + 1], g.nf1, w, g.beta, sk1[t]);
+      if (job == 2) {
 #pragma unroll
-      for (int q = 0; q < kBatchBlock; ++q)
-        if (q < nb) sw[q][t] = wts[(size_t)(b0 + q) * w_stride + j];
+        for (int q = 0; q < kBatchBlock; ++q)
+          if (q < nb) sw[q][t] = wts[(size_t)(b0 + q) * w_stride + j];
+      }
     }
     __syncthreads();
     if (mine)
-      for (int q = 0; q < n; ++q) {
+      for (int q = part; q < n; q += kSpreadParts) {
         const int d0 = ring_offset(c0, sa0[q], g.nf0);
         if (d0 >= w) continue;
         const int d1 = ring_offset(c1, sa1[q], g.nf1);
@@ -266,10 +275,115 @@ __global__ void __launch_bounds__(kSpreadTile * kSpreadTile)
       }
     __syncthreads();
   }
-  if (mine)
 #pragma unroll
-    for (int q = 0; q < kBatchBlock; ++q)
-      if (q < nb) grid[(size_t)(b0 + q) * grid_stride + (size_t)c0 + (size_t)g.nf0 * c1] = mk2<R>(re[q], im[q]);
+  for (int q = 0; q < kBatchBlock; ++q) {
+    if (q >= nb) break;
+    if (part > 0) sums[part - 1][cell] = mk2<R>(re[q], im[q]);
+    __syncthreads();
+    if (part == 0 && mine) {
+      for (int o = 0; o < kSpreadParts - 1; ++o) {
+        re[q] += sums[o][cell].x;
+        im[q] += sums[o][cell].y;
+      }
+      grid[(size_t)(b0 + q) * grid_stride + (size_t)c0 + (size_t)g.nf0 * c1] = mk2<R>(re[q], im[q]);
+    }
+    __syncthreads();
+  }
+}
+
+// The taps and window origins of every point, once for all batch items: [j][kWMax] of each axis, zero from w.
+__global__ void spread_taps_kernel(const NufftGridT<double> g, const double* __restrict__ u, int npts,
+                                   double* __restrict__ taps, int2* __restrict__ org) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= npts) return;
+  double k0[kWMax], k1[kWMax];
+#pragma unroll
+  for (int i = 0; i < kWMax; ++i) k0[i] = k1[i] = 0.0;
+  org[j] = make_int2(es_taps<double>(u[2 * j], g.nf0, g.w, g.beta, k0),
+                     es_taps<double>(u[2 * j + 1], g.nf1, g.w, g.beta, k1));
+  double* t = taps + (size_t)j * 2 * kWMax;
+#pragma unroll
+  for (int i = 0; i < kWMax; ++i) {
+    t[i] = k0[i];
+    t[kWMax + i] = k1[i];
+  }
+}
+
+// The same spread for many items, FP64: a lane is a batch item, a warp holds two rows of the tile for it,
+// so a point's taps are broadcasts and its weight is read from shared memory once for 16 cells.  With a
+// thread per cell and four items, 58 % of the threads a point visits are outside its window and every
+// contribution waits for its own loads: 576 items at 65,536 points on a 128 x 128 fine grid took
+// 28.1 ms, here 4.2.  Bound by shared memory and the FP64 pipe about equally (14 wavefronts for 18
+// FP64 instructions per row).  Points are added in their order in the tile.
+constexpr int kItemLanes = 32, kItemChunk = 32, kPadTaps = 8 + kWMax + 8;
+__global__ void __launch_bounds__(128) spread_items_kernel(const NufftGridT<double> g, double2* __restrict__ grid,
+                                                           const double* __restrict__ taps, const int2* __restrict__ org,
+                                                           const double2* __restrict__ wts, size_t grid_stride,
+                                                           size_t w_stride, const NufftBins bins, int batch) {
+  __shared__ double sk0[kItemChunk][kPadTaps], sk1[kItemChunk][kPadTaps];  // taps at 8 .. 8 + w, zeros around
+  __shared__ double2 sw[kItemChunk][kItemLanes + 1];
+  __shared__ int2 so[kItemChunk];  // the tile's first cell within each window (negative before it)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+  const int b0 = blockIdx.y * kItemLanes, nb = min(kItemLanes, batch - b0);
+  const int x0 = (tile % bins.tiles0) * kSpreadTile, y0 = (tile / bins.tiles0) * kSpreadTile;
+  const int w = g.w;
+  for (int i = tid; i < kItemChunk * 8; i += 128) {
+    const int p = i / 8, x = i % 8;
+    sk0[p][x] = sk0[p][8 + kWMax + x] = sk1[p][x] = sk1[p][8 + kWMax + x] = 0.0;
+  }
+  double re[2][kSpreadTile], im[2][kSpreadTile];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int x = 0; x < kSpreadTile; ++x) re[r][x] = im[r][x] = 0.0;
+  const int p0 = bins.start[tile], p1 = bins.start[tile + 1];
+  for (int base = p0; base < p1; base += kItemChunk) {
+    const int n = min(kItemChunk, p1 - base);
+    __syncthreads();
+    for (int i = tid; i < n * 2 * kWMax; i += 128) {
+      const int p = i / (2 * kWMax), x = i % (2 * kWMax);
+      const double t = taps[(size_t)bins.pts[base + p] * (2 * kWMax) + x];
+      (x < kWMax ? sk0[p][8 + x] : sk1[p][8 + x - kWMax]) = t;
+    }
+    const int j = lane < n ? bins.pts[base + lane] : 0;
+    if (warp == 0 && lane < n) {
+      const int2 o = org[j];
+      int d0 = ring_offset(x0, o.x, g.nf0), d1 = ring_offset(y0, o.y, g.nf1);
+      d0 = d0 > g.nf0 / 2 ? d0 - g.nf0 : d0;
+      d1 = d1 > g.nf1 / 2 ? d1 - g.nf1 : d1;
+      so[lane] = make_int2(d0, d1);
+    }
+    if (lane < n)
+      for (int b = warp; b < kItemLanes; b += 4)  // neighbouring lanes take neighbouring points
+        sw[lane][b] = b < nb ? wts[(size_t)(b0 + b) * w_stride + j] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int q = 0; q < n; ++q) {
+      const int d0 = so[q].x, d1 = so[q].y + 2 * warp;  // of column 0, of this warp's first row
+      if (d0 <= -kSpreadTile || d0 >= w || d1 < -1 || d1 >= w) continue;
+      const double2 v = sw[q][lane];
+      const double ka = sk1[q][8 + d1], kb = sk1[q][9 + d1];
+      const double2 va = make_double2(v.x * ka, v.y * ka), vb = make_double2(v.x * kb, v.y * kb);
+      const double* k0 = &sk0[q][8 + d0];
+#pragma unroll
+      for (int x = 0; x < kSpreadTile; ++x) {
+        const double k = k0[x];
+        re[0][x] += va.x * k;
+        im[0][x] += va.y * k;
+        re[1][x] += vb.x * k;
+        im[1][x] += vb.y * k;
+      }
+    }
+  }
+  if (lane >= nb) return;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int c1 = y0 + 2 * warp + r;
+    if (c1 >= g.nf1) continue;
+    double2* out = grid + (size_t)(b0 + lane) * grid_stride + (size_t)g.nf0 * c1 + x0;
+#pragma unroll
+    for (int x = 0; x < kSpreadTile; ++x)
+      if (x0 + x < g.nf0) out[x] = make_double2(re[r][x], im[r][x]);
+  }
 }
 
 // ---- the 1D type-1 NUFFT (`Nufft1`, nufft.rs:25-112), FP64 --------------------------------------
@@ -479,11 +593,24 @@ void nufft_type2(const NufftGridT<R>& g, const typename Vec2<R>::type* modes, in
 template <class R>
 void nufft_type1(const NufftGridT<R>& g, const double* u, int npts, const NufftBins& bins,
                  const typename Vec2<R>::type* wts, int batch, size_t w_stride, typename Vec2<R>::type* modes,
-                 size_t mode_stride, typename Vec2<R>::type* work, int sign, cudaStream_t st) {
+                 size_t mode_stride, typename Vec2<R>::type* work, int sign, cudaStream_t st, void* taps) {
   const size_t gs = (size_t)g.nf0 * g.nf1;
   // every cell of every tile is written (zero where no point reaches it)
-  dim3 sg(bins.tiles0 * bins.tiles1, (batch + kBatchBlock - 1) / kBatchBlock);
-  spread_tile_kernel<R><<<sg, kSpreadTile * kSpreadTile, 0, st>>>(g, work, u, wts, gs, w_stride, bins, batch);
+  bool done = false;
+  if constexpr (sizeof(R) == 8) {
+    if (taps) {
+      double* t = (double*)taps;
+      int2* org = (int2*)(t + (size_t)npts * 2 * kWMax);
+      spread_taps_kernel<<<(npts + 127) / 128, 128, 0, st>>>(g, u, npts, t, org);
+      dim3 ig(bins.tiles0 * bins.tiles1, (batch + kItemLanes - 1) / kItemLanes);
+      spread_items_kernel<<<ig, 128, 0, st>>>(g, work, t, org, wts, gs, w_stride, bins, batch);
+      done = true;
+    }
+  }
+  if (!done) {
+    dim3 sg(bins.tiles0 * bins.tiles1, (batch + kBatchBlock - 1) / kBatchBlock);
+    spread_tile_kernel<R><<<sg, kCellsPerTile * kSpreadParts, 0, st>>>(g, work, u, wts, gs, w_stride, bins, batch);
+  }
   nufft_fft2(g, work, batch, sign, st);
   dim3 eg((g.m_out0 * g.m_out1 + 255) / 256, batch);
   extract_kernel<R><<<eg, 256, 0, st>>>(g, work, modes, gs, mode_stride);
@@ -494,9 +621,16 @@ template void nufft_type2<float>(const NufftGridT<float>&, const float2*, int, s
 template void nufft_type2<double>(const NufftGridT<double>&, const double2*, int, size_t, const double*, int, double2*,
                                   size_t, double2*, int, const double*, cudaStream_t);
 template void nufft_type1<float>(const NufftGridT<float>&, const double*, int, const NufftBins&, const float2*, int,
-                                 size_t, float2*, size_t, float2*, int, cudaStream_t);
+                                 size_t, float2*, size_t, float2*, int, cudaStream_t, void*);
 template void nufft_type1<double>(const NufftGridT<double>&, const double*, int, const NufftBins&, const double2*, int,
-                                  size_t, double2*, size_t, double2*, int, cudaStream_t);
+                                  size_t, double2*, size_t, double2*, int, cudaStream_t, void*);
+
+// From 16 items on a lane per item is the faster (half of a last chunk's lanes may be idle); a fine ring
+// of fewer than 64 cells could meet a tile with both ends of a window, which the signed offset excludes.
+size_t nufft_spread_taps(const NufftGridT<double>& g, int npts, int batch) {
+  if (batch < 16 || npts <= 0 || g.nf0 < 64 || g.nf1 < 64) return 0;
+  return (size_t)npts * (2 * kWMax * sizeof(double) + sizeof(int2));
+}
 
 
 void nufft1_run(const Nufft1Grid& g, const double* pos, int npos, const NufftBins& bins, const double2* wts, int nw,

@@ -454,7 +454,9 @@ void SpiralRecon::gridding(const double2* d_data, int batch, double2* d_out) {
   double2* wts = (double2*)T.alloc((size_t)batch * npts * 16);
   weight_samples_kernel<<<grid1(npts, batch), 256, 0, st>>>(d_data, nullptr, d_w, sc, npts, wts);
   double2* work = (double2*)T.alloc((size_t)batch * g.nf0 * g.nf1 * 16);
-  nufft_type1<double>(g, d_k, npts, bins_k, wts, batch, npts, d_out, (size_t)n * n, work, -1, st);
+  const size_t tb = nufft_spread_taps(g, npts, batch);
+  nufft_type1<double>(g, d_k, npts, bins_k, wts, batch, npts, d_out, (size_t)n * n, work, -1, st,
+                      tb ? T.alloc(tb) : nullptr);
   scale_kernel<<<grid1((size_t)batch * n * n), 256, 0, st>>>(d_out, (double)n * n, (size_t)batch * n * n, d_out);
   MRSIM_CUDA(cudaGetLastError());
   MRSIM_CUDA(cudaStreamSynchronize(st));  // T's buffers are freed on return
@@ -472,7 +474,8 @@ void SpiralRecon::images(const double2* d_data, int batch, double2* d_x) {
     double2* wts = (double2*)W.alloc((size_t)batch * npts * 16);
     weight_samples_kernel<<<grid1(npts, batch), 256, 0, st>>>(d_data, d_win, d_w, sc, npts, wts);
     double2* work = (double2*)W.alloc((size_t)batch * g.nf0 * g.nf1 * 16);
-    nufft_type1<double>(g, d_k, npts, bins_k, wts, batch, npts, r, nn, work, -1, st);
+    const size_t tb = nufft_spread_taps(g, npts, batch);
+    nufft_type1<double>(g, d_k, npts, bins_k, wts, batch, npts, r, nn, work, -1, st, tb ? W.alloc(tb) : nullptr);
     if (!d_tfp) project(r, batch, st);
     MRSIM_CUDA(cudaStreamSynchronize(st));  // W's buffers are freed on return
   }

@@ -253,3 +253,18 @@ def test_one_launch_iterations_match_the_operator_in_numpy(gpu_ctx, n, band, ite
             dr, rho = rho1 * rho * dr + 2.0 * rho1 / delta * r, rho1
         assert np.linalg.norm(got[b] - x) <= 1e-8 * max(np.linalg.norm(x), 1e-300)
 
+
+
+@pytest.mark.parametrize("n,il,dw,batch", [(32, 4, 0.008, 16), (45, 5, 0.005, 33), (64, 8, 0.004, 47)])
+def test_batched_spreading_matches_single_items_and_the_oracle(gpu_ctx, n, il, dw, batch):
+    # fine grids of whole and of cut tiles, item counts around a warp's lanes; windows wrap at the rim
+    tr, k, taus = design(n, il, dw)
+    rng = np.random.default_rng(n)
+    d = rng.normal(size=(batch, len(k))) + 1j * rng.normal(size=(batch, len(k)))
+    rec = S.SpiralRecon(k, n, ctx=gpu_ctx)
+    got = rec.gridding(d)
+    assert np.array_equal(rec.gridding(d), got)
+    for b in (0, batch // 2, batch - 1):
+        assert rel_l2(got[b], rec.gridding(d[b])) <= 1e-13
+    want, _, _, _ = O.spiral_recon(k, n, d[-1:], "gridding")
+    assert rel_l2(got[-1], want[0]) <= 1e-8
