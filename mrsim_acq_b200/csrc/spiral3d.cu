@@ -230,8 +230,14 @@ __global__ void spiral_zdft_kernel(const ZArgs a) {
 }
 
 // FP64 normal equations of the kz kernel: G = F^H [F | B] over rows (t, j); F rows are the
-// sources' samples of every coil, B the targets'.  One CTA accumulates a block of rows into a
-// partial [nfeat][nfeat + nc] result; partials are summed on the host in a fixed order.
+// sources' samples of every coil, B the targets'.  A block stages kKzRows rows of one target partition
+// and its threads hold 4 x 4 entries each (a row's 8 loads from shared memory serve 16 complex
+// products; with a load of two values per product the kernel waited on shared memory and its
+// entries lived in local memory: a 16-coil volume's four fits, of up to 64 features and 80 columns over
+// 65,536 samples a partition, took 24.8 ms, here 10.2).
+// Only tiles on and above the diagonal are formed, G being Hermitian.  The threads that the units
+// leave over take rows of their own; the groups are added in order.  Bound by the FP64 pipe.
+constexpr int kKzRows = 32, kKzTile = 4;
 struct KzFitArgs {
   const float2* k;     // [q][p][nsamp] calibration samples
   const int* t_list;   // target partitions with every source in the band
@@ -240,94 +246,126 @@ struct KzFitArgs {
   double2* partial;    // [block][nfeat][nfeat + nc]
 };
 
-__global__ void __launch_bounds__(256) kz_normal_kernel(const KzFitArgs a) {
+__host__ __device__ inline int kz_units(int nfeat, int ncol) {
+  const int ti = (nfeat + kKzTile - 1) / kKzTile, tj = (ncol + kKzTile - 1) / kKzTile;
+  return ti * tj - ti * (ti - 1) / 2;
+}
+
+__global__ void __launch_bounds__(512) kz_normal_kernel(const KzFitArgs a) {
   extern __shared__ __align__(16) unsigned char kz_smem[];
   const int nfeat = a.nsrc * a.nc, ncol = nfeat + a.nc;
-  constexpr int kRows = 16;
-  double2* fr = reinterpret_cast<double2*>(kz_smem);  // [kRows][ncol]
-  const long long total = (long long)a.n_t * a.nsamp;
-  const int nent = nfeat * ncol;
-  constexpr int kPer = 24;  // entries per thread (nfeat <= 64, nc <= 64: 64 x 128 / 256 = 32 max)
-  double2 acc[kPer];
+  const int tjn = (ncol + kKzTile - 1) / kKzTile, ld = kKzTile * tjn | 1;
+  const int units = kz_units(nfeat, ncol), groups = (int)blockDim.x / units;
+  // column c at (c % 4) tjn + c / 4: neighbouring units read neighbouring values
+  double2* fr = reinterpret_cast<double2*>(kz_smem);  // [kKzRows][ld]
+  int ti = 0, tj = (int)threadIdx.x % units;
+  const int unit = tj, grp = (int)threadIdx.x / units;
+  while (tj >= tjn - ti) tj -= tjn - ti++;
+  tj += ti;
+  double re[kKzTile][kKzTile], im[kKzTile][kKzTile];
 #pragma unroll
-  for (int e = 0; e < kPer; ++e) acc[e] = make_double2(0.0, 0.0);
-  for (long long r0 = (long long)blockIdx.x * kRows; r0 < total; r0 += (long long)gridDim.x * kRows) {
+  for (int u = 0; u < kKzTile; ++u)
+#pragma unroll
+    for (int v = 0; v < kKzTile; ++v) re[u][v] = im[u][v] = 0.0;
+  const int per_t = (a.nsamp + kKzRows - 1) / kKzRows;
+  for (long long c = blockIdx.x; c < (long long)a.n_t * per_t; c += gridDim.x) {
+    const int t = a.t_list[c / per_t], j0 = (int)(c % per_t) * kKzRows;
     __syncthreads();
-    for (int idx = threadIdx.x; idx < kRows * ncol; idx += blockDim.x) {
-      const int rr = idx / ncol, col = idx % ncol;
-      const long long row = r0 + rr;
+    for (int idx = threadIdx.x; idx < kKzRows * kKzTile * tjn; idx += blockDim.x) {
+      const int rr = idx % kKzRows, col = idx / kKzRows;
       double2 v = make_double2(0.0, 0.0);
-      if (row < total) {
-        const int t = a.t_list[row / a.nsamp];
-        const int j = (int)(row % a.nsamp);
-        int p, q;
-        if (col < nfeat) {
-          p = t + a.offs[col / a.nc];
-          q = col % a.nc;
-        } else {
-          p = t;
-          q = col - nfeat;
-        }
-        const float2 s = a.k[((size_t)q * a.nz + p) * a.nsamp + j];
+      if (col < ncol && j0 + rr < a.nsamp) {
+        const int p = col < nfeat ? t + a.offs[col / a.nc] : t, q = col % a.nc;  // nfeat is a multiple of nc
+        const float2 s = a.k[((size_t)q * a.nz + p) * a.nsamp + j0 + rr];
         v = make_double2((double)s.x, (double)s.y);
       }
-      fr[rr * ncol + col] = v;
+      fr[rr * ld + col % kKzTile * tjn + col / kKzTile] = v;
     }
     __syncthreads();
-    for (int e = 0; e < kPer; ++e) {
-      const int ent = threadIdx.x + e * blockDim.x;
-      if (ent >= nent) break;
-      const int i = ent / ncol, jj = ent % ncol;
-      double re = acc[e].x, im = acc[e].y;
-      for (int rr = 0; rr < kRows; ++rr) {
-        const double2 fi = fr[rr * ncol + i], fj = fr[rr * ncol + jj];
-        re = fma(fi.x, fj.x, fma(fi.y, fj.y, re));  // conj(fi) fj
-        im = fma(fi.x, fj.y, fma(-fi.y, fj.x, im));
+    if (grp < groups)
+      for (int rr = grp; rr < kKzRows; rr += groups) {
+        double2 fi[kKzTile], fj[kKzTile];
+#pragma unroll
+        for (int u = 0; u < kKzTile; ++u) {
+          fi[u] = fr[rr * ld + u * tjn + ti];
+          fj[u] = fr[rr * ld + u * tjn + tj];
+        }
+#pragma unroll
+        for (int u = 0; u < kKzTile; ++u)
+#pragma unroll
+          for (int v = 0; v < kKzTile; ++v) {  // conj(fi) fj
+            re[u][v] = fma(fi[u].x, fj[v].x, fma(fi[u].y, fj[v].y, re[u][v]));
+            im[u][v] = fma(fi[u].x, fj[v].y, fma(-fi[u].y, fj[v].x, im[u][v]));
+          }
       }
-      acc[e] = make_double2(re, im);
-    }
   }
-  for (int e = 0; e < kPer; ++e) {
-    const int ent = threadIdx.x + e * blockDim.x;
-    if (ent >= nent) break;
-    a.partial[(size_t)blockIdx.x * nent + ent] = acc[e];
+  double2* out = a.partial + (size_t)blockIdx.x * nfeat * ncol;
+#pragma unroll
+  for (int u = 0; u < kKzTile; ++u) {
+    for (int o = 1; o < groups; ++o) {
+      __syncthreads();
+      if (grp == o)
+#pragma unroll
+        for (int v = 0; v < kKzTile; ++v) fr[unit * kKzTile + v] = make_double2(re[u][v], im[u][v]);
+      __syncthreads();
+      if (grp == 0)
+#pragma unroll
+        for (int v = 0; v < kKzTile; ++v) {
+          re[u][v] += fr[unit * kKzTile + v].x;
+          im[u][v] += fr[unit * kKzTile + v].y;
+        }
+    }
+    const int i = kKzTile * ti + u;
+    if (grp == 0 && i < nfeat)
+#pragma unroll
+      for (int v = 0; v < kKzTile; ++v) {
+        const int j = kKzTile * tj + v;
+        if (j < ncol) out[(size_t)i * ncol + j] = make_double2(re[u][v], im[u][v]);
+        if (tj > ti && j < nfeat) out[(size_t)j * ncol + i] = make_double2(re[u][v], -im[u][v]);
+      }
   }
 }
 
-// The kz kernel's system (`KzGrappa::fit`, kspace3d.rs:1299-1362): the blocks' partial normal
-// equations summed in block order, scaled by nfeat / trace, the Tikhonov term added to the
-// diagonal, then every target coil's weights by pivoted elimination (hermitian_solve.cuh).  One
-// CTA; status 1 when the trace is not positive (an empty calibration).
+// The blocks' partial normal equations summed in block order into block 0's.
+__global__ void kz_reduce_kernel(double2* __restrict__ partial, int blocks, int n_el) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n_el) return;
+  double2 g = make_double2(0.0, 0.0);
+#pragma unroll 8
+  for (int b = 0; b < blocks; ++b) {
+    const double2 p = partial[(size_t)b * n_el + e];
+    g.x = __dadd_rn(g.x, p.x);
+    g.y = __dadd_rn(g.y, p.y);
+  }
+  partial[e] = g;
+}
+
+// The kz kernel's system (`KzGrappa::fit`, kspace3d.rs:1299-1362): the normal equations scaled by
+// nfeat / trace, the Tikhonov term added to the diagonal, then every target coil's weights by pivoted
+// elimination (hermitian_solve.cuh).  One CTA, the system in shared memory (its steps are a chain; with
+// the blocks' sums in here too and the system in global memory those four took 1.65 ms, here under
+// 0.9 with the reductions); status 1 when the trace is not positive (an empty calibration).
 struct KzSolveArgs {
-  const double2* partial;  // [blocks][nfeat][ncol], ncol = nfeat + nc
-  double2* W;              // [nfeat][ncol]
-  double* scratch;         // 2 nfeat + nc * 2 nfeat
-  float2* out;             // [nc][nfeat]
+  const double2* sum;  // [nfeat][ncol], ncol = nfeat + nc
+  float2* out;         // [nc][nfeat]
   int* status;
   double lambda;
-  int blocks, nfeat, nc;
+  int nfeat, nc;
 };
 
 __global__ void __launch_bounds__(256) kz_solve_kernel(const KzSolveArgs a) {
+  extern __shared__ __align__(16) unsigned char kz_smem[];
   __shared__ double red_v[256];
   __shared__ int red_i[256];
   __shared__ double s_scale;
   __shared__ int s_bad;
   const int nf = a.nfeat, ncol = nf + a.nc;
-  const size_t n_el = (size_t)nf * ncol;
-  for (size_t e = threadIdx.x; e < n_el; e += blockDim.x) {
-    double2 g = make_double2(0.0, 0.0);
-    for (int b = 0; b < a.blocks; ++b) {
-      const double2 p = a.partial[(size_t)b * n_el + e];
-      g.x = __dadd_rn(g.x, p.x);
-      g.y = __dadd_rn(g.y, p.y);
-    }
-    a.W[e] = g;
-  }
-  __syncthreads();
+  const int n_el = nf * ncol;
+  double2* W = reinterpret_cast<double2*>(kz_smem);
+  double* scratch = reinterpret_cast<double*>(W + n_el);
   if (threadIdx.x == 0) {
     double trace = 0.0;
-    for (int i = 0; i < nf; ++i) trace = __dadd_rn(trace, a.W[(size_t)i * ncol + i].x);
+    for (int i = 0; i < nf; ++i) trace = __dadd_rn(trace, a.sum[(size_t)i * ncol + i].x);
     s_bad = !(trace > 0.0);
     s_scale = s_bad ? 0.0 : __ddiv_rn((double)nf, trace);
     if (s_bad) *a.status = 1;
@@ -335,15 +373,15 @@ __global__ void __launch_bounds__(256) kz_solve_kernel(const KzSolveArgs a) {
   __syncthreads();
   if (s_bad) return;
   const double sc = s_scale;
-  for (size_t e = threadIdx.x; e < n_el; e += blockDim.x) {
-    double2 v = a.W[e];
+  for (int e = threadIdx.x; e < n_el; e += blockDim.x) {
+    double2 v = a.sum[e];
     v.x = __dmul_rn(v.x, sc);
     v.y = __dmul_rn(v.y, sc);
-    if ((int)(e / ncol) == (int)(e % ncol)) v.x = __dadd_rn(v.x, a.lambda);
-    a.W[e] = v;
+    if (e / ncol == e % ncol) v.x = __dadd_rn(v.x, a.lambda);
+    W[e] = v;
   }
   __syncthreads();
-  hermitian_solve_block(a.W, nf, a.nc, a.scratch, a.scratch + nf, a.scratch + 2 * nf, a.out, red_v, red_i);
+  hermitian_solve_block(W, nf, a.nc, scratch, scratch + nf, scratch + 2 * nf, a.out, red_v, red_i);
 }
 
 struct KzFillJob {
@@ -1077,23 +1115,28 @@ static KzKernel kz_fit(mrsim_context* ctx, const Spiral3dTable& T, int accel, co
     a.nc = nc;
     a.nz = nz;
     a.nsamp = nsamp;
-    const int blocks = 296;
-    a.partial = (double2*)A.alloc((size_t)blocks * nfeat * ncol * sizeof(double2));
-    const size_t smem = (size_t)16 * ncol * sizeof(double2);
-    kz_normal_kernel<<<blocks, 256, smem, st>>>(a);
+    const int blocks = 296, n_el = nfeat * ncol, units = kz_units(nfeat, ncol);
+    a.partial = (double2*)A.alloc((size_t)blocks * n_el * sizeof(double2));
+    // one unit a thread: the limit above keeps the units below 512
+    const int threads = units <= 256 ? 256 : 512;
+    const size_t rows = sizeof(double2) * kKzRows * ((ncol + kKzTile) | 1);
+    const size_t nsmem = std::max(rows, sizeof(double2) * kKzTile * (size_t)units);
+    const size_t ssmem = sizeof(double2) * n_el + sizeof(double) * (2 * nfeat + (size_t)nc * 2 * nfeat);
+    constexpr int kMost = 200 * 1024;
+    MRSIM_CUDA(cudaFuncSetAttribute(kz_normal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+    MRSIM_CUDA(cudaFuncSetAttribute(kz_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+    kz_normal_kernel<<<blocks, threads, nsmem, st>>>(a);
+    kz_reduce_kernel<<<(n_el + 63) / 64, 64, 0, st>>>(a.partial, blocks, n_el);
     MRSIM_CUDA(cudaGetLastError());
     KzSolveArgs sa;
-    sa.partial = a.partial;
-    sa.W = (double2*)A.alloc((size_t)nfeat * ncol * sizeof(double2));
-    sa.scratch = (double*)A.alloc((size_t)(2 * nfeat + nc * 2 * nfeat) * sizeof(double));
+    sa.sum = a.partial;
     sa.out = (float2*)A.alloc((size_t)nc * nfeat * sizeof(float2));
     sa.status = (int*)A.alloc(sizeof(int));
     sa.lambda = kKzLambda;
-    sa.blocks = blocks;
     sa.nfeat = nfeat;
     sa.nc = nc;
     MRSIM_CUDA(cudaMemsetAsync(sa.status, 0, sizeof(int), st));
-    kz_solve_kernel<<<1, 256, 0, st>>>(sa);
+    kz_solve_kernel<<<1, 256, ssmem, st>>>(sa);
     MRSIM_CUDA(cudaGetLastError());
     int status = 0;
     const int woff = (int)K.w.size();

@@ -177,3 +177,13 @@ def test_slices_planned_on_several_threads(gpu_ctx):
     first = K3.spiral_samples_3d(*args, ctx=gpu_ctx)
     for _ in range(20):
         assert np.array_equal(K3.spiral_samples_3d(*args, ctx=gpu_ctx), first)
+
+
+@pytest.mark.parametrize("accel,rows", [(2, 3), (3, 5), (2, 8)])
+def test_kz_fits_of_ragged_sizes_match_the_oracle(gpu_ctx, accel, rows):
+    # features and columns that are no multiples of the normal equations' 4 x 4 tiles, and that are
+    args, kzo = _kz_case(K3.KzSampling(1.0, accel), rows)
+    mag, ph = K3.simulate_acquisition_3d(*args, phase=PhaseModel.none(), seed=3, kz_opts=kzo, ctx=gpu_ctx)
+    vols, _, _ = O.simulate_acquisition_3d_spiral(*args, phase=PhaseModel.none(), seed=3, kz_opts=kzo)
+    z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
+    assert rel_l2(z, vols.T.ravel()) <= 1e-5
