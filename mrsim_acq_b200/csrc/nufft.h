@@ -52,8 +52,7 @@ void nufft_type2(const NufftGridT<R>& g, const typename Vec2<R>::type* modes, in
                  const double* u, int npts, typename Vec2<R>::type* out, size_t out_stride,
                  typename Vec2<R>::type* work, int sign, const R* scale, cudaStream_t st);
 // The deterministic spread's fine-grid tiles and, per tile, the points whose kernel window can
-// reach it, in point order (CSR on the device, built on the host from the positions once per
-// point set).  A tile is 8 x 8 fine cells in 2D (a cell's scan covers (8 + w)^2 cells of
+// reach it, in point order (CSR on the device, built from the positions once per point set).  A tile is 8 x 8 fine cells in 2D (a cell's scan covers (8 + w)^2 cells of
 // windows to use w^2; a 128 x 128 fine grid still gives 256 blocks), 256 cells in 1D.
 constexpr int kSpreadTile = 8;
 constexpr int kSpreadTile1 = 256;
@@ -63,8 +62,10 @@ struct NufftBins {
   const int* pts = nullptr;
 };
 struct DevArena;
-// 2D points u (npts x 2, period n per axis) on a fine grid of nf0 x nf1 cells, kernel width w
-NufftBins nufft_bins2(DevArena& A, int nf0, int nf1, int w, const double* u_host, int npts, cudaStream_t st);
+// 2D points u (npts x 2 on the device, period n per axis) on a fine grid of nf0 x nf1 cells, kernel width
+// w; the lists in A, scratch in T
+NufftBins nufft_bins2(DevArena& A, DevArena& T, int nf0, int nf1, int w, const double* d_u, int npts,
+                      cudaStream_t st);
 // 1D positions (cells, period n) on a fine grid of nf cells
 NufftBins nufft_bins1(DevArena& A, int nf, int w, const double* pos_host, int npos, cudaStream_t st);
 
@@ -127,6 +128,8 @@ void spiral_exact(const SpiralExactArgs& a, cudaStream_t st);
 
 void segment_images(const float2* x, const float2* rate, int nvox, const double* tau_l, int L, float2* out,
                     cudaStream_t st);
+// stat[j]: the half-cell phase of sample j and 1 / voxels (`SegmentedForward::new` spiral.rs:159-170)
+void spiral_stat(const double* k, int npts, int snx, int sny, int ox, int oy, float2* stat, cudaStream_t st);
 // seg [l][point], or with by_point [point][l]
 void segment_combine(const float2* seg, int npts, int L, const int* tau_idx, const double* b, const float2* stat,
                      float2* out, bool by_point, cudaStream_t st);

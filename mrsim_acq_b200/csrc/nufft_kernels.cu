@@ -13,7 +13,10 @@
 
 #include <algorithm>
 
+#include "driver.h"
 #include "es_taps.cuh"
+#include "host_tables.h"
+#include "mrsim_internal.h"
 #include "nufft.h"
 
 namespace mrsim {
@@ -35,6 +38,17 @@ template <>
 __device__ __forceinline__ double2 mk2<double>(double a, double b) {
   return make_double2(a, b);
 }
+// In FP64 as on the host, where 65,536 samples' sines took 2 ms.
+__global__ void spiral_stat_kernel(const double* __restrict__ k, int npts, int snx, int sny, double xoff, double yoff,
+                                   float2* __restrict__ stat) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= npts) return;
+  const double ninv = 1.0 / ((double)snx * sny);
+  double sn, cs;
+  sincos(-kTau * (k[2 * j] * xoff / snx + k[2 * j + 1] * yoff / sny), &sn, &cs);
+  stat[j] = make_float2((float)(cs * ninv), (float)(sn * ninv));
+}
+
 template <class R>
 __global__ void place_kernel(const NufftGridT<R> g, const typename Vec2<R>::type* __restrict__ modes,
                              typename Vec2<R>::type* __restrict__ grid, int batch, size_t mode_stride,
@@ -208,6 +222,84 @@ __device__ __forceinline__ int ring_offset(int c, int a, int n) {
   while (d < 0) d += n;
   while (d >= n) d -= n;
   return d;
+}
+
+// ---- the points of each spread tile ---------------------------------------------------------------
+// lo[axis][j]: the ring cell one before the point's window (the window is widened by a cell each side);
+// -1 where the position is not finite (its taps are zero: it reaches no tile).
+__global__ void bins_origin_kernel(const double* __restrict__ u, int npts, int nf0, int nf1, int w, int* __restrict__ lo) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= npts) return;
+  double p;
+  const bool ok = isfinite(u[2 * j]) && isfinite(u[2 * j + 1]);
+  lo[j] = ok ? wrap(es_origin(u[2 * j], nf0, 0.5 * w, p) - 1, nf0) : -1;
+  lo[npts + j] = ok ? wrap(es_origin(u[2 * j + 1], nf1, 0.5 * w, p) - 1, nf1) : -1;
+}
+
+// One block per tile of one axis and parent list (block = parent * tiles + tile): the parent's points
+// (p_start / p_pts; NULL: all npts in order) whose `span` cells from lo[j] on meet the tile's, counted
+// (count != NULL) or stored from start[block] on, in the parent's order.
+constexpr int kBinThreads = 256;
+__global__ void __launch_bounds__(kBinThreads) bins_select_kernel(const int* __restrict__ lo, int npts,
+                                                                  const int* __restrict__ p_start,
+                                                                  const int* __restrict__ p_pts, int tiles, int nf,
+                                                                  int span, int* __restrict__ count,
+                                                                  const int* __restrict__ start, int* __restrict__ pts) {
+  __shared__ int part[kBinThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int parent = blockIdx.x / tiles, t0 = (blockIdx.x % tiles) * kSpreadTile, len = min(kSpreadTile, nf - t0);
+  const int b0 = p_start ? p_start[parent] : 0, b1 = p_start ? p_start[parent + 1] : npts;
+  int at = count ? 0 : start[blockIdx.x];
+  for (int base = b0; base < b1; base += kBinThreads) {
+    int j = -1;
+    bool hit = false;
+    if (base + tid < b1) {
+      j = p_pts ? p_pts[base + tid] : base + tid;
+      const int l = lo[j];
+      int d = t0 - l;  // from the span's first cell to the tile's, and back, around the ring
+      int e = -d;
+      if (d < 0) d += nf;
+      if (e < 0) e += nf;
+      hit = l >= 0 && (d < span || e < len);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) part[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kBinThreads / 32; ++w) {
+      before += w < warp ? part[w] : 0;
+      total += part[w];
+    }
+    if (hit && !count) pts[at + before + __popc(m & ((1u << lane) - 1u))] = j;
+    at += total;
+    __syncthreads();
+  }
+  if (count && tid == 0) count[blockIdx.x] = at;
+}
+
+// One block: start[i] = sum of count[0 .. i), start[n] the total.
+__global__ void __launch_bounds__(1024) bins_scan_kernel(const int* __restrict__ count, int n, int* __restrict__ start) {
+  __shared__ int part[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = (n + 1023) / 1024;
+  const int i0 = min(n, tid * per), i1 = min(n, i0 + per);
+  int v = 0;
+  for (int i = i0; i < i1; ++i) v += count[i];
+  int x = v;
+#pragma unroll
+  for (int h = 1; h < 32; h <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, x, h);
+    if (lane >= h) x += o;
+  }
+  if (lane == 31) part[warp] = x;
+  __syncthreads();
+  x -= v;
+  for (int w = 0; w < warp; ++w) x += part[w];
+  for (int i = i0; i < i1; ++i) {
+    start[i] = x;
+    x += count[i];
+  }
+  if (tid == 1023) start[n] = x;
 }
 
 constexpr int kSpreadChunk = 64;  // points whose taps a spread block holds at a time
@@ -625,6 +717,39 @@ template void nufft_type1<float>(const NufftGridT<float>&, const double*, int, c
 template void nufft_type1<double>(const NufftGridT<double>&, const double*, int, const NufftBins&, const double2*, int,
                                   size_t, double2*, size_t, double2*, int, cudaStream_t, void*);
 
+// The lists are made on the device, rows of tiles first and each row's tiles from its list (a pass of
+// every tile over every point would grow with their product).  On the host, with a ring walk per point
+// and axis, twice, they and the voxel and sample tables of the forward were 80 of 204 ms of a volume
+// with 65,536 points.
+NufftBins nufft_bins2(DevArena& A, DevArena& T, int nf0, int nf1, int w, const double* d_u, int npts,
+                      cudaStream_t st) {
+  NufftBins b;
+  b.tiles0 = (nf0 + kSpreadTile - 1) / kSpreadTile;
+  b.tiles1 = (nf1 + kSpreadTile - 1) / kSpreadTile;
+  const int nt = b.tiles0 * b.tiles1, span = w + 2;
+  // tiles that a span can meet on an axis (one more where the ring's last tile is cut)
+  auto most = [&](int nf, int tiles) { return std::min(tiles, (span + 6) / kSpreadTile + (nf % kSpreadTile ? 2 : 1)); };
+  const size_t m1 = most(nf1, b.tiles1), m0 = most(nf0, b.tiles0);
+  int* lo = (int*)T.alloc((size_t)npts * 2 * 4);
+  int* count = (int*)T.alloc((size_t)nt * 4);
+  int* rstart = (int*)T.alloc((size_t)(b.tiles1 + 1) * 4);
+  int* rpts = (int*)T.alloc(m1 * npts * 4);
+  int* start = (int*)A.alloc((size_t)(nt + 1) * 4);
+  int* pts = (int*)A.alloc(m0 * m1 * npts * 4);
+  bins_origin_kernel<<<(npts + 255) / 256, 256, 0, st>>>(d_u, npts, nf0, nf1, w, lo);
+  const int *lo0 = lo, *lo1 = lo + npts, *none = nullptr;
+  bins_select_kernel<<<b.tiles1, kBinThreads, 0, st>>>(lo1, npts, none, none, b.tiles1, nf1, span, count, none, nullptr);
+  bins_scan_kernel<<<1, 1024, 0, st>>>(count, b.tiles1, rstart);
+  bins_select_kernel<<<b.tiles1, kBinThreads, 0, st>>>(lo1, npts, none, none, b.tiles1, nf1, span, nullptr, rstart, rpts);
+  bins_select_kernel<<<nt, kBinThreads, 0, st>>>(lo0, npts, rstart, rpts, b.tiles0, nf0, span, count, none, nullptr);
+  bins_scan_kernel<<<1, 1024, 0, st>>>(count, nt, start);
+  bins_select_kernel<<<nt, kBinThreads, 0, st>>>(lo0, npts, rstart, rpts, b.tiles0, nf0, span, nullptr, start, pts);
+  MRSIM_CUDA(cudaGetLastError());
+  b.start = start;
+  b.pts = pts;
+  return b;
+}
+
 // From 16 items on a lane per item is the faster (half of a last chunk's lanes may be idle); a fine ring
 // of fewer than 64 cells could meet a tile with both ends of a window, which the signed offset excludes.
 size_t nufft_spread_taps(const NufftGridT<double>& g, int npts, int batch) {
@@ -650,6 +775,10 @@ void segment_images(const float2* x, const float2* rate, int nvox, const double*
                     cudaStream_t st) {
   dim3 g((nvox + 255) / 256, L);
   segment_images_kernel<<<g, 256, 0, st>>>(x, rate, nvox, tau_l, L, out);
+}
+
+void spiral_stat(const double* k, int npts, int snx, int sny, int ox, int oy, float2* stat, cudaStream_t st) {
+  spiral_stat_kernel<<<(npts + 255) / 256, 256, 0, st>>>(k, npts, snx, sny, (ox - 1.0) / 2.0, (oy - 1.0) / 2.0, stat);
 }
 
 void segment_combine(const float2* seg, int npts, int L, const int* tau_idx, const double* b, const float2* stat,

@@ -128,18 +128,6 @@ NufftBins upload_bins(DevArena& A, int tiles0, int tiles1, int npts, const std::
 }
 }  // namespace
 
-NufftBins nufft_bins2(DevArena& A, int nf0, int nf1, int w, const double* u_host, int npts, cudaStream_t st) {
-  const int tiles0 = (nf0 + kSpreadTile - 1) / kSpreadTile, tiles1 = (nf1 + kSpreadTile - 1) / kSpreadTile;
-  std::vector<int> t0, t1;
-  return upload_bins(A, tiles0, tiles1, npts, [&](int j, std::vector<int>& out) {
-    window_tiles(u_host[2 * (size_t)j], nf0, w, kSpreadTile, t0);
-    window_tiles(u_host[2 * (size_t)j + 1], nf1, w, kSpreadTile, t1);
-    out.clear();
-    for (int b : t1)
-      for (int a : t0) out.push_back(a + tiles0 * b);
-  }, st);
-}
-
 NufftBins nufft_bins1(DevArena& A, int nf, int w, const double* pos_host, int npos, cudaStream_t st) {
   const int tiles = (nf + kSpreadTile1 - 1) / kSpreadTile1;
   return upload_bins(A, tiles, 1, npos, [&](int j, std::vector<int>& out) {
@@ -199,7 +187,7 @@ void nufft2_host(mrsim_context* ctx, int type, int n0, int n1, int m_lo0, int m_
   } else {
     const float2* dw = (const float2*)A.upload(in, (size_t)npts * sizeof(float2), st);
     float2* dm = (float2*)A.alloc(nm * sizeof(float2));
-    const NufftBins bins = nufft_bins2(A, g.nf0, g.nf1, g.w, u, npts, st);
+    const NufftBins bins = nufft_bins2(A, A, g.nf0, g.nf1, g.w, du, npts, st);
     nufft_type1<float>(g, du, npts, bins, dw, 1, npts, dm, nm, work, sign, st);
     MRSIM_CUDA(cudaGetLastError());
     MRSIM_CUDA(cudaMemcpyAsync(out, dm, nm * sizeof(float2), cudaMemcpyDeviceToHost, st));
@@ -339,13 +327,8 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
   const int L = plan.l;
   const int ox = snx / nx, oy = sny / ny;
   const int sxs = ox * (nx / 2), sys = oy * (ny / 2);
-  const double xoff = (ox - 1.0) / 2.0, yoff = (oy - 1.0) / 2.0;
-  const double ninv = 1.0 / (double)n;
-  std::vector<float2> stat(npts);
   std::vector<int> tidx(npts);
   for (int j = 0; j < npts; ++j) {
-    const double ph = -kTau * (k[2 * j] * xoff / snx + k[2 * j + 1] * yoff / sny);
-    stat[j] = make_float2((float)(std::cos(ph) * ninv), (float)(std::sin(ph) * ninv));
     if (tau_idx[j] < 0 || tau_idx[j] >= ntau) fail("sample-time index out of range");
     tidx[j] = (int)tau_idx[j];
   }
@@ -367,7 +350,8 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
     nufft_type2<float>(g, imgs, L, n, du, npts, seg, npts, work, 1, nullptr, st);
   }
   const double* db = (const double*)A.upload(plan.b.data(), plan.b.size() * 8, st);
-  const float2* dstat = (const float2*)A.upload(stat.data(), stat.size() * sizeof(float2), st);
+  float2* dstat = (float2*)A.alloc((size_t)npts * sizeof(float2));
+  spiral_stat(du, npts, snx, sny, ox, oy, dstat, st);
   const int* dti = (const int*)A.upload(tidx.data(), tidx.size() * 4, st);
   float2* dout = (float2*)A.alloc((size_t)npts * sizeof(float2));
   segment_combine(seg, npts, L, dti, db, dstat, dout, tiled, st);

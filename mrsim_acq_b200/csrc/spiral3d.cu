@@ -622,9 +622,7 @@ struct SpiralPlan3 {
   std::vector<int> src_of;     // [c][p]
   std::vector<float> wc;       // [c][p][ns]
   std::vector<double> zsens;   // [q][z]
-  std::vector<float2> cis0;    // [z][plane]: e^{i phi0}
-  std::vector<float2> stat;    // [nsamp]
-  std::vector<int64_t> tau_idx;
+  mrsim_phase_model phase;     // the object phase (no preparation)
 };
 
 static void build_sources(SpiralPlan3& P, const mrsim_acquisition& acq) {
@@ -773,35 +771,46 @@ static SpiralPlan3 make_spiral_plan(const mrsim_acquisition_3d_input& in, const 
   P.zsens.resize((size_t)P.nc * P.nz);
   for (int q = 0; q < P.nc; ++q)
     for (int z = 0; z < P.nz; ++z) P.zsens[(size_t)q * P.nz + z] = coil_row_sensitivity(q / P.ring, rows, z, P.nz);
-  P.cis0.resize(P.nvox);
-  mrsim_phase_model pm;
-  std::memset(&pm, 0, sizeof pm);
-  if (in.phase) pm = *in.phase;
-  for (int z = 0; z < P.nz; ++z) {  // `phase_slice` with a zero shot (kspace.rs:1156-1180)
-    const double sx = P.snx / 2.0, sy = P.sny / 2.0, off = (P.o - 1.0) / 2.0, r2 = z - P.nz / 2.0;
-    for (int y = 0; y < P.sny; ++y)
-      for (int x = 0; x < P.snx; ++x) {
-        const double r0 = (x - sx - off) / P.o, r1 = (y - sy - off) / P.o;
-        const double* c = pm.background;
-        const double bg = c[0] + c[1] * r0 + c[2] * r1 + c[3] * r2 + c[4] * r0 * r0 + c[5] * r1 * r1 + c[6] * r2 * r2 +
-                          c[7] * r0 * r1 + c[8] * r0 * r2 + c[9] * r1 * r2;
-        const double ph = pm.global + bg;
-        P.cis0[(size_t)z * P.plane + x + (size_t)P.snx * y] = make_float2((float)std::cos(ph), (float)std::sin(ph));
-      }
-  }
-  const int sxs = P.o * (nx / 2), sys = P.o * (ny / 2);
-  (void)sxs;
-  (void)sys;
-  const double xoff = (P.o - 1.0) / 2.0, yoff = (P.o - 1.0) / 2.0, ninv = 1.0 / (double)P.plane;
-  const std::vector<double>& k = P.table.traj.k;
-  P.stat.resize(P.nsamp);
-  P.tau_idx.resize(P.nsamp);
-  for (int j = 0; j < P.nsamp; ++j) {  // `SegmentedForward::new` (spiral.rs:159-170)
-    const double ph = -kTau * (k[2 * j] * xoff / P.snx + k[2 * j + 1] * yoff / P.sny);
-    P.stat[j] = make_float2((float)(std::cos(ph) * ninv), (float)(std::sin(ph) * ninv));
-    P.tau_idx[j] = j % P.ns;
-  }
+  std::memset(&P.phase, 0, sizeof P.phase);
+  if (in.phase) P.phase = *in.phase;
   return P;
+}
+
+// The tables of a value per voxel or sample are made where they are read, in FP64 as on the host: their
+// sines and exponentials (786,432 + 131,072 + 65,536 of them at 128 x 128 x 48 with 8 coils in a ring) and
+// the points' tile lists were 80 ms of host time a volume.
+// cis0[z][y][x] = e^{i phi0}: `phase_slice` with a zero shot (kspace.rs:1156-1180)
+__global__ void spiral_phase_kernel(const mrsim_phase_model pm, int snx, int sny, int nz, int o,
+                                    float2* __restrict__ cis0) {
+  const size_t plane = (size_t)snx * sny, n = plane * nz;
+  const double sx = snx / 2.0, sy = sny / 2.0, off = (o - 1.0) / 2.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int z = (int)(i / plane), e = (int)(i % plane), x = e % snx, y = e / snx;
+    const double r0 = (x - sx - off) / o, r1 = (y - sy - off) / o, r2 = z - nz / 2.0;
+    const double* c = pm.background;
+    const double bg = c[0] + c[1] * r0 + c[2] * r1 + c[3] * r2 + c[4] * r0 * r0 + c[5] * r1 * r1 + c[6] * r2 * r2 +
+                      c[7] * r0 * r1 + c[8] * r0 * r2 + c[9] * r1 * r2;
+    double sn, cs;
+    sincos(pm.global + bg, &sn, &cs);
+    cis0[i] = make_float2((float)cs, (float)sn);
+  }
+}
+
+// amp[a][y][x] = scale x `coil_sensitivity` (kspace.rs:226-237) of a ring of `ring` coils
+__global__ void spiral_amp_kernel(double scale, int ring, int snx, int sny, int o, int n, float* __restrict__ amp) {
+  const size_t plane = (size_t)snx * sny, total = plane * ring;
+  const double off = (o - 1.0) / 2.0, c = (double)n / 2.0, r = 0.6 * n, sigma = 0.9 * n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int a = (int)(i / plane), e = (int)(i % plane);
+    double v = 1.0;
+    if (ring > 1) {
+      double sn, cs;
+      sincos(kTau * a / ring, &sn, &cs);
+      const double dx = (e % snx - off) / o - (c + r * cs), dy = (e / snx - off) / o - (c + r * sn);
+      v = exp(-(dx * dx + dy * dy) / (2.0 * sigma * sigma)) + 0.15;
+    }
+    amp[i] = (float)(scale * v);
+  }
 }
 
 // Device inputs of one acquisition's images (all volumes), plus per-element amplitudes.
@@ -846,16 +855,11 @@ static SpiralInputs upload_spiral_inputs(DevArena& A, const SpiralPlan3& P, cons
     I.decay = (float*)A.upload(d.data(), d.size() * 4, st);
     I.lna = (float*)A.upload(la.data(), la.size() * 4, st);
   }
-  std::vector<float> amp((size_t)P.ring * P.plane);
-  const double xoff = (P.o - 1.0) / 2.0, yoff = (P.o - 1.0) / 2.0;
-  for (int a = 0; a < P.ring; ++a)
-    for (int y = 0; y < P.sny; ++y)
-      for (int x = 0; x < P.snx; ++x)
-        amp[(size_t)a * P.plane + x + (size_t)P.snx * y] =
-            (float)(acq.signal_scale *
-                    coil_sensitivity(a, P.ring, ((double)x - xoff) / P.o, ((double)y - yoff) / P.o, P.n, P.n));
-  I.amp = (float*)A.upload(amp.data(), amp.size() * 4, st);
-  I.cis0 = (float2*)A.upload(P.cis0.data(), P.cis0.size() * sizeof(float2), st);
+  I.amp = (float*)A.alloc((size_t)P.ring * P.plane * 4);
+  spiral_amp_kernel<<<g3(P.ring * P.plane, 1, 1), 256, 0, st>>>(acq.signal_scale, P.ring, P.snx, P.sny, P.o, P.n, I.amp);
+  I.cis0 = (float2*)A.alloc(P.nvox * sizeof(float2));
+  spiral_phase_kernel<<<g3(P.nvox, 1, 1), 256, 0, st>>>(P.phase, P.snx, P.sny, P.nz, P.o, I.cis0);
+  MRSIM_CUDA(cudaGetLastError());
   return I;
 }
 
@@ -903,7 +907,8 @@ static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, c
   DevArena C(ctx);
   NufftGrid grid = make_nufft<float>(C, P.snx, P.sny, -P.o * (P.n / 2), -P.o * (P.n / 2), P.snx, P.sny, 1e-12, st);
   const double* d_k = (const double*)C.upload(P.table.traj.k.data(), P.table.traj.k.size() * 8, st);
-  const float2* d_stat = (const float2*)C.upload(P.stat.data(), P.stat.size() * sizeof(float2), st);
+  float2* d_stat = (float2*)C.alloc((size_t)nsamp * sizeof(float2));
+  spiral_stat(d_k, nsamp, P.snx, P.sny, P.o, P.o, d_stat, st);
   float2* k2 = (float2*)C.alloc((size_t)nvar * ring * nsrc * nz * nsamp * sizeof(float2));
   MRSIM_CUDA(cudaMemsetAsync(k2, 0, (size_t)nvar * ring * nsrc * nz * nsamp * sizeof(float2), st));
   // per slice: slots (a, s) with their plans; the plans' tables and every slice's slots go up once, so

@@ -282,9 +282,9 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
   tw_2n = (const double2*)upload_twiddles<double>(A, 2 * n, st);
   k_host.assign(k, k + 2 * (size_t)npts);
   d_k = (double*)A.upload(k, (size_t)npts * 2 * 8, st);
-  bins_k = nufft_bins2(A, g.nf0, g.nf1, g.w, k, npts, st);
   d_w = (double*)A.alloc((size_t)npts * 8);
   DevArena T(ctx);
+  bins_k = nufft_bins2(A, T, g.nf0, g.nf1, g.w, d_k, npts, st);
   // Pipe-Menon (grid_recon.rs:54-66)
   {
     std::vector<double> ones(npts, 1.0);
@@ -343,7 +343,7 @@ SpiralRecon::SpiralRecon(mrsim_context* c, const double* k, int npts_, int n_, c
     real_to_complex_kernel<<<grid1(npts), 256, 0, st>>>(d_w, sc * sc, npts, wc);
     double2* tmodes = (double2*)T.alloc((size_t)m * m * 16);
     double2* work = (double2*)T.alloc((size_t)g2.nf0 * g2.nf1 * 16);
-    const NufftBins bins2 = nufft_bins2(T, g2.nf0, g2.nf1, g2.w, u2.data(), npts, st);
+    const NufftBins bins2 = nufft_bins2(T, T, g2.nf0, g2.nf1, g2.w, du2, npts, st);
     nufft_type1<double>(g2, du2, npts, bins2, wc, 1, npts, tmodes, (size_t)m * m, work, -1, st);
     d_tf = (double2*)A.alloc((size_t)m * m * 16);
     circulant_kernel<<<grid1((size_t)m * m), 256, 0, st>>>(tmodes, n, d_tf);

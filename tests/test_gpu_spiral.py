@@ -349,3 +349,16 @@ def test_tiled_type2_matches_the_oracle(gpu_ctx, sx, sy, npts, fmax):
     want = O.spiral_segmented(inp, acq, 0, 1, k, ti, plan.tau_l, plan.b, None, False)
     assert rel_l2(got, want) <= 1e-5
     assert np.abs(got - want).max() <= 5e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n0,n1,npts", [(3, 5, 1), (9, 40, 255), (32, 33, 257), (64, 20, 5000)])
+def test_spread_lists_match_the_oracle(gpu_ctx, n0, n1, npts):
+    # rings narrower than the window, cut last tiles, positions at and beyond the period's ends
+    rng = np.random.default_rng(npts)
+    u = (rng.random((npts, 2)) - 0.5) * [n0, n1]
+    if npts > 100:
+        u[:4] = [[-n0 / 2, n1 / 2], [n0, -n1], [n0 / 2 - 1e-12, 0.0], [2.5 * n0, -1.5 * n1]]
+    w = rng.normal(size=npts) + 1j * rng.normal(size=npts)
+    lo, mo = [-(n0 // 2), -(n1 // 2)], [n0, n1]
+    got = S.Nufft2([n0, n1], lo, mo, 1e-6, ctx=gpu_ctx).type1(u, w, -1)
+    assert rel_l2(got.ravel(), O.nufft2(1, [n0, n1], lo, mo, 1e-6, u, w, -1)) <= 2e-6

@@ -187,3 +187,15 @@ def test_kz_fits_of_ragged_sizes_match_the_oracle(gpu_ctx, accel, rows):
     vols, _, _ = O.simulate_acquisition_3d_spiral(*args, phase=PhaseModel.none(), seed=3, kz_opts=kzo)
     z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
     assert rel_l2(z, vols.T.ravel()) <= 1e-5
+
+
+def test_device_tables_of_phase_and_rings_match_the_oracle(gpu_ctx):
+    # every term of the phase polynomial, a ring of three coils
+    c = case("rings")
+    phase = PhaseModel(0.4, [0.3, 0.01, -0.02, 0.05, 1e-3, -2e-3, 4e-3, 1e-3, 2e-3, -3e-3])
+    args = (c["sim"], c["acqd"], c["nv"], c["images"], c["t2"], c["t1"], c["fmap"], c["ti"],
+            c["acq"].replace(n_coils=6), c["tr"], c["ro"])
+    mag, ph = K3.simulate_acquisition_3d(*args, phase=phase, seed=3, kz_opts=c["kzo"], ctx=gpu_ctx)
+    vols, _, _ = O.simulate_acquisition_3d_spiral(*args, phase=phase, seed=3, kz_opts=c["kzo"])
+    z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
+    assert rel_l2(z, vols.T.ravel()) <= 1e-5
