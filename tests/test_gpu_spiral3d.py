@@ -199,3 +199,19 @@ def test_device_tables_of_phase_and_rings_match_the_oracle(gpu_ctx):
     vols, _, _ = O.simulate_acquisition_3d_spiral(*args, phase=phase, seed=3, kz_opts=c["kzo"])
     z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
     assert rel_l2(z, vols.T.ravel()) <= 1e-5
+
+
+@pytest.mark.parametrize("nz", [7, 10])
+def test_pocs_of_ragged_partitions_matches_the_oracle(gpu_ctx, nz):
+    # partition counts and restored partitions that are no multiples of four
+    n, o = 16, 2
+    s = n * o
+    kz = K3.KzSampling(0.75, 1)
+    args = ([s, s, nz], [n, n, nz], 1, blobs(s, s, nz, 1, 1), [T2.uniform(80.0)], None, spiral_fmap(s, s, nz), None,
+            Acquisition(do_relaxation=False, do_distortions=True, n_coils=2, signal_scale=100.0), kz_train(nz, kz),
+            spiral_ro(kz.partial_fourier, kz.accel))
+    kzo = K3.KzOptions(coil_rows=2, pocs=True)
+    mag, ph = K3.simulate_acquisition_3d(*args, phase=PhaseModel.none(), seed=3, kz_opts=kzo, ctx=gpu_ctx)
+    vols, _, _ = O.simulate_acquisition_3d_spiral(*args, phase=PhaseModel.none(), seed=3, kz_opts=kzo)
+    z = mag.astype(np.float64) * np.exp(1j * ph.astype(np.float64))
+    assert rel_l2(z, vols.T.ravel()) <= 1e-5
