@@ -83,14 +83,17 @@ size_t nufft_spread_taps(const NufftGridT<double>& g, int npts, int batch);
 // Type 2 of a batch of FP32 mode grids (packed [item][m1][m0]) at points ordered by window origin
 // (nufft_tiled.cu), sign +1: out[point][item].  grid: batch fine grids; tmp: batch x m_out1 x nf0.
 struct NufftPoints {
-  const double* u = nullptr;
-  int npts = 0, tiles0 = 0, max_items = 0;
+  int tiles0 = 0, max_items = 0;
+  bool wide = false;  // tiles of 16 x 8 origins, not 8 x 4
   int4* items = nullptr;
   int* n_items = nullptr;
   const int* pts = nullptr;
+  const int* key = nullptr;
+  const float* taps = nullptr;
 };
 bool nufft_tiled_fits(const NufftGrid& g);
-NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, cudaStream_t st);
+// batch: the most items that a call will bring (it chooses the tiles)
+NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, int batch, cudaStream_t st);
 void nufft_type2_tiled(const NufftGrid& g, const float2* modes, int batch, const NufftPoints& P, float2* out,
                        float2* grid, float2* tmp, cudaStream_t st);
 

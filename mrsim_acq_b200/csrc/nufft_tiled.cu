@@ -7,14 +7,15 @@
 //   rows      a warp reads a mode row, deapodizes it and transforms it zero-padded to the fine length;
 //             only the mode rows exist between the two passes
 //   columns   16 columns at a time through shared memory; the zero rows are never read
-//   points    a block holds the 20 x 16 fine cells around a tile of 8 x 4 window origins for 32 (or 16)
-//             batch items, and each warp serves four points of one origin at once with the items on
-//             its lanes, so a cell is read once from shared memory for the four and the grid once from
-//             L2 per tile.  The points are ordered by window origin once per trajectory, on the device.
+//   points    a block holds the fine cells around a tile of window origins for 16 batch items, and each
+//             half-warp serves four points of one origin at once with the items on its lanes, so a
+//             cell is read once from shared memory for the four and the grid from L2 once per tile.
+//             The points are ordered by window origin and their taps formed once per trajectory.
 // The taps and each point's sum are the general kernel's, operation for operation.  Bound by the FMA pipe
 // (two FMAs per tap, item and point, a quarter of them for the empty places of a group).  Results come
 // out [point][item]: the combination that follows reads an item range of a point in one run.
-// That slice takes 0.28 + 0.06 ms (16 segments of one coil: 134 + 49 us, here 58 + 17 + 10 for the order).
+// That slice takes 0.24 + 0.06 ms (16 segments of one coil: 134 + 49 us, here 51 + 17 + 22 for the order and
+// the taps).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,52 +30,75 @@ namespace mrsim {
 namespace {
 
 constexpr int kW = 13;                            // taps per axis
-constexpr int kTX = 8, kTY = 4, kCells = kTX * kTY;  // window origins of a tile
-constexpr int kRX = kTX + kW - 1, kRY = kTY + kW - 1;  // fine cells they reach
+// Window origins of a tile, and the groups of points a block takes at a time.  The wide tile reads each
+// grid cell 4.4 times instead of 10 and leaves fewer half-warps without a group; the small one gives a
+// batch of one chunk enough blocks.
+struct Small {
+  static constexpr int kTX = 8, kTY = 4, kGroups = 32;
+};
+struct Wide {
+  static constexpr int kTX = 16, kTY = 8, kGroups = 64;
+};
 constexpr int kGroup = 4;                         // points of one origin a warp serves together
-constexpr int kItemGroups = 32;                   // groups a block takes at a time
+constexpr int kItems = 16;                        // batch items of a block
+constexpr int kTapStride = 28;                    // floats a point: its taps of each axis, two unused
 
 __device__ __forceinline__ int wrap_cell(int m, int n) { return m < 0 ? m + n : (m >= n ? m - n : m); }
 
-__device__ __forceinline__ int origin(double u, int nf) {
-  double p;
-  return wrap_cell(es_origin(u, nf, 0.5 * kW, p), nf);
-}
-
-// key[j] = tile * kCells + cell of the point's origin; rank[j] its place among the points of that origin
-__global__ void points_key_kernel(const double* __restrict__ u, int npts, int nf0, int nf1, int tiles0,
-                                  int* __restrict__ count, int* __restrict__ key, int* __restrict__ rank) {
+// key[j] = tile * kCells + cell of the point's origin; rank[j] its place among the points of that
+// origin; taps[j] its taps.
+template <class T>
+__global__ void points_key_kernel(const double* __restrict__ u, int npts, int nf0, int nf1, float beta, int tiles0,
+                                  int* __restrict__ count, int* __restrict__ key, int* __restrict__ rank,
+                                  float* __restrict__ taps) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= npts) return;
-  const int a0 = origin(u[2 * j], nf0), a1 = origin(u[2 * j + 1], nf1);
-  const int k = ((a1 / kTY) * tiles0 + a0 / kTX) * kCells + (a1 % kTY) * kTX + a0 % kTX;
+  float k0[kWMax], k1[kWMax];
+  const int a0 = wrap_cell(es_taps<float>(u[2 * j], nf0, kW, beta, k0), nf0);
+  const int a1 = wrap_cell(es_taps<float>(u[2 * j + 1], nf1, kW, beta, k1), nf1);
+  const int k = ((a1 / T::kTY) * tiles0 + a0 / T::kTX) * (T::kTX * T::kTY) + (a1 % T::kTY) * T::kTX + a0 % T::kTX;
   key[j] = k;
   rank[j] = atomicAdd(&count[k], 1);  // (which point gets which place changes no result)
+  float* t = taps + (size_t)j * kTapStride;
+#pragma unroll
+  for (int i = 0; i < kW; ++i) {
+    t[i] = k0[i];
+    t[kW + i] = k1[i];
+  }
 }
 
 // One warp per tile: each origin's first group within the tile (ceil(count / kGroup) groups each) and
 // the tile's groups.  The scan over the tiles then has only their number to walk: one block over every
 // origin took 120 us at 65,536 of them.
+template <class T>
 __global__ void __launch_bounds__(256) points_tile_kernel(const int* __restrict__ count, int tiles,
                                                           int* __restrict__ local, int* __restrict__ groups) {
+  constexpr int kCells = T::kTX * T::kTY;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= tiles) return;
-  const int v = (count[t * kCells + lane] + kGroup - 1) / kGroup;
-  int x = v;
+  int base = 0;
 #pragma unroll
-  for (int h = 1; h < 32; h <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, x, h);
-    if (lane >= h) x += o;
+  for (int c = lane; c < kCells; c += 32) {
+    const int v = (count[t * kCells + c] + kGroup - 1) / kGroup;
+    int x = v;
+#pragma unroll
+    for (int h = 1; h < 32; h <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, x, h);
+      if (lane >= h) x += o;
+    }
+    local[t * kCells + c] = base + x - v;
+    base += __shfl_sync(0xffffffffu, x, 31);
   }
-  local[t * kCells + lane] = x - v;
-  if (lane == 31) groups[t] = x;
+  if (lane == 0) groups[t] = base;
 }
 
 // One block: first group of each tile, and the work items (tile, first group, groups) of up to
-// kItemGroups groups.
+// T::kGroups groups.
+template <class T>
 __global__ void __launch_bounds__(1024) points_scan_kernel(const int* __restrict__ groups, int tiles,
                                                            int* __restrict__ first, int4* __restrict__ items,
                                                            int* __restrict__ n_items) {
+  constexpr int kItemGroups = T::kGroups;
   __shared__ int part[2][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = (tiles + 1023) / 1024;
   int v[2] = {0, 0};  // groups and items of this thread's tiles
@@ -104,11 +128,13 @@ __global__ void __launch_bounds__(1024) points_scan_kernel(const int* __restrict
   }
 }
 
+template <class T>
 __global__ void points_place_kernel(const int* __restrict__ key, const int* __restrict__ rank, int npts,
                                     const int* __restrict__ first, const int* __restrict__ local,
                                     int* __restrict__ pts) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= npts) return;
+  constexpr int kCells = T::kTX * T::kTY;
   const int k = key[j];
   pts[(first[k / kCells] + local[k] + rank[j] / kGroup) * kGroup + rank[j] % kGroup] = j;
 }
@@ -197,19 +223,21 @@ __global__ void __launch_bounds__(256) mode_cols_kernel(const NufftGrid g, const
   for (int i = threadIdx.x; i < N * kCols; i += 256) dst[(size_t)(i / kCols) * nf0 + i % kCols] = s[(i / kCols) * LD + i % kCols];
 }
 
-template <int BI>
+template <class T>
 constexpr size_t points_smem() {
-  return sizeof(float2) * (size_t)kRX * kRY * (BI + 1) + sizeof(float4) * 2 * kItemGroups * kW +
-         sizeof(int) * (kItemGroups * (kGroup + 1));
+  return sizeof(float2) * (size_t)(T::kTX + kW - 1) * (T::kTY + kW - 1) * (kItems + 1) +
+         sizeof(float4) * 2 * T::kGroups * kW + sizeof(int) * (T::kGroups * (kGroup + 1));
 }
 
-// BI batch items on 32 / BI groups of a warp's lanes.
-template <int BI>
+// kItems batch items on the lanes of each half-warp.
+template <class T>
 __global__ void __launch_bounds__(256, 2) points_kernel(const NufftGrid g, const float2* __restrict__ grid,
-                                                        const double* __restrict__ u, const int4* __restrict__ items,
-                                                        const int* __restrict__ n_items, const int* __restrict__ pts,
-                                                        int tiles0, int batch, float2* __restrict__ out) {
-  constexpr int LD = BI + 1, LANES = 32 / BI;
+                                                        const float* __restrict__ taps, const int* __restrict__ key,
+                                                        const int4* __restrict__ items, const int* __restrict__ n_items,
+                                                        const int* __restrict__ pts, int tiles0, int batch,
+                                                        float2* __restrict__ out) {
+  constexpr int BI = kItems, LD = BI + 1, LANES = 32 / BI, kItemGroups = T::kGroups;
+  constexpr int kRX = T::kTX + kW - 1, kRY = T::kTY + kW - 1;  // fine cells that the tile's windows reach
   extern __shared__ __align__(16) unsigned char psm[];
   float4* k0s = reinterpret_cast<float4*>(psm);        // [group][tap] of the group's four points
   float4* k1s = k0s + kItemGroups * kW;
@@ -223,7 +251,7 @@ __global__ void __launch_bounds__(256, 2) points_kernel(const NufftGrid g, const
   const int n = *n_items;
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const int4 item = items[it];
-    const int ng = item.z, x0 = (item.x % tiles0) * kTX, y0 = (item.x / tiles0) * kTY;
+    const int ng = item.z, x0 = (item.x % tiles0) * T::kTX, y0 = (item.x / tiles0) * T::kTY;
     __syncthreads();  // every thread is done with the item before
     for (int i = tid; i < kRX * kRY * BI; i += 256) {  // neighbouring threads take neighbouring cells
       const int c = i % (kRX * kRY), b = i / (kRX * kRY);
@@ -233,20 +261,23 @@ __global__ void __launch_bounds__(256, 2) points_kernel(const NufftGrid g, const
     for (int t = tid; t < ng * kGroup; t += 256) {
       const int j = pts[item.y * kGroup + t];
       pj[t] = j;
-      float k0[kWMax], k1[kWMax];
+      if (t % kGroup == 0) {  // a group's first place is never empty
+        const int c = key[j] % (T::kTX * T::kTY);
+        at[t / kGroup] = (c / T::kTX) * kRX + c % T::kTX;
+      }
+      float k[kTapStride];
+      const float4* src = reinterpret_cast<const float4*>(taps + (size_t)max(j, 0) * kTapStride);
 #pragma unroll
-      for (int i = 0; i < kW; ++i) k0[i] = k1[i] = 0.f;
-      if (j >= 0) {
-        const int a0 = wrap_cell(es_taps<float>(u[2 * j], nf0, kW, g.beta, k0), nf0);
-        const int a1 = wrap_cell(es_taps<float>(u[2 * j + 1], nf1, kW, g.beta, k1), nf1);
-        if (t % kGroup == 0) at[t / kGroup] = (a1 - y0) * kRX + (a0 - x0);
+      for (int i = 0; i < kTapStride / 4; ++i) {
+        const float4 v = j >= 0 ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        k[4 * i] = v.x, k[4 * i + 1] = v.y, k[4 * i + 2] = v.z, k[4 * i + 3] = v.w;
       }
       float* f0 = reinterpret_cast<float*>(k0s + (t / kGroup) * kW) + t % kGroup;
       float* f1 = reinterpret_cast<float*>(k1s + (t / kGroup) * kW) + t % kGroup;
 #pragma unroll
       for (int i = 0; i < kW; ++i) {
-        f0[kGroup * i] = k0[i];
-        f1[kGroup * i] = k1[i];
+        f0[kGroup * i] = k[i];
+        f1[kGroup * i] = k[kW + i];
       }
     }
     __syncthreads();
@@ -309,14 +340,15 @@ bool nufft_tiled_fits(const NufftGrid& g) {
   return g.w == kW && g.nf0 % 64 == 0 && g.nf1 % 64 == 0 && g.nf0 <= 256 && g.nf1 <= 256;
 }
 
-NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, cudaStream_t st) {
+namespace {
+template <class T>
+NufftPoints make_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, cudaStream_t st) {
+  constexpr int kCells = T::kTX * T::kTY;
   NufftPoints P;
-  P.u = d_u;
-  P.npts = npts;
-  P.tiles0 = (g.nf0 + kTX - 1) / kTX;
-  const int tiles = P.tiles0 * ((g.nf1 + kTY - 1) / kTY), nkeys = tiles * kCells;
-  // every group holds at least one point; an item is a whole kItemGroups groups or a tile's last
-  const size_t max_items = (size_t)tiles + npts / kItemGroups + 1;
+  P.tiles0 = (g.nf0 + T::kTX - 1) / T::kTX;
+  const int tiles = P.tiles0 * ((g.nf1 + T::kTY - 1) / T::kTY), nkeys = tiles * kCells;
+  // every group holds at least one point; an item is a whole T::kGroups groups or a tile's last
+  const size_t max_items = (size_t)tiles + npts / T::kGroups + 1;
   int* count = (int*)A.alloc((size_t)nkeys * 4);
   int* key = (int*)A.alloc((size_t)npts * 4);
   int* rank = (int*)A.alloc((size_t)npts * 4);
@@ -324,17 +356,42 @@ NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int
   int* groups = (int*)A.alloc((size_t)tiles * 4);
   int* first = (int*)A.alloc((size_t)tiles * 4);
   int* pts = (int*)A.alloc((size_t)npts * kGroup * 4);
+  float* taps = (float*)A.alloc((size_t)npts * kTapStride * 4);
   P.items = (int4*)A.alloc(max_items * sizeof(int4));
   P.n_items = (int*)A.alloc(4);
   P.pts = pts;
+  P.key = key;
+  P.taps = taps;
   P.max_items = (int)max_items;
   MRSIM_CUDA(cudaMemsetAsync(count, 0, (size_t)nkeys * 4, st));
   MRSIM_CUDA(cudaMemsetAsync(pts, 0xff, (size_t)npts * kGroup * 4, st));
-  points_key_kernel<<<(npts + 255) / 256, 256, 0, st>>>(d_u, npts, g.nf0, g.nf1, P.tiles0, count, key, rank);
-  points_tile_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(count, tiles, local, groups);
-  points_scan_kernel<<<1, 1024, 0, st>>>(groups, tiles, first, P.items, P.n_items);
-  points_place_kernel<<<(npts + 255) / 256, 256, 0, st>>>(key, rank, npts, first, local, pts);
+  points_key_kernel<T><<<(npts + 255) / 256, 256, 0, st>>>(d_u, npts, g.nf0, g.nf1, g.beta, P.tiles0, count, key, rank,
+                                                           taps);
+  points_tile_kernel<T><<<(tiles + 7) / 8, 256, 0, st>>>(count, tiles, local, groups);
+  points_scan_kernel<T><<<1, 1024, 0, st>>>(groups, tiles, first, P.items, P.n_items);
+  points_place_kernel<T><<<(npts + 255) / 256, 256, 0, st>>>(key, rank, npts, first, local, pts);
   MRSIM_CUDA(cudaGetLastError());
+  return P;
+}
+
+template <class T>
+void launch_points(const NufftGrid& g, const float2* grid, const NufftPoints& P, int batch, float2* out,
+                   cudaStream_t st) {
+  constexpr size_t smem = points_smem<T>();
+  MRSIM_CUDA(cudaFuncSetAttribute(points_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int chunks = (batch + kItems - 1) / kItems;
+  const int blocks = std::max(1, std::min(P.max_items, (2 * 148 * 4 + chunks - 1) / chunks));
+  points_kernel<T><<<dim3(blocks, chunks), 256, smem, st>>>(g, grid, P.taps, P.key, P.items, P.n_items, P.pts, P.tiles0,
+                                                            batch, out);
+}
+}  // namespace
+
+NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, int batch, cudaStream_t st) {
+  // 65,536 points on a 256 x 256 fine grid: 16 items 51 us with small tiles and 55 with wide ones, 128 items
+  // 276 and 244.  The line between: three chunks give the wide tiles' blocks five items each to even out.
+  const bool wide = batch > 2 * kItems;
+  NufftPoints P = wide ? make_points<Wide>(A, g, d_u, npts, st) : make_points<Small>(A, g, d_u, npts, st);
+  P.wide = wide;
   return P;
 }
 
@@ -350,17 +407,10 @@ void nufft_type2_tiled(const NufftGrid& g, const float2* modes, int batch, const
   MRSIM_NT(launch_rows, g.nf0 / 32, g, modes, batch, tmp, st)
   MRSIM_NT(launch_cols, g.nf1 / 32, g, tmp, batch, grid, st)
 #undef MRSIM_NT
-  // 16 items a block where no more are wanted: the lanes then take two groups of points
-  auto points = [&](auto kernel, int bi, size_t smem) {
-    MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int chunks = (batch + bi - 1) / bi;
-    const int blocks = std::max(1, std::min(P.max_items, (2 * 148 * 4 + chunks - 1) / chunks));
-    kernel<<<dim3(blocks, chunks), 256, smem, st>>>(g, grid, P.u, P.items, P.n_items, P.pts, P.tiles0, batch, out);
-  };
-  if (batch <= 16)
-    points(points_kernel<16>, 16, points_smem<16>());
+  if (P.wide)
+    launch_points<Wide>(g, grid, P, batch, out, st);
   else
-    points(points_kernel<32>, 32, points_smem<32>());
+    launch_points<Small>(g, grid, P, batch, out, st);
   MRSIM_CUDA(cudaGetLastError());
 }
 

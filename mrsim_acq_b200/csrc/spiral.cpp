@@ -345,7 +345,7 @@ SegmentedInfo spiral_segmented_host(mrsim_context* ctx, const mrsim_slice_input&
   const bool tiled = nufft_tiled_fits(g);
   if (tiled) {
     float2* tmp = (float2*)A.alloc((size_t)L * g.m_out1 * g.nf0 * sizeof(float2));
-    nufft_type2_tiled(g, imgs, L, nufft_points(A, g, du, npts, st), seg, work, tmp, st);
+    nufft_type2_tiled(g, imgs, L, nufft_points(A, g, du, npts, L, st), seg, work, tmp, st);
   } else {
     nufft_type2<float>(g, imgs, L, n, du, npts, seg, npts, work, 1, nullptr, st);
   }

@@ -993,7 +993,7 @@ static void spiral_samples(const SpiralPlan3& P, const SpiralInputs& I, int g, c
   float2* work = (float2*)C.alloc((size_t)most * grid.nf0 * grid.nf1 * sizeof(float2));
   float2* tmp = tiled ? (float2*)C.alloc((size_t)most * grid.m_out1 * grid.nf0 * sizeof(float2)) : nullptr;
   NufftPoints points;
-  if (tiled) points = nufft_points(C, grid, d_k, nsamp, st);
+  if (tiled) points = nufft_points(C, grid, d_k, nsamp, most, st);
   for (int z = 0; z < nz; ++z) {
     if (tot[z] == 0) continue;
     const TsegPlan *pc = plan_at(P.cls_of[z]), *pv = plan_at(P.vox_of[z]);
