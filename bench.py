@@ -276,7 +276,7 @@ def scale_measurements(args, ctx, stream):
                                  "samples_per_step": smp, "ms_per_step": tot / steps,
                                  "value": smp / (tot / steps * 1e-3), "unit": "samples/s",
                                  "stage_ms": dict(zip(STAGES, [round(float(v), 3) for v in st])),
-                                 "note": "exact pair (per-coil kernels: a ring of 32 takes no coil-class path); "
+                                 "note": "exact pair (the ring of 32 as 7 basis rows); "
                                          "the segmented path refuses this shape (more than 16 line groups)"}
     out["stack_of_spirals"] = spiral_measurement(ctx)
     out["mixed_batch"] = mixed_batch_measurement(ctx, stream)

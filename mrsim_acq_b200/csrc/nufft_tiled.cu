@@ -11,11 +11,12 @@
 //             half-warp serves four points of one origin at once with the items on its lanes, so a
 //             cell is read once from shared memory for the four and the grid from L2 once per tile.
 //             The points are ordered by window origin and their taps formed once per trajectory.
-// The taps and each point's sum are the general kernel's, operation for operation.  Bound by the FMA pipe
-// (two FMAs per tap, item and point, a quarter of them for the empty places of a group).  Results come
-// out [point][item]: the combination that follows reads an item range of a point in one run.
-// That slice takes 0.24 + 0.06 ms (16 segments of one coil: 134 + 49 us, here 51 + 17 + 22 for the order and
-// the taps).
+// The taps and each point's sum are the general kernel's, operation for operation.  No pipe is full: at 16
+// items FMA 27 % and shared-memory loads 30 % of the elapsed time, at 128 items FMA about 43 % (a fifth of it
+// for the empty places of a group); a tile's loads and its sums alternate, at two blocks of 108 registers an
+// SM.  Results come out [point][item]: the combination that follows reads an item range of a point in one
+// run.  That slice takes 0.24 + 0.06 ms (16 segments of one coil: 134 + 49 us, here 51 + 17 + 22 for the
+// order and the taps).
 #include <cuda_runtime.h>
 
 #include <algorithm>
