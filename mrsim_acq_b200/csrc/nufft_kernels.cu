@@ -1,7 +1,7 @@
 // nufft_kernels.cu — the 2D NUFFT pair of the stack-of-spirals path on the device (reference
 // `Nufft2`, nufft.rs:125-299): exponential-of-semicircle kernel exp(beta (sqrt(1 - z^2) - 1)),
 // beta = 2.30 w, w = ceil(-log10 tol) + 1 clamped to 2..16, oversampling 2, deapodization by the
-// kernel's sampled transform.  Type 1 spreads (tiles, in point order), type 2 interpolates; the fine-grid
+// kernel's sampled transform.  Type 1 spreads (tiles, in a fixed order), type 2 interpolates; the fine-grid
 // FFT is a shared-memory radix-2 kernel (a direct DFT for lengths that are not powers of two).
 // Point positions and kernel offsets are formed in FP64 (the kernel is steep: an FP32 position
 // would cost ~1e-5 of relative accuracy); the taps and sums are FP32.
