@@ -44,7 +44,7 @@ def _flags(src: pathlib.Path) -> list[str]:
 def build(verbose: bool = False, force: bool = False) -> pathlib.Path:
     OBJ.mkdir(exist_ok=True)
     srcs = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")))
-    headers = list(CSRC.glob("*.h")) + list((HERE.parent / "include").glob("*.h"))
+    headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((HERE.parent / "include").glob("*.h"))
     newest_header = max((h.stat().st_mtime for h in headers), default=0.0)
     exe = nvcc()
 
