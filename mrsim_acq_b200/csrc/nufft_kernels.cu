@@ -226,14 +226,15 @@ __device__ __forceinline__ int ring_offset(int c, int a, int n) {
 
 // ---- the points of each spread tile ---------------------------------------------------------------
 // lo[axis][j]: the ring cell one before the point's window (the window is widened by a cell each side);
-// -1 where the position is not finite (its taps are zero: it reaches no tile).
+// -1 where either coordinate has no position (its taps are zero: it reaches no tile).
 __global__ void bins_origin_kernel(const double* __restrict__ u, int npts, int nf0, int nf1, int w, int* __restrict__ lo) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= npts) return;
-  double p;
-  const bool ok = isfinite(u[2 * j]) && isfinite(u[2 * j + 1]);
-  lo[j] = ok ? wrap(es_origin(u[2 * j], nf0, 0.5 * w, p) - 1, nf0) : -1;
-  lo[npts + j] = ok ? wrap(es_origin(u[2 * j + 1], nf1, 0.5 * w, p) - 1, nf1) : -1;
+  double p0, p1;
+  const int a0 = es_origin(u[2 * j], nf0, 0.5 * w, p0), a1 = es_origin(u[2 * j + 1], nf1, 0.5 * w, p1);
+  const bool ok = p0 >= 0.0 && p1 >= 0.0;
+  lo[j] = ok ? wrap(a0 - 1, nf0) : -1;
+  lo[npts + j] = ok ? wrap(a1 - 1, nf1) : -1;
 }
 
 // One block per tile of one axis and parent list (block = parent * tiles + tile): the parent's points

@@ -89,10 +89,11 @@ template NufftGridT<double> make_nufft<double>(DevArena&, int, int, int, int, in
 namespace {
 // The tiles of a fine ring of nf cells (tiles of `tile` cells) that the kernel window of a point
 // at period coordinate u can reach: the window's cells m0 .. m0 + w - 1 (m0 as the device forms
-// it), widened by a cell each side.  A non-finite position reaches none (its taps are zero).
+// it), widened by a cell each side.  A coordinate without a position (u or 2u not finite) reaches none
+// (its taps are zero).
 void window_tiles(double u, int nf, int w, int tile, std::vector<int>& out) {
   out.clear();
-  if (!std::isfinite(u)) return;
+  if (!std::isfinite(2.0 * u)) return;
   const double half = 0.5 * w;
   double p = std::fmod(2.0 * u, (double)nf);
   if (p < 0.0) p += nf;
