@@ -148,6 +148,21 @@ __host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps,
   return adjq_rows(nc, maps);
 }
 
+// Dynamic shared memory of the staged kernels, which hold a table of every row (forward) or line
+// (adjoint) of a tile beside their ring, and the most that a block can have beside their static tables
+// (4 KB of piece offsets at the most).  A plan whose rows or lines do not fit takes the per-thread-load
+// forward and the general adjoint, whose tables are smaller: with three compartments 1,900 lines fit
+// (15 echoes of 128 lines) and the general kernel holds 3,100 to 4,200.
+constexpr size_t kStagedSmem = 227 * 1024 - 4608;
+inline size_t ystage_q_smem(int nc, bool maps, int qg, int max_sny) {
+  return sizeof(float) * ((size_t)kFwdStages * fwdq_planes(nc, maps) * fwdq_rows(nc, maps) * 128 +
+                          (size_t)max_sny * (8 + (qg + 3) / 4 * 4));
+}
+inline size_t yadjoint_q_smem(int nq, int ty, int nc, bool maps, int max_lines) {
+  return sizeof(float2) * (size_t)kAdjStages * adjq_chunk_lines(nq) * nq * 128 +
+         sizeof(float) * (size_t)(max_lines + adjq_chunk_lines(nq)) * (2 * ty + adjq_line_floats(nc, maps));
+}
+
 // How many blocks share one tile of a y-stage (a cluster; each takes a part of the rows or lines and
 // the partial sums meet in distributed shared memory).  A plan of few tiles leaves most of the chip
 // idle and its blocks walk their rows or lines one after another: the count that makes waves times

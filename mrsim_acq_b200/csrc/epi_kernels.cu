@@ -929,6 +929,25 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           if (!(N >= 8 && N <= kXfftMaxN && (N & (N - 1)) == 0)) p->xfft = false;
         }
     }
+    for (int i = 0; i < n; ++i) p->adj_narrow = p->adj_narrow || (hu[i].snx & 1) || ((uintptr_t)hu[i].g & 15);
+    auto has_maps = [&](bool maps) {
+      for (int i = 0; i < n; ++i)
+        if (((hu[i].flags & UF_MAPS) != 0) == maps) return true;
+      return false;
+    };
+    // rows per thread of the fixed-count y-adjoint: the built-in choice, or 2 where 4 would be (the tunable)
+    auto adj_ty = [&](bool maps, bool rows, bool basis) {
+      const int ty = adjq_rows_v(p->nc, maps, rows);
+      return p->opt.adj_rows == 2 && ty == 4 && !(basis && p->adj_narrow) ? 2 : ty;
+    };
+    auto adj_fits = [&](int nq, bool rows, bool basis) {  // on nq coils or rows, for every kind of unit here
+      for (bool maps : {false, true})
+        if (has_maps(maps) &&
+            yadjoint_q_smem(nq, adj_ty(maps, rows, basis), p->nc, maps, p->max_lines) > kStagedSmem)
+          return false;
+      return true;
+    };
+    auto fwd_fits = [&](bool maps) { return ystage_q_smem(p->nc, maps, p->qg, p->max_sny) <= kStagedSmem; };
     // The coil basis (coil_basis, driver.cpp) where every unit has one of the same row count: rings of
     // 6, 7 and 9 or more coils, and of 8 where the class rows have no x-stage (rows past 128 points,
     // the DFT GEMM).  Its 4 to 7 rows replace the coils in both y-stages, whose work per voxel and
@@ -950,6 +969,8 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           nb = 0;
       }
       if ((all8 && cls8) || (any_maps && p->nc > 3)) nb = 0;
+      if (nb && !(adj_fits(nb, true, true) && (!has_maps(false) || fwd_fits(false)) && (!any_maps || fwd_fits(true))))
+        nb = 0;
       p->basis_nb = nb;
     }
     {  // the kernels read the rows a y-stage runs on as geo.ncls rows of geo.eyc and a constant one
@@ -978,6 +999,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       // registers than the 256-thread CTA leaves: those shapes keep the per-thread-load kernel
       if (p->qg == 8 && (p->nc == 8 || (pass == 1 && p->nc >= 4))) ok = false;
       if (!wide && !p->basis_nb) ok = false;
+      if (!fwd_fits(pass == 1)) ok = false;
       p->fwdq[pass] = ok;
       p->fwd_narrow[pass] = !wide;
       // coil classes: every unit with the same 8 coils in 5 classes (the ring) -> 6 accumulators
@@ -1108,12 +1130,11 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
     // 4 or 8), an even snx and 16-byte aligned h rows (cooperative 16-byte copies), and on basis rows
     // any of them (8-byte copies where some row is not so)
     int nq_all = n > 0 ? hu[0].ncoils : 0;
-    for (int i = 0; i < n; ++i) {
+    for (int i = 0; i < n; ++i)
       if (hu[i].ncoils != nq_all || (long long)hu[i].ncoils * hu[i].n_lines * hu[i].snx >= (1LL << 31)) nq_all = 0;
-      p->adj_narrow = p->adj_narrow || (hu[i].snx & 1) || ((uintptr_t)hu[i].g & 15);
-    }
     if (p->adj_narrow) nq_all = 0;
     if (nq_all != 1 && nq_all != 2 && nq_all != 4 && nq_all != 8) nq_all = 0;
+    const bool coil_rows_fit = nq_all == 0 || adj_fits(nq_all, false, false);
     // coil classes in the adjoint: every unit has the 8-coil ring (5 classes + offset), rows of
     // at most 128 points in the warp FFT, and the fixed-count y-adjoint for its shape
     {
@@ -1122,14 +1143,14 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         const UnitDesc& u = hu[i];
         cl = u.ncoils == 8 && u.geo.ncls == 5 && u.geo.coil_off != 0.f && u.geo.cls && u.geo.eyc;
       }
+      if (cl && !adj_fits(6, true, false)) cl = false;
       p->adj_cls = (cl && !p->opt.no_classes) || p->basis_nb > 0;
+      if (!coil_rows_fit) nq_all = 0;
     }
     for (int pass = 0; pass < 4; ++pass) {
       bool maps = pass & 1, grads = pass & 2;
       p->adjq[pass] = p->basis_nb ? p->basis_nb : p->adj_cls ? 6 : (maps && p->nc == 8) ? 0 : nq_all;
-      // rows per thread: the built-in choice, or 2 where 4 would be (the tunable)
-      int ty = adjq_rows_v(p->nc, maps, p->adj_cls);
-      if (p->opt.adj_rows == 2 && ty == 4 && !(p->basis_nb && p->adj_narrow)) ty = 2;
+      const int ty = adj_ty(maps, p->adj_cls, p->basis_nb > 0);
       p->adj_ty[pass] = ty;
       const int step = p->adjq[pass] ? 2 * ty : kTY;
       std::vector<int4> yt;

@@ -633,9 +633,7 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     if (p->adjq[pass]) {
       const int NQv = p->adjq[pass];
       const int TYv = p->adj_ty[pass];
-      const size_t smq = sizeof(float2) * (size_t)kAdjStages * adjq_chunk_lines(NQv) * NQv * 128 +
-                         sizeof(float) * (size_t)(p->max_lines + adjq_chunk_lines(NQv)) *
-                             (2 * TYv + adjq_line_floats(NCv, maps));
+      const size_t smq = yadjoint_q_smem(NQv, TYv, NCv, maps, p->max_lines);
       bool launched = false;
       const bool virt = p->adj_cls;
       const bool small = p->adj_small[pass];

@@ -542,8 +542,7 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     const bool maps = pass == 1;
     const int QG = p->qg, NCv = p->nc;
     if (p->fwdq[pass]) {
-      const size_t smq = sizeof(float) * ((size_t)kFwdStages * fwdq_planes(NCv, maps) * fwdq_rows(NCv, maps) * 128 +
-                                          (size_t)p->max_sny * (8 + (QG + 3) / 4 * 4));
+      const size_t smq = ystage_q_smem(NCv, maps, QG, p->max_sny);
       bool launched = false;
       const int NVv = p->fwd_nv[pass];
       const bool narrow = p->fwd_narrow[pass];
