@@ -87,6 +87,10 @@ __device__ __forceinline__ float2 phase_turns2(float2 s, float2 f, float2 t_hi, 
 // one slice is five launches of 3 to 8 us; the overlap takes the launch gaps and table setups out of
 // its chain (39.9 -> 21.0 us).  Launches of more than kChainTiles tiles keep kernels without the wait,
 // which cost a 1200-unit step 1.5 % and gave it nothing.
+// A chained kernel may be resident while an earlier one of its chain still writes (the y-adjoint while
+// the statics kernel forms the phase, every link having triggered at its start), so what a kernel of
+// the chain writes is not read-only for its lifetime: it is read by plain loads or asynchronous copies,
+// never through __ldg, which is for the tables and planes that copies alone write.
 constexpr int kChainTiles = 4 * 296;
 __device__ __forceinline__ void grid_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void grid_wait() { cudaGridDependencySynchronize(); }

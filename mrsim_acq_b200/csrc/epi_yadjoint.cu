@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   for (int ty = 0; ty < TY; ++ty) {
     const int y = min(y0 + rg * TY + ty, sny - 1);
     const int i = xs_ + snx * y;
-    a[ty] = u.phase ? __ldg(u.phase + i) : 0.f;
+    a[ty] = !u.phase ? 0.f : SPLIT ? u.phase[i] : __ldg(u.phase + i);  // (see grid_wait)
     f[ty] = distort ? __ldg(u.fmap + i) : 0.f;
     la[ty] = (MAPS && u.log_amp) ? __ldg(u.log_amp + i) : 0.f;
     if (MAPS) {
