@@ -608,6 +608,13 @@ void epi_operator_set_fieldmap(EpiOperator* op, const float* fmap) {
 // Selects the y-stages: 0 the exact per-line phasors, 1 / 2 the time-segmented tensor-core
 // contractions in split f16 / split bf16 (built here: segmentation, tables, tensor maps).
 void epi_operator_set_segmented(EpiOperator* op, int precision) {
+  // what fails here leaves the operator as it was: the copy of the fieldmap is kept once it is whole
+  if (precision && op->h_fmap.empty()) {
+    std::vector<float> f((size_t)op->nz * op->snx * op->sny);
+    MRSIM_CUDA(cudaMemcpyAsync(f.data(), op->d_fmap, f.size() * 4, cudaMemcpyDeviceToHost, op->ctx->stream));
+    MRSIM_CUDA(cudaStreamSynchronize(op->ctx->stream));
+    op->h_fmap = std::move(f);
+  }
   // the segmented y-stages write coil or class rows: a plan on basis rows is built again without
   // them, and with them again when the exact path returns
   std::unique_ptr<EpiPlan> was;
@@ -618,16 +625,10 @@ void epi_operator_set_segmented(EpiOperator* op, int precision) {
                               (int)op->plan->host_statics.size(), &o));
     std::swap(was, op->plan);
   }
-  if (precision && op->h_fmap.empty()) {
-    op->h_fmap.resize((size_t)op->nz * op->snx * op->sny);
-    MRSIM_CUDA(cudaMemcpyAsync(op->h_fmap.data(), op->d_fmap, op->h_fmap.size() * 4, cudaMemcpyDeviceToHost,
-                               op->ctx->stream));
-    MRSIM_CUDA(cudaStreamSynchronize(op->ctx->stream));
-  }
   TsPlan* fresh = nullptr;
   try {
     fresh = precision ? ts_plan_build(*op, precision) : nullptr;
-  } catch (...) {  // refused: the operator stays as it was
+  } catch (...) {
     if (was) std::swap(was, op->plan);
     throw;
   }
