@@ -1076,8 +1076,9 @@ int mrsim_spiral_recon_image(mrsim_spiral_recon* rec, const double* samples, int
   if (batch <= 0) return guarded([] { mrsim::fail("batch must be positive"); });
   const size_t np = rec ? (size_t)rec->impl->npts : 0, nn = rec ? (size_t)rec->impl->n * rec->impl->n : 0;
   return recon_call(rec, samples, np * batch, out, nn * batch, [&](double2* i, double2* o) {
-    for (int64_t b0 = 0; b0 < batch; b0 += mrsim::kMaxBatch) {
-      const int nb = (int)std::min<int64_t>(mrsim::kMaxBatch, batch - b0);
+    const int most = rec->impl->max_batch();
+    for (int64_t b0 = 0; b0 < batch; b0 += most) {
+      const int nb = (int)std::min<int64_t>(most, batch - b0);
       rec->impl->images(i + b0 * np, nb, o + b0 * nn);
     }
   });

@@ -1360,8 +1360,9 @@ void spiral3d_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, 
       double2* h = (double2*)C.alloc((size_t)nc * nz * nn * sizeof(double2));
       MRSIM_CUDA(cudaMemsetAsync(h, 0, (size_t)nc * nz * nn * sizeof(double2), st));
       double2* himg = (double2*)C.alloc((size_t)nc * nb * nn * sizeof(double2));
-      for (size_t b0 = 0; b0 < (size_t)nc * nb; b0 += kMaxBatch) {
-        const int cnt = (int)std::min<size_t>(kMaxBatch, (size_t)nc * nb - b0);
+      const size_t most = (size_t)rec.max_batch();
+      for (size_t b0 = 0; b0 < (size_t)nc * nb; b0 += most) {
+        const int cnt = (int)std::min<size_t>(most, (size_t)nc * nb - b0);
         rec.images(hs + b0 * nsamp, cnt, himg + b0 * nn);
       }
       for (int q = 0; q < nc; ++q)

@@ -550,8 +550,9 @@ void SpiralRecon::rings(const double2* d_coil, int n_part, int ncoils, int ring,
   dim3 rg((unsigned)std::min(4096, (npts + 255) / 256), ring, n_part);
   ring_data_kernel<<<rg, 256, 0, st>>>(d_coil, dz, ncoils, ring, npts, data);
   double2* imgs = (double2*)T.alloc((size_t)batch * nn * 16);
-  for (int b0 = 0; b0 < batch; b0 += kMaxBatch) {
-    const int nb = std::min(kMaxBatch, batch - b0);
+  const int most = max_batch();
+  for (int b0 = 0; b0 < batch; b0 += most) {
+    const int nb = std::min(most, batch - b0);
     images(data + (size_t)b0 * npts, nb, imgs + (size_t)b0 * nn);
   }
   ring_combine_kernel<<<grid1(nn, n_part), 256, 0, st>>>(imgs, dsens, dz2, ring, (int)nn, d_out);

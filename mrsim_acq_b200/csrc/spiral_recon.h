@@ -18,7 +18,6 @@ constexpr double kLsKappa = 100.0;
 constexpr int kPowerIterations = 1000;
 constexpr double kPowerTol = 1e-10;
 constexpr double kLambdaMargin = 1.1;
-constexpr int kMaxBatch = 592;  // images per pass through the Chebyshev iteration: four waves of 148
 
 // The iterations as one launch each, for n = 32, 64, 96, 128 (spiral_iter.cu): tables permuted from
 // the circulant's transform and the band (NULL: none); norms [batch][2] = |r|^2 before and after; out
@@ -61,6 +60,13 @@ struct SpiralRecon {
   // with the call that made it, so its memory comes from the context's pool.
   SpiralRecon(mrsim_context* ctx, const double* k, int npts, int n, const mrsim_acquisition& win_acq,
               int iterations, double kappa, bool band_limited, bool call_scoped = false);
+  // Images per pass through the Chebyshev iteration.  As one launch, four waves of 148 blocks, where a
+  // pass's samples, fine grids and images stay below 8 GB; else 256: the launches per step fill the
+  // chip with fewer, and their padded grids (128 n^2 bytes an image) are 34 GB for 256 at n = 1024.
+  int max_batch() const {
+    const size_t per = ((size_t)npts + (size_t)g.nf0 * g.nf1 + (size_t)n * n) * 16;
+    return d_tfp && 592 * per <= ((size_t)8 << 30) ? 592 : 256;
+  }
   Scratch scratch(DevArena& T, int batch) const;
   void project(double2* x, int batch, cudaStream_t st) const;
   void normal(const double2* x, double2* out, int batch, const Scratch& s, cudaStream_t st) const;
