@@ -46,7 +46,7 @@ def slab_inputs(sim_dims, acq_dims, n_volumes: int, images: Sequence[np.ndarray]
         if v is None:
             return None
         return [T2.of_map(np.ascontiguousarray(np.asarray(m.map).reshape(nz, plane)[z0:z1]).reshape(-1))
-                if m.is_map else m for m in v]
+                if m.map is not None else m for m in v]
 
     return dict(sim_dims=(snx, sny, z1 - z0), acq_dims=(acq_dims[0], acq_dims[1], z1 - z0), n_volumes=n_volumes,
                 images=imgs, fmap=f, t2=maps(t2), t_inhom=maps(t_inhom), slice_z=list(range(z0, z1)), nz_full=nz)
