@@ -1,8 +1,7 @@
-// epi_device.h — what the EPI kernels share (epi_ystage.cu, epi_yadjoint.cu, epi_kernels.cu): packed
+// epi_device.h — what the EPI kernels share (epi_ystage.cu, epi_yadjoint.cu, epi_ythin.cu, epi_kernels.cu): packed
 // arithmetic, the reduced phase, asynchronous copies, and the shapes of the staged kernels' tiles.
 #pragma once
 
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "mrsim_internal.h"
@@ -13,8 +12,6 @@
 #pragma nv_diag_suppress 128
 
 namespace mrsim {
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -85,8 +82,10 @@ __device__ __forceinline__ float2 phase_turns2(float2 s, float2 f, float2 t_hi, 
 // kernel of the chain waits, so what a kernel sees after it is what in-order launches give; copies and
 // kernels that do not call grid_begin are waited for before a launch starts, as always.  A step of
 // one slice is five launches of 3 to 8 us; the overlap takes the launch gaps and table setups out of
-// its chain (39.9 -> 21.0 us).  Launches of more than kChainTiles tiles keep kernels without the wait,
-// which cost a 1200-unit step 1.5 % and gave it nothing.
+// its chain (39.9 -> 21.0 us).  Chained are the y-stages and x-stages of at most kChainTiles tiles and
+// the statics of at most 148 units.  Above that the y-stages run instances without the wait (with it a
+// 1200-unit step took 1.5 % longer and gained nothing), and the x-stages and statics, whose wait then
+// returns at once, plain launches.
 // A chained kernel may be resident while an earlier one of its chain still writes (the y-adjoint while
 // the statics kernel forms the phase, every link having triggered at its start), so what a kernel of
 // the chain writes is not read-only for its lifetime: it is read by plain loads or asynchronous copies,
@@ -167,43 +166,50 @@ inline size_t yadjoint_q_smem(int nq, int ty, int nc, bool maps, int max_lines) 
          sizeof(float) * (size_t)(max_lines + adjq_chunk_lines(nq)) * (2 * ty + adjq_line_floats(nc, maps));
 }
 
-// How many blocks share one tile of a y-stage (a cluster; each takes a part of the rows or lines and
-// the partial sums meet in distributed shared memory).  A plan of few tiles leaves most of the chip
-// idle and its blocks walk their rows or lines one after another: the count that makes waves times
-// steps smallest, with two blocks resident per SM, `steps` row or line steps in a tile and about
-// `setup` steps' worth of tables and reduction in a block.  Fixed by the whole plan, so that ranges of
-// its units give the same bits.
-inline int split_blocks(long long tiles, int steps, int max_split, double setup) {
-  int best = 1;
-  double least = 1e300;
-  for (int s = 1; s <= max_split; s *= 2) {
-    const double waves = (double)((tiles * s + 295) / 296);
-    const double cost = waves * ((double)steps / s + (s > 1 ? setup : 0.5 * setup));
-    if (cost < 0.9 * least) {  // a gain worth the exchange
-      least = cost;
-      best = s;
-    }
-  }
-  return best;
+// The thin y kernels (ystage_thin_kernel, yadjoint_thin_kernel), for plans of few tiles: blocks of 32
+// columns x 4 G lines (forward) or rows (adjoint), whose 8 warps form the terms of different rows or
+// lines side by side and then add them in the same order as the full kernels, operation for operation:
+// a slab computed alone has the bits that it has in its series, whichever form each plan takes.
+constexpr int kThinCols = 32;
+__host__ __device__ __forceinline__ constexpr int thin_rows(int g) { return 32 / g; }  // rows of a forward chunk
+constexpr int kThinLines = 16;  // lines of an adjoint chunk
+__host__ __device__ __forceinline__ constexpr int thin_stages(int nq) { return nq <= 4 ? 3 : 2; }
+inline size_t ystage_thin_smem(int g, int nc, int qg, int max_sny) {
+  return sizeof(float) * ((size_t)kFwdStages * fwdq_planes(nc, false) * thin_rows(g) * kThinCols +
+                          2 * (size_t)thin_rows(g) * 4 * g * kThinCols + (size_t)max_sny * (4 * g + (qg + 3) / 4 * 4));
+}
+inline size_t yadjoint_thin_smem(int g, int nq, int nc, int max_lines) {
+  return sizeof(float2) * ((size_t)thin_stages(nq) * kThinLines * nq * kThinCols +
+                           (size_t)kThinLines * 4 * g * kThinCols) +
+         sizeof(float) * (size_t)(max_lines + kThinLines) * (4 * g + adjq_line_floats(nc, false));
+}
+//
+// thin_groups: G for a plan of `tiles` full tiles of `outs` lines or rows by 128 columns, 0 for the full
+// kernels.  G = 1 makes eight blocks of a full tile, G = 2 four that read less.  Forward and adjoint of n
+// slices of 64 x 64 on 128 x 128 (8 n and 16 n tiles), 8 coils, 3 compartments, in us, G = 1 / 2 / full:
+// n = 1: 17 / 20 / 35 and 14 / 18 / 27; 3: 18 / 17 / 40 and 23 / 18 / 41; 6: 28 / 26 / 38 and 37 / 28 / 42;
+// 12: 50 / 40 / 59 and 66 / 51 / 47; 24: 85 / 68 / 64 and 120 / 87 / 71; one coil: 14 / 15 / 22 and
+// 7 / 8 / 12, n = 8: 23 / 25 / 50 and 17 / 16 / 26, n = 16: 34 / 32 / 52 and 30 / 25 / 28.  So: two blocks
+// an SM of G = 1, then a full tile an SM.
+inline int thin_groups(long long tiles, int outs) {
+  const long long t = tiles * outs / 8;
+  return t <= 37 ? 1 : t <= 148 ? 2 : 0;
 }
 
-// A launch of 256-thread blocks in clusters of `cluster` (1: none) that may start while the kernel
-// before it still runs (`overlap`); the kernel calls grid_begin and grid_wait.
+// A launch of 256-thread blocks that may start while the kernel before it still runs (`overlap`); the
+// kernel calls grid_begin and grid_wait.
 template <class K, class... A>
-void launch_chained(K kernel, dim3 blocks, int cluster, size_t smem, cudaStream_t st, bool overlap, A... args) {
+void launch_chained(K kernel, dim3 blocks, size_t smem, cudaStream_t st, bool overlap, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = blocks;
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = (unsigned)cluster;
-  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
   MRSIM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
@@ -220,6 +226,13 @@ void set_smem(K kernel, size_t bytes) {
                                     227 * 1024 - (int)fa.sharedSizeBytes));
 }
 
+}  // namespace
+
+// The thin kernels' launches of a pass: n tiles (epi_ythin.cu).
+void launch_ystage_thin(const EpiPlan* p, int pass, const int4* tiles, int n, cudaStream_t st);
+void launch_yadjoint_thin(const EpiPlan* p, int pass, const int4* tiles, int n, cudaStream_t st);
+
+namespace {
 // The tiles of units [u0, u1) in a list with per-unit starts `start` (empty: the whole list).
 struct TileRange {
   int t0, n;

@@ -31,6 +31,7 @@
 //   xgemm_kernel                       radix-2 FFT (other powers of two), DFT GEMM (other widths)
 //   yadjoint_q_kernel / yadjoint_kernel  y-adjoint (epi_yadjoint.cu: fixed coil or class count; any
 //                                      coil count)
+//   ystage_thin_kernel / yadjoint_thin_kernel  both for plans of few tiles (epi_ythin.cu), same bits
 // The class-mode and packed (f32x2) paths are exact rearrangements: equal ey rows, and lanes that
 // round like the scalar operations.
 #include <cuda_runtime.h>
@@ -1011,23 +1012,43 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       }
       p->fwd_nv[pass] = p->basis_nb ? p->basis_nb : (cl && !p->opt.no_classes) ? 6 : 0;
     }
-    for (int pass = 0; pass < 2; ++pass) {
-      std::vector<int4> tiles;
-      const int step = p->fwdq[pass] ? 8 : kT;
-      p->y_start[pass].assign(n + 1, 0);
-      for (int i = 0; i < n; ++i) {
-        p->y_start[pass][i] = (int)tiles.size();
-        if (((hu[i].flags & UF_MAPS) != 0) != (pass == 1)) continue;
-        for (int l = 0; l < hu[i].n_lines; l += step)
-          for (int x0 = 0; x0 < hu[i].snx; x0 += 128)
-            for (int q0 = 0; q0 < (p->basis_nb ? 1 : hu[i].ncoils); q0 += p->qg) tiles.push_back(make_int4(i, l, x0, q0));
+    // coil classes through the forward x-stage: every unit's y-stage runs in class mode and the
+    // rows have at most 128 points
+    {
+      bool fc = p->xfft && p->xfft_e >= 1 && p->xfft_e <= 4 && n > 0;
+      for (int pass = 0; pass < 2 && fc; ++pass) {
+        bool any = false;
+        for (int i = 0; i < n && !any; ++i) any = ((hu[i].flags & UF_MAPS) != 0) == (pass == 1);
+        if (any && p->fwd_nv[pass] != 6) fc = false;
       }
-      p->y_start[pass][n] = (int)tiles.size();
+      p->fwd_cls = fc || p->basis_nb > 0;
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+      auto make_tiles = [&](int lines, int cols) {
+        std::vector<int4> t;
+        p->y_start[pass].assign(n + 1, 0);
+        for (int i = 0; i < n; ++i) {
+          p->y_start[pass][i] = (int)t.size();
+          if (((hu[i].flags & UF_MAPS) != 0) != (pass == 1)) continue;
+          for (int l = 0; l < hu[i].n_lines; l += lines)
+            for (int x0 = 0; x0 < hu[i].snx; x0 += cols)
+              for (int q0 = 0; q0 < (p->basis_nb ? 1 : hu[i].ncoils); q0 += p->qg) t.push_back(make_int4(i, l, x0, q0));
+        }
+        p->y_start[pass][n] = (int)t.size();
+        return t;
+      };
+      std::vector<int4> tiles = make_tiles(p->fwdq[pass] ? 8 : kT, 128);
+      const bool small = p->fwdq[pass] && pass == 0 && !p->fwd_narrow[pass] && (int)tiles.size() <= kChainTiles;
+      p->fwd_chain[pass] = small;
+      // (not where the full kernel expands classes to coils)
+      if (small && !(p->fwd_nv[pass] && !p->fwd_cls)) {
+        const int g = thin_groups((long long)tiles.size(), 8);
+        if (g && ystage_thin_smem(g, p->nc, p->qg, p->max_sny) <= kStagedSmem) {
+          p->fwd_thin[pass] = g;
+          tiles = make_tiles(4 * g, kThinCols);
+        }
+      }
       p->n_ytiles[pass] = (int)tiles.size();
-      // (not where this kernel expands classes to coils, whose epilogue holds every class of a line)
-      p->fwd_small[pass] = p->fwdq[pass] && pass == 0 && !p->fwd_narrow[pass] && p->n_ytiles[pass] <= kChainTiles;
-      if (p->fwd_small[pass])
-        p->fwd_split[pass] = split_blocks(p->n_ytiles[pass], p->max_sny, std::min(8, p->max_sny / 16), 16.0);
       arrays.add(&p->d_ytiles[pass], tiles.data(), sizeof(int4) * tiles.size());
     }
     // x-stage tiles of 32 rows, or where those would not fill the chip (two blocks per SM) of one line of
@@ -1086,18 +1107,6 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->n_ftiles = (int)ft.size();
       arrays.add(&p->d_ftiles, ft.data(), sizeof(int4) * ft.size());
     }
-    // coil classes through the forward x-stage: every unit's y-stage runs in class mode and the
-    // rows have at most 128 points
-    {
-      bool fc = p->xfft && p->xfft_e >= 1 && p->xfft_e <= 4 && n > 0;
-      for (int pass = 0; pass < 2 && fc; ++pass) {
-        bool any = false;
-        for (int i = 0; i < n && !any; ++i) any = ((hu[i].flags & UF_MAPS) != 0) == (pass == 1);
-        if (any && p->fwd_nv[pass] != 6) fc = false;
-      }
-      p->fwd_cls = fc || p->basis_nb > 0;
-      if (p->fwd_nv[0] && !p->fwd_cls) p->fwd_small[0] = false;
-    }
     // x-stage GEMM tiles, from host copies of the line tables (one copy per distinct table)
     std::map<const LineRec*, std::vector<LineRec>> host_lines;
     for (int dir = 0; dir < 2 && !p->xfft; ++dir) {
@@ -1152,24 +1161,33 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->adjq[pass] = p->basis_nb ? p->basis_nb : p->adj_cls ? 6 : (maps && p->nc == 8) ? 0 : nq_all;
       const int ty = adj_ty(maps, p->adj_cls, p->basis_nb > 0);
       p->adj_ty[pass] = ty;
-      const int step = p->adjq[pass] ? 2 * ty : kTY;
-      std::vector<int4> yt;
-      p->a_start[pass].assign(n + 1, 0);
-      for (int i = 0; i < n; ++i) {
-        p->a_start[pass][i] = (int)yt.size();
-        bool um = (hu[i].flags & UF_MAPS) != 0;
-        bool ug = (hu[i].flags & (UF_WANT_FMAP_GRAD | UF_WANT_R2_GRAD)) != 0;
-        if (um != maps || ug != grads) continue;
-        for (int y0 = 0; y0 < hu[i].sny; y0 += step)
-          for (int x0 = 0; x0 < hu[i].snx; x0 += 128) yt.push_back(make_int4(i, y0, x0, 0));
+      auto make_tiles = [&](int rows, int cols) {
+        std::vector<int4> t;
+        p->a_start[pass].assign(n + 1, 0);
+        for (int i = 0; i < n; ++i) {
+          p->a_start[pass][i] = (int)t.size();
+          bool um = (hu[i].flags & UF_MAPS) != 0;
+          bool ug = (hu[i].flags & (UF_WANT_FMAP_GRAD | UF_WANT_R2_GRAD)) != 0;
+          if (um != maps || ug != grads) continue;
+          for (int y0 = 0; y0 < hu[i].sny; y0 += rows)
+            for (int x0 = 0; x0 < hu[i].snx; x0 += cols) t.push_back(make_int4(i, y0, x0, 0));
+        }
+        p->a_start[pass][n] = (int)t.size();
+        return t;
+      };
+      const int full = p->adjq[pass] ? 2 * ty : kTY;
+      std::vector<int4> yt = make_tiles(full, 128);
+      const bool small = p->adjq[pass] && !maps && !p->adj_narrow && ty == adjq_rows_v(p->nc, maps, p->adj_cls) &&
+                         (int)yt.size() <= kChainTiles;
+      p->adj_chain[pass] = small;
+      if (small) {
+        const int g = thin_groups((long long)yt.size(), full);
+        if (g && yadjoint_thin_smem(g, p->adjq[pass], p->nc, p->max_lines) <= kStagedSmem) {
+          p->adj_thin[pass] = g;
+          yt = make_tiles(4 * g, kThinCols);
+        }
       }
-      p->a_start[pass][n] = (int)yt.size();
       p->n_atiles[pass] = (int)yt.size();
-      p->adj_small[pass] = p->adjq[pass] && !maps && !p->adj_narrow && ty == adjq_rows_v(p->nc, maps, p->adj_cls) &&
-                           p->n_atiles[pass] <= kChainTiles;
-      if (p->adj_small[pass])
-        p->adj_split[pass] = split_blocks(p->n_atiles[pass], p->max_lines,
-                                          std::min(8, p->max_lines / adjq_chunk_lines(p->adjq[pass])), 8.0);
       arrays.add(&p->d_atiles[pass], yt.data(), sizeof(int4) * yt.size());
     }
     if (!p->basis_nb && (p->adj_cls || p->fwd_cls)) {  // the class x-stage tiles: 4 lines x the 8 coils
@@ -1198,7 +1216,7 @@ void epi_plan_statics(const EpiPlan* p, cudaStream_t st, int u0, int u1) {
   if (u1 == u0) return;
   // a few voxels per thread: eight blocks per unit, or more where the units are few
   const int per_unit = std::max(8, 592 / (u1 - u0));
-  launch_chained(statics_kernel, dim3(std::min(per_unit, (p->max_static_n + 255) / 256), u1 - u0), 1, 0, st,
+  launch_chained(statics_kernel, dim3(std::min(per_unit, (p->max_static_n + 255) / 256), u1 - u0), 0, st,
                  u1 - u0 <= 148, (const StaticDesc*)(p->d_statics + u0));
 }
 
@@ -1229,7 +1247,7 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
   case EV: {                                                                              \
     auto k = xfft_basis_kernel<EV, ADJ>;                                                  \
     set_smem(k, sm);                                                                      \
-    launch_chained(k, dim3((unsigned)count), 1, sm, st, count <= kChainTiles, p->d_units, tiles, p->basis_nb);  \
+    launch_chained(k, dim3((unsigned)count), sm, st, count <= kChainTiles, p->d_units, tiles, p->basis_nb);  \
     break;                                                                                \
   }
 #define MRSIM_XBA(ADJ) MRSIM_XB(1, ADJ) MRSIM_XB(2, ADJ) MRSIM_XB(3, ADJ) MRSIM_XB(4, ADJ) \
@@ -1252,10 +1270,10 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
     const unsigned g = (unsigned)R.n;
 #define MRSIM_XC(ADJ)                                                                             \
   switch (p->xfft_e) {                                                                            \
-    case 1: launch_chained(xfft_warp_kernel<1, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
-    case 2: launch_chained(xfft_warp_kernel<2, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
-    case 3: launch_chained(xfft_warp_kernel<3, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
-    default: launch_chained(xfft_warp_kernel<4, ADJ, true>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, true>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, true>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, true>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    default: launch_chained(xfft_warp_kernel<4, ADJ, true>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
   }
     if (adj) {
       MRSIM_XC(true)
@@ -1274,14 +1292,14 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
       const unsigned g = (unsigned)p->fe_count[E];
 #define MRSIM_XE(ADJ)                                                                               \
   switch (E) {                                                                                      \
-    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
-    default: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;           \
+    default: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;          \
   }
       if (adj) {
         MRSIM_XE(true)
@@ -1300,14 +1318,14 @@ void launch_xstage(const EpiPlan* p, cudaStream_t st, int u0, int u1, bool adj) 
     const unsigned g = (unsigned)R.n;
 #define MRSIM_XF(ADJ)                                                                             \
   switch (p->xfft_e) {                                                                            \
-    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
-    case 8: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 1, 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 1: launch_chained(xfft_warp_kernel<1, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 2: launch_chained(xfft_warp_kernel<2, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 3: launch_chained(xfft_warp_kernel<3, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 4: launch_chained(xfft_warp_kernel<4, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 5: launch_chained(xfft_warp_kernel<5, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 6: launch_chained(xfft_warp_kernel<6, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 7: launch_chained(xfft_warp_kernel<7, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
+    case 8: launch_chained(xfft_warp_kernel<8, ADJ, false>, dim3(g), 0, st, g <= kChainTiles, p->d_units, tiles); break;         \
     default: xfft_kernel<ADJ><<<g, 256, 0, st>>>(p->d_units, tiles);                              \
   }
     if (adj) {

@@ -227,9 +227,8 @@ __global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restric
 // the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
 // or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
 // NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
-// SPLIT: a small launch, chained to the kernel before it: the blocks of a cluster share the tile's lines; each leaves its sums in shared memory and
-// adds up, over the cluster in rank order, and stores the rows rank, rank + blocks, ... of the tile.
-template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW, bool SPLIT>
+// CHAIN: a small launch, chained to the kernel before it.
+template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW, bool CHAIN>
 __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
                                                             const int4* __restrict__ tiles) {
   extern __shared__ __align__(16) float smem[];
@@ -240,10 +239,8 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   constexpr int STAGE = JC * NQ * 128;        // float2 per stage
   constexpr int PIECES = JC * NQ * 64;        // 16-byte pieces per stage
   constexpr int PPT = (PIECES + 255) / 256;   // pieces per thread
-  if (SPLIT) grid_begin();
-  const int nsplit = SPLIT ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
-  const int rank = SPLIT ? (int)cooperative_groups::this_cluster().block_rank() : 0;
-  const int4 tl = tiles[SPLIT ? blockIdx.x / nsplit : blockIdx.x];  // unit, y0, x0
+  if (CHAIN) grid_begin();
+  const int4 tl = tiles[blockIdx.x];  // unit, y0, x0
   const UnitDesc& u = units[tl.x];
   const int snx = u.snx, sny = u.sny, ncomp = u.ncomp, nlines = u.n_lines;
   const int y0 = tl.y, x0 = tl.z;
@@ -257,8 +254,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   const int col = tid & 127, rg = tid >> 7;
   const int x = x0 + col;
   const bool xok = x < snx;
-  const int nch_all = (nlines + JC - 1) / JC;
-  const int cb = SPLIT ? nch_all * rank / nsplit : 0, nchunks = SPLIT ? nch_all * (rank + 1) / nsplit : nch_all;
+  const int nchunks = (nlines + JC - 1) / JC;
 
   // This thread's 16-byte pieces k = tid + 256 i of a chunk: row r = k / 64 = (line jj, coil q),
   // column pair 2 (k % 64); the destination is float2 2k of the stage.  The source offset of
@@ -298,16 +294,15 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
     cp_async_commit();
   };
-  if (!SPLIT) {  // (as in the forward: a small launch fills its tables first)
+  if (!CHAIN) {  // (as in the forward: a small launch fills its tables first)
 #pragma unroll
-    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
+    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(c, c);
   }
 
   const int ys = u.ny / 2;
   const int oy = sny / u.ny;
   const int sys = oy * ys;
-  const int line0 = SPLIT ? cb * JC : 0, line1 = SPLIT ? nchunks * JC : nlp;  // this block's lines
-  for (int idx = line0 * ROWS + tid; idx < line1 * ROWS; idx += 256) {
+  for (int idx = tid; idx < nlp * ROWS; idx += 256) {
     const int j = idx / ROWS, r = idx % ROWS;
     const int y = y0 + r;
     float v = 0.f;
@@ -323,7 +318,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
     Bt[idx] = v;
   }
-  for (int j = line0 + tid; j < line1; j += 256) {
+  for (int j = tid; j < nlp; j += 256) {
     float* e = Lt + j * LF;
     if (j >= nlines) {
 #pragma unroll
@@ -349,10 +344,10 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
   }
 
-  if (SPLIT) {
+  if (CHAIN) {
     grid_wait();
 #pragma unroll
-    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(cb + c, c);
+    for (int c = 0; c < kAdjStages - 1; ++c) issue_chunk(c, c);
   }
   // per-thread constants of its 4 rows
   const bool distort = (u.flags & UF_DISTORT) != 0;
@@ -377,7 +372,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
   for (int ty = 0; ty < TY; ++ty) {
     const int y = min(y0 + rg * TY + ty, sny - 1);
     const int i = xs_ + snx * y;
-    a[ty] = !u.phase ? 0.f : SPLIT ? u.phase[i] : __ldg(u.phase + i);  // (see grid_wait)
+    a[ty] = !u.phase ? 0.f : CHAIN ? u.phase[i] : __ldg(u.phase + i);  // (see grid_wait)
     f[ty] = distort ? __ldg(u.fmap + i) : 0.f;
     la[ty] = (MAPS && u.log_amp) ? __ldg(u.log_amp + i) : 0.f;
     if (MAPS) {
@@ -415,7 +410,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
 
   int s_use = 0, s_issue = kAdjStages - 1;  // stages of chunk c and of chunk c + stages - 1
-  for (int c = cb; c < nchunks; ++c) {
+  for (int c = 0; c < nchunks; ++c) {
     cp_async_wait_n<kAdjStages - 2>();
     __syncthreads();  // chunk c landed for every thread; every thread is done with chunk c - 1
     issue_chunk(c + kAdjStages - 1, s_issue);
@@ -541,7 +536,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
     }
   }
   cp_async_wait0();
-  if (!SPLIT && !xok) return;
+  if (!xok) return;
   if (PK) {
 #pragma unroll
     for (int ty = 0; ty < TY; ++ty)
@@ -557,50 +552,6 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
       }
   }
   const size_t plane = (size_t)snx * sny;
-  if (SPLIT) {
-    constexpr int NF = GRADS ? 4 : 2;  // sums per compartment
-    __syncthreads();                   // every thread is done with the ring
-    float* part = smem;                // [row][compartment][sum][thread]
-#pragma unroll
-    for (int ty = 0; ty < TY; ++ty)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        float* o = part + (ty * NC + c) * NF * 256 + tid;
-        o[0] = cg[ty][c].x;
-        o[256] = cg[ty][c].y;
-        if (GRADS) {
-          o[512] = Uy[ty][GRADS ? c : 0];
-          o[768] = Vx[ty][GRADS ? c : 0];
-        }
-      }
-    cooperative_groups::this_cluster().sync();
-    for (int ty = rank; ty < TY; ty += nsplit) {
-      const int y = y0 + rg * TY + ty;
-      const bool store = xok && y < sny;
-      const size_t i = store ? (size_t)x + (size_t)snx * y : 0;
-      float fg = 0.f;
-      for (int c = 0; c < ncomp; ++c) {
-        float t[NF];
-#pragma unroll
-        for (int k = 0; k < NF; ++k) t[k] = 0.f;
-        for (int r = 0; r < nsplit; ++r) {
-          const float* o = cooperative_groups::this_cluster().map_shared_rank(part, r) + (ty * NC + c) * NF * 256 + tid;
-#pragma unroll
-          for (int k = 0; k < NF; ++k) t[k] += o[256 * k];
-        }
-        if (!store) continue;
-        u.comp_grad[c * plane + i] = make_float2(t[0], t[1]);
-        if (GRADS) {
-          const float m = __ldg(u.comp + (size_t)c * u.comp_stride + i);
-          fg = fmaf(m, t[NF - 2], fg);
-          if (u.r2_grad) u.r2_grad[c * plane + i] = -2.0f * m * t[NF - 1];
-        }
-      }
-      if (GRADS && store && u.fmap_grad) u.fmap_grad[i] = distort ? 4.0f * 3.14159265358979f * fg : 0.f;
-    }
-    cooperative_groups::this_cluster().sync();  // no block leaves while another reads its sums
-    return;
-  }
 #pragma unroll
   for (int ty = 0; ty < TY; ++ty) {
     const int y = y0 + rg * TY + ty;
@@ -630,22 +581,24 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     const int4* tiles = p->d_atiles[pass] + R.t0;
     const bool maps = pass & 1, grads = (pass & 2) != 0;
     const int NCv = p->nc;
+    if (p->adj_thin[pass]) {
+      launch_yadjoint_thin(p, pass, tiles, R.n, st);
+      continue;
+    }
     if (p->adjq[pass]) {
       const int NQv = p->adjq[pass];
       const int TYv = p->adj_ty[pass];
       const size_t smq = yadjoint_q_smem(NQv, TYv, NCv, maps, p->max_lines);
       bool launched = false;
       const bool virt = p->adj_cls;
-      const bool small = p->adj_small[pass];
-      const int split = p->adj_split[pass];
-      const size_t smsplit = std::max(smq, sizeof(float) * 256 * (size_t)TYv * NCv * (grads ? 4 : 2));
+      const bool chain = p->adj_chain[pass];
       // the built-in rows per thread, and 2 rows where the built-in choice is 4
 #define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
   if (NQv == NQV && NCv == NCV && maps == M && grads == G && virt == V && p->adj_narrow == W) { \
-    if (TYv == adjq_rows_v(NCV, M, V) && !M && !W && small) {                           \
+    if (TYv == adjq_rows_v(NCV, M, V) && !M && !W && chain) {                         \
       auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, !M && !W>;   \
-      set_smem(k, smsplit);                                                             \
-      launch_chained(k, dim3((unsigned)R.n * split), split, smsplit, st, true, p->d_units, tiles);   \
+      set_smem(k, smq);                                                                 \
+      launch_chained(k, dim3((unsigned)R.n), smq, st, true, p->d_units, tiles);         \
       launched = true;                                                                  \
     } else if (TYv == adjq_rows_v(NCV, M, V)) {                                         \
       auto k = yadjoint_q_kernel<NQV, adjq_rows_v(NCV, M, V), NCV, M, G, V, W, false>;  \

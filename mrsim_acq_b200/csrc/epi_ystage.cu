@@ -203,10 +203,8 @@ __global__ void __launch_bounds__(128, 4) ystage_kernel(const UnitDesc* __restri
 // the layout the class-mode x-stage expands) instead of the coil rows; 2 writes basis rows (the
 // unit's eyc holds the coil basis, whose last row is constant), G_v = s T_v for every row.
 // NARROW: some plane or row is not on a 16-byte boundary, so the ring fills by 4-byte copies.
-// SPLIT: a small launch, chained to the kernel before it, in which the blocks of a cluster share the tile's rows (not with classes expanded to coils here); each
-// leaves its sums in shared memory and adds up a share of the (line, row) pairs over the cluster, in
-// rank order.  One slice of one coil (64 lines on 128 x 128) has 8 tiles: 23.2 us walked whole.
-template <int QG, int NV, int NC, bool MAPS, bool NARROW, bool SPLIT>
+// CHAIN: a small launch, chained to the kernel before it.
+template <int QG, int NV, int NC, bool MAPS, bool NARROW, bool CHAIN>
 __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __restrict__ units,
                                                           const Tile* __restrict__ tiles, int cls_rows) {
   constexpr int T = 4, TL = 8;
@@ -222,10 +220,8 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   extern __shared__ __align__(16) float smem[];
   float* ring = smem;                           // [stage][plane][RC][128]
   float* Bt = ring + kFwdStages * STAGE;        // [sny][TL]
-  if (SPLIT) grid_begin();
-  const int nsplit = SPLIT ? (int)cg::this_cluster().num_blocks() : 1;
-  const int rank = SPLIT ? (int)cg::this_cluster().block_rank() : 0;
-  const Tile tl = tiles[SPLIT ? blockIdx.x / nsplit : blockIdx.x];
+  if (CHAIN) grid_begin();
+  const Tile tl = tiles[blockIdx.x];
   const UnitDesc& u = units[tl.unit];
   const int snx = u.snx, sny = u.sny, ncomp = u.ncomp;
   float* Ey = Bt + sny * TL;                    // [sny][QGP]: ey per coil, or per class and 1
@@ -247,8 +243,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   }
   __syncthreads();
   const int x0 = tl.x0;
-  const int nch_all = (sny + RC - 1) / RC;
-  const int cb = SPLIT ? nch_all * rank / nsplit : 0, nch = SPLIT ? nch_all * (rank + 1) / nsplit : nch_all;
+  const int nch = (sny + RC - 1) / RC;
   auto issue_rows = [&](int c) {
     if (NARROW && c < nch) {
       float* dst = ring + (c % kFwdStages) * STAGE;
@@ -279,17 +274,16 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   };
   // the first rows fly while the tables fill; a small launch fills its tables while the kernel before
   // it still runs instead
-  if (!SPLIT) {
+  if (!CHAIN) {
 #pragma unroll
-    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(cb + c);
+    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(c);
   }
 
   const int nl = min(TL, u.n_lines - tl.line0);
   const int ys = u.ny / 2;
   const int oy = sny / u.ny;
   const int sys = oy * ys;
-  const int row0 = SPLIT ? cb * RC : 0, row1 = SPLIT ? min(sny, nch * RC) : sny;  // this block's rows
-  for (int idx = row0 * TL + tid; idx < row1 * TL; idx += 256) {
+  for (int idx = tid; idx < sny * TL; idx += 256) {
     const int y = idx / TL, j = idx % TL;
     float v = 0.f;
     if (j < nl) {
@@ -304,7 +298,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
     }
     Bt[idx] = v;
   }
-  for (int idx = row0 * QGP + tid; idx < QGP * row1; idx += 256) {
+  for (int idx = tid; idx < QGP * sny; idx += 256) {
     const int y = idx / QGP, qq = idx % QGP;
     if (NV) {
       const int nc = u.geo.ncls;
@@ -328,10 +322,10 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
       for (int c = 0; c < kMaxComp; ++c) rel_s[j][c] = 0.f;
     }
   }
-  if (SPLIT) {
+  if (CHAIN) {
     grid_wait();
 #pragma unroll
-    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(cb + c);
+    for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(c);
   }
   __syncthreads();
 
@@ -369,7 +363,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
 #pragma unroll
     for (int qq = 0; qq < NA; ++qq) acc[j][qq] = make_float2(0.f, 0.f);
 
-  for (int c = cb; c < nch; ++c) {
+  for (int c = 0; c < nch; ++c) {
     cp_async_wait_n<kFwdStages - 2>();
     __syncthreads();  // rows of chunk c landed; every thread is done with chunk c - 1
     issue_rows(c + kFwdStages - 1);
@@ -468,26 +462,6 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
     }
   }
   cp_async_wait0();
-  if (SPLIT) {
-    __syncthreads();  // every thread is done with the ring
-    float2* part = reinterpret_cast<float2*>(smem);
-#pragma unroll
-    for (int j = 0; j < T; ++j)
-#pragma unroll
-      for (int v = 0; v < NA; ++v) part[(j * NA + v) * 256 + tid] = acc[j][v];
-    cg::this_cluster().sync();
-    for (int p = rank; p < T * NA; p += nsplit) {
-      const int j = p / NA, v = p % NA;
-      float2 sum = cg::this_cluster().map_shared_rank(part, 0)[p * 256 + tid];
-      for (int r = 1; r < nsplit; ++r) sum = fadd2(sum, cg::this_cluster().map_shared_rank(part, r)[p * 256 + tid]);
-      const int q = NV ? v : tl.q0 + v;
-      if (!xok || jb + j >= nl || (!NV && q >= u.ncoils)) continue;
-      const float sv = u.signal_scale * (NV && v == NA - 1 && cls_rows == 1 ? off : 1.f);
-      u.g[((size_t)q * u.n_lines + tl.line0 + jb + j) * snx + x] = make_float2(sum.x * sv, sum.y * sv);
-    }
-    cg::this_cluster().sync();  // no block leaves while another reads its sums
-    return;
-  }
   if (!xok) return;
   const float s = u.signal_scale;
   if (NV && cls_rows) {
@@ -541,20 +515,23 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     const Tile* tiles = (const Tile*)p->d_ytiles[pass] + R.t0;
     const bool maps = pass == 1;
     const int QG = p->qg, NCv = p->nc;
+    if (p->fwd_thin[pass]) {
+      launch_ystage_thin(p, pass, p->d_ytiles[pass] + R.t0, R.n, st);
+      continue;
+    }
     if (p->fwdq[pass]) {
       const size_t smq = ystage_q_smem(NCv, maps, QG, p->max_sny);
       bool launched = false;
       const int NVv = p->fwd_nv[pass];
       const bool narrow = p->fwd_narrow[pass];
-      const bool small = p->fwd_small[pass];
-      const int split = p->fwd_split[pass], rows_kind = p->basis_nb ? 2 : p->fwd_cls ? 1 : 0;
-      const size_t smsplit = std::max(smq, sizeof(float2) * 256 * kT * (size_t)std::max(NVv, QG));
+      const bool chain = p->fwd_chain[pass];
+      const int rows_kind = p->basis_nb ? 2 : p->fwd_cls ? 1 : 0;
 #define MRSIM_YFW(QGV, NVV, NCV, M, W)                                                  \
   if (QG == QGV && NVv == NVV && NCv == NCV && maps == M && narrow == W) {              \
-    if (!M && !W && small) {                                                            \
+    if (!M && !W && chain) {                                                          \
       auto k = ystage_q_kernel<QGV, NVV, NCV, M, W, !M && !W>;                          \
-      set_smem(k, smsplit);                                                             \
-      launch_chained(k, dim3((unsigned)R.n * split), split, smsplit, st, true, p->d_units, tiles, rows_kind);  \
+      set_smem(k, smq);                                                                 \
+      launch_chained(k, dim3((unsigned)R.n), smq, st, true, p->d_units, tiles, rows_kind);  \
     } else {                                                                            \
       auto k = ystage_q_kernel<QGV, NVV, NCV, M, W, false>;                             \
       set_smem(k, smq);                                                                 \

@@ -209,9 +209,9 @@ struct EpiPlan {
   // ... and accumulating coil classes: their count plus the coil offset row, or 0
   int fwd_nv[2] = {0, 0};
   bool fwd_narrow[2] = {false, false};  // ... its rows copied 4 bytes at a time (16 otherwise)
-  // small launches: chained to the kernel before, with this many blocks (a cluster) to a tile
-  bool fwd_small[2] = {false, false}, adj_small[4] = {false, false, false, false};
-  int fwd_split[2] = {1, 1}, adj_split[4] = {1, 1, 1, 1};
+  // small launches: chained to the kernel before; few tiles: the groups of the thin kernels, or 0
+  bool fwd_chain[2] = {false, false}, adj_chain[4] = {false, false, false, false};
+  int fwd_thin[2] = {0, 0}, adj_thin[4] = {0, 0, 0, 0};
   bool adj_narrow = false;                // the fixed-count y-adjoint's rows 8 at a time
   // y-adjoint pass (maps | grads << 1) served by the fixed-coil-count kernel: its coil count, or 0
   // for the general kernel

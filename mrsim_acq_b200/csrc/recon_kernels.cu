@@ -269,104 +269,119 @@ __global__ void __launch_bounds__(256) recon_combine_kernel(const ReconJob* __re
   }
 }
 
-// The same by FFTs, for matrices of 32 E points per axis (E <= 4): a cluster of blocks per (unit, echo),
-// each taking every S-th coil.  A coil's k-space is windowed and row-transformed by a warp per row as it
-// is read, column-transformed in shared memory, and added to the block's Roemer sums in registers;
-// the cluster adds those in rank order.  With xs = nx/2 and ys = ny/2 multiples of 16 the centred
-// transform is the plain one between sign flips: e^{-i2pi (k - s)(x - s)/n} = (-1)^(k + x) e^{-i2pi kx/n}.
-// One cluster of S = 1 per unit fills the chip from 592 units on; fewer units share their coils among up to
-// 8 blocks.  600 units of 64 x 64 x 8 coils: 208 us, 0.76 TB/s of k-space; as direct sums 2142
-// us (64-term sums at 12 % of the FMA rate).
+// The same by FFTs, for matrices of 32 E points per axis (E <= 4): a cluster of S blocks per (unit, echo)
+// takes S coils at a time, a block each.  A coil's k-space is windowed and row-transformed by a warp per
+// row as it is read and column-transformed in shared memory; then every block adds the coils' images, in
+// coil order, to the Roemer sums of its share of the pixels, so the sums are the same for every S.
+// With xs = nx/2 and ys = ny/2 multiples of 16 the centred transform is the plain one between sign flips:
+// e^{-i2pi (k - s)(x - s)/n} = (-1)^(k + x) e^{-i2pi kx/n}.
+// One block a unit fills the chip from 592 units on; fewer units share their coils among up to 8 blocks.  600
+// units of 64 x 64 x 8 coils: 205 us, 0.77 TB/s of k-space (as direct sums 2142 us: 64-term sums at 12 %
+// of the FMA rate); one slice of 8 coils 16 us; 32 partitions of 32 coils 57 us.
 template <int EX, int EY>
 struct ReconShape {
   static constexpr int NX = 32 * EX, NY = 32 * EY, LD = NX + 1;
   static constexpr int T = NX * NY >= 8192 ? 512 : 256, NW = T / 32, NP = NX * NY / T;
-  static constexpr size_t smem = sizeof(float2) * ((size_t)NY * LD + NX + NY);
+  // images of a block of a cluster: two where they fit, so that one is read while the next is formed
+  static constexpr int NB = NY * LD <= 6 * 1024 ? 2 : 1;
+  static constexpr size_t smem(bool multi) { return sizeof(float2) * ((size_t)(multi ? NB : 1) * NY * LD + NX + NY); }
 };
 
-template <int EX, int EY>
+template <int EX, int EY, int S>
 __global__ void __launch_bounds__(ReconShape<EX, EY>::T) recon_fft_kernel(const ReconJob* __restrict__ jobs) {
   using R = ReconShape<EX, EY>;
   constexpr int NX = R::NX, NY = R::NY, LD = R::LD, T = R::T, NW = R::NW, NP = R::NP;
   constexpr int LX = log2_c(EX), LY = log2_c(EY);
   constexpr bool PX = (EX & (EX - 1)) == 0, PY = (EY & (EY - 1)) == 0;
   extern __shared__ __align__(16) float2 sm[];
-  float2* img = sm;             // [NY][LD]
-  float2* twx = img + NY * LD;  // e^{-i2pi j/NX}
+  constexpr int NB = S > 1 ? R::NB : 1;
+  float2* twx = sm;        // e^{-i2pi j/NX}
   float2* twy = twx + NX;
+  float2* imgs = twy + NY;  // [NB][NY][LD]
   const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int rank = S > 1 ? (int)cl.block_rank() : 0;
   const ReconJob& J = jobs[blockIdx.x / S];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nc = J.nc;
   for (int i = tid; i < NX; i += T) twx[i] = J.ex_tab[i];
   for (int i = tid; i < NY; i += T) twy[i] = J.ey_tab[i];
-  float2 acc[NP];
+  const float* __restrict__ sens = J.sens;
+  float2* const coil_images = J.coil_images;
+  constexpr int MP = (NP + S - 1) / S;  // this block's pixels: tid + (first + p) T
+  const int first = rank * MP;
+  float2 acc[MP];
 #pragma unroll
-  for (int p = 0; p < NP; ++p) acc[p] = make_float2(0.f, 0.f);
+  for (int p = 0; p < MP; ++p) acc[p] = make_float2(0.f, 0.f);
+  auto sync = [&] {
+    if (S == 1)
+      __syncthreads();
+    else
+      cl.sync();
+  };
   __syncthreads();
   const int k2 = (int)(__brev(lane) >> 27);
-  for (int q = rank; q < nc; q += S) {
-    const float2* kq = J.k + (size_t)q * NX * NY;
-    for (int ky = warp; ky < NY; ky += NW) {
-      float2 b[EX];
+  for (int q0 = 0; q0 < nc; q0 += S) {
+    const int q = q0 + rank;
+    float2* img = imgs + (NB == 2 ? (q0 / S & 1) * NY * LD : 0);
+    if (q < nc) {  // (the whole block)
+      const float2* kq = J.k + (size_t)q * NX * NY;
+      for (int ky = warp; ky < NY; ky += NW) {
+        float2 b[EX];
 #pragma unroll
-      for (int m = 0; m < EX; ++m) {
-        const int kx = lane + 32 * m;
-        float2 v = kq[ky * NX + kx];
-        float w = J.window ? J.window[ky * NX + kx] : 1.f;
-        w = ((kx + ky) & 1) ? -w : w;
-        b[PX ? bitrev_c(m, LX) : m] = make_float2(v.x * w, v.y * w);
+        for (int m = 0; m < EX; ++m) {
+          const int kx = lane + 32 * m;
+          float2 v = kq[ky * NX + kx];
+          float w = J.window ? J.window[ky * NX + kx] : 1.f;
+          w = ((kx + ky) & 1) ? -w : w;
+          b[PX ? bitrev_c(m, LX) : m] = make_float2(v.x * w, v.y * w);
+        }
+        warp_row_fft<EX, true>(b, twx, lane);
+#pragma unroll
+        for (int k1 = 0; k1 < EX; ++k1) img[ky * LD + k1 + EX * k2] = b[k1];
       }
-      warp_row_fft<EX, true>(b, twx, lane);
+      __syncthreads();
+      for (int x = warp; x < NX; x += NW) {
+        float2 b[EY];
 #pragma unroll
-      for (int k1 = 0; k1 < EX; ++k1) img[ky * LD + k1 + EX * k2] = b[k1];
+        for (int m = 0; m < EY; ++m) b[PY ? bitrev_c(m, LY) : m] = img[(lane + 32 * m) * LD + x];
+        warp_row_fft<EY, true>(b, twy, lane);
+#pragma unroll
+        for (int k1 = 0; k1 < EY; ++k1) img[(k1 + EY * k2) * LD + x] = b[k1];
+      }
     }
-    __syncthreads();
-    for (int x = warp; x < NX; x += NW) {
-      float2 b[EY];
+    sync();  // the round's images are whole
+    // (a pixel's images and sensitivities are loaded before they are added: the loads of the round fly)
+    const int nq = min(S, nc - q0);
 #pragma unroll
-      for (int m = 0; m < EY; ++m) b[PY ? bitrev_c(m, LY) : m] = img[(lane + 32 * m) * LD + x];
-      warp_row_fft<EY, true>(b, twy, lane);
+    for (int p = 0; p < MP; ++p) {
+      if (NP % S != 0 && first + p >= NP) break;
+      const int i = tid + (first + p) * T, y = i / NX, x = i % NX;
+      float2 v[S];
+      float s[S];
 #pragma unroll
-      for (int k1 = 0; k1 < EY; ++k1) img[(k1 + EY * k2) * LD + x] = b[k1];
+      for (int r = 0; r < S; ++r)
+        if (S == 1 || r < nq) {
+          v[r] = (S > 1 ? cl.map_shared_rank(img, r) : img)[y * LD + x];
+          s[r] = sens[(size_t)(q0 + r) * NX * NY + i];
+        }
+#pragma unroll
+      for (int r = 0; r < S; ++r)
+        if (S == 1 || r < nq) {
+          if ((x + y) & 1) v[r] = make_float2(-v[r].x, -v[r].y);
+          if (coil_images) coil_images[(size_t)(q0 + r) * NX * NY + i] = v[r];
+          acc[p].x = fmaf(s[r], v[r].x, acc[p].x);
+          acc[p].y = fmaf(s[r], v[r].y, acc[p].y);
+        }
     }
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int i = tid + p * T, y = i / NX, x = i % NX;
-      float2 v = img[y * LD + x];
-      if ((x + y) & 1) v = make_float2(-v.x, -v.y);
-      if (J.coil_images) J.coil_images[(size_t)q * NX * NY + i] = v;
-      const float s = J.sens[(size_t)q * NX * NY + i];
-      acc[p].x = fmaf(s, v.x, acc[p].x);
-      acc[p].y = fmaf(s, v.y, acc[p].y);
-    }
-    __syncthreads();
+    if (NB == 1) sync();  // every block has read them
   }
-  if (S == 1) {
+  if (NB == 2) sync();  // (no block leaves while another reads its images)
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int i = tid + p * T;
-      const float inv = J.inv_ssum[i];
-      J.combined[i] = make_float2(acc[p].x * inv, acc[p].y * inv);
-    }
-    return;
-  }
-  float2* part = img;  // [pixel]
-#pragma unroll
-  for (int p = 0; p < NP; ++p) part[tid + p * T] = acc[p];
-  cl.sync();
-  for (int i = rank * T + tid; i < NX * NY; i += S * T) {
-    float2 v = cl.map_shared_rank(part, 0)[i];
-    for (int r = 1; r < S; ++r) {
-      const float2 o = cl.map_shared_rank(part, r)[i];
-      v.x += o.x;
-      v.y += o.y;
-    }
+  for (int p = 0; p < MP; ++p) {
+    if (NP % S != 0 && first + p >= NP) break;
+    const int i = tid + (first + p) * T;
     const float inv = J.inv_ssum[i];
-    J.combined[i] = make_float2(v.x * inv, v.y * inv);
+    J.combined[i] = make_float2(acc[p].x * inv, acc[p].y * inv);
   }
-  cl.sync();  // no block leaves while another reads its sums
 }
 
 __global__ void window_copy_kernel(const ReconJob* __restrict__ jobs) {
@@ -390,15 +405,19 @@ namespace {
 template <int EX, int EY>
 void launch_recon_fft(const ReconJob* d_jobs, int n_jobs, int nc, cudaStream_t st) {
   using R = ReconShape<EX, EY>;
-  auto k = recon_fft_kernel<EX, EY>;
-  if (R::smem > 48 * 1024)
-    MRSIM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem));
   int S = 1;
   while (2 * S <= std::min(8, nc) && (long long)n_jobs * 2 * S <= 592) S *= 2;
+  auto k = S == 8   ? recon_fft_kernel<EX, EY, 8>
+           : S == 4 ? recon_fft_kernel<EX, EY, 4>
+           : S == 2 ? recon_fft_kernel<EX, EY, 2>
+                    : recon_fft_kernel<EX, EY, 1>;
+  const size_t smem = R::smem(S > 1);
+  if (smem > 48 * 1024)
+    MRSIM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(n_jobs * S));
   cfg.blockDim = dim3(R::T);
-  cfg.dynamicSmemBytes = R::smem;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeClusterDimension;
