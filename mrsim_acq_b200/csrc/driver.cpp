@@ -571,7 +571,9 @@ EpiOperator* epi_operator_create(mrsim_context* ctx, const mrsim_acquisition_inp
       sd.out = op->d_phase + ui * plane;
     }
   }
-  op->plan.reset(epi_plan_create(units.data(), (int)units.size(), statics.data(), (int)statics.size()));
+  const HostLines tables = op->line_tables();
+  op->plan.reset(epi_plan_create(units.data(), (int)units.size(), statics.data(), (int)statics.size(), nullptr, nullptr,
+                                 &tables));
   if (in.images) upload_series_images(op.get(), in.images);
   MRSIM_CUDA(cudaStreamSynchronize(st));
   return op.release();
@@ -620,9 +622,10 @@ void epi_operator_set_segmented(EpiOperator* op, int precision) {
   std::unique_ptr<EpiPlan> was;
   if ((precision != 0 && op->plan->basis_nb > 0) || (precision == 0 && op->plan->opt.no_basis)) {
     EpiPlanOptions o = op->plan->opt;
+    const HostLines tables = op->line_tables();
     o.no_basis = precision != 0 ? 1 : 0;
     was.reset(epi_plan_create(op->plan->host_units.data(), op->plan->n_units, op->plan->host_statics.data(),
-                              (int)op->plan->host_statics.size(), &o));
+                              (int)op->plan->host_statics.size(), &o, nullptr, &tables));
     std::swap(was, op->plan);
   }
   TsPlan* fresh = nullptr;
@@ -662,16 +665,19 @@ EpiBatch* epi_batch_create(mrsim_context* ctx, int n, const mrsim_acquisition_in
   b->ctx = ctx;
   std::vector<UnitDesc> units;
   std::vector<StaticDesc> statics;
+  HostLines tables;
   for (int i = 0; i < n; ++i) {
     if (!inputs[i]) fail("series " + std::to_string(i) + " is NULL");
     b->ops.emplace_back(epi_operator_create(ctx, *inputs[i], acq, echo_times_ms, n_echoes, nullptr, 0, grads));
     const EpiPlan& p = *b->ops.back()->plan;
+    tables[b->ops.back()->d_lines] = b->ops.back()->h_lines.data();
     b->unit0.push_back((int)units.size());
     units.insert(units.end(), p.host_units.begin(), p.host_units.end());
     statics.insert(statics.end(), p.host_statics.begin(), p.host_statics.end());
     b->samples += b->ops.back()->samples_per_step;
   }
-  b->plan.reset(epi_plan_create(units.data(), (int)units.size(), statics.data(), (int)statics.size()));
+  b->plan.reset(epi_plan_create(units.data(), (int)units.size(), statics.data(), (int)statics.size(), nullptr, nullptr,
+                                &tables));
   MRSIM_CUDA(cudaStreamSynchronize(ctx->stream));
   return b.release();
 }
@@ -714,8 +720,9 @@ bool parse_choice(const std::string& v, TuneChoice& c) {
   return true;
 }
 void apply_choice(EpiOperator* op, const TuneChoice& c) {
+  const HostLines tables = op->line_tables();
   op->plan.reset(epi_plan_create(op->plan->host_units.data(), op->plan->n_units, op->plan->host_statics.data(),
-                                 (int)op->plan->host_statics.size(), &c.opt));
+                                 (int)op->plan->host_statics.size(), &c.opt, nullptr, &tables));
   epi_operator_set_segmented(op, c.segmented);
 }
 }  // namespace

@@ -68,6 +68,7 @@ struct EpiOperator {
   mrsim_acquisition acq{};
   std::vector<double> tes;
   std::vector<LineRec> h_lines;
+  HostLines line_tables() const { return {{d_lines, h_lines.data()}}; }
   std::vector<float> h_fmap;
   float t2u[kMaxComp] = {0}, tiu[kMaxComp] = {0};
   bool maps = false, any_eddy = false;

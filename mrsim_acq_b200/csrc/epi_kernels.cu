@@ -876,7 +876,7 @@ struct PlanArrays {
 }  // namespace
 
 EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns, const EpiPlanOptions* opt,
-                         mrsim_context* ctx) {
+                         mrsim_context* ctx, const HostLines* lines) {
   EpiPlan* p = new EpiPlan();
   PlanArrays arrays;
   try {
@@ -1107,8 +1107,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       p->n_ftiles = (int)ft.size();
       arrays.add(&p->d_ftiles, ft.data(), sizeof(int4) * ft.size());
     }
-    // x-stage GEMM tiles, from host copies of the line tables (one copy per distinct table)
-    std::map<const LineRec*, std::vector<LineRec>> host_lines;
+    // x-stage GEMM tiles, from host copies of the line tables (one readback per table that has none)
+    std::map<const LineRec*, std::vector<LineRec>> read;
+    HostLines known = lines ? *lines : HostLines();
     for (int dir = 0; dir < 2 && !p->xfft; ++dir) {
       std::vector<XTile> xt;
       p->g_start[dir].assign(n + 1, 0);
@@ -1116,20 +1117,16 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
         p->g_start[dir][i] = (int)xt.size();
         const int nl = hu[i].n_lines;
         if (nl == 0) continue;
-        auto it = host_lines.find(hu[i].lines);
-        if (it == host_lines.end()) {
-          std::vector<LineRec> L(nl);
-          // the table's upload may still be queued on the context's stream
-          if (ctx) {
-            MRSIM_CUDA(cudaMemcpyAsync(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost, ctx->stream));
-            MRSIM_CUDA(cudaStreamSynchronize(ctx->stream));
-          } else {
-            MRSIM_CUDA(cudaDeviceSynchronize());
-            MRSIM_CUDA(cudaMemcpy(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost));
-          }
-          it = host_lines.emplace(hu[i].lines, std::move(L)).first;
+        const LineRec*& table = known[hu[i].lines];
+        if (!table) {
+          if (!ctx) fail("a plan needs its units' line tables");
+          std::vector<LineRec>& L = read[hu[i].lines];
+          L.resize(nl);
+          MRSIM_CUDA(cudaMemcpyAsync(L.data(), hu[i].lines, sizeof(LineRec) * nl, cudaMemcpyDeviceToHost, ctx->stream));
+          MRSIM_CUDA(cudaStreamSynchronize(ctx->stream));
+          table = L.data();
         }
-        append_xtiles(xt, hu[i], i, it->second.data(), dir);
+        append_xtiles(xt, hu[i], i, table, dir);
       }
       p->g_start[dir][n] = (int)xt.size();
       p->n_gtiles[dir] = (int)xt.size();

@@ -4,8 +4,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
 #include <mutex>
 #include <stdexcept>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -227,9 +229,12 @@ struct EpiPlan {
   ~EpiPlan();
 };
 // With `ctx` its arrays come from the context's pool and are freed on its stream, after the work
-// queued there: for a plan that runs on that stream and ends with the call.
+// queued there: for a plan that runs on that stream and ends with the call.  lines: host copies of the
+// units' line tables, by device address; with `ctx` a table that is not there is read back on its stream.
+using HostLines = std::map<const LineRec*, const LineRec*>;
 EpiPlan* epi_plan_create(const UnitDesc* units, int n, const StaticDesc* statics, int ns,
-                         const EpiPlanOptions* opt = nullptr, mrsim_context* ctx = nullptr);
+                         const EpiPlanOptions* opt = nullptr, mrsim_context* ctx = nullptr,
+                         const HostLines* lines = nullptr);
 // The x-stage tiles of one unit (dir 0 forward, 1 adjoint); `lines` is a host copy of its table.
 void append_xtiles(std::vector<XTile>& out, const UnitDesc& u, int unit_index, const LineRec* lines, int dir);
 // Each launcher covers units [u0, u1) of the plan (u1 < 0: every unit).
