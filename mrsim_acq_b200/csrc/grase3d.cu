@@ -50,18 +50,19 @@ struct ZdftArgs {
 // A thread serves ZT partitions of its column: with kZTile of them a slice's sample is read once for all
 // (it was read once per partition: 3.2 GB through L2 for 32 coils x 32 partitions x 3 compartments of
 // 64 x 64: 640 us, here 149).  Per-shot images and per-echo sources give partitions different ones: ZT = 1.  The
-// tile's z kernel sits in shared memory ([z][partition]); the sums run in z order.
+// tile's z kernel sits in shared memory ([z][partition]) where it fits (SHARED: 3,632 partitions); the
+// sums run in z order.
 constexpr int kZTile = 8;
-template <int ZT>
+template <int ZT, bool SHARED>
 __global__ void __launch_bounds__(256) grase_zdft_kernel(const ZdftArgs a) {
   extern __shared__ __align__(16) float2 zks[];
   const int per = a.nx * a.ny, nz = a.nz;
   const int p0 = blockIdx.y * ZT;
   const int gq = blockIdx.z;  // gl * nc + q
   const int gl = gq / a.nc, q = gq % a.nc;
-  for (int t = threadIdx.x; t < nz * ZT; t += blockDim.x) {
+  for (int t = threadIdx.x; SHARED && t < nz * ZT; t += blockDim.x) {
     const int z = t / ZT, p = p0 + t % ZT;
-    zks[t] = p < nz ? a.zk[p * nz + z] : make_float2(0.f, 0.f);
+    zks[t] = p < nz ? a.zk[(size_t)p * nz + z] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   const size_t zstride = (size_t)a.nc * per;
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256) grase_zdft_kernel(const ZdftArgs a) {
           const float2 k = Kc[z * zstride];
 #pragma unroll
           for (int t = 0; t < ZT; ++t) {
-            const float2 e = zks[z * ZT + t];
+            const float2 e = SHARED ? zks[z * ZT + t] : __ldg(a.zk + (size_t)min(p0 + t, nz - 1) * nz + z);
             ar[t] += k.x * e.x - k.y * e.y;
             ai[t] += k.x * e.y + k.y * e.x;
           }
@@ -105,15 +106,16 @@ __global__ void __launch_bounds__(256) grase_zdft_kernel(const ZdftArgs a) {
 }
 
 // slices[gl][z][q] = (1/nz) sum_p k3[gl][q][p] conj(zk[p][z]), kZTile slices to a thread as above
+template <bool SHARED>
 __global__ void __launch_bounds__(256) grase_izdft_kernel(const float2* __restrict__ k3, const float2* __restrict__ zk,
                                                           int nx, int ny, int nz, int nc, float2* __restrict__ slices) {
   extern __shared__ __align__(16) float2 zks[];
   const int per = nx * ny;
   const int z0 = blockIdx.y * kZTile;
   const int gq = blockIdx.z, gl = gq / nc, q = gq % nc;
-  for (int t = threadIdx.x; t < nz * kZTile; t += blockDim.x) {
+  for (int t = threadIdx.x; SHARED && t < nz * kZTile; t += blockDim.x) {
     const int p = t / kZTile, z = z0 + t % kZTile;
-    zks[t] = z < nz ? zk[p * nz + z] : make_float2(0.f, 0.f);
+    zks[t] = z < nz ? zk[(size_t)p * nz + z] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   const float inv = 1.0f / (float)nz;
@@ -126,7 +128,14 @@ __global__ void __launch_bounds__(256) grase_izdft_kernel(const float2* __restri
       const float2 k = k3[(((size_t)gl * nc + q) * nz + p) * per + i];
 #pragma unroll
       for (int t = 0; t < kZTile; t += 2) {
-        const float4 e = *reinterpret_cast<const float4*>(zks + p * kZTile + t);
+        float4 e;
+        if (SHARED) {
+          e = *reinterpret_cast<const float4*>(zks + p * kZTile + t);
+        } else {
+          const float2 e0 = __ldg(zk + (size_t)p * nz + min(z0 + t, nz - 1));
+          const float2 e1 = __ldg(zk + (size_t)p * nz + min(z0 + t + 1, nz - 1));
+          e = make_float4(e0.x, e0.y, e1.x, e1.y);
+        }
         ar[t] += k.x * e.x + k.y * e.y;
         ai[t] += k.y * e.x - k.x * e.y;
         ar[t + 1] += k.x * e.z + k.y * e.w;
@@ -140,13 +149,30 @@ __global__ void __launch_bounds__(256) grase_izdft_kernel(const float2* __restri
   }
 }
 
-// the tile's z kernel in shared memory, opted in past 48 KB (more than 768 partitions)
+// Bytes of a tile's z kernel in shared memory, opted in past 48 KB; 0 where it does not fit.
 template <class K>
-size_t z_smem(K kernel, int nz) {
-  const size_t n = sizeof(float2) * kZTile * (size_t)nz;
+size_t z_smem(K kernel, int zt, int nz) {
+  const size_t n = sizeof(float2) * zt * (size_t)nz;
+  if (n > 227 * 1024) return 0;
   if (n > 48 * 1024)
     MRSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   return n;
+}
+
+template <int ZT>
+void launch_zdft(const ZdftArgs& a, dim3 grid, cudaStream_t st) {
+  if (const size_t n = z_smem(grase_zdft_kernel<ZT, true>, ZT, a.nz))
+    grase_zdft_kernel<ZT, true><<<grid, 256, n, st>>>(a);
+  else
+    grase_zdft_kernel<ZT, false><<<grid, 256, 0, st>>>(a);
+}
+
+void launch_izdft(dim3 grid, const float2* k3, const float2* zk, int nx, int ny, int nz, int nc, float2* slices,
+                  cudaStream_t st) {
+  if (const size_t n = z_smem(grase_izdft_kernel<true>, kZTile, nz))
+    grase_izdft_kernel<true><<<grid, 256, n, st>>>(k3, zk, nx, ny, nz, nc, slices);
+  else
+    grase_izdft_kernel<false><<<grid, 256, 0, st>>>(k3, zk, nx, ny, nz, nc, slices);
 }
 
 // combined [gl][z][ny][nx] -> magnitude / phase at vox * nv + g
@@ -496,10 +522,9 @@ static void grase_kspace(const GrasePlan& P, const GraseInputs& I, const mrsim_a
   for (int c = 0; c < P.ncomp; ++c)
     for (int p = 1; p < nz; ++p) one_source = one_source && P.src_of[(size_t)c * nz + p] == P.src_of[(size_t)c * nz];
   if (one_source)
-    grase_zdft_kernel<kZTile><<<grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), 256,
-                                z_smem(grase_zdft_kernel<kZTile>, nz), st>>>(a);
+    launch_zdft<kZTile>(a, grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), st);
   else
-    grase_zdft_kernel<1><<<grid3(per, nz, ngl * nc), 256, z_smem(grase_zdft_kernel<1>, nz), st>>>(a);
+    launch_zdft<1>(a, grid3(per, nz, ngl * nc), st);
   MRSIM_CUDA(cudaGetLastError());
 }
 
@@ -595,8 +620,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     grase_kspace(Pc, Ic, acq_cal, in.phase, nullptr, 0, 1, Pc.mask, k3, ctx);
     grase_noise(C, Pc, k3, 0, 1, cal_seed ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
     float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
-    grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
-        k3, d_zk, nx, ny, nz, nc, sl);
+    launch_izdft(grid3(per, (nz + kZTile - 1) / kZTile, nc), k3, d_zk, nx, ny, nz, nc, sl, st);
     std::vector<float2*> refs;
     for (int z = 0; z < nz; ++z) refs.push_back(sl + (size_t)z * nc * per);
     W = fit_grappa(A, refs, nx, ny, nc, acq_cal, accel, (int)acq.acs_lines, st);
@@ -620,8 +644,7 @@ void grase_acquire(mrsim_context* ctx, const mrsim_acquisition_3d_input& in, con
     grase_kspace(P, I, acq, in.phase, d_lw, g0, g1, P.mask, k3, ctx, &V);
     grase_noise(C, P, k3, g0, g1, seed, P.mask, acq, st);
     float2* sl = (float2*)C.alloc((size_t)ngl * nz * nc * per * sizeof(float2));
-    grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
-        k3, d_zk, nx, ny, nz, nc, sl);
+    launch_izdft(grid3(per, (nz + kZTile - 1) / kZTile, ngl * nc), k3, d_zk, nx, ny, nz, nc, sl, st);
     float2* comb = (float2*)C.alloc((size_t)ngl * nz * per * sizeof(float2));
     std::vector<ReconJob> jobs;
     for (int gl = 0; gl < ngl; ++gl)
@@ -870,8 +893,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       grase_kspace(Pc, Ic, ae, in.phase, d_lw, 0, 1, Pc.mask, k3, ctx);
       grase_noise(C, Pc, k3, 0, 1, (seed ^ echo_salt((uint64_t)e)) ^ kSeedSaltGrappaCal, Pc.mask, acq_cal, st);
       float2* sl = (float2*)C.alloc((size_t)nz * nc * per * sizeof(float2));
-      grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
-          k3, d_zk, nx, ny, nz, nc, sl);
+      launch_izdft(grid3(per, (nz + kZTile - 1) / kZTile, nc), k3, d_zk, nx, ny, nz, nc, sl, st);
       std::vector<float2*> refs;
       for (int z = 0; z < nz; ++z) refs.push_back(sl + (size_t)z * nc * per);
       W[e] = fit_grappa(A, refs, nx, ny, nc, acq_cal, accel, (int)acq.acs_lines, st);
@@ -902,8 +924,7 @@ void ge_acquire(mrsim_context* ctx, const mrsim_acquisition_ge_input& in, const 
       // the noise and spikes of echo e on its own streams (echo 0 unsalted)
       grase_noise(E, Pg, k3, g, g + 1, seed ^ echo_salt((uint64_t)e), Pg.mask, acq, st);
       float2* sl = (float2*)E.alloc((size_t)nz * nc * per * sizeof(float2));
-      grase_izdft_kernel<<<grid3(per, (nz + kZTile - 1) / kZTile, nc), 256, z_smem(grase_izdft_kernel, nz), st>>>(
-          k3, d_zk, nx, ny, nz, nc, sl);
+      launch_izdft(grid3(per, (nz + kZTile - 1) / kZTile, nc), k3, d_zk, nx, ny, nz, nc, sl, st);
       float2* comb = (float2*)E.alloc((size_t)nz * per * sizeof(float2));
       std::vector<ReconJob> jobs;
       for (int z = 0; z < nz; ++z) {
