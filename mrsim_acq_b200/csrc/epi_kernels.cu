@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
   float2* pt = pm + 2 * N;    // post-twiddle per kx (nx <= N)
   float2* rb = pt + N;        // [8][NP]
   float2* st = rb + 8 * NP;   // forward: basis rows [line][r][x]; adjoint: coil rows [line][coil][x]
-  __shared__ float co[kMaxCoils * kBasisPad];
+  __shared__ __align__(16) float co[kMaxCoils * kBasisPad];  // (read as float4)
   __shared__ int lrow[kBasisRows], lpol[kBasisRows];
   __shared__ float ldec[kBasisRows];
   const int4 t = tiles[blockIdx.x];
