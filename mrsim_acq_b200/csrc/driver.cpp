@@ -73,9 +73,12 @@ DevArena::~DevArena() {
 // within 0.6 of it) that they span few dimensions: the constant row (the coil offset's) and at most
 // six more carry every coil of any ring.  Pivoted Gram-Schmidt in FP64 from the constant row takes
 // rows until what remains of every coil is below 1e-9: 7 rows for 12 to 64 coils (2e-10 to 4e-10
-// left; a float32 table of the factors carries 3e-8), 6 for 8 and 10, 4 for 6.  Returns the row
-// count padded to one the kernels are built for (4, 6, 7), or 0 when 7 rows do not suffice; rows
-// [nb - 1][sny] scaled to a largest value of 1, coef [coil][kBasisPad].
+// left), 6 for 8 and 10, 4 for 6.  The kernels use the rows and coefficients rounded to float32, which
+// rebuild the factors to 3e-8 to 5e-8 at most and 1.7e-8 rms, about what a float32 table of the factors
+// carries (3e-8 and 1.7e-8).  What the pair's sums on these rows cost is said at kConstBlock
+// (epi_device.h).  Returns the row count padded to one the kernels are built for (4, 6, 7), or 0 when 7
+// rows do not suffice; rows [nb - 1][sny] scaled to a largest value of 1, coef [coil][kBasisPad] with the
+// constant row's in the last place too.
 static int coil_basis(const std::vector<double>& ey, int ncoils, int sny, std::vector<float>& rows,
                       std::vector<float>& coef) {
   constexpr int kMaxRows = 7;
@@ -141,7 +144,7 @@ static int coil_basis(const std::vector<double>& ey, int ncoils, int sny, std::v
     const double* e = &ey[(size_t)q * sny];
     double mean = 0.0;
     for (int y = 0; y < sny; ++y) mean += e[y];
-    coef[(size_t)q * kBasisPad + nb - 1] = (float)(mean / sny);
+    coef[(size_t)q * kBasisPad + nb - 1] = coef[(size_t)q * kBasisPad + kBasisPad - 1] = (float)(mean / sny);
     for (size_t r = 0; r < B.size(); ++r) {
       double d = 0.0;
       for (int y = 0; y < sny; ++y) d += B[r][y] * e[y];

@@ -125,6 +125,16 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src,
 }
 
 constexpr int kT = 4;   // lines per tile of ystage_kernel
+
+// On basis rows every coil's sample is mostly the constant row's sum, so that sum's rounding is nearly
+// the same in every coil and does not average out over the coils in the adjoint, as the coils' own sums'
+// did.  It is therefore added up in blocks of 16 rows, and those in blocks of 64.  What the adjoint makes
+// of the forward's rounding (32 coils, 64 x 64 on 128 x 128, in FP32 on the CPU): one chain of rows 1.4e-7,
+// blocks of 32 7.4e-8, of 16 6.3e-8, exact sums 2.8e-8, per-coil sums 1.9e-8, beside 1.8e-7 from the sines in
+// all of them; the adjoint's own blocks (adj_blocked) give more back.  The pair against 64 bits, 128 x 128 on
+// 256 x 256, 32 coils, k-space and compartment gradients: per-coil sums 2.55e-7 and 4.00e-7, basis rows in
+// one chain 2.57e-7 and 4.26e-7, now 2.19e-7 and 3.57e-7.
+constexpr int kConstBlock = 16, kConstBlocks = 64;
 constexpr int kTY = 4;  // rows per tile of yadjoint_kernel
 
 // ystage_q_kernel: ring stages, and input planes and rows per stage
@@ -157,13 +167,28 @@ __host__ __device__ __forceinline__ constexpr int adjq_rows_v(int nc, bool maps,
 // forward and the general adjoint, whose tables are smaller: with three compartments 1,900 lines fit
 // (15 echoes of 128 lines) and the general kernel holds 3,100 to 4,200.
 constexpr size_t kStagedSmem = 227 * 1024 - 4608;
-inline size_t ystage_q_smem(int nc, bool maps, int qg, int max_sny) {
+inline size_t ystage_q_smem(int nc, bool maps, int qg, int max_sny, bool basis) {
   return sizeof(float) * ((size_t)kFwdStages * fwdq_planes(nc, maps) * fwdq_rows(nc, maps) * 128 +
-                          (size_t)max_sny * (8 + (qg + 3) / 4 * 4));
+                          (size_t)max_sny * (8 + (qg + 3) / 4 * 4) + (basis ? 2 * 8 * 256 : 0));
 }
 inline size_t yadjoint_q_smem(int nq, int ty, int nc, bool maps, int max_lines) {
   return sizeof(float2) * (size_t)kAdjStages * adjq_chunk_lines(nq) * nq * 128 +
          sizeof(float) * (size_t)(max_lines + adjq_chunk_lines(nq)) * (2 * ty + adjq_line_floats(nc, maps));
+}
+// On basis rows the adjoint adds its lines in blocks of 16 too, whose whole sums are in shared memory,
+// where they leave two blocks an SM (about 170 lines with gradients of three compartments, 430 without):
+// what the forward's rounding costs the pair more than per-coil sums, this one gives back.  The rule is
+// a unit's own lines and the built-in rows per thread, so every form and grouping takes the same one.
+constexpr int kLineBlock = 32;
+constexpr size_t kBlockedSmem = 108 * 1024;
+__host__ __device__ __forceinline__ constexpr size_t adj_sum_bytes(int ty, int nc, bool grads) {
+  return (size_t)1024 * ty * nc * (grads ? 4 : 2);
+}
+__host__ __device__ __forceinline__ constexpr bool adj_blocked(int nq, int nc, bool maps, bool grads, int lines) {
+  return (size_t)8 * kAdjStages * adjq_chunk_lines(nq) * nq * 128 +
+             (size_t)4 * (lines + adjq_chunk_lines(nq)) * (2 * adjq_rows(nc, maps) + adjq_line_floats(nc, maps)) +
+             adj_sum_bytes(adjq_rows(nc, maps), nc, grads) <=
+         kBlockedSmem;
 }
 
 // The thin y kernels (ystage_thin_kernel, yadjoint_thin_kernel), for plans of few tiles: blocks of 32

@@ -113,6 +113,12 @@ __global__ void statics_kernel(const StaticDesc* descs) {
   }
 }
 
+// Chains in which a column's coils are added to the constant basis row (coil q in chain q mod 4), before
+// the chains are added.  That row is nearly all of H, and its rounding is common to every voxel of a
+// column, which a coil's own was not: H of 32 coils is off by 9.3e-8 in one chain, 7.8e-8 in four (7.9e-8
+// by per-coil sums).
+constexpr int kCoilChains = 4;
+
 // ---------------------------------------------------------------------------------------------
 // x-stage as a register-tiled complex GEMM.  A tile is up to 32 rows (lines of ONE readout polarity
 // x coils) by 64 output columns; K runs over the contraction in chunks of 32 staged in shared memory.
@@ -256,22 +262,32 @@ __global__ void __launch_bounds__(256) xgemm_kernel(const UnitDesc* __restrict__
     for (int e = threadIdx.x; e < T.nl * 64; e += 256) {
       const int jj = e >> 6, c = e & 63, col = T.col0 + c;
       if (col >= N) continue;
-      float2 G[kBasisPad - 1], sum = make_float2(0.f, 0.f);
+      float2 G[kBasisPad - 2], last = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int b = 0; b < kBasisPad - 1; ++b) G[b] = make_float2(0.f, 0.f);
-      for (int q = 0; q < T.nq; ++q) {
+      for (int b = 0; b < kBasisPad - 2; ++b) G[b] = make_float2(0.f, 0.f);
+      float2 chain[kCoilChains];
+#pragma unroll
+      for (int k = 0; k < kCoilChains; ++k) chain[k] = make_float2(0.f, 0.f);
+      auto add = [&](int q, float2& l) {
         const float2 h = Bs[jj * T.nq + q][c];
         const float* co = u.geo.bco + (T.q0 + q) * kBasisPad;
-        const float2 w = fmul2(dup2(s * u.geo.ex[(size_t)(T.q0 + q) * snx + col]), h);
-        sum = fadd2(sum, h);
+        const float ex = s * u.geo.ex[(size_t)(T.q0 + q) * snx + col];
+        const float2 w = fmul2(dup2(ex), h);
+        l = ffma2(dup2(fmaf(ex, co[kBasisPad - 1], so)), h, l);
 #pragma unroll
-        for (int b = 0; b < kBasisPad - 1; ++b)
-          if (b < nb) G[b] = ffma2(dup2(co[b]), w, G[b]);
-      }
+        for (int b = 0; b < kBasisPad - 2; ++b)
+          if (b < nb - 1) G[b] = ffma2(dup2(co[b]), w, G[b]);
+      };
+      for (int q = 0; q < T.nq; q += kCoilChains)
+#pragma unroll
+        for (int k = 0; k < kCoilChains; ++k)
+          if (q + k < T.nq) add(q + k, chain[k]);
+      last = fadd2(fadd2(chain[0], chain[1]), fadd2(chain[2], chain[3]));
       const size_t base = (size_t)T.line[jj] * snx + col, rs = (size_t)u.n_lines * snx;
 #pragma unroll
-      for (int b = 0; b < kBasisPad - 1; ++b)
-        if (b < nb) u.g[base + b * rs] = b == nb - 1 ? ffma2(dup2(so), sum, G[b]) : G[b];
+      for (int b = 0; b < kBasisPad - 2; ++b)
+        if (b < nb - 1) u.g[base + b * rs] = G[b];
+      u.g[base + (nb - 1) * rs] = last;
     }
   }
 }
@@ -779,24 +795,37 @@ __global__ void __launch_bounds__(256, E > 4 ? 2 : ADJ ? 3 : 4) xfft_basis_kerne
       for (int e = threadIdx.x; e < nj * N; e += 256) {
         const int jl = e / N, x = e % N;
         const size_t base = (size_t)(j0 + jl) * N + x, rs = (size_t)nl * N;
-        float2 G[kBasisPad - 1], sum = make_float2(0.f, 0.f);
+        float2 G[kBasisPad - 2], last = q0 > 0 ? gbuf[base + (nb - 1) * rs] : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int v = 0; v < kBasisPad - 1; ++v)  // past the first 32 coils: on from this thread's own sums
-          G[v] = q0 > 0 && v < nb ? gbuf[base + v * rs] : make_float2(0.f, 0.f);
+        for (int v = 0; v < kBasisPad - 2; ++v)  // past the first 32 coils: on from this thread's own sums
+          G[v] = q0 > 0 && v < nb - 1 ? gbuf[base + v * rs] : make_float2(0.f, 0.f);
         const float2* hr = st + (size_t)jl * nq * N + x;
-        for (int q = 0; q < nq; ++q) {
+        float2 chain[kCoilChains];
+#pragma unroll
+        for (int k = 0; k < kCoilChains; ++k) chain[k] = make_float2(0.f, 0.f);
+        auto add = [&](int q, float2& l) {
           const float2 h = hr[q * N];
           const float4 c0 = *reinterpret_cast<const float4*>(co + (q0 + q) * kBasisPad);
           const float4 c1 = *reinterpret_cast<const float4*>(co + (q0 + q) * kBasisPad + 4);
           const float cf[kBasisPad] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-          const float2 w = fmul2(dup2(s * __ldg(exg + (q0 + q) * N + x)), h);
-          sum = fadd2(sum, h);
+          const float ex = s * __ldg(exg + (q0 + q) * N + x);
+          const float2 w = fmul2(dup2(ex), h);
+          l = ffma2(dup2(fmaf(ex, cf[kBasisPad - 1], so)), h, l);
 #pragma unroll
-          for (int v = 0; v < kBasisPad - 1; ++v) G[v] = ffma2(dup2(cf[v]), w, G[v]);
-        }
+          for (int v = 0; v < kBasisPad - 2; ++v) G[v] = ffma2(dup2(cf[v]), w, G[v]);
+        };
+        int q = 0;
+        for (; q + kCoilChains <= nq; q += kCoilChains)
 #pragma unroll
-        for (int v = 0; v < kBasisPad - 1; ++v)
-          if (v < nb) gbuf[base + v * rs] = v == nb - 1 ? ffma2(dup2(so), sum, G[v]) : G[v];
+          for (int k = 0; k < kCoilChains; ++k) add(q + k, chain[k]);
+#pragma unroll
+        for (int k = 0; k < kCoilChains - 1; ++k)
+          if (q + k < nq) add(q + k, chain[k]);
+        last = fadd2(last, fadd2(fadd2(chain[0], chain[1]), fadd2(chain[2], chain[3])));
+#pragma unroll
+        for (int v = 0; v < kBasisPad - 2; ++v)
+          if (v < nb - 1) gbuf[base + v * rs] = G[v];
+        gbuf[base + (nb - 1) * rs] = last;
       }
       __syncthreads();  // before the next coils' rows overwrite these
     }
@@ -948,7 +977,9 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           return false;
       return true;
     };
-    auto fwd_fits = [&](bool maps) { return ystage_q_smem(p->nc, maps, p->qg, p->max_sny) <= kStagedSmem; };
+    auto fwd_fits = [&](bool maps, bool basis) {
+      return ystage_q_smem(p->nc, maps, p->qg, p->max_sny, basis) <= kStagedSmem;
+    };
     // The coil basis (coil_basis, driver.cpp) where every unit has one of the same row count: rings of
     // 6, 7 and 9 or more coils, and of 8 where the class rows have no x-stage (rows past 128 points,
     // the DFT GEMM).  Its 4 to 7 rows replace the coils in both y-stages, whose work per voxel and
@@ -970,7 +1001,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
           nb = 0;
       }
       if ((all8 && cls8) || (any_maps && p->nc > 3)) nb = 0;
-      if (nb && !(adj_fits(nb, true, true) && (!has_maps(false) || fwd_fits(false)) && (!any_maps || fwd_fits(true))))
+      if (nb && !(adj_fits(nb, true, true) && (!has_maps(false) || fwd_fits(false, true)) && (!any_maps || fwd_fits(true, true))))
         nb = 0;
       p->basis_nb = nb;
     }
@@ -1000,7 +1031,7 @@ EpiPlan* epi_plan_create(const UnitDesc* hu, int n, const StaticDesc* hs, int ns
       // registers than the 256-thread CTA leaves: those shapes keep the per-thread-load kernel
       if (p->qg == 8 && (p->nc == 8 || (pass == 1 && p->nc >= 4))) ok = false;
       if (!wide && !p->basis_nb) ok = false;
-      if (!fwd_fits(pass == 1)) ok = false;
+      if (!fwd_fits(pass == 1, p->basis_nb > 0)) ok = false;
       p->fwdq[pass] = ok;
       p->fwd_narrow[pass] = !wide;
       // coil classes: every unit with the same 8 coils in 5 classes (the ring) -> 6 accumulators

@@ -223,12 +223,13 @@ __global__ void __launch_bounds__(128) yadjoint_kernel(const UnitDesc* __restric
 //     accumulator update is one FMA.
 
 
-// VIRT: the h rows are the NQ = classes + 1 class rows of the class-mode x-adjoint (scale, ex and
+// VIRT = 1: the h rows are the NQ = classes + 1 class rows of the class-mode x-adjoint (scale, ex and
 // the coil offset already applied), so amp_v(y) = ey_v(y) for the classes and 1 for the offset row;
-// or the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis).
+// VIRT = 2: the NQ basis rows of the basis x-adjoint (the unit's eyc holds the coil basis); the constant
+// row, which carries most of H, is added last, so that one sum alone rounds at its size.
 // NARROW: odd rows (or g off a 16-byte boundary), so the ring fills by 8-byte copies.
 // CHAIN: a small launch, chained to the kernel before it.
-template <int NQ, int TY, int NC, bool MAPS, bool GRADS, bool VIRT, bool NARROW, bool CHAIN>
+template <int NQ, int TY, int NC, bool MAPS, bool GRADS, int VIRT, bool NARROW, bool CHAIN>
 __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjoint_q_kernel(const UnitDesc* __restrict__ units,
                                                             const int4* __restrict__ tiles) {
   extern __shared__ __align__(16) float smem[];
@@ -409,8 +410,43 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
       if (GRADS) Uy[ty][GRADS ? c : 0] = Vx[ty][GRADS ? c : 0] = 0.f;
     }
 
+  // basis rows: the sums of whole blocks of kLineBlock lines, [sum][thread], and their additions
+  static_assert(kLineBlock % JC == 0, "whole chunks in a block");
+  float2* const whole = reinterpret_cast<float2*>(Lt + (size_t)nlp * LF) + tid;
+  const bool blocked = VIRT == 2 && adj_blocked(NQ, NC, MAPS, GRADS, nlines);
+  auto each_sum = [&](auto f) {  // f(sum, its place)
+    int k = 0;
+    if (PK) {
+#pragma unroll
+      for (int pp = 0; pp < NPR; ++pp)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          f(pcx[pp][c], whole[256 * k++]);
+          f(pcy[pp][c], whole[256 * k++]);
+          if (GRADS) {
+            f(puy[pp][c], whole[256 * k++]);
+            f(pvx[pp][c], whole[256 * k++]);
+          }
+        }
+    } else {
+#pragma unroll
+      for (int ty = 0; ty < TY; ++ty)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          f(cg[ty][c], whole[256 * k++]);
+          if (GRADS) {
+            float2 t = make_float2(Uy[ty][GRADS ? c : 0], Vx[ty][GRADS ? c : 0]);
+            f(t, whole[256 * k++]);
+            Uy[ty][GRADS ? c : 0] = t.x;
+            Vx[ty][GRADS ? c : 0] = t.y;
+          }
+        }
+    }
+  };
+  if (VIRT == 2 && blocked) each_sum([](float2& acc, float2& w) { w = acc; });  // (zeros)
+
   int s_use = 0, s_issue = kAdjStages - 1;  // stages of chunk c and of chunk c + stages - 1
-  for (int c = 0; c < nchunks; ++c) {
+  auto add_chunk = [&](int c) {
     cp_async_wait_n<kAdjStages - 2>();
     __syncthreads();  // chunk c landed for every thread; every thread is done with chunk c - 1
     issue_chunk(c + kAdjStages - 1, s_issue);
@@ -427,7 +463,7 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
       const float thi = e0.x, tlo = e0.y, trf = e0.z, tinh = e0.w;
       if (PK) {
         float2 Hx[NPR], Hy[NPR];  // [pair] = rows (2p, 2p + 1); starts from the offset row (amplitude 1)
-        {
+        if (VIRT == 1) {
           const float2 h = hs[(jj * NQ + NQ - 1) * 128];
 #pragma unroll
           for (int pp = 0; pp < NPR; ++pp) {
@@ -442,8 +478,16 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
 #pragma unroll
           for (int pp = 0; pp < NPR; ++pp) {
             const float2 am = make_float2(amp[2 * pp][q], amp[(2 * pp + 1) % TY][q]);
-            Hx[pp] = ffma2(am, hx, Hx[pp]);
-            Hy[pp] = ffma2(am, hy, Hy[pp]);
+            Hx[pp] = VIRT == 2 && q == 0 ? fmul2(am, hx) : ffma2(am, hx, Hx[pp]);
+            Hy[pp] = VIRT == 2 && q == 0 ? fmul2(am, hy) : ffma2(am, hy, Hy[pp]);
+          }
+        }
+        if (VIRT == 2) {
+          const float2 h = hs[(jj * NQ + NQ - 1) * 128];
+#pragma unroll
+          for (int pp = 0; pp < NPR; ++pp) {
+            Hx[pp] = fadd2(Hx[pp], dup2(h.x));
+            Hy[pp] = fadd2(Hy[pp], dup2(h.y));
           }
         }
         float2 btp[NPR];
@@ -534,9 +578,23 @@ __global__ void __launch_bounds__(256, (VIRT && !MAPS && TY == 2) ? 3 : 2) yadjo
         }
       }
     }
+  };
+  if (VIRT == 2 && blocked) {
+    for (int c0 = 0; c0 < nchunks; c0 += kLineBlock / JC) {
+      const int c1 = min(nchunks, c0 + kLineBlock / JC);
+      for (int c = c0; c < c1; ++c) add_chunk(c);
+      if (c1 < nchunks)
+        each_sum([](float2& acc, float2& w) {
+          w = fadd2(w, acc);
+          acc = make_float2(0.f, 0.f);
+        });
+    }
+  } else {
+    for (int c = 0; c < nchunks; ++c) add_chunk(c);
   }
   cp_async_wait0();
   if (!xok) return;
+  if (VIRT == 2 && blocked) each_sum([](float2& acc, float2& w) { acc = fadd2(w, acc); });
   if (PK) {
 #pragma unroll
     for (int ty = 0; ty < TY; ++ty)
@@ -588,9 +646,10 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     if (p->adjq[pass]) {
       const int NQv = p->adjq[pass];
       const int TYv = p->adj_ty[pass];
-      const size_t smq = yadjoint_q_smem(NQv, TYv, NCv, maps, p->max_lines);
+      size_t smq = yadjoint_q_smem(NQv, TYv, NCv, maps, p->max_lines);
+      if (p->basis_nb) smq = std::max(smq, std::min(smq + adj_sum_bytes(TYv, NCv, grads), kBlockedSmem));
       bool launched = false;
-      const bool virt = p->adj_cls;
+      const int virt = p->basis_nb ? 2 : p->adj_cls ? 1 : 0;
       const bool chain = p->adj_chain[pass];
       // the built-in rows per thread, and 2 rows where the built-in choice is 4
 #define MRSIM_AQW(NQV, NCV, M, G, V, W)                                                 \
@@ -613,11 +672,12 @@ void epi_plan_adjoint_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
     }                                                                                   \
   }
 #define MRSIM_AQV(NQV, NCV, M, G, V) MRSIM_AQW(NQV, NCV, M, G, V, false)
-#define MRSIM_AQ(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, false)
+#define MRSIM_AQ(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, 0)
 #define MRSIM_AQC(NCV, M, G) MRSIM_AQ(1, NCV, M, G) MRSIM_AQ(2, NCV, M, G) MRSIM_AQ(4, NCV, M, G) MRSIM_AQ(8, NCV, M, G)
 #define MRSIM_AQN(M, G) MRSIM_AQC(1, M, G) MRSIM_AQC(2, M, G) MRSIM_AQC(3, M, G) MRSIM_AQC(4, M, G)
-#define MRSIM_AQK(M, G) MRSIM_AQL(4, M, G) MRSIM_AQL(6, M, G) MRSIM_AQL(7, M, G)
-#define MRSIM_AQB(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, true) MRSIM_AQW(NQV, NCV, M, G, true, true)
+#define MRSIM_AQK(M, G) MRSIM_AQL(4, M, G) MRSIM_AQL(6, M, G) MRSIM_AQL(7, M, G) \
+  MRSIM_AQV(6, 1, M, G, 1) MRSIM_AQV(6, 2, M, G, 1) MRSIM_AQV(6, 3, M, G, 1) MRSIM_AQV(6, 4, M, G, 1)
+#define MRSIM_AQB(NQV, NCV, M, G) MRSIM_AQV(NQV, NCV, M, G, 2) MRSIM_AQW(NQV, NCV, M, G, 2, true)
 #define MRSIM_AQL(NQV, M, G) MRSIM_AQB(NQV, 1, M, G) MRSIM_AQB(NQV, 2, M, G) MRSIM_AQB(NQV, 3, M, G) MRSIM_AQB(NQV, 4, M, G)
       MRSIM_AQN(false, false) MRSIM_AQN(true, false) MRSIM_AQN(false, true) MRSIM_AQN(true, true)
       MRSIM_AQC(8, false, false) MRSIM_AQC(8, false, true)

@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   constexpr int NA = NV ? NV : QG;             // accumulators per line
   constexpr int NPL = fwdq_planes(NC, MAPS);
   constexpr int RC = fwdq_rows(NC, MAPS);
+  static_assert(kConstBlock % RC == 0, "whole chunks in a block");
   constexpr int STAGE = NPL * RC * 128;        // floats per stage
   constexpr int PIECES = NPL * RC * 32;        // 16-byte pieces per stage
   constexpr int PPT = (PIECES + 255) / 256;
@@ -225,6 +226,9 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   const UnitDesc& u = units[tl.unit];
   const int snx = u.snx, sny = u.sny, ncomp = u.ncomp;
   float* Ey = Bt + sny * TL;                    // [sny][QGP]: ey per coil, or per class and 1
+  // basis rows: the constant row's whole blocks, of kConstBlock and of kConstBlocks rows, [line][thread]
+  float2* const whole = reinterpret_cast<float2*>(Ey + sny * QGP);
+  const bool blocked = NV == 4 || NV == 7 || (NV && cls_rows == 2);  // (six rows may be class rows)
   __shared__ const float* plane_s[NPL];
   __shared__ float rel_s[TL][kMaxComp];
   __shared__ float tinh_s[TL], trf_s[TL], thi_s[TL], tlo_s[TL];
@@ -362,10 +366,24 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   for (int j = 0; j < T; ++j)
 #pragma unroll
     for (int qq = 0; qq < NA; ++qq) acc[j][qq] = make_float2(0.f, 0.f);
+  if (blocked)
+#pragma unroll
+    for (int j = 0; j < 2 * T; ++j) whole[j * 256 + tid] = make_float2(0.f, 0.f);
 
   for (int c = 0; c < nch; ++c) {
     cp_async_wait_n<kFwdStages - 2>();
     __syncthreads();  // rows of chunk c landed; every thread is done with chunk c - 1
+    if (blocked && c * RC % kConstBlock == 0)
+#pragma unroll
+      for (int j = 0; j < T; ++j) {
+        float2 b = fadd2(whole[j * 256 + tid], acc[j][NA - 1]);
+        acc[j][NA - 1] = make_float2(0.f, 0.f);
+        if (c * RC % kConstBlocks == 0) {
+          whole[(T + j) * 256 + tid] = fadd2(whole[(T + j) * 256 + tid], b);
+          b = make_float2(0.f, 0.f);
+        }
+        whole[j * 256 + tid] = b;
+      }
     issue_rows(c + kFwdStages - 1);
     const float* S = ring + (c % kFwdStages) * STAGE + col;
     const int rn = min(RC, sny - c * RC);
@@ -463,6 +481,10 @@ __global__ void __launch_bounds__(256, 2) ystage_q_kernel(const UnitDesc* __rest
   }
   cp_async_wait0();
   if (!xok) return;
+  if (blocked)
+#pragma unroll
+    for (int j = 0; j < T; ++j)
+      acc[j][NA - 1] = fadd2(whole[(T + j) * 256 + tid], fadd2(whole[j * 256 + tid], acc[j][NA - 1]));
   const float s = u.signal_scale;
   if (NV && cls_rows) {
 #pragma unroll
@@ -520,7 +542,7 @@ void epi_plan_forward_ystage(const EpiPlan* p, cudaStream_t st, int u0, int u1) 
       continue;
     }
     if (p->fwdq[pass]) {
-      const size_t smq = ystage_q_smem(NCv, maps, QG, p->max_sny);
+      const size_t smq = ystage_q_smem(NCv, maps, QG, p->max_sny, p->basis_nb > 0);
       bool launched = false;
       const int NVv = p->fwd_nv[pass];
       const bool narrow = p->fwd_narrow[pass];

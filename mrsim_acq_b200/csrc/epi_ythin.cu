@@ -107,9 +107,11 @@ __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __r
   grid_wait();
 #pragma unroll
   for (int c = 0; c < kFwdStages - 1; ++c) issue_rows(c);
-  float2 acc[NO];
+  // block, blocks: the constant row's whole blocks of kConstBlock and of kConstBlocks rows
+  float2 acc[NO], block = make_float2(0.f, 0.f), blocks = block;
 #pragma unroll
   for (int o = 0; o < NO; ++o) acc[o] = make_float2(0.f, 0.f);
+  const bool blocked = NV == 4 || NV == 7 || (NV && cls_rows == 2);  // (six rows may be class rows)
   for (int c = 0; c < nch; ++c) {
     cp_async_wait_n<kFwdStages - 2>();
     __syncthreads();  // rows of chunk c landed; every warp is done with chunk c - 1 and its terms
@@ -144,8 +146,7 @@ __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __r
     const float* e = Ey + c * RC * QGP + o0;
     const float2* w = terms + jl * CW + lane;
     const int rn = min(RC, sny - c * RC);
-#pragma unroll 8
-    for (int r = 0; r < rn; ++r) {
+    auto add_row = [&](int r) {
       const float2 t = w[r * TL * CW];
 #pragma unroll
       for (int o = 0; o < NO; ++o) {
@@ -154,6 +155,25 @@ __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __r
           acc[o] = fadd2(acc[o], t);  // the offset or constant row is all ones
         else if (NA % CS == 0 || qq < NA)
           acc[o] = ffma2(dup2(NV ? e[r * QGP + o * CS] : fmaf(exq[NV ? 0 : o], e[r * QGP + o * CS], off)), t, acc[o]);
+      }
+    };
+    for (int r = 0; r < rn; r += kConstBlock) {
+      if (blocked)
+#pragma unroll
+        for (int o = 0; o < NO; ++o)
+          if (o0 + o * CS == NA - 1) {
+            block = fadd2(block, acc[o]);
+            acc[o] = make_float2(0.f, 0.f);
+            if ((c * RC + r) % kConstBlocks == 0) {
+              blocks = fadd2(blocks, block);
+              block = make_float2(0.f, 0.f);
+            }
+          }
+      if (r + kConstBlock <= rn) {
+#pragma unroll
+        for (int k = 0; k < kConstBlock; ++k) add_row(r + k);
+      } else {
+        for (int k = r; k < rn; ++k) add_row(k);
       }
     }
   }
@@ -165,7 +185,8 @@ __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __r
     const int qq = o0 + o * CS, q = NV ? qq : tl.w + qq;
     if (qq >= NA || (!NV && q >= u.ncoils)) break;
     const float sv = NV && qq == NA - 1 && cls_rows == 1 ? s * off : s;
-    u.g[((size_t)q * u.n_lines + tl.y + jl) * snx + x] = make_float2(sv * acc[o].x, sv * acc[o].y);
+    const float2 t = blocked && qq == NA - 1 ? fadd2(blocks, fadd2(block, acc[o])) : acc[o];
+    u.g[((size_t)q * u.n_lines + tl.y + jl) * snx + x] = make_float2(sv * t.x, sv * t.y);
   }
 }
 
@@ -174,7 +195,7 @@ __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __r
 // it forms their Z into shared memory; then each warp adds the chunk's lines of one row, in order, to the
 // row's sums (G = 1: to the compartment gradients, or to the t- and trf-weighted sums).
 // That slice is 16 tiles of the full kernel, 12 us with its x-stage; here 128 blocks, 7 us.
-template <int G, int NQ, int NC, bool GRADS, bool VIRT>
+template <int G, int NQ, int NC, bool GRADS, int VIRT>
 __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* __restrict__ units,
                                                                const int4* __restrict__ tiles) {
   constexpr int CW = kThinCols, JL = kThinLines, NST = thin_stages(NQ), LF = adjq_line_floats(NC, false);
@@ -274,6 +295,28 @@ __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* _
     cg[c] = make_float2(0.f, 0.f);
     if (GRADS) Uy[GRADS ? c : 0] = Vx[GRADS ? c : 0] = 0.f;
   }
+  // basis rows: the sums of whole blocks of kLineBlock lines (adj_blocked)
+  static_assert(kLineBlock % JL == 0, "whole chunks in a block");
+  const bool blocked = VIRT == 2 && adj_blocked(NQ, NC, false, GRADS, nlines);
+  float2 wcg[NC];
+  float wUy[GRADS ? NC : 1], wVx[GRADS ? NC : 1];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    wcg[c] = make_float2(0.f, 0.f);
+    if (GRADS) wUy[GRADS ? c : 0] = wVx[GRADS ? c : 0] = 0.f;
+  }
+  auto fold = [&] {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      wcg[c] = fadd2(wcg[c], cg[c]);
+      cg[c] = make_float2(0.f, 0.f);
+      if (GRADS) {
+        wUy[GRADS ? c : 0] += Uy[GRADS ? c : 0];
+        wVx[GRADS ? c : 0] += Vx[GRADS ? c : 0];
+        Uy[GRADS ? c : 0] = Vx[GRADS ? c : 0] = 0.f;
+      }
+    }
+  };
   for (int c = 0; c < nchunks; ++c) {
     cp_async_wait_n<NST - 2>();
     __syncthreads();  // chunk c landed; every warp is done with chunk c - 1 and its terms
@@ -286,7 +329,7 @@ __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* _
       const float4 b4 = *reinterpret_cast<const float4*>(Bt + j * ROWS + rb);
       const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
       float2 H[4];
-      if (VIRT) {  // as the full kernel: from the last row (amplitude 1) on
+      if (VIRT == 1) {  // as the full kernel: from the offset row (amplitude 1) on
         const float2 h = hs[(jj * NQ + NQ - 1) * CW];
 #pragma unroll
         for (int ty = 0; ty < 4; ++ty) H[ty] = h;
@@ -296,10 +339,15 @@ __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* _
         for (int ty = 0; ty < 4; ++ty) H[ty] = fmul2(dup2(amp[ty][0]), h);
       }
 #pragma unroll
-      for (int q = VIRT ? 0 : 1; q < (VIRT ? NQ - 1 : NQ); ++q) {
+      for (int q = VIRT == 1 ? 0 : 1; q < (VIRT ? NQ - 1 : NQ); ++q) {
         const float2 h = hs[(jj * NQ + q) * CW];
 #pragma unroll
         for (int ty = 0; ty < 4; ++ty) H[ty] = ffma2(dup2(amp[ty][q]), h, H[ty]);
+      }
+      if (VIRT == 2) {  // the constant row last
+        const float2 h = hs[(jj * NQ + NQ - 1) * CW];
+#pragma unroll
+        for (int ty = 0; ty < 4; ++ty) H[ty] = fadd2(H[ty], h);
       }
 #pragma unroll
       for (int tp = 0; tp < 4; tp += 2) {
@@ -318,6 +366,7 @@ __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* _
     __syncthreads();
     const float2* z = terms + row * CW + lane;
     const float* e = Lt + c * JL * LF + 4;
+    if (blocked && c * JL % kLineBlock == 0) fold();
     if (half == 0) {
 #pragma unroll
       for (int jj = 0; jj < JL; ++jj) {
@@ -340,6 +389,17 @@ __global__ void __launch_bounds__(256, 2) yadjoint_thin_kernel(const UnitDesc* _
   }
   cp_async_wait0();
   if (!xok || y0 + row >= sny) return;
+  if (blocked) {
+    fold();
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      cg[c] = wcg[c];
+      if (GRADS) {
+        Uy[GRADS ? c : 0] = wUy[GRADS ? c : 0];
+        Vx[GRADS ? c : 0] = wVx[GRADS ? c : 0];
+      }
+    }
+  }
   const size_t plane = (size_t)snx * sny, i = (size_t)x + (size_t)snx * (y0 + row);
   float fg = 0.f;
 #pragma unroll
@@ -381,7 +441,8 @@ void launch_ystage_thin(const EpiPlan* p, int pass, const int4* tiles, int n, cu
 
 void launch_yadjoint_thin(const EpiPlan* p, int pass, const int4* tiles, int n, cudaStream_t st) {
   const int G = p->adj_thin[pass], NQv = p->adjq[pass], NCv = p->nc;
-  const bool grads = (pass & 2) != 0, virt = p->adj_cls;
+  const bool grads = (pass & 2) != 0;
+  const int virt = p->basis_nb ? 2 : p->adj_cls ? 1 : 0;
   const size_t sm = yadjoint_thin_smem(G, NQv, NCv, p->max_lines);
   bool launched = false;
 #define MRSIM_AT(NQV, NCV, GR, V)                                                                        \
@@ -391,9 +452,8 @@ void launch_yadjoint_thin(const EpiPlan* p, int pass, const int4* tiles, int n, 
     launch_chained(k, dim3((unsigned)n), sm, st, true, p->d_units, tiles);                               \
     launched = true;                                                                                     \
   }
-#define MRSIM_ATC(NCV, GR) MRSIM_AT(1, NCV, GR, false) MRSIM_AT(2, NCV, GR, false) MRSIM_AT(4, NCV, GR, false) \
-  MRSIM_AT(8, NCV, GR, false)
-#define MRSIM_ATV(NCV, GR) MRSIM_AT(4, NCV, GR, true) MRSIM_AT(6, NCV, GR, true) MRSIM_AT(7, NCV, GR, true)
+#define MRSIM_ATC(NCV, GR) MRSIM_AT(1, NCV, GR, 0) MRSIM_AT(2, NCV, GR, 0) MRSIM_AT(4, NCV, GR, 0) MRSIM_AT(8, NCV, GR, 0)
+#define MRSIM_ATV(NCV, GR) MRSIM_AT(6, NCV, GR, 1) MRSIM_AT(4, NCV, GR, 2) MRSIM_AT(6, NCV, GR, 2) MRSIM_AT(7, NCV, GR, 2)
 #define MRSIM_ATN(GR) MRSIM_ATC(1, GR) MRSIM_ATC(2, GR) MRSIM_ATC(3, GR) MRSIM_ATC(4, GR) MRSIM_ATC(8, GR) \
   MRSIM_ATV(1, GR) MRSIM_ATV(2, GR) MRSIM_ATV(3, GR) MRSIM_ATV(4, GR)
   MRSIM_ATN(false) MRSIM_ATN(true)

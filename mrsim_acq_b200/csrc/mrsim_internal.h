@@ -62,7 +62,8 @@ struct GeoTab {
   const float* eyc;   // [class][sny] the class rows
   // coil basis: every coil's ey row as a combination of nbas rows, the last of them constant,
   //   ey_q(y) = sum_{r < nbas - 1} bco[q][r] bas_r(y) + bco[q][nbas - 1]
-  // (coil_basis, driver.cpp; nbas = 0: none).  bco rows are kBasisPad floats.
+  // (coil_basis, driver.cpp; nbas = 0: none).  bco rows are kBasisPad floats, the constant row's coefficient
+  // in the last of them too.
   int nbas;
   const float* bas;   // [nbas - 1][sny]
   const float* bco;   // [coil][kBasisPad]
