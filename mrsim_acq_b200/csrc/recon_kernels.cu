@@ -275,16 +275,19 @@ __global__ void __launch_bounds__(256) recon_combine_kernel(const ReconJob* __re
 // coil order, to the Roemer sums of its share of the pixels, so the sums are the same for every S.
 // With xs = nx/2 and ys = ny/2 multiples of 16 the centred transform is the plain one between sign flips:
 // e^{-i2pi (k - s)(x - s)/n} = (-1)^(k + x) e^{-i2pi kx/n}.
+// The twiddles carry their rounding along: it is the forward x-transform's too, and would add up with it
+// (one slice of 8 coils against 64 bits: direct sums 1.45e-7, FFT with float32 twiddles 1.53e-7, with both
+// parts 1.22e-7).
 // One block a unit fills the chip from 592 units on; fewer units share their coils among up to 8 blocks.  600
-// units of 64 x 64 x 8 coils: 205 us, 0.77 TB/s of k-space (as direct sums 2142 us: 64-term sums at 12 %
-// of the FMA rate); one slice of 8 coils 16 us; 32 partitions of 32 coils 57 us.
+// units of 64 x 64 x 8 coils: 241 us, 0.65 TB/s of k-space (as direct sums 2142 us: 64-term sums at 12 %
+// of the FMA rate); one slice of 8 coils 16 us; 32 partitions of 32 coils 59 us.
 template <int EX, int EY>
 struct ReconShape {
   static constexpr int NX = 32 * EX, NY = 32 * EY, LD = NX + 1;
   static constexpr int T = NX * NY >= 8192 ? 512 : 256, NW = T / 32, NP = NX * NY / T;
   // images of a block of a cluster: two where they fit, so that one is read while the next is formed
   static constexpr int NB = NY * LD <= 6 * 1024 ? 2 : 1;
-  static constexpr size_t smem(bool multi) { return sizeof(float2) * ((size_t)(multi ? NB : 1) * NY * LD + NX + NY); }
+  static constexpr size_t smem(bool multi) { return sizeof(float2) * ((size_t)(multi ? NB : 1) * NY * LD + 2 * NX + 2 * NY); }
 };
 
 template <int EX, int EY, int S>
@@ -295,15 +298,15 @@ __global__ void __launch_bounds__(ReconShape<EX, EY>::T) recon_fft_kernel(const 
   constexpr bool PX = (EX & (EX - 1)) == 0, PY = (EY & (EY - 1)) == 0;
   extern __shared__ __align__(16) float2 sm[];
   constexpr int NB = S > 1 ? R::NB : 1;
-  float2* twx = sm;        // e^{-i2pi j/NX}
-  float2* twy = twx + NX;
-  float2* imgs = twy + NY;  // [NB][NY][LD]
+  float2* twx = sm;             // e^{-i2pi j/NX}, then what their rounding took
+  float2* twy = twx + 2 * NX;
+  float2* imgs = twy + 2 * NY;  // [NB][NY][LD]
   const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   const int rank = S > 1 ? (int)cl.block_rank() : 0;
   const ReconJob& J = jobs[blockIdx.x / S];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nc = J.nc;
-  for (int i = tid; i < NX; i += T) twx[i] = J.ex_tab[i];
-  for (int i = tid; i < NY; i += T) twy[i] = J.ey_tab[i];
+  for (int i = tid; i < 2 * NX; i += T) twx[i] = J.ex_tab[i];
+  for (int i = tid; i < 2 * NY; i += T) twy[i] = J.ey_tab[i];
   const float* __restrict__ sens = J.sens;
   float2* const coil_images = J.coil_images;
   constexpr int MP = (NP + S - 1) / S;  // this block's pixels: tid + (first + p) T
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(ReconShape<EX, EY>::T) recon_fft_kernel(const 
           w = ((kx + ky) & 1) ? -w : w;
           b[PX ? bitrev_c(m, LX) : m] = make_float2(v.x * w, v.y * w);
         }
-        warp_row_fft<EX, true>(b, twx, lane);
+        warp_row_fft<EX, true, true>(b, twx, lane);
 #pragma unroll
         for (int k1 = 0; k1 < EX; ++k1) img[ky * LD + k1 + EX * k2] = b[k1];
       }
@@ -343,7 +346,7 @@ __global__ void __launch_bounds__(ReconShape<EX, EY>::T) recon_fft_kernel(const 
         float2 b[EY];
 #pragma unroll
         for (int m = 0; m < EY; ++m) b[PY ? bitrev_c(m, LY) : m] = img[(lane + 32 * m) * LD + x];
-        warp_row_fft<EY, true>(b, twy, lane);
+        warp_row_fft<EY, true, true>(b, twy, lane);
 #pragma unroll
         for (int k1 = 0; k1 < EY; ++k1) img[(k1 + EY * k2) * LD + x] = b[k1];
       }

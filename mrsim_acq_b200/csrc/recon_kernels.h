@@ -21,8 +21,8 @@ struct ReconJob {
   float2* k;                // [coil][ny][nx], GRAPPA fills it in place
   const float2* grappa_w;   // [d-1][co][6 nc] for this slice and echo time, or NULL
   const float* window;      // [ny][nx] or NULL
-  const float2* ex_tab;     // e^{-i 2 pi m / nx}, m = 0..nx-1
-  const float2* ey_tab;     // e^{-i 2 pi m / ny}
+  const float2* ex_tab;     // e^{-i 2 pi m / nx}, m = 0..nx-1, then what rounding to float32 took from each
+  const float2* ey_tab;     // e^{-i 2 pi m / ny} likewise
   const float* sens;        // [coil][ny][nx] coil sensitivities on the acquired grid
   const float* inv_ssum;    // [ny][nx] 1 / max(sum_q s_q^2, 1e-12)
   float2* coil_images;      // capture [coil][ny][nx] or NULL

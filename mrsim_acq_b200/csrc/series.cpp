@@ -27,12 +27,19 @@ ReconTables build_recon_tables(DevArena& A, int nx, int ny, int nc, const mrsim_
   const size_t per = (size_t)nx * ny;
   // one allocation and one copy: DFT tables, sensitivities, Roemer denominator, window
   const bool win = acq.window_kind != MRSIM_WINDOW_NONE;
-  const size_t o_sens = 2 * ((size_t)nx + ny), o_inv = o_sens + nc * per, o_win = o_inv + per;
+  const size_t o_sens = 4 * ((size_t)nx + ny), o_inv = o_sens + nc * per, o_win = o_inv + per;
   std::vector<float> host(o_win + (win ? per : 0));
   float2* ex = (float2*)host.data();
-  float2* ey = ex + nx;
-  for (int m = 0; m < nx; ++m) ex[m] = make_float2((float)std::cos(-kTau * m / nx), (float)std::sin(-kTau * m / nx));
-  for (int m = 0; m < ny; ++m) ey[m] = make_float2((float)std::cos(-kTau * m / ny), (float)std::sin(-kTau * m / ny));
+  float2* ey = ex + 2 * nx;
+  auto table = [](float2* t, int n) {
+    for (int m = 0; m < n; ++m) {
+      const double c = std::cos(-kTau * m / n), s = std::sin(-kTau * m / n);
+      t[m] = make_float2((float)c, (float)s);
+      t[n + m] = make_float2((float)(c - t[m].x), (float)(s - t[m].y));
+    }
+  };
+  table(ex, nx);
+  table(ey, ny);
   // `coil_sensitivity` on the acquired grid and the Roemer denominator (kspace.rs:1343-1373)
   T.sens_host.assign(nc * per, 0.f);
   std::vector<double> ssum(per, 0.0);
@@ -62,7 +69,7 @@ ReconTables build_recon_tables(DevArena& A, int nx, int ny, int nc, const mrsim_
             (float)window_at(acq, ((double)kx - xs) / (double)nx, ((double)ky - ys) / (double)ny);
   float* d = (float*)A.upload(host.data(), host.size() * 4, st);
   T.ex_tab = (float2*)d;
-  T.ey_tab = T.ex_tab + nx;
+  T.ey_tab = T.ex_tab + 2 * nx;
   T.sens = d + o_sens;
   T.inv_ssum = d + o_inv;
   if (win) T.window = d + o_win;
