@@ -11,7 +11,8 @@ namespace {
 // order, to every coil or row (G = 1: to half of them).  The chain of a tile is thus its additions, not
 // its rows' phases.
 // One slice of one coil (64 lines on 128 x 128) is 8 tiles of the full kernel, 23 us; here 64 blocks.
-// Bound by latency: two warps a scheduler, whose phases, exchange and additions alternate.
+// Bound by latency: two to four warps a scheduler, whose phases, exchange and additions alternate (4 slices
+// of 8 coils: FMA pipe 20 %, shared memory 57 % of the cycles).
 template <int G, int QG, int NV, int NC>
 __global__ void __launch_bounds__(256, 2) ystage_thin_kernel(const UnitDesc* __restrict__ units,
                                                              const int4* __restrict__ tiles, int cls_rows) {

@@ -406,8 +406,9 @@ __global__ void spread_taps_kernel(const NufftGridT<double> g, const double* __r
 // so a point's taps are broadcasts and its weight is read from shared memory once for 16 cells.  With a
 // thread per cell and four items, 58 % of the threads a point visits are outside its window and every
 // contribution waits for its own loads: 576 items at 65,536 points on a 128 x 128 fine grid took
-// 28.1 ms, here 4.2.  Bound by shared memory and the FP64 pipe about equally (14 wavefronts for 18
-// FP64 instructions per row).  Points are added in their order in the tile.
+// 28.1 ms, here 4.2.  No pipe is full (shared memory 38 %, FP64 27 %, issue 46 % of the cycles, at 26 %
+// occupancy): a chunk's loads and its sums alternate at its barriers.  Points are added in their order in
+// the tile.
 constexpr int kItemLanes = 32, kItemChunk = 32, kPadTaps = 8 + kWMax + 8;
 __global__ void __launch_bounds__(128) spread_items_kernel(const NufftGridT<double> g, double2* __restrict__ grid,
                                                            const double* __restrict__ taps, const int2* __restrict__ org,

@@ -389,7 +389,8 @@ void launch_points(const NufftGrid& g, const float2* grid, const NufftPoints& P,
 
 NufftPoints nufft_points(DevArena& A, const NufftGrid& g, const double* d_u, int npts, int batch, cudaStream_t st) {
   // 65,536 points on a 256 x 256 fine grid: 16 items 51 us with small tiles and 55 with wide ones, 128 items
-  // 276 and 244.  The line between: three chunks give the wide tiles' blocks five items each to even out.
+  // 276 and 244.  The line between is set, not measured: three chunks give the wide tiles' blocks five items each to even
+  // out.
   const bool wide = batch > 2 * kItems;
   NufftPoints P = wide ? make_points<Wide>(A, g, d_u, npts, st) : make_points<Small>(A, g, d_u, npts, st);
   P.wide = wide;

@@ -186,7 +186,7 @@ __global__ void seg_combine_kernel(const float2* __restrict__ seg, const int* __
 // The same from the tiled transforms' [point][item] rows: a warp takes 32 points of one slot and brings
 // 16 segments of them at a time through shared memory, the table rows beside them, so that both are
 // read in runs; a thread per point read a cache line of each per segment (128 items at 65,536 points:
-// 55 us, here 26).  Bound by L2.  The sum's order is the same.
+// 55 us, here 26).  L1 48 %, issue 39 %, DRAM 19 % of their rates.  The sum's order is the same.
 constexpr int kCombineWarps = 4, kCombineSegs = 16;
 __global__ void __launch_bounds__(32 * kCombineWarps)
     seg_combine_points_kernel(const float2* __restrict__ seg, int items, const int* __restrict__ slot_base,
@@ -279,7 +279,8 @@ __global__ void spiral_zdft_kernel(const ZArgs a) {
 // entries lived in local memory: a 16-coil volume's four fits, of up to 64 features and 80 columns over
 // 65,536 samples a partition, took 24.8 ms, here 10.2).
 // Only tiles on and above the diagonal are formed, G being Hermitian.  The threads that the units
-// leave over take rows of their own; the groups are added in order.  Bound by the FP64 pipe.
+// leave over take rows of their own; the groups are added in order.  Shared memory is at 40 to 53 % and the FP64 pipe at 32 to 39 %
+// of their rates: a chunk's loads and its products alternate.
 constexpr int kKzRows = 32, kKzTile = 4;
 struct KzFitArgs {
   const float2* k;     // [q][p][nsamp] calibration samples
@@ -481,7 +482,8 @@ __global__ void to_double_kernel(const float2* __restrict__ in, size_t n, double
 // z-DFT table and the low-resolution weights are in shared memory, four outputs share each load of a
 // voxel's values (which live in local memory), and a block is small, so that those stay in L1.  With every
 // partition in every iteration, the table from global memory and a cosine per term, 12 of 48
-// partitions restored for 65,536 voxels took 7.0 ms, here 1.4.  Bound by the FP64 pipe and L1.
+// partitions restored for 65,536 voxels took 7.0 ms, here 1.4.  FP64 pipe and L1 at 42 % each (19 % of the
+// warps resident): latency of the voxels' values.
 constexpr int kPocsThreads = 64;
 __global__ void __launch_bounds__(kPocsThreads) pocs_kernel(const double2* __restrict__ h, int lo,
                                                             const double2* __restrict__ zk, int nz, int nn,

@@ -21,8 +21,9 @@
 // A cluster of C blocks holds one image, n / C rows each; column lines cross the blocks through
 // distributed shared memory.  C = 1 holds n <= 64 (198 KB with the direction's rows) and fills the
 // chip from the batch; 96 and 128 need 2 and 4.  The power iteration has one image, so it takes 8
-// blocks: its steps are a chain, and eight SMs shorten each.  Bound by the FP64 pipe (about 2.2 MFLOP
-// a step at n = 64) and, in the power iteration, by the barriers.  Measured at n = 64: 576 images x 80
+// blocks: its steps are a chain, and eight SMs shorten each.  Bound by shared memory (96 % of its cycles
+// while the blocks run, FP64 pipe 25 to 40 %; about 2.2 MFLOP a step at n = 64) and, in the power
+// iteration, by the latency of its exchanges (no pipe above 2 %).  Measured at n = 64: 576 images x 80
 // steps 14.8 ms (6.8 of about 37 TFLOP/s, 0.18; before 125 ms of kernels), 1000 power steps 9.5 ms
 // (before 1000 x 19 launches and a host wait each, about 200 ms).
 #include <cooperative_groups.h>
